@@ -2,7 +2,7 @@
 
 Outputs, next to the Python package they serve (git-ignored, shipped with the tree):
   vllm_gguf_plugin/libgguf_b200.so   the C-ABI kernel library (include/gguf_b200.h)
-  vllm_gguf_plugin/_C_gguf.abi3.so   torch stable-ABI library `_C_gguf` calling the C-ABI
+  vllm_gguf_plugin/_C_gguf.abi3.so   torch library `_C_gguf` and the module's eager functions, calling the C-ABI
 
 quantize_q8_1.cu and gemv1.cu (the decode GEMV that quantizes its activations itself) are
 compiled with --use_fast_math: the two fp32 divisions of the q8_1 quantization must be the same
@@ -78,7 +78,7 @@ def build_torch_shim(force: bool = False) -> Path:
         return so
     cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-DUSE_CUDA", str(src), "-o", str(so),
            f"-I{troot / 'include'}", f"-I{sysconfig.get_paths()['include']}", f"-I{CUDA}/include",
-           f"-L{OUT}", "-lgguf_b200", f"-L{troot / 'lib'}", "-ltorch", "-ltorch_cpu", "-lc10",
+           f"-L{OUT}", "-lgguf_b200", f"-L{troot / 'lib'}", "-ltorch_python", "-ltorch", "-ltorch_cuda", "-ltorch_cpu", "-lc10_cuda", "-lc10",
            "-Wl,-rpath,$ORIGIN", f"-Wl,-rpath,{troot / 'lib'}"]
     subprocess.check_call(cmd)
     return so

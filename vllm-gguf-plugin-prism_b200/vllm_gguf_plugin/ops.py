@@ -27,6 +27,7 @@ from __future__ import annotations
 import os
 
 import torch
+from torch.compiler import is_compiling
 
 # GGML type ids (gguf.GGMLQuantizationType; the reference keeps them in triton/gemm/utils.py:5-24)
 GGML_TYPE_Q4_0 = 2
@@ -62,6 +63,7 @@ except ImportError as exc:  # no silent fallback: the CUDA extension IS the prod
 
 _CUDA_AVAILABLE = True
 _CUDA_ENABLED = True
+_OP_GEMV, _OP_MMQ, _OP_DEQUANT_MATMUL = 0, 1, 4   # GGUF_B200_OP_* of include/gguf_b200.h
 
 # (values per block, bytes per block) -- gguf.GGML_QUANT_SIZES for the supported types
 QUANT_SIZES = {
@@ -153,6 +155,12 @@ def _ggml_moe_a8_vec_fake(X, W, topk_ids, top_k, quant_type, row, tokens):
 # --- public API (reference: ops.py:181-286) ---
 
 
+def _mul_mat(W, X, quant_type, row, op):
+    """An eager product without the dispatcher's overhead; None while compiling or tracing, and for anything that is not
+    a plain CUDA tensor."""
+    return None if is_compiling() else _C_gguf.mul_mat(W, X, quant_type, row, op)
+
+
 def ggml_dequantize(W: torch.Tensor, quant_type: int, m: int, n: int, dtype: torch.dtype | None) -> torch.Tensor:
     _require(quant_type, _CUDA_DEQUANT_TYPES, "ggml_dequantize")
     return torch.ops._C_gguf.ggml_dequantize(W, quant_type, m, n, dtype)
@@ -160,18 +168,21 @@ def ggml_dequantize(W: torch.Tensor, quant_type: int, m: int, n: int, dtype: tor
 
 def ggml_mul_mat_vec_a8(W: torch.Tensor, X: torch.Tensor, quant_type: int, row: int) -> torch.Tensor:
     _require(quant_type, _CUDA_GEMV_QUANT_TYPES, "ggml_mul_mat_vec_a8")
-    return torch.ops._C_gguf.ggml_mul_mat_vec_a8(W, X, quant_type, row)
+    y = _mul_mat(W, X, quant_type, row, _OP_GEMV)
+    return torch.ops._C_gguf.ggml_mul_mat_vec_a8(W, X, quant_type, row) if y is None else y
 
 
 def ggml_mul_mat_a8(W: torch.Tensor, X: torch.Tensor, quant_type: int, row: int) -> torch.Tensor:
     _require(quant_type, _CUDA_GEMM_QUANT_TYPES, "ggml_mul_mat_a8")
-    return torch.ops._C_gguf.ggml_mul_mat_a8(W, X, quant_type, row)
+    y = _mul_mat(W, X, quant_type, row, _OP_MMQ)
+    return torch.ops._C_gguf.ggml_mul_mat_a8(W, X, quant_type, row) if y is None else y
 
 
 def ggml_dequant_matmul(W: torch.Tensor, X: torch.Tensor, quant_type: int, row: int) -> torch.Tensor:
     """x @ dequantize(W).T in one kernel, unquantized fp16/bf16 activations (IQ2_XXS, IQ4_XS)."""
     _require(quant_type, _DEQUANT_MATMUL_TYPES, "ggml_dequant_matmul")
-    return torch.ops._C_gguf.dequant_matmul(W, X, quant_type, row)
+    y = _mul_mat(W, X, quant_type, row, _OP_DEQUANT_MATMUL)
+    return torch.ops._C_gguf.dequant_matmul(W, X, quant_type, row) if y is None else y
 
 
 def ggml_dequantize_rows(W: torch.Tensor, ids: torch.Tensor, quant_type: int, dtype: torch.dtype | None) -> torch.Tensor:

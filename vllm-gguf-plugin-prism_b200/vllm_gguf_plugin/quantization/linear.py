@@ -13,8 +13,10 @@ objects are plain classes/functions, so the kernels stay testable on a box witho
 from __future__ import annotations
 
 import torch
+from torch.compiler import is_compiling
 
 from .. import ops
+from .._C_gguf import linear as _native_linear
 from .utils import (
     DEQUANT_TYPES,
     IMATRIX_QUANT_TYPES,
@@ -133,6 +135,7 @@ class GGUFLinearMethod(LinearMethodBase):
         fallback = extra_weight_attrs.pop("weight_loader", None)
         weight = torch.nn.Parameter(torch.empty(0, dtype=torch.uint8), requires_grad=False)
         weight.shard_id = []
+        weight.gguf_one_type = None
         weight.shard_offset_map = {}
         weight.output_partition_sizes = list(output_partition_sizes)
         weight.input_size_per_partition = input_size_per_partition
@@ -204,10 +207,24 @@ class GGUFLinearMethod(LinearMethodBase):
             w.shard_id[:] = order
         w.data = data
         w._shards = {}
+        # the block type of all stacked rows, when one call can take them together
+        wtype = layer.weight_type
+        types = {wtype.shard_weight_type.get(i, wtype.weight_type) for i in w.shard_id}
+        same_width = len({o[2] for o in w.shard_offset_map.values()}) == 1
+        w.gguf_one_type = types.pop() if len(types) == 1 and same_width else None
 
     def apply(self, layer: torch.nn.Module, x: torch.Tensor, bias: torch.Tensor | None = None) -> torch.Tensor:
         if self.layout is not None:
             x = self.layout.input_to_gguf(x)
+        if not is_compiling():
+            # An eager call goes to the native dispatcher in one step: same routing as `_fused_mul_mat_gguf`, none of
+            # the layers in between (custom op, operator dispatch), which cost more than a decode GEMV runs for.
+            weight = layer.weight
+            one_type = weight.gguf_one_type if weight.shard_id else layer.weight_type.weight_type
+            if one_type is not None:
+                out = _native_linear(x, weight, one_type)
+                if out is not None:
+                    return out if bias is None else out.add_(bias)
         shard_id = layer.weight.shard_id
         if shard_id:
             shard_id = ["q", "k", "v"] if "q" in shard_id else shard_id
