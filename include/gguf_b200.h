@@ -80,6 +80,12 @@ int gguf_b200_dequantize_rows(const void* W, int type, const int64_t* row_ids, i
  * accepted and merely disables the split. */
 int64_t gguf_b200_workspace_bytes(int op, int type, int64_t M, int64_t N, int64_t K);
 
+/* Scratch bytes with which an op is fastest, never less than the above: for batches of a few tokens
+ * (gguf_b200_mul_mat_vec_a8 from three on, gguf_b200_mul_mat_a8 from three to sixteen) it adds what the
+ * small-batch kernel needs, its activation tiles and partial sums; without that room these calls take
+ * several passes of the one- and two-vector kernel, or the tiled kernel. */
+int64_t gguf_b200_scratch_bytes(int op, int type, int64_t M, int64_t N, int64_t K);
+
 /* Decode GEMV: Y[M][N] = q8_1(X) . dequant(W)^T, weights read once for up to 8 vectors.
  * Replaces: ggml_mul_mat_vec_a8, gguf_kernel.cu:104-218 (+ mmvq.cuh). */
 int gguf_b200_mul_mat_vec_a8(const void* W, const void* X, void* Y, void* workspace, int64_t workspace_bytes,
@@ -122,15 +128,16 @@ int gguf_b200_moe_a8(const void* X, const void* W, void* Y, void* workspace, int
                      int64_t n_experts, int type, int dtype, int64_t tokens, int64_t top_k, int64_t N, int64_t K,
                      void* stream);
 
-/* The whole MoE step of one layer in one call: expert alignment, gate/up expert GEMM, activation,
- * down expert GEMM, routing weights and the sum over the top_k experts.
- * Replaces: the tiled branch of _fused_moe_gguf, quantization/fused_moe.py:56-95 (moe_align_block_size,
- * ggml_moe_a8, apply_moe_activation, ggml_moe_a8, mul_ by the routing weights, moe_sum: six library
- * ops there).  Here the activation runs inside the second GEMM's activation quantizer and the routing
+/* The whole MoE step of one layer in one call: expert alignment, gate/up expert product, activation,
+ * down expert product, routing weights and the sum over the top_k experts.  Up to 64 tokens, and for types
+ * without a tiled kernel, on the small-batch kernel (integer dot products); otherwise on the tiled one.
+ * Replaces: both branches of _fused_moe_gguf, quantization/fused_moe.py:56-133 (moe_align_block_size,
+ * ggml_moe_a8 or ggml_moe_a8_vec, apply_moe_activation, the second product, mul_ by the routing weights,
+ * moe_sum: six library ops there).  Here the activation runs inside the second GEMM's activation quantizer and the routing
  * weights inside its epilogue; the alignment and the final sum are small kernels of this library.
  *   X [tokens][H]; W13 [E][2I][H/QK*ts] (gate rows, then up rows, of every expert); W2 [E][H][I/QK*ts];
  *   topk_ids int32 [tokens*top_k] and topk_weights float [tokens*top_k] on the device; Y [tokens][H].
- *   act: 1 = silu, 2 = gelu (erf form).  Types 2, 3, 6, 7, 8, 12, 13, 14; n_experts <= 256; I % 8 == 0.
+ *   act: 1 = silu, 2 = gelu (erf form).  All types; n_experts <= 256; I % 8 == 0.
  *   A slot whose expert id is outside [0, n_experts) contributes nothing (expert-parallel masking).
  * Workspace: gguf_b200_fused_moe_workspace_bytes (slot lists, both intermediate matrices, activations). */
 int64_t gguf_b200_fused_moe_workspace_bytes(int type13, int type2, int dtype, int64_t tokens, int64_t top_k,

@@ -869,3 +869,55 @@ def test_moe_down_projection_full_size_close_to_reference(ref):
     torch.cuda.synchronize()
     assert capi.last_status() == 0
     assert rel_l2(y.float().cpu(), r.float().cpu()) <= REL_L2_TOL
+
+
+# ---------------------------------------------------------------- small-batch kernel ----------
+
+# (rows, K, tokens): one chunk; rows beyond the last alignment class and a row tile's edge; column tiles of 1, 2, 3 and 4;
+# a K that ends inside a chunk (32-value blocks); row tiles shared by many CTAs; more tokens than one pass takes
+SMALL_SHAPES = [(7, 256, 4), (128, 256, 3), (259, 768, 16), (300, 800, 9), (1000, 2048, 13), (130, 8192, 20), (640, 4096, 33)]
+
+
+@pytest.mark.parametrize("name", TYPES)
+def test_small_batches_equal_single_vectors(name):
+    """Three to sixteen tokens at once (tensor-core integer products) against the same rows one by one (dp4a)."""
+    from vllm_gguf_plugin import ops
+
+    t = TYPES[name]
+    for N, K, M in SMALL_SHAPES:
+        if K % synth.QUANT_SIZES[t][0]:
+            continue
+        _, w = dev_w(t, N, K, seed=N + K)
+        for dtype, tol in ((torch.float32, 2e-6), (torch.float16, 3e-4)):
+            x = dev_x(M, K, seed=M, dtype=dtype)
+            want = torch.cat([ops.ggml_mul_mat_vec_a8(w, x[i:i + 1].contiguous(), t, N) for i in range(M)])
+            got = ops.ggml_mul_mat_vec_a8(w, x, t, N)
+            assert rel_l2(got.float().cpu(), want.float().cpu()) <= tol, (N, K, M, dtype)
+            assert torch.equal(got, ops.ggml_mul_mat_vec_a8(w, x, t, N))     # the parts are added in a fixed order
+    torch.cuda.synchronize()
+    assert capi.last_status() == 0
+
+
+@pytest.mark.parametrize("case", [(2, 2, 64, 8, 1, 2048, 1024), (12, 14, 8, 4, 46, 1024, 512), (10, 11, 8, 2, 33, 512, 512), (16, 21, 4, 2, 30, 512, 256),
+                                  (23, 20, 8, 2, 100, 512, 256), (8, 8, 3, 3, 64, 256, 768)])
+def test_small_moe_step_matches_separate_products(case):
+    """The step on the small-batch kernel against one GEMV per (token, expert), the activation and the weighted sum."""
+    from vllm_gguf_plugin import ops
+
+    t13, t2, E, k, T, H, I = case
+    w13 = torch.from_numpy(np.stack([synth.make_weight(t13, 2 * I, H, seed=e) for e in range(E)])).to(DEV)
+    w2 = torch.from_numpy(np.stack([synth.make_weight(t2, H, I, seed=100 + e) for e in range(E)])).to(DEV)
+    x = (dev_x(T, H, seed=T).float() / 32).half()
+    twn, idn = synth.make_routing(T, E, k, T)
+    tw, ids = torch.from_numpy(twn).to(DEV), torch.from_numpy(idn).to(DEV).int()
+    ids[0, 0] = -1                                                             # not a valid expert: contributes nothing
+    y1 = ops.ggml_moe_a8_vec(x, w13, ids, k, t13, 2 * I, T)
+    a = (torch.nn.functional.silu(y1[:, :I].float()).half() * y1[:, I:]).contiguous()
+    a[0] = 0
+    y2 = ops.ggml_moe_a8_vec(a, w2, ids, 1, t2, H, T * k).view(T, k, H)
+    y2[0, 0] = 0
+    want = (y2.float() * tw.view(T, k, 1)).half().float().sum(1)
+    got = ops.ggml_fused_moe(x, w13, w2, tw, ids, t13, t2, "silu")
+    torch.cuda.synchronize()
+    assert capi.last_status() == 0
+    assert rel_l2(got.float().cpu(), want.cpu()) <= 2e-3

@@ -62,6 +62,38 @@ static int check_common(const void* W, const void* X, const void* Y, int type, i
   return E_OK;
 }
 
+// ---- batches of a few tokens (smallm.cu) ----
+static int64_t small_tiles(int64_t M) { return ((M < smallm_max_tokens() ? M : smallm_max_tokens()) + 7) / 8; }
+static int64_t small_bytes(int64_t M, int64_t N, int64_t K) { return smallm_scratch_bytes(small_tiles(M), 1, N, K); }
+// Up to two tokens the register-resident GEMV is faster (14336x4096 Q4_K, two tokens: 11.1 us against 16; IQ3_S 22.5 against
+// 22.7), from three on it would need a second pass over the weights (20.2, 42.6 us at four; 16.3, 22.7 here).
+static int64_t small_min_tokens() { return 3; }
+static bool small_fits(int64_t N, int64_t K) { return N < (int64_t)1 << 24 && K < (int64_t)1 << 24; }
+// Y = q8_1(X) . dequant(W)^T, in passes of up to smallm_max_tokens() tokens
+static int small_dense(const void* W, const void* X, void* Y, void* ws, int type, int dtype, int sum_mode, int64_t M, int64_t N, int64_t K,
+                       int64_t pitch, int64_t ldy, int* st, cudaStream_t s) {
+  const int64_t esz = dtype == DT_F32 ? 4 : 2, most = smallm_max_tokens();
+  for (int64_t m0 = 0; m0 < M; m0 += most) {
+    SmallArgs a{};
+    a.w = W;
+    a.x = static_cast<const uint8_t*>(X) + m0 * K * esz;
+    a.y = static_cast<uint8_t*>(Y) + m0 * ldy * esz;
+    a.ws = ws;
+    a.type = type; a.dtype = dtype; a.sum_mode = sum_mode;
+    a.m = M - m0 < most ? M - m0 : most;
+    a.n = N; a.k = K;
+    a.pitch = pitch; a.ldy = ldy;
+    a.tiles = (a.m + 7) / 8;
+    a.experts = a.max_passes = 1;
+    a.x_div = 1;
+    a.rows_out = a.m;
+    a.status = st;
+    const int rc = launch_smallm(a, s);
+    if (rc) return rc;
+  }
+  return E_OK;
+}
+
 }  // namespace gguf_b200
 
 extern "C" {
@@ -140,6 +172,9 @@ int gguf_b200_dequantize_rows(const void* W, int type, const int64_t* row_ids, i
 // tiled kernel (about 25 us on a 14336x4096 matrix whatever the batch) is faster.  Q6_K has the multi-vector kernel.
 static int64_t mmq_gemv_max_tokens(int type) { return type == T_Q6_K ? 16 : 4; }
 
+// ... and that the small-batch kernel serves instead, given room for its activation tiles
+static int64_t mmq_small_max_tokens() { return 16; }
+
 // activation matrix of the tensor-core kernels, rounded so that what follows it stays aligned
 static int64_t mmq_b_bytes(int type, int64_t M, int64_t K) { return round_up(M * mmq_ldb(type, K) * 2, 256); }
 
@@ -156,6 +191,13 @@ int64_t gguf_b200_workspace_bytes(int op, int type, int64_t M, int64_t N, int64_
   return 0;
 }
 
+int64_t gguf_b200_scratch_bytes(int op, int type, int64_t M, int64_t N, int64_t K) {
+  const int64_t least = gguf_b200_workspace_bytes(op, type, M, N, K);
+  const bool small = type_size(type) && N > 0 && K > 0 && M >= small_min_tokens() &&
+                     (op == GGUF_B200_OP_GEMV || (op == GGUF_B200_OP_MMQ && M <= mmq_small_max_tokens()));
+  return small && small_bytes(M, N, K) > least ? small_bytes(M, N, K) : least;
+}
+
 int gguf_b200_mul_mat_vec_a8(const void* W, const void* X, void* Y, void* ws, int64_t ws_bytes, int type, int dtype,
                              int64_t M, int64_t N, int64_t K, void* stream) {
   int rc = check_common(W, X, Y, type, dtype, M, N, K);
@@ -168,6 +210,8 @@ int gguf_b200_mul_mat_vec_a8(const void* W, const void* X, void* Y, void* ws, in
   // one or two vectors: ONE launch, the GEMV kernel quantizes the activations itself (same codes)
   rc = launch_gemv_fused(W, X, Y, type, dtype, M, N, K, gemv_sum_mode(type), st, s);
   if (rc <= 0) return rc;
+  if (M >= small_min_tokens() && small_fits(N, K) && ws_bytes >= small_bytes(M, N, K))
+    return small_dense(W, X, Y, ws, type, dtype, gemv_sum_mode(type), M, N, K, K / block_size(type) * type_size(type), N, st, s);
   // the Q4_K / Q5_K GEMV takes its min term from the quantized codes (sum_mode 1), all others from the fp16 sum
   rc = launch_quantize_q8_1(X, dtype, ws, M, K, Q8_MODE_SOA, gemv_sum_mode(type), 0, CORR_NONE, nullptr, 1, 0, s);
   if (rc) return rc;
@@ -391,6 +435,8 @@ int gguf_b200_mul_mat_a8(const void* W, const void* X, void* Y, void* ws, int64_
   int* st = status_ptr();
   if (!st) return E_CUDA;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (M >= small_min_tokens() && M <= mmq_small_max_tokens() && small_fits(N, K) && ws_bytes >= small_bytes(M, N, K))
+    return small_dense(W, X, Y, ws, type, dtype, type == T_Q5_0 ? 1 : 0, M, N, K, K / block_size(type) * type_size(type), N, st, s);
   if (M <= mmq_gemv_max_tokens(type)) {
     // GEMV kernels with the tiled kernels' formulas: min / offset terms from the stored fp16 sum of the
     // inputs -- except Q5_0, whose tiled kernel folds the -16 into the codes (no sum term at all:
@@ -510,11 +556,38 @@ FusedMoeLayout fused_moe_layout(int type13, int type2, int dtype, int64_t tokens
   L.total = o;
   return L;
 }
+// Up to this many tokens (and always for types without a tiled kernel) the step runs on the small-batch kernel: an expert
+// then sees a handful of tokens, and reading the weights of the experts in use is what it costs.
+constexpr int64_t kMoeSmallTokens = 64;
+bool moe_small(int type13, int type2, int64_t tokens) { return tokens <= kMoeSmallTokens || !is_mmq_type(type13) || !is_mmq_type(type2); }
+struct MoeSmallLayout {
+  int pass_tiles;
+  int64_t tiles, passes, o_sorted, o_passes, o_npass, o_y1, o_y2, o_ws, total;
+};
+MoeSmallLayout moe_small_layout(int dtype, int64_t tokens, int64_t top_k, int64_t E, int64_t H, int64_t I) {
+  MoeSmallLayout L{};
+  const int64_t slots = tokens * top_k, esz = dtype == DT_F32 ? 4 : 2;
+  L.pass_tiles = slots <= 8 * E ? 1 : slots <= 16 * E ? 2 : 4;   // an expert's share of the slots, on average, in one pass
+  L.tiles = moe_plan_tiles(slots, (int)E);
+  L.passes = moe_plan_passes(slots, (int)E, L.pass_tiles);
+  int64_t o = 0;
+  auto take = [&](int64_t bytes) { const int64_t at = o; o += round_up(bytes, 256); return at; };
+  L.o_sorted = take(L.tiles * 8 * 4);
+  L.o_passes = take(L.passes * 16);
+  L.o_npass = take(8);
+  L.o_y1 = take(slots * 2 * I * esz);
+  L.o_y2 = take(slots * H * esz);
+  const int64_t a = smallm_scratch_bytes(L.tiles, L.passes, 2 * I, H), b = smallm_scratch_bytes(L.tiles, L.passes, H, I);
+  L.o_ws = take(a > b ? a : b);
+  L.total = o;
+  return L;
+}
 }  // namespace
 
 int64_t gguf_b200_fused_moe_workspace_bytes(int type13, int type2, int dtype, int64_t tokens, int64_t top_k, int64_t n_experts,
                                             int64_t H, int64_t I) {
-  if (!is_mmq_type(type13) || !is_mmq_type(type2) || tokens < 0 || top_k <= 0 || n_experts <= 0 || n_experts > 256 || H <= 0 || I <= 0) return 0;
+  if (!type_size(type13) || !type_size(type2) || tokens < 0 || top_k <= 0 || n_experts <= 0 || n_experts > 256 || H <= 0 || I <= 0) return 0;
+  if (moe_small(type13, type2, tokens)) return moe_small_layout(dtype, tokens, top_k, n_experts, H, I).total;
   return fused_moe_layout(type13, type2, dtype, tokens, top_k, n_experts, H, I).total;
 }
 
@@ -525,11 +598,50 @@ int gguf_b200_fused_moe(const void* X, const void* W13, const void* W2, void* Y,
   if (rc) return rc;
   rc = check_common(W2, X, Y, type2, dtype, tokens, H, I);
   if (rc) return rc;
-  if (!is_mmq_type(type13) || !is_mmq_type(type2)) return E_BAD_TYPE;
   if (top_k <= 0 || n_experts <= 0 || (act != 1 && act != 2) || I % 8 != 0) return E_BAD_SHAPE;
   if (n_experts > 256) return E_TOO_LARGE;
   if (tokens == 0) return E_OK;
   if (!topk_ids || !topk_weights || !ws || !aligned16(ws)) return E_BAD_POINTER;
+  if (moe_small(type13, type2, tokens)) {
+    const MoeSmallLayout L = moe_small_layout(dtype, tokens, top_k, n_experts, H, I);
+    if (ws_bytes < L.total) return E_WORKSPACE;
+    if (!small_fits(n_experts * 2 * I, H) || !small_fits(n_experts * H, I)) return E_TOO_LARGE;
+    int* st = status_ptr();
+    if (!st) return E_CUDA;
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    uint8_t* base = static_cast<uint8_t*>(ws);
+    int32_t* sorted = reinterpret_cast<int32_t*>(base + L.o_sorted);
+    int32_t* npass = reinterpret_cast<int32_t*>(base + L.o_npass);
+    const int64_t slots = tokens * top_k;
+    rc = launch_moe_plan(topk_ids, slots, (int)n_experts, L.pass_tiles, sorted, base + L.o_passes, npass, s);
+    if (rc) return rc;
+    auto gemm = [&](const void* x, int64_t x_div, int act_mode, const void* w, int type, int64_t N, int64_t K, void* y, const float* scale) {
+      SmallArgs a{};
+      a.w = w; a.x = x; a.y = y; a.ws = base + L.o_ws;
+      a.type = type; a.dtype = dtype; a.sum_mode = gemv_sum_mode(type);
+      a.m = slots; a.n = N; a.k = K;
+      a.pitch = K / block_size(type) * type_size(type);
+      a.ldy = N;
+      a.tiles = L.tiles;
+      a.experts = n_experts;
+      a.max_passes = L.passes;
+      a.passes = base + L.o_passes;
+      a.n_passes = npass;
+      a.sorted = sorted;
+      a.pass_tiles = L.pass_tiles;
+      a.rows_out = slots;
+      a.x_div = x_div;
+      a.act = act_mode;
+      a.row_scale = scale;
+      a.status = st;
+      return launch_smallm(a, s);
+    };
+    rc = gemm(X, top_k, 0, W13, type13, 2 * I, H, base + L.o_y1, nullptr);
+    if (rc) return rc;
+    rc = gemm(base + L.o_y1, 1, act, W2, type2, H, I, base + L.o_y2, topk_weights);
+    if (rc) return rc;
+    return launch_moe_sum(base + L.o_y2, Y, topk_ids, (int)n_experts, tokens, top_k, H, dtype, s);
+  }
   const FusedMoeLayout L = fused_moe_layout(type13, type2, dtype, tokens, top_k, n_experts, H, I);
   if (ws_bytes < L.total) return E_WORKSPACE;
   int* st = status_ptr();

@@ -134,10 +134,47 @@ int mmq_moe_block_size();
 
 int64_t q8_soa_bytes(int64_t M, int64_t K);
 
+// Small-batch product on the 8-bit tensor instruction (smallm.cu), dense or per expert.  The activations are quantized into
+// tiles of eight columns by launch_quantize_frag, which launch_smallm calls first.
+struct SmallArgs {
+  const void* w;             // packed weights (expert 0), rows `pitch` bytes apart
+  const void* x;             // activations, element type dtype
+  void* y;                   // element type dtype, rows ldy elements apart
+  void* ws;                  // smallm_scratch_bytes(tiles, max_passes, n, k), 256-byte aligned
+  int type, dtype, sum_mode; // sum_mode: see gemv_sum_mode
+  int64_t m, n, k;           // tokens (dense), weight rows, values per row
+  int64_t pitch, ldy;
+  int64_t tiles;             // column tiles of eight (MoE: room for)
+  int64_t experts, max_passes;   // dense: 1, 1
+  // MoE (null passes = dense): written on the device by launch_moe_plan
+  const void* passes;        // int4 {expert, first column tile, column tiles, 0}
+  const int32_t* n_passes;   // [0] passes, [1] column tiles in use
+  const int32_t* sorted;     // output row of every column, rows_out in padding columns
+  int pass_tiles;            // column tiles of a pass (1, 2 or 4)
+  int64_t rows_out;
+  int64_t x_div;             // column c takes activation row sorted[c] / x_div
+  int act;                   // 1 silu, 2 gelu: the rows of x are [gate | up] of 2k values (see launch_quantize_q8_1)
+  const float* row_scale;
+  int* status;
+};
+int launch_smallm(const SmallArgs& a, cudaStream_t stream);
+int launch_quantize_frag(const SmallArgs& a, void* out, int* counters, int64_t n_counters, cudaStream_t stream);
+int64_t smallm_scratch_bytes(int64_t tiles, int64_t passes, int64_t n, int64_t k);
+int smallm_max_tokens();
+int smallm_table_bytes(int type);
+bool smallm_pairs_with_sum(int type);
+int smallm_order(int type);      // order of a block's values in the tiles (smallm_decode.cuh)
+
 // fused MoE step (moe_fused.cu)
 int64_t moe_align_sorted_len(int64_t slots, int n_experts, int block);
 int launch_moe_align(const int32_t* topk_ids, int64_t slots, int n_experts, int block, int32_t* scratch, int32_t* sorted_ids,
                      int32_t* expert_ids, int32_t* n_post_pad, cudaStream_t stream);
+// the same lists for the small-batch kernel: columns in tiles of eight, passes of up to pass_tiles tiles of one expert.
+// sorted[8 * tiles] (padded with `slots`), passes int4[max_passes], n_passes[2]
+int64_t moe_plan_tiles(int64_t slots, int n_experts);                       // room for column tiles
+int64_t moe_plan_passes(int64_t slots, int n_experts, int pass_tiles);
+int launch_moe_plan(const int32_t* topk_ids, int64_t slots, int n_experts, int pass_tiles, int32_t* sorted, void* passes, int32_t* n_passes,
+                    cudaStream_t stream);
 int launch_moe_sum(const void* y, void* out, const int32_t* topk_ids, int n_experts, int64_t tokens, int64_t top_k, int64_t h,
                    int dtype, cudaStream_t stream);
 

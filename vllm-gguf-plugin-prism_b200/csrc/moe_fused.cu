@@ -103,6 +103,76 @@ int launch_moe_align(const int32_t* topk_ids, int64_t slots, int n_experts, int 
   return E_OK;
 }
 
+// ---- lists of the small-batch form (smallm.cu) ----
+// One CTA, one warp per expert in turn: slots are few there (at most a few hundred), so that one launch that scans them twice
+// is cheaper than three that scan them once.
+__global__ void __launch_bounds__(1024) moe_plan_kernel(const int32_t* __restrict__ topk_ids, int slots, int n_experts, int pass_tiles,
+                                                        int32_t* __restrict__ sorted, int4* __restrict__ passes, int32_t* __restrict__ n_passes) {
+  pdl_trigger();
+  pdl_wait();
+  __shared__ int32_t s_cnt[256], s_tile[257], s_pass[257];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int e = warp; e < n_experts; e += 32) {
+    int c = 0;
+    for (int s = lane; s < slots; s += 32) c += topk_ids[s] == e ? 1 : 0;
+    c = __reduce_add_sync(0xffffffffu, c);
+    if (lane == 0) s_cnt[e] = c;
+  }
+  __syncthreads();
+  if (warp == 0) {   // exclusive prefix sums of the experts' column tiles and passes
+    int tiles = 0, ps = 0;
+    for (int e0 = 0; e0 < n_experts; e0 += 32) {
+      const int e = e0 + lane, nt = e < n_experts ? (s_cnt[e] + 7) / 8 : 0, np = (nt + pass_tiles - 1) / pass_tiles;
+      int a = nt, b = np;
+#pragma unroll
+      for (int m = 1; m < 32; m <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, a, m), v = __shfl_up_sync(0xffffffffu, b, m);
+        if (lane >= m) { a += u; b += v; }
+      }
+      if (e < n_experts) {
+        s_tile[e] = tiles + a - nt;
+        s_pass[e] = ps + b - np;
+      }
+      tiles += __shfl_sync(0xffffffffu, a, 31);
+      ps += __shfl_sync(0xffffffffu, b, 31);
+    }
+    if (lane == 0) {
+      n_passes[0] = ps;
+      n_passes[1] = tiles;
+    }
+  }
+  __syncthreads();
+  for (int e = warp; e < n_experts; e += 32) {
+    const int nt = (s_cnt[e] + 7) / 8, t0 = s_tile[e];
+    for (int i = lane; i < (nt + pass_tiles - 1) / pass_tiles; i += 32)
+      passes[s_pass[e] + i] = make_int4(e, t0 + i * pass_tiles, nt - i * pass_tiles < pass_tiles ? nt - i * pass_tiles : pass_tiles, 0);
+    int pos = 8 * t0;
+    for (int s0 = 0; s0 < slots && nt > 0; s0 += 32) {
+      const int s = s0 + lane;
+      const bool mine = s < slots && topk_ids[s] == e;
+      const unsigned m = __ballot_sync(0xffffffffu, mine);
+      if (mine) sorted[pos + __popc(m & ((1u << lane) - 1u))] = s;
+      pos += __popc(m);
+    }
+    for (int i = pos + lane; i < 8 * (t0 + nt); i += 32) sorted[i] = slots;
+  }
+}
+
+int64_t moe_plan_tiles(int64_t slots, int n_experts) {
+  const int64_t worst = slots / 8 + n_experts;      // every expert may leave one tile unfilled
+  return slots < worst ? slots : worst;
+}
+int64_t moe_plan_passes(int64_t slots, int n_experts, int pass_tiles) {
+  const int64_t worst = slots / (8 * pass_tiles) + n_experts;
+  return slots < worst ? slots : worst;
+}
+int launch_moe_plan(const int32_t* topk_ids, int64_t slots, int n_experts, int pass_tiles, int32_t* sorted, void* passes, int32_t* n_passes,
+                    cudaStream_t stream) {
+  if (n_experts < 1 || n_experts > 256 || slots > 1 << 20) return E_BAD_SHAPE;
+  return launch_pdl(moe_plan_kernel, dim3(1), dim3(1024), 0, stream, topk_ids, (int)slots, n_experts, pass_tiles, sorted, static_cast<int4*>(passes),
+                    n_passes) == cudaSuccess ? E_OK : E_CUDA;
+}
+
 template <typename T>
 __global__ void __launch_bounds__(256) moe_sum_kernel(const T* __restrict__ y, T* __restrict__ out, const int32_t* __restrict__ topk_ids,
                                                       int n_experts, int64_t tokens, int top_k, int64_t h) {

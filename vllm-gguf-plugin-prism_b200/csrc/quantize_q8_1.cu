@@ -235,6 +235,123 @@ __global__ void __launch_bounds__(256) quantize_f16x8_kernel(const in_t* __restr
   }
 }
 
+// Activation tiles of the small-batch kernel (smallm.cu): column tile = eight activation rows, chunk = 256 values.  A tile
+// holds eight blocks of 256 code bytes -- lane (column g, t) of a warp finds the eight codes of its fragment in the eight
+// bytes at 8 * lane, in the order the weight format dictates (smallm_decode.cuh) --, then per block and column the pair
+// {d8, -1.5 * 2^23 * d8} ({d8, s8} for the formats that round their products to fp16), then the s8 of the chunk as two tf32
+// parts in the order of a tensor-instruction fragment.  Four lanes quantize a block as in quantize_f16x8_kernel.  Also clears the consumer's arrival counters.
+template <typename in_t>
+__global__ void __launch_bounds__(256) quantize_frag_kernel(const in_t* __restrict__ x, uint8_t* __restrict__ out, int64_t rows, int64_t K,
+                                                            int tiles, int nc, int order, int with_sum, int sum_mode, const int32_t* __restrict__ sorted,
+                                                            const int32_t* __restrict__ n_used, int x_div, int act, int64_t x_ld,
+                                                            int* __restrict__ counters, int n_counters) {
+  pdl_trigger();
+  pdl_wait();
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_counters; i += gridDim.x * blockDim.x) counters[i] = 0;
+  const int used = n_used ? n_used[1] : tiles;                    // column tiles in use
+  const int nb = nc * 8;                                          // blocks of a column
+  const int total = used * nb;                                    // one warp per (tile, block)
+  const bool vec = K % 8 == 0 && x_ld % 8 == 0;
+  for (int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < total; i += gridDim.x * (blockDim.x >> 5)) {
+    const int tile = i / nb, kb = i - tile * nb;
+    const int col = tile * 8 + g, k = kb * 32 + 8 * t;
+    int64_t src = col;
+    bool have = src < rows;
+    if (sorted) {
+      const int id = sorted[col];
+      have = id < rows;
+      src = have ? id / x_div : 0;
+    }
+    float v[8];
+    const in_t* xr = x + src * x_ld + k;
+    if (have && k + 8 <= K && vec && sizeof(in_t) == 2) {
+      const uint4 a = *reinterpret_cast<const uint4*>(xr);
+      const in_t* e = reinterpret_cast<const in_t*>(&a);
+      if (act) {
+        const uint4 b = *reinterpret_cast<const uint4*>(xr + K);
+        const in_t* f = reinterpret_cast<const in_t*>(&b);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = act_mul<in_t>(act, to_float<in_t>(e[j]), to_float<in_t>(f[j]));
+      } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = to_float<in_t>(e[j]);
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        v[j] = !(have && k + j < K) ? 0.f : act ? act_mul<in_t>(act, to_float<in_t>(xr[j]), to_float<in_t>(xr[K + j])) : to_float<in_t>(xr[j]);
+    }
+    float amax = 0.f, sm[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      amax = fmaxf(amax, fabsf(v[j]));
+      sm[j] = v[j] + __shfl_xor_sync(0xffffffffu, v[j], 2, 32);          // i ^ 16
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) sm[j] += __shfl_xor_sync(0xffffffffu, sm[j], 1, 32);   // i ^ 8
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2, 32));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1, 32));
+    float s4[4], s2[2];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) s4[j] = sm[j] + sm[j + 4];               // i ^ 4
+#pragma unroll
+    for (int j = 0; j < 2; ++j) s2[j] = s4[j] + s4[j + 2];               // i ^ 2
+    const float sum = s2[0] + s2[1];                                      // i ^ 1
+    const float d = amax / 127;
+    uint32_t w0 = 0, w1 = 0;
+    int qs = 0;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int8_t qq = amax == 0.0f ? 0 : roundf(v[j] / d);
+      qs += qq;
+      if (j < 4) w0 |= ((uint32_t)qq & 0xFFu) << (8 * j);
+      else w1 |= ((uint32_t)qq & 0xFFu) << (8 * (j - 4));
+    }
+    qs += __shfl_xor_sync(0xffffffffu, qs, 2, 32);
+    qs += __shfl_xor_sync(0xffffffffu, qs, 1, 32);
+    uint8_t* blk = out + ((size_t)(kb >> 3) * tiles + tile) * 3072;
+    uint8_t* codes = blk + (kb & 7) * 256 + g * 32;
+    if (order == 1) {
+      *reinterpret_cast<uint2*>(codes + 8 * t) = make_uint2(w0, w1);
+    } else if (order == 0) {   // word v of the block goes to lane v % 4, half v / 4; this lane has the words 2t, 2t + 1
+      *reinterpret_cast<uint32_t*>(codes + 8 * ((2 * t) & 3) + 4 * (t >> 1)) = w0;
+      *reinterpret_cast<uint32_t*>(codes + 8 * ((2 * t + 1) & 3) + 4 * (t >> 1)) = w1;
+    } else {                   // words i and 4 + i byte-interleaved for lane i
+      const uint32_t other = __shfl_xor_sync(0xffffffffu, t < 2 ? w1 : w0, 2, 32);
+      const uint32_t lo = t < 2 ? w0 : other, hi = t < 2 ? other : w1;
+      *reinterpret_cast<uint2*>(codes + 8 * (t < 2 ? 2 * t : 2 * t - 3)) = make_uint2(__byte_perm(lo, hi, 0x5140), __byte_perm(lo, hi, 0x7362));
+    }
+    if (t == 0) {
+      const float d8 = __half2float(__float2half(d));
+      const float s8 = sum_mode ? d8 * (float)qs : __half2float(__float2half(sum));
+      *reinterpret_cast<float2*>(blk + 2048 + (kb & 7) * 64 + g * 8) = make_float2(d8, with_sum ? s8 : -12582912.f * d8);
+      const float hi = __uint_as_float(__float_as_uint(s8) & 0xFFFFE000u), lo = s8 - hi;
+      float* f = reinterpret_cast<float*>(blk + 2560 + (g * 4 + (kb & 3)) * 16 + 4 * ((kb >> 2) & 1));   // {hi, hi of block + 4, lo, lo of block + 4}
+      f[0] = hi;
+      f[2] = __uint_as_float(__float_as_uint(lo) & 0xFFFFE000u);
+    }
+  }
+}
+
+int launch_quantize_frag(const SmallArgs& a, void* out, int* counters, int64_t n_counters, cudaStream_t stream) {
+  const int nc = (int)((a.k + 255) / 256), order = smallm_order(a.type);
+  const int64_t rows = a.passes ? a.rows_out : a.m, x_ld = a.act ? 2 * a.k : a.k;
+  const int64_t want = (a.tiles * nc * 8 + 7) / 8;
+  const dim3 grid((unsigned)(want > 148 * 8 ? 148 * 8 : want));
+  uint8_t* o = static_cast<uint8_t*>(out);
+  auto go = [&](auto kern, auto* x) {
+    return launch_pdl(kern, grid, dim3(256), 0, stream, x, o, rows, a.k, (int)a.tiles, nc, order, smallm_pairs_with_sum(a.type) ? 1 : 0, a.sum_mode, a.sorted, a.n_passes, (int)a.x_div,
+                      a.act, x_ld, counters, (int)n_counters) == cudaSuccess ? E_OK : E_CUDA;
+  };
+  switch (a.dtype) {
+    case DT_F32: return go(quantize_frag_kernel<float>, static_cast<const float*>(a.x));
+    case DT_F16: return go(quantize_frag_kernel<__half>, static_cast<const __half*>(a.x));
+    case DT_BF16: return go(quantize_frag_kernel<__nv_bfloat16>, static_cast<const __nv_bfloat16*>(a.x));
+  }
+  return E_BAD_DTYPE;
+}
+
 template <int MODE>
 static int launch_mode(const void* x, int x_dtype, void* out, int64_t M, int64_t K, int sum_mode, int64_t ldb,
                        int corr_mode, const int32_t* gid, int64_t gdiv, int64_t glim, cudaStream_t stream, Q8Tp wt = Q8Tp{}) {

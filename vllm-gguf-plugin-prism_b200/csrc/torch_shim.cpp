@@ -119,7 +119,7 @@ static Tensor matmul_common(const Tensor& W, const Tensor& X, int64_t type, int6
   const int64_t M = X.size(0);
   Tensor Y = new_tensor({M, row}, X.scalar_type(), X.device());
   if (M == 0 || row == 0) return Y;
-  const int64_t ws_bytes = gguf_b200_workspace_bytes(op, (int)type, M, row, K);
+  const int64_t ws_bytes = gguf_b200_scratch_bytes(op, (int)type, M, row, K);
   const Scratch ws(ws_bytes);
   void* s = current_stream(X.get_device());
   int rc;
@@ -192,7 +192,7 @@ Tensor ggml_moe_a8_vec(const Tensor& X, const Tensor& W, const Tensor& topk_ids,
   return Y;
 }
 
-// The tiled MoE step in one call (see gguf_b200_fused_moe).  act: 1 silu, 2 gelu.
+// The MoE step in one call (see gguf_b200_fused_moe).  act: 1 silu, 2 gelu.
 Tensor fused_moe(const Tensor& X, const Tensor& W13, const Tensor& W2, const Tensor& topk_weights, const Tensor& topk_ids, int64_t type13,
                  int64_t type2, int64_t act) {
   const c10::cuda::CUDAGuard guard(X.device());
@@ -330,7 +330,22 @@ PyObject* py_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
+// moe(x, W13, W2, topk_weights, topk_ids, type13, type2, act): the whole expert step
+PyObject* py_moe(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  TORCH_CHECK(n == 8, "moe takes 8 arguments");
+  const Tensor* t[5];
+  for (int i = 0; i < 5; ++i)
+    if (!(t[i] = plain_cuda(a[i]))) Py_RETURN_NONE;
+  if (!modes_off()) Py_RETURN_NONE;
+  const long type13 = PyLong_AsLong(a[5]), type2 = PyLong_AsLong(a[6]), act = PyLong_AsLong(a[7]);
+  if (PyErr_Occurred()) return nullptr;
+  return THPVariable_Wrap(fused_moe(*t[0], *t[1], *t[2], *t[3], *t[4], type13, type2, act));
+  END_HANDLE_TH_ERRORS
+}
+
 PyMethodDef methods[] = {
+    {"moe", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(&py_moe)), METH_FASTCALL, nullptr},
     {"mul_mat", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(&py_mul_mat)), METH_FASTCALL, nullptr},
     {"embed", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(&py_embed)), METH_FASTCALL, nullptr},
     {"linear", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(&py_linear)), METH_FASTCALL, nullptr},

@@ -13,6 +13,7 @@ matters, and stay with IEEE defaults.
 from __future__ import annotations
 
 import os
+import re
 import subprocess
 import sys
 import sysconfig
@@ -25,7 +26,7 @@ OUT = PKG / "vllm_gguf_plugin"
 OBJ = PKG / "build"
 CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-CU_FILES = ["capi.cu", "quantize_q8_1.cu", "dequantize.cu", "gemv.cu", "gemv1.cu", "mmq.cu", "noalloc.cu", "tp.cu", "moe_fused.cu"]
+CU_FILES = ["capi.cu", "quantize_q8_1.cu", "dequantize.cu", "gemv.cu", "gemv1.cu", "smallm.cu", "smallm_inst_a.cu", "smallm_inst_b.cu", "smallm_inst_c.cu", "mmq.cu", "noalloc.cu", "tp.cu", "moe_fused.cu"]
 FAST_MATH = {"quantize_q8_1.cu", "gemv1.cu"}
 
 
@@ -36,8 +37,15 @@ def _stale(target: Path, deps) -> bool:
     return any(Path(d).stat().st_mtime > t for d in deps)
 
 
-def _headers():
-    return list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.h")) + list((PKG.parent / "include").glob("*.h"))
+def _includes(src: Path, seen=None) -> set:
+    """The source and the project headers it includes, directly or not."""
+    seen = set() if seen is None else seen
+    if src not in seen:
+        seen.add(src)
+        for name in re.findall(r'^#include "([^"]+)"', src.read_text(), flags=re.M):
+            if (src.parent / name).exists():
+                _includes((src.parent / name).resolve(), seen)
+    return seen
 
 
 def _nvcc(src: Path, obj: Path, verbose: bool):
@@ -52,12 +60,11 @@ def _nvcc(src: Path, obj: Path, verbose: bool):
 def build_kernels(force: bool = False, verbose: bool = False) -> Path:
     OBJ.mkdir(exist_ok=True)
     so = OUT / "libgguf_b200.so"
-    hdrs = _headers()
     srcs = [CSRC / f for f in CU_FILES if (CSRC / f).exists()]
     jobs = []
     for src in srcs:
         obj = OBJ / (src.stem + ".o")
-        if force or _stale(obj, [src, *hdrs]):
+        if force or _stale(obj, _includes(src)):
             jobs.append((src, obj))
     if jobs:
         with ThreadPoolExecutor(max_workers=min(len(jobs), os.cpu_count() or 4)) as ex:

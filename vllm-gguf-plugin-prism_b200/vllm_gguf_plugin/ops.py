@@ -18,7 +18,7 @@ Differences from the reference, all deliberate:
   instead of 4; callers already feed it to ``moe_align_block_size`` (fused_moe.py:64-68);
 * ``ggml_dequantize_rows`` is new: the embedding look-up (index_select of rows + ggml_dequantize,
   quantization/vocal_embeds.py:88-96) as one kernel;
-* ``ggml_fused_moe`` is new: the whole tiled MoE step of a layer in one call;
+* ``ggml_fused_moe`` is new: the whole MoE step of a layer in one call;
 * ``ggml_dequant_matmul`` is new: the fused form of "ggml_dequantize then x @ W.T" that the
   reference uses for IQ types above the GEMV batch threshold (quantization/linear.py:50-54).
 """
@@ -214,14 +214,18 @@ MOE_ACTIVATIONS = {"silu": 1, "gelu": 2}
 
 def ggml_fused_moe(X: torch.Tensor, W13: torch.Tensor, W2: torch.Tensor, topk_weights: torch.Tensor, topk_ids: torch.Tensor,
                    quant_type: int, quant_type2: int, activation: str) -> torch.Tensor:
-    """The tiled MoE step of one layer in one call: alignment, gate/up expert GEMM, activation, down
-    expert GEMM, routing weights and the top-k sum (the reference runs six ops for it,
-    quantization/fused_moe.py:56-95).  X [T, H] -> [T, H]."""
-    _require(quant_type, _CUDA_GEMM_QUANT_TYPES, "ggml_fused_moe")
-    _require(quant_type2, _CUDA_GEMM_QUANT_TYPES, "ggml_fused_moe")
-    return torch.ops._C_gguf.fused_moe(X, W13, W2, topk_weights.to(torch.float32).contiguous(),
-                                       topk_ids.to(torch.int32).contiguous(), quant_type, quant_type2,
-                                       MOE_ACTIVATIONS[activation])
+    """The MoE step of one layer in one call: alignment, gate/up expert product, activation, down expert product, routing
+    weights and the top-k sum (the reference runs six ops for it, quantization/fused_moe.py:56-133).  X [T, H] -> [T, H].
+    Up to 64 tokens, and for the code-book types, on the small-batch kernel; above that on the tiled one."""
+    _require(quant_type, _CUDA_GEMV_QUANT_TYPES, "ggml_fused_moe")
+    _require(quant_type2, _CUDA_GEMV_QUANT_TYPES, "ggml_fused_moe")
+    if topk_weights.dtype != torch.float32 or not topk_weights.is_contiguous():
+        topk_weights = topk_weights.to(torch.float32).contiguous()
+    if topk_ids.dtype != torch.int32 or not topk_ids.is_contiguous():
+        topk_ids = topk_ids.to(torch.int32).contiguous()
+    act = MOE_ACTIVATIONS[activation]
+    y = None if is_compiling() else _C_gguf.moe(X, W13, W2, topk_weights, topk_ids, quant_type, quant_type2, act)
+    return torch.ops._C_gguf.fused_moe(X, W13, W2, topk_weights, topk_ids, quant_type, quant_type2, act) if y is None else y
 
 
 def ggml_moe_a8_vec(

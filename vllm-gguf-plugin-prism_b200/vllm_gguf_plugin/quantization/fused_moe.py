@@ -14,6 +14,7 @@ import os
 
 import torch
 import torch.nn.functional as F
+from torch.compiler import is_compiling
 
 from .. import ops
 from .utils import MMQ_QUANT_TYPES, MMVQ_QUANT_TYPES, logger
@@ -98,15 +99,15 @@ def _fused_moe_gguf(
     weight_type2: int,
     activation: str,
 ) -> torch.Tensor:
-    out_hidden_states = torch.empty_like(x)
     num_tokens, _ = x.shape
     E, N, _ = w1.shape
     top_k = topk_ids.shape[1]
+    if (activation in ops.MOE_ACTIVATIONS and E <= 256 and w2.shape[0] == E and (N // 2) % 8 == 0 and x.shape[0] > 0
+            and int(weight_type) in ops.QUANT_SIZES and int(weight_type2) in ops.QUANT_SIZES
+            and os.environ.get("VLLM_GGUF_FUSED_MOE", "1") == "1"):
+        # one call: alignment, both expert products, activation, routing weights and top-k sum
+        return ops.ggml_fused_moe(x, w1, w2, topk_weights, topk_ids, weight_type, weight_type2, activation)
     if weight_type2 in MMQ_QUANT_TYPES and weight_type in MMQ_QUANT_TYPES and x.shape[0] > 64:
-        if (activation in ops.MOE_ACTIVATIONS and E <= 256 and w2.shape[0] == E and (N // 2) % 8 == 0
-                and os.environ.get("VLLM_GGUF_FUSED_MOE", "1") == "1"):
-            # one call: alignment, both expert GEMMs, activation, routing weights and top-k sum
-            return ops.ggml_fused_moe(x, w1, w2, topk_weights, topk_ids, weight_type, weight_type2, activation)
         # the reference's sequence of separate ops (fused_moe.py:64-95)
         block_size = ops.ggml_moe_get_block_size(weight_type)
         sorted_token_ids, expert_ids, num_tokens_post_padded = _align(topk_ids, block_size, E)
@@ -124,6 +125,7 @@ def _fused_moe_gguf(
         raise NotImplementedError(
             f"no GGUF MoE kernel for quantization types ({int(weight_type)}, {int(weight_type2)})")
     out = out.reshape(num_tokens, top_k, w2.shape[1]).mul_(topk_weights.view(num_tokens, top_k, 1).to(out.dtype))
+    out_hidden_states = torch.empty_like(x)
     ops.moe_sum(out, out_hidden_states)
     return out_hidden_states
 
@@ -215,5 +217,6 @@ class GGUFMoEMethod(FusedMoEMethodBase):
             raise NotImplementedError("Apply router weight on input is not supported for fused GGUF MoE method.")
         activation = getattr(layer, "activation", "silu")
         activation = getattr(activation, "value", activation)
-        return fused_moe_gguf(x, layer.w13_weight, layer.w2_weight, topk_weights, topk_ids,
+        step = fused_moe_gguf if is_compiling() else _fused_moe_gguf   # eager: no custom-op dispatch in between
+        return step(x, layer.w13_weight, layer.w2_weight, topk_weights, topk_ids,
                               layer.w13_weight_type.weight_type, layer.w2_weight_type.weight_type, activation)
