@@ -921,3 +921,47 @@ def test_small_moe_step_matches_separate_products(case):
     torch.cuda.synchronize()
     assert capi.last_status() == 0
     assert rel_l2(got.float().cpu(), want.cpu()) <= 2e-3
+
+
+# ragged last tiles, one and two accumulators, two instructions per stage, tiles whole / cut evenly / in runs over all SMs
+TILED_SHAPES = [(7, 256, 20), (259, 768, 100), (2048, 1280, 40), (77, 4096, 513), (1000, 2048, 300), (8192, 1024, 129), (14336, 512, 385)]
+
+
+@pytest.mark.parametrize("name", sorted(TYPES))
+def test_tiled_product_of_every_shape(name):
+    """The tensor-core product against row-by-row products (or, for the types it multiplies dequantized, against those weights)."""
+    from vllm_gguf_plugin import ops
+
+    t = TYPES[name]
+    quantized = name in MMQ_TYPES
+    if name == "Q5_0":
+        pytest.skip("its tiled and row formulas differ by the rounding of the offset; see test_mmq_parity")
+    for N, K, M in TILED_SHAPES:
+        _, w = dev_w(t, N, K, seed=N + K)
+        x = (dev_x(M, K, seed=M).float() / 8).half()
+        run = ops.ggml_mul_mat_a8 if quantized else ops.ggml_dequant_matmul
+        y = run(w, x, t, N)
+        if quantized:
+            want = torch.cat([ops.ggml_mul_mat_vec_a8(w, x[i:i + 16].float().contiguous(), t, N) for i in range(0, M, 16)])
+        else:
+            want = (x.double() @ capi.dequantize(w, t, N, K, torch.float16).double().T).float()
+        assert rel_l2(y.float().cpu(), want.cpu()) <= REL_L2_TOL, (N, K, M)
+        assert torch.equal(y, run(w, x, t, N))          # shared tiles are added in a fixed order
+    torch.cuda.synchronize()
+    assert capi.last_status() == 0
+
+
+@pytest.mark.parametrize("pad", [16, 4096 + 32])
+@pytest.mark.parametrize("name", ["Q4_K", "Q6_K"])
+def test_moe_experts_with_a_gap_between_them(name, pad):
+    """Expert matrices that do not lie back to back give what packed ones give."""
+    t, E, N, K, T, top_k = TYPES[name], 4, 264, 512, 40, 2
+    w = torch.from_numpy(np.stack([synth.make_weight(t, N, K, seed=e) for e in range(E)])).to(DEV)
+    x = dev_x(T, K, seed=T)
+    _, idn = synth.make_routing(T, E, top_k, T)
+    s, e, n = (torch.from_numpy(v).to(DEV) for v in synth.moe_align_block_size(idn, 64, E))
+    buf = torch.zeros(E * (N * w.shape[2] + pad), dtype=torch.uint8, device=DEV)
+    spread = buf.as_strided((E, N, w.shape[2]), (N * w.shape[2] + pad, w.shape[2], 1))
+    spread.copy_(w)
+    assert torch.equal(capi.moe_a8(x, spread, s, e, n, t, N, top_k, T), capi.moe_a8(x, w, s, e, n, t, N, top_k, T))
+    assert capi.last_status() == 0

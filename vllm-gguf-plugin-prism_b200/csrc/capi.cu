@@ -3,6 +3,8 @@
 // synchronisation (except gguf_b200_last_status), no exceptions.
 #include "../../include/gguf_b200.h"
 
+#include <math.h>
+
 #include "common.cuh"
 #include "kernels.h"
 
@@ -94,6 +96,46 @@ static int small_dense(const void* W, const void* X, void* Y, void* ws, int type
   return E_OK;
 }
 
+static bool is_dequant_matmul_type(int t) {
+  return t == T_IQ2_XXS || t == T_IQ2_XS || t == T_IQ2_S || t == T_IQ3_XXS || t == T_IQ3_S || t == T_IQ1_S || t == T_IQ1_M || t == T_IQ4_NL || t == T_IQ4_XS;
+}
+// activation matrix of the tensor-core kernels, rounded so that what follows it stays aligned
+static int64_t mmq_b_bytes(int type, int64_t M, int64_t K) { return round_up(M * mmq_ldb(type, K) * 2, 256); }
+
+// The tensor-core GEMM on q8_1 activations (quantize != 0) or on the activations as they are.
+static int tiled_dense(bool quantize, const void* W, const void* X, void* Y, void* ws, int64_t ws_bytes, int type, int dtype, int64_t M, int64_t N,
+                       int64_t K, int64_t pitch, int64_t ldy, const MmqTp* tp, int* st, cudaStream_t s) {
+  MmqArgs a{};
+  a.w = W; a.y = Y;
+  a.type = type; a.out_dtype = dtype;
+  a.M = M; a.N = N; a.K = K;
+  a.pitch = pitch; a.ldy = ldy;
+  a.status = st;
+  a.tp = tp;
+  // whatever the caller gave beyond the activation matrix may hold the parts of shared tiles
+  const int64_t used = quantize ? mmq_b_bytes(type, M, K) : 0;
+  const MmqShare share = mmq_share(type, M, N, K);
+  if (share.part_bytes > 0 && ws && aligned16(ws) && ws_bytes >= used + share.counter_bytes + share.part_bytes) {
+    a.counter = reinterpret_cast<int*>(static_cast<uint8_t*>(ws) + used);
+    a.part = static_cast<uint8_t*>(ws) + used + share.counter_bytes;
+    a.part_bytes = share.part_bytes;
+  }
+  if (quantize) {
+    a.ldb = mmq_ldb(type, K);
+    a.corr_mode = mmq_corr_mode(type);
+    a.perm = mmq_perm(type, K, pitch);
+    a.b = ws; a.b_dtype = DT_F16;
+    const int rc = launch_quantize_q8_1(X, dtype, ws, M, K, Q8_MODE_F16, 0, a.ldb, a.corr_mode, nullptr, 1, 0, s, a.perm, nullptr, 0, 0, a.counter,
+                                        a.counter ? share.n_counters : 0);
+    if (rc) return rc;
+  } else {
+    a.b = X; a.b_dtype = dtype; a.ldb = K;
+    a.corr_mode = CORR_NONE;
+    a.zero_counters = share.n_counters;
+  }
+  return launch_mmq(a, s);
+}
+
 }  // namespace gguf_b200
 
 extern "C" {
@@ -175,8 +217,7 @@ static int64_t mmq_gemv_max_tokens(int type) { return type == T_Q6_K ? 16 : 4; }
 // ... and that the small-batch kernel serves instead, given room for its activation tiles
 static int64_t mmq_small_max_tokens() { return 16; }
 
-// activation matrix of the tensor-core kernels, rounded so that what follows it stays aligned
-static int64_t mmq_b_bytes(int type, int64_t M, int64_t K) { return round_up(M * mmq_ldb(type, K) * 2, 256); }
+static int64_t moe_list_bytes(int64_t n_sorted) { return round_up((n_sorted / mmq_moe_block_size() + 1) * 16 + 16, 256); }
 
 int64_t gguf_b200_workspace_bytes(int op, int type, int64_t M, int64_t N, int64_t K) {
   if (!type_size(type) || M < 0 || K <= 0) return 0;
@@ -185,17 +226,27 @@ int64_t gguf_b200_workspace_bytes(int op, int type, int64_t M, int64_t N, int64_
     case GGUF_B200_OP_MOE_VEC: return q8_soa_bytes(M, K);
     /* dense GEMM: + room for the fp32 partial tiles of a split over K (small N, long K) */
     case GGUF_B200_OP_MMQ: return M <= mmq_gemv_max_tokens(type) ? M * mmq_ldb(type, K) * 2 : mmq_b_bytes(type, M, K) + mmq_split_scratch_bytes(M, N > 0 ? N : 0, K);
-    case GGUF_B200_OP_MOE: return M * mmq_ldb(type, K) * 2;  /* M = length of sorted_token_ids */
+    /* M = length of sorted_token_ids; behind the activations, the work list */
+    case GGUF_B200_OP_MOE: return mmq_b_bytes(type, M, K) + moe_list_bytes(M);
     case GGUF_B200_OP_DEQUANT_MATMUL: return mmq_split_scratch_bytes(M, N > 0 ? N : 0, K);
   }
   return 0;
 }
 
 int64_t gguf_b200_scratch_bytes(int op, int type, int64_t M, int64_t N, int64_t K) {
-  const int64_t least = gguf_b200_workspace_bytes(op, type, M, N, K);
-  const bool small = type_size(type) && N > 0 && K > 0 && M >= small_min_tokens() &&
-                     (op == GGUF_B200_OP_GEMV || (op == GGUF_B200_OP_MMQ && M <= mmq_small_max_tokens()));
-  return small && small_bytes(M, N, K) > least ? small_bytes(M, N, K) : least;
+  int64_t most = gguf_b200_workspace_bytes(op, type, M, N, K);
+  if (!type_size(type) || N <= 0 || K <= 0 || M <= 0) return most;
+  auto at_least = [&](int64_t b) { if (b > most) most = b; };
+  if (M >= small_min_tokens() && (op == GGUF_B200_OP_GEMV || (op == GGUF_B200_OP_MMQ && M <= mmq_small_max_tokens()))) at_least(small_bytes(M, N, K));
+  if (op == GGUF_B200_OP_MMQ || op == GGUF_B200_OP_DEQUANT_MATMUL) {
+    const MmqShare share = mmq_share(type, M, N, K);
+    at_least((op == GGUF_B200_OP_MMQ ? mmq_b_bytes(type, M, K) : 0) + share.counter_bytes + share.part_bytes);
+  }
+  if (op == GGUF_B200_OP_MOE) {
+    const MmqShare share = mmq_share_moe(N, M / mmq_moe_block_size() + 1, mmq_moe_block_size());
+    at_least(mmq_b_bytes(type, M, K) + moe_list_bytes(M) + share.counter_bytes + share.part_bytes);
+  }
+  return most;
 }
 
 int gguf_b200_mul_mat_vec_a8(const void* W, const void* X, void* Y, void* ws, int64_t ws_bytes, int type, int dtype,
@@ -343,7 +394,7 @@ int gguf_b200_matmul_tp(int op, const void* W, const void* X, void* const* y_pee
   int rc = check_common(W, X, y_peers[rank], type, dtype, M, N_local, K);
   if (rc || M == 0 || N_local == 0) return rc;
   if (op == GGUF_B200_OP_DEQUANT_MATMUL) {
-    if (type != T_IQ2_XXS && type != T_IQ4_XS && type != T_IQ4_NL) return E_BAD_TYPE;
+    if (!is_dequant_matmul_type(type)) return E_BAD_TYPE;
     if (dtype != DT_F16 && dtype != DT_BF16) return E_BAD_DTYPE;
     if (K % 64 != 0) return E_BAD_SHAPE;
   } else if (!is_mmq_type(type)) {
@@ -362,37 +413,12 @@ int gguf_b200_matmul_tp(int op, const void* W, const void* X, void* const* y_pee
     tp.y_peer[r] = y_peers[r];
     tp.flag_peer[r] = flag_peers[r];
   }
-  MmqArgs a{};
-  a.w = W; a.y = nullptr;
-  a.type = type; a.out_dtype = dtype;
-  a.M = M; a.N = N_local; a.K = K;
-  a.rows_out = M;
-  a.status = st;
-  a.tp = &tp;
-  if (op == GGUF_B200_OP_DEQUANT_MATMUL) {
-    a.b = X; a.b_dtype = dtype; a.ldb = K;
-    a.corr_mode = CORR_NONE;
-    if (ws && aligned16(ws) && ws_bytes > 0) {
-      a.part = ws;
-      a.part_bytes = ws_bytes;
-    }
-    return launch_mmq(a, s);
+  const bool quantize = op == GGUF_B200_OP_MMQ;
+  if (quantize) {
+    if (!ws || !aligned16(ws)) return E_BAD_POINTER;
+    if (ws_bytes < M * mmq_ldb(type, K) * 2) return E_WORKSPACE;
   }
-  if (!ws || !aligned16(ws)) return E_BAD_POINTER;
-  const int64_t ldb = mmq_ldb(type, K);
-  if (ws_bytes < M * ldb * 2) return E_WORKSPACE;
-  const int perm = mmq_perm(type, N_local, K, false, 0);
-  rc = launch_quantize_q8_1(X, dtype, ws, M, K, Q8_MODE_F16, 0, ldb, mmq_corr_mode(type), nullptr, 1, 0, s, perm);
-  if (rc) return rc;
-  a.perm = perm;
-  a.b = ws; a.b_dtype = DT_F16; a.ldb = ldb;
-  a.corr_mode = mmq_corr_mode(type);
-  const int64_t used = mmq_b_bytes(type, M, K);
-  if (ws_bytes > used) {
-    a.part = static_cast<uint8_t*>(ws) + used;
-    a.part_bytes = ws_bytes - used;
-  }
-  return launch_mmq(a, s);
+  return tiled_dense(quantize, W, X, nullptr, ws, ws_bytes, type, dtype, M, N_local, K, K / block_size(type) * type_size(type), 0, &tp, st, s);
 }
 
 int gguf_b200_tp_wait(const uint32_t* flags_local, const uint32_t* epochs_local, int slot, int world, void* stream) {
@@ -443,49 +469,24 @@ int gguf_b200_mul_mat_a8(const void* W, const void* X, void* Y, void* ws, int64_
     // load_tiles_q5_0 + vec_dot_q8_0_q8_1_impl, vecdotq.cuh:676-749), i.e. 16 * d8 * sum(q8)
     rc = launch_quantize_q8_1(X, dtype, ws, M, K, Q8_MODE_SOA, type == T_Q5_0 ? 1 : 0, 0, CORR_NONE, nullptr, 1, 0, s);
     if (rc) return rc;
-    return launch_gemv(W, ws, Y, type, dtype, M, N, K, st, s);
+    rc = launch_gemv(W, ws, Y, type, dtype, M, N, K, st, s);
+    if (rc != E_TOO_LARGE) return rc;
   }
-  const int perm = mmq_perm(type, N, K, false, 0);
-  rc = launch_quantize_q8_1(X, dtype, ws, M, K, Q8_MODE_F16, 0, ldb, mmq_corr_mode(type), nullptr, 1, 0, s, perm);
-  if (rc) return rc;
-  MmqArgs a{};
-  a.perm = perm;
-  a.w = W; a.b = ws; a.y = Y;
-  a.type = type; a.out_dtype = dtype; a.b_dtype = DT_F16;
-  a.M = M; a.N = N; a.K = K; a.ldb = ldb;
-  a.corr_mode = mmq_corr_mode(type);
-  a.rows_out = M;
-  a.status = st;
-  // whatever the caller gave beyond the activation matrix may hold split-K partial tiles
-  const int64_t used = mmq_b_bytes(type, M, K);
-  if (ws_bytes > used) {
-    a.part = static_cast<uint8_t*>(ws) + used;
-    a.part_bytes = ws_bytes - used;
-  }
-  return launch_mmq(a, s);
+  return tiled_dense(true, W, X, Y, ws, ws_bytes, type, dtype, M, N, K, K / block_size(type) * type_size(type), N, nullptr, st, s);
 }
 
 int gguf_b200_dequant_matmul(const void* W, const void* X, void* Y, void* ws, int64_t ws_bytes, int type, int dtype,
                              int64_t M, int64_t N, int64_t K, void* stream) {
   int rc = check_common(W, X, Y, type, dtype, M, N, K);
   if (rc || M == 0 || N == 0) return rc;
-  if (type != T_IQ2_XXS && type != T_IQ4_XS && type != T_IQ4_NL) return E_BAD_TYPE;
+  if (!is_dequant_matmul_type(type)) return E_BAD_TYPE;
   if (dtype != DT_F16 && dtype != DT_BF16) return E_BAD_DTYPE;
   if (K % 64 != 0) return E_BAD_SHAPE;
   int* st = status_ptr();
   if (!st) return E_CUDA;
-  MmqArgs a{};
-  a.w = W; a.b = X; a.y = Y;
-  a.type = type; a.out_dtype = dtype; a.b_dtype = dtype;
-  a.M = M; a.N = N; a.K = K; a.ldb = K;
-  a.corr_mode = CORR_NONE;
-  a.rows_out = M;
-  a.status = st;
-  if (ws && aligned16(ws) && ws_bytes > 0) {   // optional: room for split-K partial tiles
-    a.part = ws;
-    a.part_bytes = ws_bytes;
-  }
-  return launch_mmq(a, static_cast<cudaStream_t>(stream));
+  // (the workspace is optional: room for the parts of shared tiles)
+  return tiled_dense(false, W, X, Y, ws, ws_bytes, type, dtype, M, N, K, K / block_size(type) * type_size(type), N, nullptr, st,
+                     static_cast<cudaStream_t>(stream));
 }
 
 int gguf_b200_moe_a8(const void* X, const void* W, void* Y, void* ws, int64_t ws_bytes, const int32_t* sorted_token_ids,
@@ -506,53 +507,74 @@ int gguf_b200_moe_a8(const void* X, const void* W, void* Y, void* ws, int64_t ws
   if (n_sorted == 0) return E_OK;
   if (!sorted_token_ids || !expert_ids || !num_tokens_post_padded) return E_BAD_POINTER;
   if (!ws || !aligned16(ws)) return E_BAD_POINTER;
-  const int64_t ldb = mmq_ldb(type, K);
-  if (ws_bytes < n_sorted * ldb * 2) return E_WORKSPACE;
+  const int64_t used = mmq_b_bytes(type, n_sorted, K), list = moe_list_bytes(n_sorted);
+  if (ws_bytes < used + list) return E_WORKSPACE;
+  if (!small_fits(n_experts * N, K)) return E_TOO_LARGE;
+  const int64_t pitch = K / block_size(type) * type_size(type);
+  if (expert_stride_bytes < N * pitch && n_experts > 1) return E_BAD_SHAPE;
   int* st = status_ptr();
   if (!st) return E_CUDA;
-  // quantize + gather: row p of the fp16 matrix = activations of token sorted_token_ids[p] / top_k
-  const int perm = mmq_perm(type, N, K, true, expert_stride_bytes);
-  rc = launch_quantize_q8_1(X, dtype, ws, n_sorted, K, Q8_MODE_F16, 0, ldb, mmq_corr_mode(type), sorted_token_ids, top_k,
-                            rows_out, s, perm);
-  if (rc) return rc;
+  const int blk = mmq_moe_block_size();
+  uint8_t* base = static_cast<uint8_t*>(ws);
   MmqArgs a{};
-  a.perm = perm;
   a.w = W; a.b = ws; a.y = Y;
   a.type = type; a.out_dtype = dtype; a.b_dtype = DT_F16;
-  a.M = n_sorted; a.N = N; a.K = K; a.ldb = ldb;
+  a.M = n_sorted; a.N = N; a.K = K;
+  a.pitch = pitch; a.ldb = mmq_ldb(type, K); a.ldy = N;
   a.corr_mode = mmq_corr_mode(type);
-  a.sorted_ids = sorted_token_ids;
-  a.expert_ids = expert_ids;
-  a.n_post_pad = num_tokens_post_padded;
-  a.n_sorted = n_sorted;
-  a.expert_stride_bytes = expert_stride_bytes;
-  a.top_k = top_k;
+  a.expert_gap = n_experts > 1 ? expert_stride_bytes - N * pitch : 0;
+  a.perm = a.expert_gap ? 0 : mmq_perm(type, K, pitch);
+  a.passes = base + used;
+  a.n_passes = reinterpret_cast<const int32_t*>(base + used + list - 16);
+  a.sorted = sorted_token_ids;
+  a.experts = n_experts;
+  a.max_passes = n_sorted / blk + 1;
+  a.pass_rows = blk;
   a.rows_out = rows_out;
-  a.n_experts = n_experts;
-  a.moe_block = mmq_moe_block_size();
   a.status = st;
+  const MmqShare share = mmq_share_moe(N, a.max_passes, blk);
+  if (ws_bytes >= used + list + share.counter_bytes + share.part_bytes) {
+    a.counter = reinterpret_cast<int*>(base + used + list);
+    a.part = base + used + list + share.counter_bytes;
+    a.part_bytes = share.part_bytes;
+  }
+  rc = launch_moe_blocks(expert_ids, num_tokens_post_padded, n_sorted, (int)n_experts, blk, base + used, const_cast<int32_t*>(a.n_passes), s);
+  if (rc) return rc;
+  // quantize + gather: row p of the fp16 matrix = activations of token sorted_token_ids[p] / top_k
+  rc = launch_quantize_q8_1(X, dtype, ws, n_sorted, K, Q8_MODE_F16, 0, a.ldb, a.corr_mode, sorted_token_ids, top_k, rows_out, s, a.perm, nullptr, 0, 0,
+                            a.counter, a.counter ? share.n_counters : 0, a.n_passes);
+  if (rc) return rc;
   return launch_mmq(a, s);
 }
 
 namespace {
 struct FusedMoeLayout {
-  int64_t n_sorted, o_counts, o_sorted, o_experts, o_npp, o_y1, o_y2, o_xb, total;
+  int pass_rows;
+  int64_t passes, o_sorted, o_passes, o_npass, o_y1, o_y2, o_xb, o_counter, o_part, part_bytes, total;
 };
 FusedMoeLayout fused_moe_layout(int type13, int type2, int dtype, int64_t tokens, int64_t top_k, int64_t E, int64_t H, int64_t I) {
   FusedMoeLayout L{};
-  const int blk = mmq_moe_block_size();
   const int64_t slots = tokens * top_k, esz = dtype == DT_F32 ? 4 : 2;
-  L.n_sorted = moe_align_sorted_len(slots, (int)E, blk);
+  // Rows per pass: an expert's average share and three standard deviations, so that nearly every expert's weights are decoded
+  // once.  (Up to 112 rows a tensor instruction takes the same time, so a pass is never made smaller than 64.)
+  const double mean = (double)slots / (double)E;
+  int64_t rows = round_up((int64_t)(mean + 3.0 * sqrt(mean)) + 1, 16);
+  if (rows > 256) rows = round_up((int64_t)(mean / (int64_t)((mean + 191) / 192)) + 1, 16);
+  L.pass_rows = (int)(rows < 64 ? 64 : (rows > 256 ? 256 : rows));
+  L.passes = moe_plan_passes(slots, (int)E, L.pass_rows);
   int64_t o = 0;
   auto take = [&](int64_t bytes) { const int64_t at = o; o += round_up(bytes, 256); return at; };
-  L.o_counts = take(2 * E * 4);
-  L.o_sorted = take(L.n_sorted * 4);
-  L.o_experts = take(L.n_sorted / blk * 4);
-  L.o_npp = take(4);
+  L.o_sorted = take(slots * 4);
+  L.o_passes = take(L.passes * 16);
+  L.o_npass = take(8);
   L.o_y1 = take(slots * 2 * I * esz);
   L.o_y2 = take(slots * H * esz);
-  const int64_t xb1 = L.n_sorted * mmq_ldb(type13, H) * 2, xb2 = L.n_sorted * mmq_ldb(type2, I) * 2;
+  const int64_t xb1 = slots * mmq_ldb(type13, H) * 2, xb2 = slots * mmq_ldb(type2, I) * 2;
   L.o_xb = take(xb1 > xb2 ? xb1 : xb2);
+  const MmqShare a = mmq_share_moe(2 * I, L.passes, L.pass_rows), b = mmq_share_moe(H, L.passes, L.pass_rows);
+  L.o_counter = take(a.counter_bytes > b.counter_bytes ? a.counter_bytes : b.counter_bytes);
+  L.part_bytes = a.part_bytes;
+  L.o_part = take(L.part_bytes);
   L.total = o;
   return L;
 }
@@ -568,8 +590,8 @@ MoeSmallLayout moe_small_layout(int dtype, int64_t tokens, int64_t top_k, int64_
   MoeSmallLayout L{};
   const int64_t slots = tokens * top_k, esz = dtype == DT_F32 ? 4 : 2;
   L.pass_tiles = slots <= 8 * E ? 1 : slots <= 16 * E ? 2 : 4;   // an expert's share of the slots, on average, in one pass
-  L.tiles = moe_plan_tiles(slots, (int)E);
-  L.passes = moe_plan_passes(slots, (int)E, L.pass_tiles);
+  L.tiles = moe_plan_rows(slots, (int)E, 8) / 8;
+  L.passes = moe_plan_passes(slots, (int)E, 8 * L.pass_tiles);
   int64_t o = 0;
   auto take = [&](int64_t bytes) { const int64_t at = o; o += round_up(bytes, 256); return at; };
   L.o_sorted = take(L.tiles * 8 * 4);
@@ -613,7 +635,7 @@ int gguf_b200_fused_moe(const void* X, const void* W13, const void* W2, void* Y,
     int32_t* sorted = reinterpret_cast<int32_t*>(base + L.o_sorted);
     int32_t* npass = reinterpret_cast<int32_t*>(base + L.o_npass);
     const int64_t slots = tokens * top_k;
-    rc = launch_moe_plan(topk_ids, slots, (int)n_experts, L.pass_tiles, sorted, base + L.o_passes, npass, s);
+    rc = launch_moe_plan(topk_ids, slots, (int)n_experts, 8, 8 * L.pass_tiles, sorted, base + L.o_passes, npass, s);
     if (rc) return rc;
     auto gemm = [&](const void* x, int64_t x_div, int act_mode, const void* w, int type, int64_t N, int64_t K, void* y, const float* scale) {
       SmallArgs a{};
@@ -644,58 +666,54 @@ int gguf_b200_fused_moe(const void* X, const void* W13, const void* W2, void* Y,
   }
   const FusedMoeLayout L = fused_moe_layout(type13, type2, dtype, tokens, top_k, n_experts, H, I);
   if (ws_bytes < L.total) return E_WORKSPACE;
+  if (!small_fits(n_experts * 2 * I, H) || !small_fits(n_experts * H, I)) return E_TOO_LARGE;
   int* st = status_ptr();
   if (!st) return E_CUDA;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   uint8_t* base = static_cast<uint8_t*>(ws);
   int32_t* sorted = reinterpret_cast<int32_t*>(base + L.o_sorted);
-  int32_t* experts = reinterpret_cast<int32_t*>(base + L.o_experts);
-  int32_t* npp = reinterpret_cast<int32_t*>(base + L.o_npp);
-  void* y1 = base + L.o_y1;
-  void* y2 = base + L.o_y2;
+  int32_t* npass = reinterpret_cast<int32_t*>(base + L.o_npass);
   void* xb = base + L.o_xb;
   const int64_t slots = tokens * top_k;
-  const int blk = mmq_moe_block_size();
-  // 1. expert-sorted, block-padded slot lists
-  rc = launch_moe_align(topk_ids, slots, (int)n_experts, blk, reinterpret_cast<int32_t*>(base + L.o_counts), sorted, experts, npp, s);
+  // 1. expert-sorted slots and the passes over them
+  rc = launch_moe_plan(topk_ids, slots, (int)n_experts, 1, L.pass_rows, sorted, base + L.o_passes, npass, s);
   if (rc) return rc;
   // 2. gate/up projection of every routed slot.  Rows of y1 / y2 that belong to slots without a valid
   //    expert are never written and never read (the final sum skips them), so nothing is zero-filled.
-  const int64_t rb13 = H / block_size(type13) * type_size(type13), rb2 = I / block_size(type2) * type_size(type2);
-  auto gemm = [&](const void* x, int64_t x_rows_div, const void* w, int type, int64_t N, int64_t K, int64_t row_bytes, void* y,
-                  const float* scale, int act_mode, int64_t x_ld) -> int {
-    const int64_t ldb = mmq_ldb(type, K);
-    const int64_t estride = N * row_bytes;
-    const int perm = mmq_perm(type, N, K, true, estride);
-    int r = launch_quantize_q8_1(x, dtype, xb, L.n_sorted, K, Q8_MODE_F16, 0, ldb, mmq_corr_mode(type), sorted, x_rows_div, slots, s,
-                                 perm, nullptr, act_mode, x_ld);
-    if (r) return r;
+  auto gemm = [&](const void* x, int64_t x_rows_div, const void* w, int type, int64_t N, int64_t K, void* y, const float* scale, int act_mode,
+                  int64_t x_ld) -> int {
     MmqArgs a{};
-    a.perm = perm;
     a.w = w; a.b = xb; a.y = y;
     a.type = type; a.out_dtype = dtype; a.b_dtype = DT_F16;
-    a.M = L.n_sorted; a.N = N; a.K = K; a.ldb = ldb;
+    a.M = slots; a.N = N; a.K = K;
+    a.pitch = K / block_size(type) * type_size(type);
+    a.ldb = mmq_ldb(type, K);
+    a.ldy = N;
     a.corr_mode = mmq_corr_mode(type);
-    a.sorted_ids = sorted;
-    a.expert_ids = experts;
-    a.n_post_pad = npp;
-    a.n_sorted = L.n_sorted;
-    a.expert_stride_bytes = estride;
-    a.top_k = x_rows_div;
+    a.perm = mmq_perm(type, K, a.pitch);
+    a.passes = base + L.o_passes;
+    a.n_passes = npass;
+    a.sorted = sorted;
+    a.experts = n_experts;
+    a.max_passes = L.passes;
+    a.pass_rows = L.pass_rows;
     a.rows_out = slots;
-    a.n_experts = n_experts;
-    a.moe_block = blk;
     a.row_scale = scale;
     a.status = st;
-    return launch_mmq(a, s);
+    a.counter = reinterpret_cast<int*>(base + L.o_counter);
+    a.part = base + L.o_part;
+    a.part_bytes = L.part_bytes;
+    const int r = launch_quantize_q8_1(x, dtype, xb, slots, K, Q8_MODE_F16, 0, a.ldb, a.corr_mode, sorted, x_rows_div, slots, s, a.perm, nullptr, act_mode,
+                                       x_ld, a.counter, mmq_share_moe(N, L.passes, L.pass_rows).n_counters, npass);
+    return r ? r : launch_mmq(a, s);
   };
-  rc = gemm(X, top_k, W13, type13, 2 * I, H, rb13, y1, nullptr, 0, 0);
+  rc = gemm(X, top_k, W13, type13, 2 * I, H, base + L.o_y1, nullptr, 0, 0);
   if (rc) return rc;
   // 3. down projection: its activation quantizer applies act(gate) * up on the fly, its epilogue the routing weights
-  rc = gemm(y1, 1, W2, type2, H, I, rb2, y2, topk_weights, act, 2 * I);
+  rc = gemm(base + L.o_y1, 1, W2, type2, H, I, base + L.o_y2, topk_weights, act, 2 * I);
   if (rc) return rc;
   // 4. sum over the top_k slots of every token
-  return launch_moe_sum(y2, Y, topk_ids, (int)n_experts, tokens, top_k, H, dtype, s);
+  return launch_moe_sum(base + L.o_y2, Y, topk_ids, (int)n_experts, tokens, top_k, H, dtype, s);
 }
 
 int gguf_b200_moe_a8_vec(const void* X, const void* W, void* Y, void* ws, int64_t ws_bytes, const int32_t* topk_ids,

@@ -33,13 +33,15 @@ struct Q8Tp {
 // input row gather_ids[r] / gather_div; ids outside [0, gather_limit) give a zero row.
 int launch_quantize_q8_1(const void* x, int x_dtype, void* out, int64_t M, int64_t K, int mode, int sum_mode,
                          int64_t ldb, int corr_mode, const int32_t* gather_ids, int64_t gather_div, int64_t gather_limit,
-                         cudaStream_t stream, int perm = 0, const Q8Tp* tp = nullptr, int act = 0, int64_t x_ld = 0);
+                         cudaStream_t stream, int perm = 0, const Q8Tp* tp = nullptr, int act = 0, int64_t x_ld = 0,
+                         int* zero = nullptr, int64_t n_zero = 0, const int32_t* n_used = nullptr);
+// zero, n_zero (F16 mode, aligned rows): words to clear for the kernel behind it; n_used: [1] = rows of the output in use (null: M).
 // act (F16 mode): 0 = none; 1 = silu, 2 = gelu: the input rows are [gate | up] of x_ld = 2K values and act(gate) * up is quantized
 // leading dimension (elements) of the fp16 activation matrix of the tensor-core kernels
 int64_t mmq_ldb(int type, int64_t K);
 int mmq_corr_mode(int type);
 // value order the tensor-core kernel will expect in the fp16 activation matrix for this problem
-int mmq_perm(int type, int64_t N, int64_t K, bool moe, int64_t expert_stride_bytes);
+int mmq_perm(int type, int64_t K, int64_t pitch);
 
 // row_ids != null: row gather -- out row r (K values, K a multiple of 256) = weight row row_ids[r] of weight_rows
 int launch_dequantize(const void* w, int type, void* out, int out_dtype, int64_t n_elems, int q4k_contract,
@@ -104,32 +106,38 @@ struct MmqTp {
   unsigned* flag_peer[8];
 };
 struct MmqArgs {
-  const void* w;            // packed weights (expert 0 for MoE)
-  const void* b;            // activation matrix, K-major, element type b_dtype (DT_F16 / DT_BF16)
-  void* y;                  // output [rows_out][N], element type out_dtype
+  const void* w;            // packed weights (expert 0), rows `pitch` bytes apart
+  const void* b;            // activation matrix, K-major, element type b_dtype (DT_F16 / DT_BF16), ldb elements between rows
+  void* y;                  // output, element type out_dtype, ldy elements between rows
   int type, out_dtype, b_dtype;
-  int64_t M;                // activation rows (tokens)
-  int64_t N, K;             // weight rows, weight columns (values)
-  int64_t ldb;              // leading dimension of b in elements
-  int64_t kext;             // contraction length in elements incl. correction columns (multiple of 64)
-  int corr_mode;            // which correction the appended columns hold
+  int64_t M;                // activation rows
+  int64_t N, K;             // weight rows, values per row
+  int64_t pitch, ldb, ldy;
+  int corr_mode;            // which correction the columns behind K hold
   int perm;                 // value order inside each group of four of b: 0 natural, 1 = (0,2,1,3) (see mmq_perm)
-  // MoE gather (null sorted_ids = dense)
-  const int32_t* sorted_ids;
-  const int32_t* expert_ids;
-  const int32_t* n_post_pad;
-  int64_t n_sorted, expert_stride_bytes, top_k, rows_out;
-  int64_t n_experts;        // experts in w (0: unknown, ids are only limited to [0, 255] as in the reference)
-  int moe_block;
+  // MoE (null passes = dense): the work list of launch_moe_plan / launch_moe_blocks
+  const void* passes;       // int4 {expert, first activation row, rows}
+  const int32_t* n_passes;
+  const int32_t* sorted;    // output row of every activation row (>= rows_out: padding)
+  int64_t experts, max_passes, pass_rows, rows_out;
+  int64_t expert_gap;       // MoE: bytes between one expert's matrix and the next
   const float* row_scale;   // MoE: output row r is multiplied by row_scale[r] (routing weights); null: no scaling
   int* status;
   const MmqTp* tp;          // null: plain output y
-  void* part;               // optional fp32 scratch for split-K partial tiles (16-byte aligned), part_bytes long
+  // Optional: room for tiles that several CTAs share (mmq_share_bytes).  `counter` must be zero when the kernel starts.
+  int* counter;
+  int64_t zero_counters;    // > 0: so many words of it are cleared here first
+  void* part;               // 16-byte aligned, part_bytes long
   int64_t part_bytes;
 };
-// bytes of fp32 scratch a dense M x N x K problem can use for split K (0: it never splits)
-int64_t mmq_split_scratch_bytes(int64_t M, int64_t N, int64_t K);
 int launch_mmq(const MmqArgs& a, cudaStream_t stream);
+// scratch with which every CTA gets an equal share of the chunks: n_counters words, then partial tiles
+struct MmqShare { int64_t n_counters, counter_bytes, part_bytes; };
+MmqShare mmq_share(int type, int64_t M, int64_t N, int64_t K);   // all zero where sharing does not pay
+MmqShare mmq_share_moe(int64_t N, int64_t max_passes, int64_t pass_rows);
+// fp32 scratch that a dense M x N x K problem used to split K with (what gguf_b200_workspace_bytes reports)
+int64_t mmq_split_scratch_bytes(int64_t M, int64_t N, int64_t K);
+int launch_zero(int* p, int64_t n, cudaStream_t stream);
 int mmq_moe_block_size();
 
 int64_t q8_soa_bytes(int64_t M, int64_t K);
@@ -166,15 +174,16 @@ bool smallm_pairs_with_sum(int type);
 int smallm_order(int type);      // order of a block's values in the tiles (smallm_decode.cuh)
 
 // fused MoE step (moe_fused.cu)
-int64_t moe_align_sorted_len(int64_t slots, int n_experts, int block);
-int launch_moe_align(const int32_t* topk_ids, int64_t slots, int n_experts, int block, int32_t* scratch, int32_t* sorted_ids,
-                     int32_t* expert_ids, int32_t* n_post_pad, cudaStream_t stream);
-// the same lists for the small-batch kernel: columns in tiles of eight, passes of up to pass_tiles tiles of one expert.
-// sorted[8 * tiles] (padded with `slots`), passes int4[max_passes], n_passes[2]
-int64_t moe_plan_tiles(int64_t slots, int n_experts);                       // room for column tiles
-int64_t moe_plan_passes(int64_t slots, int n_experts, int pass_tiles);
-int launch_moe_plan(const int32_t* topk_ids, int64_t slots, int n_experts, int pass_tiles, int32_t* sorted, void* passes, int32_t* n_passes,
-                    cudaStream_t stream);
+// The routed slots (token * top_k + j) sorted by expert, every expert's run starting at a multiple of `align` rows, and a work list
+// of passes of up to pass_rows rows of one expert.  passes: int4 {expert, first row / align, rows / align rounded up (align > 1) or
+// rows, 0}; sorted[row] = slot, `slots` in padding rows; n_passes: [0] passes, [1] rows in use / align.
+int64_t moe_plan_rows(int64_t slots, int n_experts, int align);              // room for rows
+int64_t moe_plan_passes(int64_t slots, int n_experts, int pass_rows);
+int launch_moe_plan(const int32_t* topk_ids, int64_t slots, int n_experts, int align, int pass_rows, int32_t* sorted, void* passes,
+                    int32_t* n_passes, cudaStream_t stream);
+// passes of `block` rows from a caller's block-aligned lists (expert ids outside [0, n_experts) and blocks beyond n_post_pad left out)
+int launch_moe_blocks(const int32_t* expert_ids, const int32_t* n_post_pad, int64_t n_sorted, int n_experts, int block, void* passes,
+                      int32_t* n_passes, cudaStream_t stream);
 int launch_moe_sum(const void* y, void* out, const int32_t* topk_ids, int n_experts, int64_t tokens, int64_t top_k, int64_t h,
                    int dtype, cudaStream_t stream);
 

@@ -17,6 +17,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "tables.cuh"
 
 namespace gguf_b200 {
 
@@ -55,32 +56,51 @@ __device__ __forceinline__ uint32_t shift_of(const uint8_t* p) { return (uint32_
 // ld.shared (through a generic pointer the look-ups travel the global-memory pipeline).  The
 // look-ups are plain (non-volatile) asm: their index comes from weight bytes that are read long
 // after the barrier that published the tables.
+// A table is replicated, entry i of copy c at index copies * i + c, and a thread reads copy (lane mod copies): the lanes
+// that share a 128-byte access phase then sit in different columns of the 128 bytes whatever entries they look up (random
+// look-ups into a single copy averaged 2.5 to 3 bank conflicts per access).  The addresses below already point at this
+// thread's copy; the larger code books have room for fewer copies.
 struct DecodeCtx {
-  // The two IQ2_XXS tables are replicated, entry i of copy c at index COPIES * i + c -- the sign table
-  // (16-byte entries) eight times, the selector table (8-byte entries) sixteen times -- and a thread
-  // reads copy (lane mod COPIES): the lanes that share a 128-byte access phase then sit in different
-  // columns of the 128 bytes whatever entries they look up (random look-ups into a single copy averaged
-  // 2.5 to 3 bank conflicts per access).  `sel` and `sgn` already point at this thread's copy.
-  uint32_t sel;       // IQ2_XXS: per grid entry (8 bytes), the byte-permute selectors of its four value pairs (see Decoder<T_IQ2_XXS>)
-  uint32_t sgn;       // IQ2_XXS: per 7-bit sign index (16 bytes), the sign-bit masks of the four value pairs
-  uint32_t kv;        // IQ4_NL / IQ4_XS: the 16 levels, one signed byte each
-  __device__ __forceinline__ uint2 sel_at(uint32_t i) const {
-    uint2 v;
-    asm("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(sel + 128u * i));
-    return v;
-  }
-  __device__ __forceinline__ uint4 sgn_at(uint32_t i) const {
-    uint4 v;
-    asm("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(sgn + 128u * i));
-    return v;
-  }
-  __device__ __forceinline__ float level(uint32_t i) const {
-    int v;
-    asm("ld.shared.s8 %0, [%1];" : "=r"(v) : "r"(kv + i));
-    return (float)v;
-  }
+  uint32_t grid;      // code book: byte-permute selectors of value pairs (IQ2), magnitudes (IQ3), codes (IQ1)
+  uint32_t sgn;       // per sign index, the sign-bit masks of the four value pairs (16 bytes)
 };
-// Shared-memory tables of the IQ2_XXS decoder, built once per CTA from the format's grid and
+template <int TYPE> struct DecodeTables {   // GRID entries of GB bytes in GC copies; SGN sign entries in SC copies
+  static constexpr int GRID = 0, GB = 0, GC = 0, SGN = 0, SC = 0;
+};
+template <> struct DecodeTables<T_IQ2_XXS> { static constexpr int GRID = 256, GB = 8, GC = 16, SGN = 128, SC = 8; };
+template <> struct DecodeTables<T_IQ2_XS> { static constexpr int GRID = 512, GB = 8, GC = 4, SGN = 128, SC = 8; };
+template <> struct DecodeTables<T_IQ2_S> { static constexpr int GRID = 1024, GB = 8, GC = 2, SGN = 256, SC = 4; };
+template <> struct DecodeTables<T_IQ3_XXS> { static constexpr int GRID = 256, GB = 4, GC = 16, SGN = 128, SC = 8; };
+template <> struct DecodeTables<T_IQ3_S> { static constexpr int GRID = 512, GB = 4, GC = 8, SGN = 256, SC = 4; };
+template <> struct DecodeTables<T_IQ1_S> { static constexpr int GRID = 2048, GB = 4, GC = 2, SGN = 0, SC = 0; };
+template <> struct DecodeTables<T_IQ1_M> : DecodeTables<T_IQ1_S> {};
+template <int TYPE> __host__ __device__ constexpr int decoder_table_bytes() {
+  using D = DecodeTables<TYPE>;
+  return D::GRID * D::GB * D::GC + D::SGN * 16 * D::SC;
+}
+template <int TYPE> __device__ __forceinline__ DecodeCtx decoder_context(const uint8_t* tab, int lane) {
+  using D = DecodeTables<TYPE>;
+  DecodeCtx cx{0, 0};
+  if constexpr (D::GRID > 0) cx.grid = smem_u32(tab) + (uint32_t)(D::GB * (lane & (D::GC - 1)));
+  if constexpr (D::SGN > 0) cx.sgn = smem_u32(tab) + (uint32_t)(D::GRID * D::GB * D::GC + 16 * (lane & (D::SC - 1)));
+  return cx;
+}
+template <int TYPE> __device__ __forceinline__ uint2 grid64(const DecodeCtx& cx, uint32_t i) {
+  uint2 v;
+  asm("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(cx.grid + (uint32_t)(8 * DecodeTables<TYPE>::GC) * i));
+  return v;
+}
+template <int TYPE> __device__ __forceinline__ uint32_t grid32(const DecodeCtx& cx, uint32_t i) {
+  uint32_t v;
+  asm("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(cx.grid + (uint32_t)(4 * DecodeTables<TYPE>::GC) * i));
+  return v;
+}
+template <int TYPE> __device__ __forceinline__ uint4 sign_masks(const DecodeCtx& cx, uint32_t i) {
+  uint4 v;
+  asm("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(cx.sgn + (uint32_t)(16 * DecodeTables<TYPE>::SC) * i));
+  return v;
+}
+// Shared-memory tables of the IQ2 decoders, built once per CTA from the formats' grid and
 // sign tables.  A grid entry holds eight magnitudes, each one of {8, 25, 43}; with the three
 // products d*8, d*25, d*43 of a 32-value group rounded to 16 bits and parked in two registers,
 // every PAIR of decoded values is one byte-permute whose 16-bit selector depends only on the grid
@@ -103,34 +123,50 @@ __device__ __forceinline__ uint4 iq2xxs_pair_signs(uint32_t sign_bits) {
   return make_uint4(m[0], m[1], m[2], m[3]);
 }
 
-template <int TYPE, typename ab_t> struct Decoder;
+template <int TYPE> __device__ __forceinline__ void decoder_fill_tables(uint8_t* tab) {
+  using D = DecodeTables<TYPE>;
+  if constexpr (D::GRID > 0) {
+    for (int i = threadIdx.x; i < D::GRID * D::GC; i += blockDim.x) {
+      const int e = i / D::GC;
+      if constexpr (TYPE == T_IQ2_XXS) reinterpret_cast<uint2*>(tab)[i] = iq2xxs_pair_selectors(d_iq2xxs_grid[e]);
+      if constexpr (TYPE == T_IQ2_XS) reinterpret_cast<uint2*>(tab)[i] = iq2xxs_pair_selectors(d_iq2xs_grid[e]);
+      if constexpr (TYPE == T_IQ2_S) reinterpret_cast<uint2*>(tab)[i] = iq2xxs_pair_selectors(d_iq2s_grid[e]);
+      if constexpr (TYPE == T_IQ3_XXS) reinterpret_cast<uint32_t*>(tab)[i] = d_iq3xxs_grid[e];
+      if constexpr (TYPE == T_IQ3_S) reinterpret_cast<uint32_t*>(tab)[i] = d_iq3s_grid[e];
+      if constexpr (TYPE == T_IQ1_S || TYPE == T_IQ1_M) reinterpret_cast<uint32_t*>(tab)[i] = d_iq1s_grid[e];
+    }
+  }
+  if constexpr (D::SGN > 0) {
+    uint4* sgn = reinterpret_cast<uint4*>(tab + D::GRID * D::GB * D::GC);
+    for (int i = threadIdx.x; i < D::SGN * D::SC; i += blockDim.x) {
+      const int e = i / D::SC;
+      sgn[i] = iq2xxs_pair_signs(D::SGN == 128 ? (uint32_t)d_ksigns_iq2xs[e] : (uint32_t)e);
+    }
+  }
+}
 
-// Raw-byte staging of the tensor-core kernel: KC values of every row of the tile are copied to
-// shared memory at once (coalesced 16-byte pieces), RBC bytes per row, in slots of SLOT bytes.
-// SLOT leaves room for the 16-byte rounding of the start and is an odd multiple of 16 so that
-// the 128 rows of a tile spread over all shared-memory banks.
-// TMA variant of the staging (row bytes a multiple of 16 and chunk starts 16-byte aligned): a
-// chunk of KC_T values per row is one 2-D box of RBC_T bytes x 128 rows, stored densely.  RBC_T
-// is an odd multiple of 16 for every supported type, so dense rows are bank-conflict free as well.
-template <int TYPE> struct TmaGeom {
-  static constexpr bool OK = TYPE == T_Q4_0 || TYPE == T_Q8_0 || TYPE == T_Q4_K || TYPE == T_Q5_K || TYPE == T_IQ4_XS;
-  static constexpr int KC_T = TYPE == T_IQ4_XS ? 512 : 256;
-  static constexpr int RBC_T = KC_T / BlockTraits<TYPE>::QK * BlockTraits<TYPE>::TS;   // 144, 176 or 272
-};
-template <int TYPE> struct RawGeom {
-  static constexpr int KC = TYPE == T_IQ2_XXS ? 512 : 256;   // multiples of 256: every producer group meets every chunk
-  static constexpr int RBC = KC / BlockTraits<TYPE>::QK * BlockTraits<TYPE>::TS;
-  static constexpr int S16 = (RBC + 30) / 16 + 1;
-  static constexpr int SLOT = (S16 % 2 ? S16 : S16 + 1) * 16;
-};
+template <int TYPE, typename ab_t> struct Decoder;
+// types that are multiplied as dequantized weights of either 16-bit type (activations as they are)
+template <int TYPE> __host__ __device__ constexpr bool decoder_bf16() {
+  return TYPE == T_IQ2_XXS || TYPE == T_IQ2_XS || TYPE == T_IQ2_S || TYPE == T_IQ3_XXS || TYPE == T_IQ3_S || TYPE == T_IQ1_S || TYPE == T_IQ1_M ||
+         TYPE == T_IQ4_NL || TYPE == T_IQ4_XS;
+}
 
 // Types whose two 32-value units of a 64-value stage (units 2j and 2j + 1 of a 256-value super-block, always
 // whole) are cut from the same words of the block: load() depends on the unit only through u >> 1.
 template <int TYPE> __host__ __device__ constexpr bool decoder_pair_load() { return TYPE == T_Q2_K || TYPE == T_Q3_K || TYPE == T_Q5_K || TYPE == T_Q6_K; }
 
+// one fp16 of each of four blocks TS bytes apart, zero from block `left` on
+template <int TS> __device__ __forceinline__ uint2 block_halves(uint32_t a, int left) {
+  uint32_t v[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) v[j] = j < left ? lds16(a + TS * j) : 0u;
+  return make_uint2(v[0] | (v[1] << 16), v[2] | (v[3] << 16));
+}
+
 // ---- Q4_0: value = half(q * d), q unsigned (see Stage64<T_Q4_0>); unit = one 18-byte block ----
 template <typename ab_t> struct Decoder<T_Q4_0, ab_t> {
-  static constexpr int CORR_OFF = 0;   // byte offset in a block of the fp16 that is the block's correction value (-1: none / computed)
+  static constexpr bool CORR = true;   // correction columns
   static constexpr int RW = 7;   // 18 bytes at 2-byte alignment: <= 6 words (+1 for the shifts)
   static __device__ __forceinline__ void load(const uint8_t* row, int u, uint32_t (&raw)[RW]) {
     ldg_cover<RW - 1>(row + (int64_t)u * 18, 18, raw);
@@ -150,21 +186,15 @@ template <typename ab_t> struct Decoder<T_Q4_0, ab_t> {
       out[8 + i] = h2_as_u32(hmul2_rn(__hsub2(ints_plus_1024((t >> 4) & 0xF, (t >> 12) & 0xF), off), d2));
     }
   }
-  // correction columns [32c, 32c+32): A'[n, g] = d of block g (pairs with -8 * s8 on the B side)
-  static __device__ __forceinline__ void corr(const uint8_t* row, int c, int64_t K, uint32_t (&out)[16]) {
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      const int64_t g = 32 * (int64_t)c + 2 * i;
-      const uint32_t a = g * 32 < K ? ldg16(row + g * 18) : 0u;
-      const uint32_t b = (g + 1) * 32 < K ? ldg16(row + (g + 1) * 18) : 0u;
-      out[i] = a | (b << 16);
-    }
+  // d of the four blocks 4 * half .. of the chunk, of which `left` exist
+  static __device__ __forceinline__ uint2 corr(const uint8_t* chunk, int half, int left) {
+    return block_halves<18>(smem_u32(chunk) + 0 + 72 * half, left - 4 * half);
   }
 };
 
 // ---- Q8_0: value = half(q * d); unit = one 34-byte block ---------------------------------------
 template <typename ab_t> struct Decoder<T_Q8_0, ab_t> {
-  static constexpr int CORR_OFF = -1;   // byte offset in a block of the fp16 that is the block's correction value (-1: none / computed)
+  static constexpr bool CORR = false;   // correction columns
   static constexpr int RW = 11;  // 34 bytes: <= 10 words (+1)
   static __device__ __forceinline__ void load(const uint8_t* row, int u, uint32_t (&raw)[RW]) {
     ldg_cover<RW - 1>(row + (int64_t)u * 34, 34, raw);
@@ -183,7 +213,6 @@ template <typename ab_t> struct Decoder<T_Q8_0, ab_t> {
       out[i] = h2_as_u32(hmul2_rn(__hsub2(ints_plus_1024(t & 0xFF, t >> 8), off), d2));
     }
   }
-  static __device__ __forceinline__ void corr(const uint8_t*, int, int64_t, uint32_t (&)[16]) {}
 };
 
 // 6-bit (scale, min) pair j of a Q4_K super-block from its 12 packed bytes held in three
@@ -200,10 +229,18 @@ __device__ __forceinline__ void q4k_scale_min(uint32_t w0, uint32_t w1, uint32_t
   }
 }
 
+// half(dmin * m) of the sub-blocks 4 * half .. 4 * half + 3 of a Q4_K / Q5_K super-block with header h
+__device__ __forceinline__ uint2 q4k_pair_mins(uint4 h, int half) {
+  const uint32_t mn = half ? ((h.w >> 4) & 0x0F0F0F0Fu) | ((h.z >> 2) & 0x30303030u) : h.z & 0x3F3F3F3Fu;   // four bytes
+  const __half2 dmin = __half2half2(__ushort_as_half((unsigned short)(h.x >> 16))), off = __floats2half2_rn(1024.f, 1024.f);
+  const __half2 a = __hsub2(u32_as_h2(__byte_perm(mn, 0x64646464u, 0x4140)), off), b = __hsub2(u32_as_h2(__byte_perm(mn, 0x64646464u, 0x4342)), off);
+  return make_uint2(h2_as_u32(hmul2_rn(dmin, a)), h2_as_u32(hmul2_rn(dmin, b)));
+}
+
 // ---- Q4_K: A = half(d1 * q) with d1 = half(d * sc); the -dmin*m part is a correction column ----
 // unit u: super-block u>>3, sub-block j = u&7: nibble (j&1) of the 32 bytes qs[32*(j>>1) ..]
 template <typename ab_t> struct Decoder<T_Q4_K, ab_t> {
-  static constexpr int CORR_OFF = -1;   // byte offset in a block of the fp16 that is the block's correction value (-1: none / computed)
+  static constexpr bool CORR = true;   // correction columns
   static constexpr int RW = 12;  // header (16 bytes) + 32 bytes of nibbles, all 16-byte aligned
   static __device__ __forceinline__ void load(const uint8_t* row, int u, uint32_t (&raw)[RW]) {
     const uint8_t* blk = row + (int64_t)(u >> 3) * 144;
@@ -227,33 +264,13 @@ template <typename ab_t> struct Decoder<T_Q4_K, ab_t> {
       out[2 * i + 1] = h2_as_u32(hmul2_rn(__hsub2(ints_plus_1024((w >> 16) & 0xF, (w >> 24) & 0xF), off), dv));
     }
   }
-  // correction columns [32c, 32c+32): A'[n, g] = half(dmin * m_g)  (pairs with -s8 on the B side)
-  static __device__ __forceinline__ void corr(const uint8_t* row, int c, int64_t K, uint32_t (&out)[16]) {
-#pragma unroll
-    for (int sb = 0; sb < 4; ++sb) {
-      const int64_t sbi = 4 * (int64_t)c + sb;  // super-block index: 8 groups each
-      if (sbi * 256 >= K) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) out[4 * sb + i] = 0;
-        continue;
-      }
-      const uint4 hdr = __ldg(reinterpret_cast<const uint4*>(row + sbi * 144));
-      const __half dmin = __ushort_as_half((unsigned short)(hdr.x >> 16));
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        int sc, ma, mb;
-        q4k_scale_min(hdr.y, hdr.z, hdr.w, 2 * i, sc, ma);
-        q4k_scale_min(hdr.y, hdr.z, hdr.w, 2 * i + 1, sc, mb);
-        out[4 * sb + i] = (uint32_t)__half_as_ushort(__hmul_rn(dmin, __int2half_rn(ma))) |
-                          ((uint32_t)__half_as_ushort(__hmul_rn(dmin, __int2half_rn(mb))) << 16);
-      }
-    }
-  }
+  // half(dmin * m) of the four sub-blocks 4 * half .. of the chunk (pairs with -s8 on the B side)
+  static __device__ __forceinline__ uint2 corr(const uint8_t* blk, int half, int) { return q4k_pair_mins(lds128s(smem_u32(blk)), half); }
 };
 
 // ---- Q4_1: A = half(q * d); the min term m * s8 is a correction column (B side: +s8) -----------------
 template <typename ab_t> struct Decoder<T_Q4_1, ab_t> {
-  static constexpr int CORR_OFF = 2;   // byte offset in a block of the fp16 that is the block's correction value (-1: none / computed)
+  static constexpr bool CORR = true;   // correction columns
   static constexpr int RW = 5;   // 20 bytes, 4-byte aligned
   static __device__ __forceinline__ void load(const uint8_t* row, int u, uint32_t (&raw)[RW]) {
     const uint32_t sb = smem_u32(row + (int64_t)u * 20);
@@ -272,15 +289,9 @@ template <typename ab_t> struct Decoder<T_Q4_1, ab_t> {
       out[8 + 2 * k + 1] = h2_as_u32(hmul2_rn(__hsub2(u32_as_h2(__byte_perm(ch, 0x64646464u, 0x4342)), off), d2));
     }
   }
-  // correction columns [32c, 32c+32): A'[n, g] = m of block g
-  static __device__ __forceinline__ void corr(const uint8_t* row, int c, int64_t K, uint32_t (&out)[16]) {
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      const int64_t g = 32 * (int64_t)c + 2 * i;
-      const uint32_t a = g * 32 < K ? ldg16(row + g * 20 + 2) : 0u;
-      const uint32_t b = (g + 1) * 32 < K ? ldg16(row + (g + 1) * 20 + 2) : 0u;
-      out[i] = a | (b << 16);
-    }
+  // m of the four blocks 4 * half .. of the chunk, of which `left` exist
+  static __device__ __forceinline__ uint2 corr(const uint8_t* chunk, int half, int left) {
+    return block_halves<20>(smem_u32(chunk) + 2 + 80 * half, left - 4 * half);
   }
 };
 
@@ -301,7 +312,7 @@ __device__ __forceinline__ void q5_word(uint32_t q, uint32_t qh, int k, __half2 
 
 // ---- Q5_0: value = half((q - 16) * d), 22-byte blocks (2-byte aligned): d | qh[4] | qs[16] ------------
 template <typename ab_t> struct Decoder<T_Q5_0, ab_t> {
-  static constexpr int CORR_OFF = -1;   // byte offset in a block of the fp16 that is the block's correction value (-1: none / computed)
+  static constexpr bool CORR = false;   // correction columns
   static constexpr int RW = 8;   // 22 bytes at 2-byte alignment: <= 6 words (+ shifts)
   static __device__ __forceinline__ void load(const uint8_t* row, int u, uint32_t (&raw)[RW]) {
     ldg_cover<7>(row + (int64_t)u * 22, 22, raw);
@@ -318,12 +329,11 @@ template <typename ab_t> struct Decoder<T_Q5_0, ab_t> {
       q5_word(q, qh, k, off, d2, out[2 * k], out[2 * k + 1], out[8 + 2 * k], out[8 + 2 * k + 1]);
     }
   }
-  static __device__ __forceinline__ void corr(const uint8_t*, int, int64_t, uint32_t (&)[16]) {}
 };
 
 // ---- Q5_1: A = half(q * d), 24-byte blocks (8-byte aligned): d | m | qh[4] | qs[16]; correction column m ----
 template <typename ab_t> struct Decoder<T_Q5_1, ab_t> {
-  static constexpr int CORR_OFF = 2;   // byte offset in a block of the fp16 that is the block's correction value (-1: none / computed)
+  static constexpr bool CORR = true;   // correction columns
   static constexpr int RW = 6;
   static __device__ __forceinline__ void load(const uint8_t* row, int u, uint32_t (&raw)[RW]) {
     const uint32_t sb = smem_u32(row + (int64_t)u * 24);
@@ -336,14 +346,9 @@ template <typename ab_t> struct Decoder<T_Q5_1, ab_t> {
 #pragma unroll
     for (int k = 0; k < 4; ++k) q5_word(raw[2 + k], qh, k, off, d2, out[2 * k], out[2 * k + 1], out[8 + 2 * k], out[8 + 2 * k + 1]);
   }
-  static __device__ __forceinline__ void corr(const uint8_t* row, int c, int64_t K, uint32_t (&out)[16]) {
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      const int64_t g = 32 * (int64_t)c + 2 * i;
-      const uint32_t a = g * 32 < K ? ldg16(row + g * 24 + 2) : 0u;
-      const uint32_t b = (g + 1) * 32 < K ? ldg16(row + (g + 1) * 24 + 2) : 0u;
-      out[i] = a | (b << 16);
-    }
+  // m of the four blocks 4 * half .. of the chunk, of which `left` exist
+  static __device__ __forceinline__ uint2 corr(const uint8_t* chunk, int half, int left) {
+    return block_halves<24>(smem_u32(chunk) + 2 + 96 * half, left - 4 * half);
   }
 };
 
@@ -351,7 +356,7 @@ template <typename ab_t> struct Decoder<T_Q5_1, ab_t> {
 // 176-byte blocks (16-byte aligned): d | dmin | scales[12] | qh[32] | qs[128].  unit u: sub-block j = u&7:
 // nibble (j&1) of qs[32*(j>>1) + l], bit j of qh[l], l = 0..31.
 template <typename ab_t> struct Decoder<T_Q5_K, ab_t> {
-  static constexpr int CORR_OFF = -1;   // byte offset in a block of the fp16 that is the block's correction value (-1: none / computed)
+  static constexpr bool CORR = true;   // correction columns
   static constexpr int RW = 20;  // header (16) + 32 bytes of nibbles + 32 bytes of high bits
   static __device__ __forceinline__ void load(const uint8_t* row, int u, uint32_t (&raw)[RW]) {
     const uint8_t* blk = row + (int64_t)(u >> 3) * 176;
@@ -378,28 +383,8 @@ template <typename ab_t> struct Decoder<T_Q5_K, ab_t> {
       out[2 * i + 1] = h2_as_u32(hmul2_rn(__hsub2(ints_plus_1024(c2, c3), off), dv));
     }
   }
-  // correction columns [32c, 32c+32): A'[n, g] = half(dmin * m_g)  (pairs with -s8 on the B side)
-  static __device__ __forceinline__ void corr(const uint8_t* row, int c, int64_t K, uint32_t (&out)[16]) {
-#pragma unroll
-    for (int sb = 0; sb < 4; ++sb) {
-      const int64_t sbi = 4 * (int64_t)c + sb;
-      if (sbi * 256 >= K) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) out[4 * sb + i] = 0;
-        continue;
-      }
-      const uint4 hdr = __ldg(reinterpret_cast<const uint4*>(row + sbi * 176));
-      const __half dmin = __ushort_as_half((unsigned short)(hdr.x >> 16));
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        int sc, ma, mb;
-        q4k_scale_min(hdr.y, hdr.z, hdr.w, 2 * i, sc, ma);
-        q4k_scale_min(hdr.y, hdr.z, hdr.w, 2 * i + 1, sc, mb);
-        out[4 * sb + i] = (uint32_t)__half_as_ushort(__hmul_rn(dmin, __int2half_rn(ma))) |
-                          ((uint32_t)__half_as_ushort(__hmul_rn(dmin, __int2half_rn(mb))) << 16);
-      }
-    }
-  }
+  // half(dmin * m) of the four sub-blocks 4 * half .. of the chunk (pairs with -s8 on the B side)
+  static __device__ __forceinline__ uint2 corr(const uint8_t* blk, int half, int) { return q4k_pair_mins(lds128s(smem_u32(blk)), half); }
 };
 
 // ---- Q6_K: value = half(d * half(sc * (code - 32))) ------------------------------------------
@@ -410,7 +395,7 @@ template <typename ab_t> struct Decoder<T_Q5_K, ab_t> {
 // Raw: [0..17] the 64 bytes of ql of the half (+ cover), [18..27] 32 bytes of qh (+ cover), [28..30] the four
 // scale bytes of the pair (+ cover), [31] d.
 template <typename ab_t> struct Decoder<T_Q6_K, ab_t> {
-  static constexpr int CORR_OFF = -1;   // byte offset in a block of the fp16 that is the block's correction value (-1: none / computed)
+  static constexpr bool CORR = false;   // correction columns
   static constexpr int RW = 32;
   static __device__ __forceinline__ void load(const uint8_t* row, int u, uint32_t (&raw)[RW]) {
     const uint8_t* blk = row + (int64_t)(u >> 3) * 210;
@@ -447,7 +432,6 @@ template <typename ab_t> struct Decoder<T_Q6_K, ab_t> {
       out[2 * wi + 1] = h2_as_u32(hmul2_rn(d2, hmul2_rn(s2, __hsub2(p1, off))));
     }
   }
-  static __device__ __forceinline__ void corr(const uint8_t*, int, int64_t, uint32_t (&)[16]) {}
 };
 
 // ---- Q2_K: value = fp32 (d*sc)*q - dmin*m rounded once (the dequantized weight itself: the 16-value
@@ -457,7 +441,7 @@ template <typename ab_t> struct Decoder<T_Q6_K, ab_t> {
 // as four halves, and every pair of weights is one byte-permute whose selector is the pair's two
 // 2-bit codes times 0x22 plus 0x1010 (code c picks bytes 2c, 2c+1).
 template <typename ab_t> struct Decoder<T_Q2_K, ab_t> {
-  static constexpr int CORR_OFF = -1;
+  static constexpr bool CORR = false;   // correction columns
   static constexpr int RW = 10;   // 32 code bytes, the word holding the two scale bytes, (d, dmin): all 4-byte aligned
   static __device__ __forceinline__ void load(const uint8_t* row, int u, uint32_t (&raw)[RW]) {
     const uint32_t sb = smem_u32(row + (int64_t)(u >> 3) * 84);
@@ -486,7 +470,6 @@ template <typename ab_t> struct Decoder<T_Q2_K, ab_t> {
       }
     }
   }
-  static __device__ __forceinline__ void corr(const uint8_t*, int, int64_t, uint32_t (&)[16]) {}
 };
 
 // ---- Q3_K: value = d * ((sc6 - 32) * (c - 4)), c = 2 low bits | hmask bit << 2; unit = 32-value group
@@ -496,7 +479,7 @@ template <typename ab_t> struct Decoder<T_Q2_K, ab_t> {
 // half 128 + c (0x5800 | c << 3), one HFMA2 gives (c - 4) * sc exactly (|.| <= 128; the addend
 // -132 * sc has 11 significant bits) and the multiplication by d rounds once.
 template <typename ab_t> struct Decoder<T_Q3_K, ab_t> {
-  static constexpr int CORR_OFF = -1;
+  static constexpr bool CORR = false;   // correction columns
   static constexpr int RW = 26;   // [0..9] code words, [10..19] hmask words, [20..24] the 12 scale bytes, [25] d
   static __device__ __forceinline__ void load(const uint8_t* row, int u, uint32_t (&raw)[RW]) {
     const uint8_t* blk = row + (int64_t)(u >> 3) * 110;
@@ -536,12 +519,30 @@ template <typename ab_t> struct Decoder<T_Q3_K, ab_t> {
       }
     }
   }
-  static __device__ __forceinline__ void corr(const uint8_t*, int, int64_t, uint32_t (&)[16]) {}
 };
+
+// byte k of w (unsigned) as the float 2^23 + byte, without a conversion instruction
+__device__ __forceinline__ float byte_2p23(uint32_t w, int k) { return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440u | k)); }
+// The sixteen IQ4 levels plus 128 in four registers: two byte-permutes look four indices up in a half of the table each (the
+// nibbles of q3, bit 3 cleared, are the selectors), a third takes the half that each index's top bit names.  Four bytes, in the
+// order of the nibbles.
+__device__ __forceinline__ uint32_t iq4_levels4(uint32_t q3, uint32_t sel) {
+  return __byte_perm(__byte_perm(0x3F2D1801u, 0x766A5D4Fu, q3), __byte_perm(0xA6998D81u, 0xF1D9C5B5u, q3), sel);
+}
+// A word of IQ4 indices (values 4i.. in the low nibbles, 16 + 4i.. in the high ones) -> the two pairs of each, scaled in fp32 and rounded once
+template <typename ab_t> __device__ __forceinline__ void iq4_word(uint32_t w, float dl, uint32_t* lo, uint32_t* hi) {
+  const uint32_t q3 = w & 0x77777777u, sel = ((w & 0x88888888u) >> 1) | 0x32103210u;
+  const uint32_t a = iq4_levels4(q3, sel), b = iq4_levels4(q3 >> 16, sel >> 16);   // bytes (4i, 16+4i, 4i+1, 17+4i) and (4i+2, ...)
+  auto v = [&](uint32_t x, int k) { return dl * (byte_2p23(x, k) - 8388736.f); };   // 2^23 + 128
+  lo[0] = pack2<ab_t>(v(a, 0), v(a, 2));
+  lo[1] = pack2<ab_t>(v(b, 0), v(b, 2));
+  hi[0] = pack2<ab_t>(v(a, 1), v(a, 3));
+  hi[1] = pack2<ab_t>(v(b, 1), v(b, 3));
+}
 
 // ---- IQ4_XS: fp32 d*(ls-32)*level rounded once to ab_t; unit = 32-value group ib = u&7 -----------
 template <typename ab_t> struct Decoder<T_IQ4_XS, ab_t> {
-  static constexpr int CORR_OFF = -1;   // byte offset in a block of the fp16 that is the block's correction value (-1: none / computed)
+  static constexpr bool CORR = false;
   static constexpr int RW = 6;   // header (8 bytes) + 16 index bytes, 8-byte aligned
   static __device__ __forceinline__ void load(const uint8_t* row, int u, uint32_t (&raw)[RW]) {
     const uint8_t* blk = row + (int64_t)(u >> 3) * 136;
@@ -549,51 +550,38 @@ template <typename ab_t> struct Decoder<T_IQ4_XS, ab_t> {
     const uint2 h = lds64(sb), a = lds64(sb + 8 + 16 * (u & 7)), b = lds64(sb + 16 + 16 * (u & 7));
     raw[0] = h.x; raw[1] = h.y; raw[2] = a.x; raw[3] = a.y; raw[4] = b.x; raw[5] = b.y;
   }
-  static __device__ __forceinline__ void decode(const uint8_t*, int u, const uint32_t (&raw)[RW], const DecodeCtx& cx, uint32_t (&out)[16]) {
+  static __device__ __forceinline__ void decode(const uint8_t*, int u, const uint32_t (&raw)[RW], const DecodeCtx&, uint32_t (&out)[16]) {
     const int ib = u & 7;
     const float d = __half2float(__ushort_as_half((unsigned short)(raw[0] & 0xffff)));
     const int ls = (int)(((raw[1] >> (4 * ib)) & 0xF) | ((((raw[0] >> 16) >> (2 * ib)) & 3) << 4)) - 32;
     const float dl = d * (float)ls;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {  // bytes 4i..4i+3: values 4i.. (low nibbles) and 16+4i.. (high)
-      const uint32_t w = raw[2 + i];
-      out[2 * i] = pack2<ab_t>(dl * cx.level(w & 0xF), dl * cx.level((w >> 8) & 0xF));
-      out[2 * i + 1] = pack2<ab_t>(dl * cx.level((w >> 16) & 0xF), dl * cx.level((w >> 24) & 0xF));
-      out[8 + 2 * i] = pack2<ab_t>(dl * cx.level((w >> 4) & 0xF), dl * cx.level((w >> 12) & 0xF));
-      out[8 + 2 * i + 1] = pack2<ab_t>(dl * cx.level((w >> 20) & 0xF), dl * cx.level((w >> 28) & 0xF));
-    }
+    for (int i = 0; i < 4; ++i) iq4_word<ab_t>(raw[2 + i], dl, out + 2 * i, out + 8 + 2 * i);
   }
-  static __device__ __forceinline__ void corr(const uint8_t*, int, int64_t, uint32_t (&)[16]) {}
 };
 
 // ---- IQ4_NL: fp32 d*level rounded once to ab_t; unit = one 18-byte block (2-byte aligned) ----------
 template <typename ab_t> struct Decoder<T_IQ4_NL, ab_t> {
-  static constexpr int CORR_OFF = -1;   // byte offset in a block of the fp16 that is the block's correction value (-1: none / computed)
+  static constexpr bool CORR = false;
   static constexpr int RW = 7;
   static __device__ __forceinline__ void load(const uint8_t* row, int u, uint32_t (&raw)[RW]) {
     ldg_cover<RW - 1>(row + (int64_t)u * 18, 18, raw);
     raw[RW - 1] = 0;
   }
-  static __device__ __forceinline__ void decode(const uint8_t* row, int u, const uint32_t (&raw)[RW], const DecodeCtx& cx, uint32_t (&out)[16]) {
+  static __device__ __forceinline__ void decode(const uint8_t* row, int u, const uint32_t (&raw)[RW], const DecodeCtx&, uint32_t (&out)[16]) {
     const uint32_t sh = shift_of(row + (int64_t)u * 18);
     const float d = __half2float(__ushort_as_half((unsigned short)(word_at(raw, 0, sh) & 0xFFFFu)));
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {  // stream half-word 1+i holds qs[2i], qs[2i+1]
-      const int h = 1 + i;
-      const uint32_t wv = word_at(raw, h >> 1, sh);
-      const uint32_t t = (h & 1) ? (wv >> 16) : (wv & 0xFFFFu);
-      out[i] = pack2<ab_t>(d * cx.level(t & 0xF), d * cx.level((t >> 8) & 0xF));
-      out[8 + i] = pack2<ab_t>(d * cx.level((t >> 4) & 0xF), d * cx.level((t >> 12) & 0xF));
-    }
+    for (int i = 0; i < 4; ++i)   // the indices start 2 bytes into the block
+      iq4_word<ab_t>(__funnelshift_r(word_at(raw, i, sh), word_at(raw, i + 1, sh), 16), d, out + 2 * i, out + 8 + 2 * i);
   }
-  static __device__ __forceinline__ void corr(const uint8_t*, int, int64_t, uint32_t (&)[16]) {}
 };
 
 // ---- IQ2_XXS: fp32 d*(0.5+s)*0.25*grid*sign rounded once; unit = 32-value group ib = u&7 ----------
 // (value = +-round(d * magnitude): the product is formed in fp32 and rounded once, as in the
 // reference; multiplying by -1.f afterwards is exact, so flipping the sign bit is the same)
 template <typename ab_t> struct Decoder<T_IQ2_XXS, ab_t> {
-  static constexpr int CORR_OFF = -1;   // byte offset in a block of the fp16 that is the block's correction value (-1: none / computed)
+  static constexpr bool CORR = false;   // correction columns
   static constexpr int RW = 5;   // [0] word holding d, [1..3] the group's 8 bytes (+ cover), [4] pad
   static __device__ __forceinline__ void load(const uint8_t* row, int u, uint32_t (&raw)[RW]) {
     const uint8_t* blk = row + (int64_t)(u >> 3) * 66;
@@ -611,15 +599,169 @@ template <typename ab_t> struct Decoder<T_IQ2_XXS, ab_t> {
     const uint32_t r0 = pack2<ab_t>(d * 8.f, d * 25.f), r1 = pack2<ab_t>(d * 43.f, 0.f);
 #pragma unroll
     for (int il = 0; il < 4; ++il) {
-      const uint2 sel = cx.sel_at((idx >> (8 * il)) & 0xFF);
-      const uint4 sg = cx.sgn_at((aux >> (7 * il)) & 127);
+      const uint2 sel = grid64<T_IQ2_XXS>(cx, (idx >> (8 * il)) & 0xFF);
+      const uint4 sg = sign_masks<T_IQ2_XXS>(cx, (aux >> (7 * il)) & 127);
       out[4 * il + 0] = __byte_perm(r0, r1, sel.x) ^ sg.x;
       out[4 * il + 1] = __byte_perm(r0, r1, sel.x >> 16) ^ sg.y;
       out[4 * il + 2] = __byte_perm(r0, r1, sel.y) ^ sg.z;
       out[4 * il + 3] = __byte_perm(r0, r1, sel.y >> 16) ^ sg.w;
     }
   }
-  static __device__ __forceinline__ void corr(const uint8_t*, int, int64_t, uint32_t (&)[16]) {}
+};
+
+// ---- the other code-book formats (bit-identical to the standalone dequantize: one fp32 product, one rounding) ----
+// 8 values of an IQ2 entry whose three possible magnitudes are parked in r0, r1 (see Decoder<T_IQ2_XXS>)
+__device__ __forceinline__ void iq2_entry(uint2 sel, uint4 sg, uint32_t r0, uint32_t r1, uint32_t* out) {
+  out[0] = __byte_perm(r0, r1, sel.x) ^ sg.x;
+  out[1] = __byte_perm(r0, r1, sel.x >> 16) ^ sg.y;
+  out[2] = __byte_perm(r0, r1, sel.y) ^ sg.z;
+  out[3] = __byte_perm(r0, r1, sel.y >> 16) ^ sg.w;
+}
+template <typename ab_t> struct Decoder<T_IQ2_XS, ab_t> {   // half d | u16 qs[32] | u8 scales[8], 74 bytes
+  static constexpr bool CORR = false;
+  static constexpr int RW = 5;   // [0] d, [1..3] the group's 8 bytes (+ cover), [4] its scale byte
+  static __device__ __forceinline__ void load(const uint8_t* blk, int u, uint32_t (&raw)[RW]) {
+    ldg_cover<1>(blk, 2, raw);
+    ldg_cover<3>(blk + 2 + 8 * u, 8, raw + 1);
+    raw[4] = lds8(smem_u32(blk) + 66 + u);
+  }
+  static __device__ __forceinline__ void decode(const uint8_t* blk, int u, const uint32_t (&raw)[RW], const DecodeCtx& cx, uint32_t (&out)[16]) {
+    const float dh = __half2float(__ushort_as_half((unsigned short)((raw[0] >> shift_of(blk)) & 0xFFFFu)));
+    const uint32_t sh = shift_of(blk + 2 + 8 * u);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const float d = dh * (0.5f + (float)((raw[4] >> (4 * h)) & 0xF)) * 0.25f;
+      const uint32_t r0 = pack2<ab_t>(d * 8.f, d * 25.f), r1 = pack2<ab_t>(d * 43.f, 0.f), q = word_at(raw + 1, h, sh);
+#pragma unroll
+      for (int l = 0; l < 2; ++l)
+        iq2_entry(grid64<T_IQ2_XS>(cx, (q >> (16 * l)) & 511u), sign_masks<T_IQ2_XS>(cx, (q >> (16 * l + 9)) & 127u), r0, r1, out + 8 * h + 4 * l);
+    }
+  }
+};
+template <typename ab_t> struct Decoder<T_IQ2_S, ab_t> {   // half d | u8 qs[32] | u8 signs[32] | u8 qh[8] | u8 scales[8], 82 bytes
+  static constexpr bool CORR = false;
+  static constexpr int RW = 7;
+  static __device__ __forceinline__ void load(const uint8_t* blk, int u, uint32_t (&raw)[RW]) {
+    ldg_cover<1>(blk, 2, raw);
+    ldg_cover<2>(blk + 2 + 4 * u, 4, raw + 1);
+    ldg_cover<2>(blk + 34 + 4 * u, 4, raw + 3);
+    raw[5] = lds8(smem_u32(blk) + 66 + u);
+    raw[6] = lds8(smem_u32(blk) + 74 + u);
+  }
+  static __device__ __forceinline__ void decode(const uint8_t* blk, int u, const uint32_t (&raw)[RW], const DecodeCtx& cx, uint32_t (&out)[16]) {
+    const float dh = __half2float(__ushort_as_half((unsigned short)((raw[0] >> shift_of(blk)) & 0xFFFFu)));
+    const uint32_t q = word_at(raw + 1, 0, shift_of(blk + 2 + 4 * u)), sg = word_at(raw + 3, 0, shift_of(blk + 34 + 4 * u));
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const float d = dh * (0.5f + (float)((raw[6] >> (4 * h)) & 0xF)) * 0.25f;
+      const uint32_t r0 = pack2<ab_t>(d * 8.f, d * 25.f), r1 = pack2<ab_t>(d * 43.f, 0.f);
+#pragma unroll
+      for (int l2 = 0; l2 < 2; ++l2) {
+        const int l = 2 * h + l2;
+        iq2_entry(grid64<T_IQ2_S>(cx, ((q >> (8 * l)) & 0xFFu) | ((raw[5] << (8 - 2 * l)) & 0x300u)), sign_masks<T_IQ2_S>(cx, (sg >> (8 * l)) & 0xFFu), r0,
+                  r1, out + 4 * l);
+      }
+    }
+  }
+};
+// 8 values of two IQ3 entries: magnitude bytes, scaled in fp32 (d * (2^23 + byte) - d * 2^23 is d * byte rounded once)
+template <typename ab_t> __device__ __forceinline__ void iq3_entries(uint32_t g0, uint32_t g1, uint4 sg, float d, float off, uint32_t* out) {
+  auto v = [&](uint32_t g, int k) { return fmaf(d, byte_2p23(g, k), off); };
+  out[0] = pack2<ab_t>(v(g0, 0), v(g0, 1)) ^ sg.x;
+  out[1] = pack2<ab_t>(v(g0, 2), v(g0, 3)) ^ sg.y;
+  out[2] = pack2<ab_t>(v(g1, 0), v(g1, 1)) ^ sg.z;
+  out[3] = pack2<ab_t>(v(g1, 2), v(g1, 3)) ^ sg.w;
+}
+template <typename ab_t> struct Decoder<T_IQ3_XXS, ab_t> {   // half d | u8 qs[64] | u32 scale_and_signs[8], 98 bytes
+  static constexpr bool CORR = false;
+  static constexpr int RW = 6;
+  static __device__ __forceinline__ void load(const uint8_t* blk, int u, uint32_t (&raw)[RW]) {
+    ldg_cover<1>(blk, 2, raw);
+    ldg_cover<3>(blk + 2 + 8 * u, 8, raw + 1);
+    ldg_cover<2>(blk + 66 + 4 * u, 4, raw + 4);
+  }
+  static __device__ __forceinline__ void decode(const uint8_t* blk, int u, const uint32_t (&raw)[RW], const DecodeCtx& cx, uint32_t (&out)[16]) {
+    const float dh = __half2float(__ushort_as_half((unsigned short)((raw[0] >> shift_of(blk)) & 0xFFFFu)));
+    const uint32_t sh = shift_of(blk + 2 + 8 * u), aux = word_at(raw + 4, 0, shift_of(blk + 66 + 4 * u));
+    const float d = dh * (0.5f + (float)(aux >> 28)) * 0.5f, off = -8388608.f * d;
+#pragma unroll
+    for (int l = 0; l < 4; ++l) {
+      const uint32_t e = word_at(raw + 1, l >> 1, sh) >> (16 * (l & 1));
+      iq3_entries<ab_t>(grid32<T_IQ3_XXS>(cx, e & 0xFFu), grid32<T_IQ3_XXS>(cx, (e >> 8) & 0xFFu), sign_masks<T_IQ3_XXS>(cx, (aux >> (7 * l)) & 127u), d,
+                        off, out + 4 * l);
+    }
+  }
+};
+template <typename ab_t> struct Decoder<T_IQ3_S, ab_t> {   // half d | u8 qs[64] | u8 qh[8] | u8 signs[32] | u8 scales[4], 110 bytes
+  static constexpr bool CORR = false;
+  static constexpr int RW = 8;
+  static __device__ __forceinline__ void load(const uint8_t* blk, int u, uint32_t (&raw)[RW]) {
+    ldg_cover<1>(blk, 2, raw);
+    ldg_cover<3>(blk + 2 + 8 * u, 8, raw + 1);
+    ldg_cover<2>(blk + 74 + 4 * u, 4, raw + 4);
+    raw[6] = lds8(smem_u32(blk) + 66 + u);
+    raw[7] = lds8(smem_u32(blk) + 106 + (u >> 1));
+  }
+  static __device__ __forceinline__ void decode(const uint8_t* blk, int u, const uint32_t (&raw)[RW], const DecodeCtx& cx, uint32_t (&out)[16]) {
+    const float dh = __half2float(__ushort_as_half((unsigned short)((raw[0] >> shift_of(blk)) & 0xFFFFu)));
+    const uint32_t sh = shift_of(blk + 2 + 8 * u), sg = word_at(raw + 4, 0, shift_of(blk + 74 + 4 * u));
+    const float d = dh * (0.5f + (float)((raw[7] >> (4 * (u & 1))) & 0xFu)) * 0.5f, off = -8388608.f * d;
+#pragma unroll
+    for (int l = 0; l < 4; ++l) {
+      const uint32_t e = word_at(raw + 1, l >> 1, sh) >> (16 * (l & 1));
+      iq3_entries<ab_t>(grid32<T_IQ3_S>(cx, (e & 0xFFu) | ((raw[6] << (8 - 2 * l)) & 256u)), grid32<T_IQ3_S>(cx, ((e >> 8) & 0xFFu) | ((raw[6] << (7 - 2 * l)) & 256u)),
+                        sign_masks<T_IQ3_S>(cx, (sg >> (8 * l)) & 0xFFu), d, off, out + 4 * l);
+    }
+  }
+};
+// 8 values of an IQ1 entry (codes 0, 1, 2 in nibbles: values 0-3 low, 4-7 high): the group has three possible values d * (code +
+// delta), rounded once each and parked in r0, r1; a pair is one byte-permute whose selector is its codes times 0x22 plus 0x1010
+__device__ __forceinline__ void iq1_entry(uint32_t g, uint32_t r0, uint32_t r1, uint32_t* out) {
+  const uint32_t s0 = (g & 0x0F0F0F0Fu) * 0x22u + 0x10101010u, s1 = ((g >> 4) & 0x0F0F0F0Fu) * 0x22u + 0x10101010u;
+  out[0] = __byte_perm(r0, r1, s0);
+  out[1] = __byte_perm(r0, r1, s0 >> 16);
+  out[2] = __byte_perm(r0, r1, s1);
+  out[3] = __byte_perm(r0, r1, s1 >> 16);
+}
+template <typename ab_t> struct Decoder<T_IQ1_S, ab_t> {   // half d | u8 qs[32] | u16 qh[8], 50 bytes
+  static constexpr bool CORR = false;
+  static constexpr int RW = 4;
+  static __device__ __forceinline__ void load(const uint8_t* blk, int u, uint32_t (&raw)[RW]) {
+    ldg_cover<1>(blk, 2, raw);
+    ldg_cover<2>(blk + 2 + 4 * u, 4, raw + 1);
+    ldg_cover<1>(blk + 34 + 2 * u, 2, raw + 3);
+  }
+  static __device__ __forceinline__ void decode(const uint8_t* blk, int u, const uint32_t (&raw)[RW], const DecodeCtx& cx, uint32_t (&out)[16]) {
+    const float dh = __half2float(__ushort_as_half((unsigned short)((raw[0] >> shift_of(blk)) & 0xFFFFu)));
+    const uint32_t q = word_at(raw + 1, 0, shift_of(blk + 2 + 4 * u)), qh = (raw[3] >> shift_of(blk + 34 + 2 * u)) & 0xFFFFu;
+    const float d = dh * (float)(2u * ((qh >> 12) & 7u) + 1u), delta = qh & 0x8000u ? -1.125f : -0.875f;
+    const uint32_t r0 = pack2<ab_t>(d * delta, d * (1.f + delta)), r1 = pack2<ab_t>(d * (2.f + delta), 0.f);
+#pragma unroll
+    for (int l = 0; l < 4; ++l) iq1_entry(grid32<T_IQ1_S>(cx, ((q >> (8 * l)) & 0xFFu) | (((qh >> (3 * l)) & 7u) << 8)), r0, r1, out + 4 * l);
+  }
+};
+template <typename ab_t> struct Decoder<T_IQ1_M, ab_t> {   // u8 qs[32] | u8 qh[16] | u16 scales[4], 56 bytes (8-byte aligned)
+  static constexpr bool CORR = false;
+  static constexpr int RW = 4;
+  static __device__ __forceinline__ void load(const uint8_t* blk, int u, uint32_t (&raw)[RW]) {
+    const uint32_t sb = smem_u32(blk);
+    raw[0] = lds32(sb + 4 * u);
+    raw[1] = (lds32(sb + 32 + 4 * (u >> 1)) >> (16 * (u & 1))) & 0xFFFFu;
+    const uint2 s = lds64(sb + 48);
+    raw[2] = s.x; raw[3] = s.y;
+  }
+  static __device__ __forceinline__ void decode(const uint8_t*, int u, const uint32_t (&raw)[RW], const DecodeCtx& cx, uint32_t (&out)[16]) {
+    const uint32_t s16 = ((raw[2] >> 12) & 0x000Fu) | ((raw[2] >> 24) & 0x00F0u) | ((raw[3] >> 4) & 0x0F00u) | ((raw[3] >> 16) & 0xF000u);
+    const float dh = __half2float(__ushort_as_half((unsigned short)s16));
+    const uint32_t s2 = ((u & 4) ? raw[3] : raw[2]) >> (16 * ((u >> 1) & 1) + 6 * (u & 1));
+#pragma unroll
+    for (int l = 0; l < 4; ++l) {
+      const uint32_t h = raw[1] >> (4 * l);
+      const float d = dh * (float)(2u * ((s2 >> (3 * (l >> 1))) & 7u) + 1u), delta = h & 8u ? -1.125f : -0.875f;
+      iq1_entry(grid32<T_IQ1_M>(cx, ((raw[0] >> (8 * l)) & 0xFFu) | ((h & 7u) << 8)), pack2<ab_t>(d * delta, d * (1.f + delta)),
+                pack2<ab_t>(d * (2.f + delta), 0.f), out + 4 * l);
+    }
+  }
 };
 
 // =============================================================================================
@@ -638,6 +780,9 @@ template <typename ab_t> struct Decoder<T_IQ2_XXS, ab_t> {
 // activation matrix is written in the same order (quantize_q8_1.cu), so the contraction is
 // unchanged.
 // =============================================================================================
+// Where the stage's number only moves addresses and shifts it is a run-time argument (one copy of the code for all four groups: the
+// kernel's first pass over its instructions costs more than a stage); where it moves words between registers it is a template
+// argument of stage<SC>().
 template <int TYPE, typename ab_t> struct Stage64 {
   static constexpr bool FAST = false;
   static constexpr int PERM = 0;
@@ -647,18 +792,24 @@ __device__ __forceinline__ uint4 lds128(const uint8_t* p) { return lds128s(smem_
 __device__ __forceinline__ __half2 h2const(float v) { return __floats2half2_rn(v, v); }
 
 // ---- Q4_K: chunk = one 144-byte super-block; stage SC = sub-blocks 2SC (low nibbles) and 2SC+1 ----
+// the scales of the sub-blocks 2 * sc and 2 * sc + 1 of a Q4_K / Q5_K super-block, times d
+__device__ __forceinline__ void q4k_pair_scales(uint4 h, int sc, __half& d0, __half& d1) {
+  const __half dall = __ushort_as_half((unsigned short)(h.x & 0xffff));
+  const int sh = 16 * (sc & 1);
+  const uint32_t a = h.y >> sh, c = h.w >> sh;
+  const uint32_t s2 = sc < 2 ? a & 0x3F3Fu : (c & 0x0F0Fu) | ((a >> 2) & 0x3030u);
+  d0 = __hmul_rn(dall, __int2half_rn((int)(s2 & 0xFFu)));
+  d1 = __hmul_rn(dall, __int2half_rn((int)(s2 >> 8)));
+}
 template <> struct Stage64<T_Q4_K, __half> {
   static constexpr bool FAST = true;
   static constexpr int PERM = 1;
-  template <int SC> static __device__ __forceinline__ void decode(const uint8_t* blk, uint32_t (&out)[32]) {
+  static __device__ __forceinline__ void decode(const uint8_t* blk, int sc, uint32_t (&out)[32]) {
     const uint4 h = lds128(blk);
-    const uint4 qa = lds128(blk + 16 + 32 * SC), qb = lds128(blk + 32 + 32 * SC);
+    const uint4 qa = lds128(blk + 16 + 32 * sc), qb = lds128(blk + 32 + 32 * sc);
     const uint32_t w[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
-    const __half dall = __ushort_as_half((unsigned short)(h.x & 0xffff));
-    int sc0, sc1, m;
-    q4k_scale_min(h.y, h.z, h.w, 2 * SC, sc0, m);
-    q4k_scale_min(h.y, h.z, h.w, 2 * SC + 1, sc1, m);
-    const __half d0 = __hmul_rn(dall, __int2half_rn(sc0)), d1 = __hmul_rn(dall, __int2half_rn(sc1));
+    __half d0, d1;
+    q4k_pair_scales(h, sc, d0, d1);
     const __half2 s0 = __half2half2(d0), s1 = __half2half2(d1);
     const float big = fmaxf(fabsf(__half2float(d0)), fabsf(__half2float(d1)));
     if (big < 32.f) {
@@ -693,17 +844,14 @@ template <> struct Stage64<T_Q4_K, __half> {
 template <> struct Stage64<T_Q5_K, __half> {
   static constexpr bool FAST = true;
   static constexpr int PERM = 1;
-  template <int SC> static __device__ __forceinline__ void decode(const uint8_t* blk, uint32_t (&out)[32]) {
+  static __device__ __forceinline__ void decode(const uint8_t* blk, int sc, uint32_t (&out)[32]) {
     const uint4 h = lds128(blk);
     const uint4 ha = lds128(blk + 16), hb = lds128(blk + 32);
-    const uint4 qa = lds128(blk + 48 + 32 * SC), qb = lds128(blk + 64 + 32 * SC);
+    const uint4 qa = lds128(blk + 48 + 32 * sc), qb = lds128(blk + 64 + 32 * sc);
     const uint32_t w[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
     const uint32_t hw[8] = {ha.x, ha.y, ha.z, ha.w, hb.x, hb.y, hb.z, hb.w};
-    const __half dall = __ushort_as_half((unsigned short)(h.x & 0xffff));
-    int sc0, sc1, m;
-    q4k_scale_min(h.y, h.z, h.w, 2 * SC, sc0, m);
-    q4k_scale_min(h.y, h.z, h.w, 2 * SC + 1, sc1, m);
-    const __half d0 = __hmul_rn(dall, __int2half_rn(sc0)), d1 = __hmul_rn(dall, __int2half_rn(sc1));
+    __half d0, d1;
+    q4k_pair_scales(h, sc, d0, d1);
     const __half2 s0 = __half2half2(d0), s1 = __half2half2(d1);
     const float big = fmaxf(fabsf(__half2float(d0)), fabsf(__half2float(d1)));
     if (big < 32.f) {
@@ -712,7 +860,7 @@ template <> struct Stage64<T_Q5_K, __half> {
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const uint32_t a = w[j], b = w[j] >> 8;
-        const uint32_t x = hw[j] >> (2 * SC), y = hw[j] >> (2 * SC + 8);   // fifth bits of values (4j, 4j+2) / (4j+1, 4j+3) at bits 0 and 16
+        const uint32_t x = hw[j] >> (2 * sc), y = hw[j] >> (2 * sc + 8);   // fifth bits of values (4j, 4j+2) / (4j+1, 4j+3) at bits 0 and 16
         out[2 * j] = h2_as_u32(__hfma2(u32_as_h2((a & 0x000F000Fu) | ((x << 4) & 0x00100010u) | 0x64006400u), s0, c0));
         out[2 * j + 1] = h2_as_u32(__hfma2(u32_as_h2((b & 0x000F000Fu) | ((y << 4) & 0x00100010u) | 0x64006400u), s0, c0));
         out[16 + 2 * j] = h2_as_u32(__hfma2(u32_as_h2((a & 0x00F000F0u) | ((x << 7) & 0x01000100u) | 0x54005400u), s1, c1));
@@ -723,7 +871,7 @@ template <> struct Stage64<T_Q5_K, __half> {
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const uint32_t a = w[j], b = w[j] >> 8;
-        const uint32_t x = hw[j] >> (2 * SC), y = hw[j] >> (2 * SC + 8);
+        const uint32_t x = hw[j] >> (2 * sc), y = hw[j] >> (2 * sc + 8);
         out[2 * j] = h2_as_u32(hmul2_rn(__hsub2(u32_as_h2((a & 0x000F000Fu) | ((x << 4) & 0x00100010u) | 0x64006400u), o0), s0));
         out[2 * j + 1] = h2_as_u32(hmul2_rn(__hsub2(u32_as_h2((b & 0x000F000Fu) | ((y << 4) & 0x00100010u) | 0x64006400u), o0), s0));
         out[16 + 2 * j] = h2_as_u32(hmul2_rn(__hsub2(u32_as_h2((a & 0x00F000F0u) | ((x << 7) & 0x01000100u) | 0x54005400u), o1), s1));
@@ -764,7 +912,7 @@ template <> struct Stage64<T_Q4_0, __half> {
       }
     }
   }
-  template <int SC> static __device__ __forceinline__ void decode(const uint8_t* chunk, uint32_t (&out)[32]) {
+  template <int SC> static __device__ __forceinline__ void stage(const uint8_t* chunk, uint32_t (&out)[32]) {
     constexpr int A0 = (36 * SC) & ~15, O = (36 * SC - A0) / 4;   // aligned start, word offset of block 2SC
     uint32_t W[12];
 #pragma unroll
@@ -780,6 +928,14 @@ template <> struct Stage64<T_Q4_0, __half> {
     block(qa, u32_as_h2(da | (da << 16)), out);
     block(qb, u32_as_h2(db | (db << 16)), out + 16);
   }
+  static __device__ __forceinline__ void decode(const uint8_t* chunk, int sc, uint32_t (&out)[32]) {
+    switch (sc) {
+      case 0: stage<0>(chunk, out); break;
+      case 1: stage<1>(chunk, out); break;
+      case 2: stage<2>(chunk, out); break;
+      default: stage<3>(chunk, out); break;
+    }
+  }
 };
 
 // ---- Q8_0: chunk = 8 blocks of 34 bytes; stage SC = blocks 2SC, 2SC+1 at byte 68*SC ----------------
@@ -791,7 +947,7 @@ template <> struct Stage64<T_Q8_0, __half> {
     const __half2 o = h2const(1152.f);
     return h2_as_u32(hmul2_rn(__hsub2(u32_as_h2(__byte_perm(w, 0x64646464u, sel)), o), d2));
   }
-  template <int SC> static __device__ __forceinline__ void decode(const uint8_t* chunk, uint32_t (&out)[32]) {
+  template <int SC> static __device__ __forceinline__ void stage(const uint8_t* chunk, uint32_t (&out)[32]) {
     constexpr int A0 = (68 * SC) & ~15, O = (68 * SC - A0) / 4;
     uint32_t W[20];
 #pragma unroll
@@ -812,6 +968,14 @@ template <> struct Stage64<T_Q8_0, __half> {
     for (int t = 0; t < 16; ++t) {
       const uint32_t wv = W[O + 9 + (t >> 1)] ^ 0x80808080u;
       out[16 + t] = pair(wv, (t & 1) ? 0x4342u : 0x4140u, d2b);
+    }
+  }
+  static __device__ __forceinline__ void decode(const uint8_t* chunk, int sc, uint32_t (&out)[32]) {
+    switch (sc) {
+      case 0: stage<0>(chunk, out); break;
+      case 1: stage<1>(chunk, out); break;
+      case 2: stage<2>(chunk, out); break;
+      default: stage<3>(chunk, out); break;
     }
   }
 };

@@ -1,0 +1,705 @@
+// Kernel of the tensor-core GEMM (see mmq.cu); instantiated by mmq_inst_*.cu.
+#pragma once
+
+#include <cuda.h>
+
+#include <type_traits>
+
+#include "kernels.h"
+#include "mmq_decode.cuh"
+#include "raw_stream.cuh"
+
+namespace gguf_b200 {
+
+constexpr int MMQ_ROWS = 128;
+constexpr int MMQ_BK = 64;                           // values per stage (128 bytes of activations: one swizzle row)
+constexpr int MMQ_GROUPS = 4;                        // producer groups of 128 threads, one thread per weight row
+constexpr int MMQ_PRODUCER_WARPS = 4 * MMQ_GROUPS;
+constexpr int MMQ_THREADS = (MMQ_PRODUCER_WARPS + 3) * 32;   // + B loader, MMA issuer, raw-weight loader
+// Tensor memory: up to 128 tokens a tile, two accumulators of 128 columns and eight A slots of 32; beyond, 384 columns of
+// accumulator -- two of 192, or one of 384 -- and four A slots.  The stages' barriers are a ring of eight in both cases: a
+// group's stages are eight apart, so by the time it waits for a phase it has seen the one before complete.
+constexpr int MMQ_A_COLS = 32, MMQ_BARS = 8;
+constexpr int MMQ_MAX_RAW = 8;
+// Correction values of eight chunks (64 fp16) per row, rows an odd number of 16-byte units apart
+constexpr int MMQ_CORR_CHUNKS = 8, MMQ_CORR_ROW = 144, MMQ_CORR_BYTES = MMQ_ROWS * MMQ_CORR_ROW;
+
+struct MmqParams {
+  RawPlan raw;
+  const uint8_t* w;
+  int64_t w_bytes;
+  void* y;
+  int64_t ldy;
+  int dtype;              // of y
+  int n, m;               // weight rows, tokens
+  int k, kpad;
+  int nc, corr;           // 256-value chunks of a row; 1: a stage of corrections behind every eight of them
+  int rt, tt, tn;         // row tiles, token tiles, tokens per tile (a multiple of 16, at most 256)
+  int sa, a_col0;         // A slots: how many (4 or 8), first column
+  int nbuf, d_step;       // accumulators, columns between them
+  int sb, raw_stages;     // ring depths
+  int raw_off, aux_off, corr_off;   // shared memory behind the B ring
+  uint32_t idesc;
+  float* part;            // partial tiles, two slots of 128 x tn per CTA; null: every tile is one CTA's
+  int waste;              // idle chunks of a CTA up to which whole tiles are dealt out all the same
+  int* counter;           // arrivals per tile, zero at the start
+  int* status;
+  // MoE (passes != null): pass = {expert, first activation row, rows}
+  const int4* passes;
+  const int32_t* n_passes;
+  const int32_t* sorted;  // output row of every activation row
+  int rows_out;
+  const float* row_scale;
+  // tensor-parallel output (tp_world > 0): see MmqTp
+  int tp_world, tp_slot;
+  int64_t tp_col_off;
+  unsigned* tp_epoch;
+  void* tp_y[8];
+  unsigned* tp_flag[8];
+};
+
+// ---- tcgen05 wrappers -------------------------------------------------------------------
+__device__ __forceinline__ void tmem_alloc(uint32_t* slot_smem, uint32_t ncols) {
+  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot_smem)), "r"(ncols) : "memory");
+}
+__device__ __forceinline__ void tmem_relinquish() { asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
+  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+}
+__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void umma_commit(uint64_t* bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+// one lane of a converged warp (the same one every time)
+__device__ __forceinline__ bool elect_one() {
+  uint32_t pred;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(pred));
+  return pred != 0;
+}
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+// 32 registers -> 32 consecutive columns of this thread's lane (warp w owns lanes 32 * (w % 4) ...)
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
+      "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
+      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+        "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]),
+        "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]),
+        "r"(r[30]), "r"(r[31])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+// D[tmem] (+)= A[tmem] * B[smem]: A is 128 lanes x 8 columns (16 fp16 values per row, two per column)
+__device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t b_hi, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 b;\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "mov.b64 b, {%2, %3};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %4, p;\n\t}"
+      ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// K-major, 128-byte swizzle: rows of 128 B, 8-row groups 1024 B apart (stride byte offset),
+// leading byte offset unused by swizzled K-major layouts (1), descriptor version 1 (sm_100).
+__device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t saddr) {
+  uint64_t d = 0;
+  d |= (uint64_t)((saddr >> 4) & 0x3FFF);
+  d |= (uint64_t)1 << 16;
+  d |= (uint64_t)(1024 >> 4) << 32;
+  d |= (uint64_t)1 << 46;
+  d |= (uint64_t)2 << 61;
+  return d;
+}
+// kind::f16 instruction descriptor: fp32 accumulator, A/B format (0 = f16, 1 = bf16), both K-major
+__host__ __device__ inline uint32_t umma_idesc(int m, int n, int fmt) {
+  return (1u << 4) | ((uint32_t)fmt << 7) | ((uint32_t)fmt << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
+}
+
+// CTAs of the tensor-parallel launch in flight per call slot that have stored their tiles
+static __device__ unsigned g_mmq_tp_done[64];
+
+// End of a tensor-parallel launch, called by every thread of a CTA after its stores to the peers:
+// CTA barrier, thread 0 fences system-wide and counts the CTA off; the last CTA of the grid
+// increments this rank's launch counter and raises the slot's flag on every rank.  The flags only
+// grow (one increment per rank and launch), so replays of a captured graph need no reset.
+__device__ __forceinline__ void tp_finish(unsigned* epoch, unsigned* const* flag, int world, int slot, unsigned total_ctas) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence_system();
+    unsigned* done = &g_mmq_tp_done[slot & 63];
+    const unsigned prev = atomicAdd(done, 1u);
+    if (prev == total_ctas - 1) {
+      *done = 0;
+      __threadfence_system();
+      epoch[slot] += 1;
+      __threadfence_system();
+      for (int r = 0; r < world; ++r) atomicAdd_system(flag[r] + slot, 1u);
+    }
+  }
+}
+
+// A CTA's work: the units (tile, chunk) [u0, u1) in parts of one tile each.  Every role of the CTA walks the same parts.
+struct MmqPart {
+  int u, u1;                 // next unit, end
+  int tile, c0, c1;          // chunks [c0, c1) of the tile
+};
+struct MmqTile {
+  int n0;                    // first row
+  int x0, rows;              // first activation row, rows that count
+  int row0;                  // MoE: first row of the expert's matrix among all rows
+};
+__device__ __forceinline__ MmqTile mmq_tile(const MmqParams& p, int tile) {
+  MmqTile t;
+  if (p.passes) {
+    const int ps = (int)((unsigned)tile / (unsigned)p.rt);
+    const int4 info = p.passes[ps];
+    t.n0 = (tile - ps * p.rt) * MMQ_ROWS;
+    t.row0 = info.x * p.n;
+    t.x0 = info.y;
+    t.rows = info.z;
+  } else {
+    const int r = (int)((unsigned)tile / (unsigned)p.tt);   // token tiles of a row tile are neighbours: they share its weights in L2
+    t.n0 = r * MMQ_ROWS;
+    t.row0 = 0;
+    t.x0 = (tile - r * p.tt) * p.tn;
+    t.rows = p.m - t.x0 < p.tn ? p.m - t.x0 : p.tn;
+  }
+  return t;
+}
+// The stages of a part come in blocks: four per chunk, and behind every run of chunks with the same c / 8 one stage of their
+// correction columns (formats without them: one block).  End of the block that starts at chunk c:
+__device__ __forceinline__ int mmq_block_end(const MmqParams& p, const MmqPart& q, int c) {
+  const int e = (c | (MMQ_CORR_CHUNKS - 1)) + 1;
+  return p.corr && e < q.c1 ? e : q.c1;
+}
+__device__ __forceinline__ bool mmq_next_part(const MmqParams& p, MmqPart& q) {
+  if (q.u >= q.u1) return false;
+  q.tile = (int)((unsigned)q.u / (unsigned)p.nc);
+  q.c0 = q.u - q.tile * p.nc;
+  q.c1 = q.u1 - q.u < p.nc - q.c0 ? q.c0 + (q.u1 - q.u) : p.nc;
+  q.u += q.c1 - q.c0;
+  return true;
+}
+
+// bits of v in a 16-bit output type
+__device__ __forceinline__ uint16_t mmq_bits16(int dtype, float v) {
+  return dtype == DT_F16 ? __half_as_ushort(__float2half_rn(v)) : __bfloat16_as_ushort(__float2bfloat16_rn(v));
+}
+// one value of an output row in the forms that are not the usual one: fp32, or this rank's column block of every rank's matrix
+__device__ __forceinline__ void mmq_store(const MmqParams& p, int64_t orow, int n, float v, float scale) {
+  if (p.tp_world > 0) {
+    const int64_t at = orow * p.ldy + p.tp_col_off + n;
+    for (int rk = 0; rk < p.tp_world; ++rk) {
+      if (p.dtype == DT_F32) static_cast<float*>(p.tp_y[rk])[at] = v;
+      else static_cast<uint16_t*>(p.tp_y[rk])[at] = mmq_bits16(p.dtype, v);
+    }
+  } else {
+    static_cast<float*>(p.y)[orow * p.ldy + n] = p.row_scale ? v * scale : v;
+  }
+}
+
+template <int TYPE, typename ab_t, bool FAST>
+__global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_constant__ CUtensorMap bmap, const __grid_constant__ CUtensorMap wmap,
+                                                             const __grid_constant__ MmqParams p) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));   // swizzle atoms
+  using Dec = Decoder<TYPE, ab_t>;
+  const int b_stage = p.tn * MMQ_BK * 2;
+  uint8_t* sB = smem;
+  uint8_t* sRaw = smem + p.raw_off;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + p.aux_off);
+  uint64_t* full = bars;                     // [8] stage i % 8: A slot and activation box filled: the four warps of a group + the B loader
+  uint64_t* empty = bars + 8;                // [8] the MMAs that read them are done
+  uint64_t* corr_full = bars + 16;           // every warp's correction values of a block of chunks are in shared memory
+  uint64_t* corr_free = bars + 17;           // ... and have been taken out
+  uint64_t* accum = bars + 24;               // [2] an accumulator is complete
+  uint64_t* drained = bars + 26;             // [2] ... and has been read
+  uint64_t* raw_full = bars + 28;            // [8]
+  uint64_t* raw_empty = bars + 36;           // [8] read by the two groups that decode it
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 44);
+  volatile int* gave_up = reinterpret_cast<volatile int*>(tmem_slot + 1);   // set by any thread whose wait ran out
+  volatile int* s_flag = gave_up + 1;        // [2]: the last to arrive at the tile of the part just read out / of the CTA's first part
+  uint8_t* s_tab = smem + p.aux_off + 512;   // decoder tables
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < MMQ_BARS; ++s) {
+      mbar_init(&full[s], MMQ_PRODUCER_WARPS / MMQ_GROUPS + 1);
+      mbar_init(&empty[s], 1);
+    }
+    mbar_init(corr_full, MMQ_PRODUCER_WARPS);
+    mbar_init(corr_free, MMQ_PRODUCER_WARPS / MMQ_GROUPS);
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(&accum[s], 1);
+      mbar_init(&drained[s], MMQ_PRODUCER_WARPS);
+    }
+    for (int s = 0; s < MMQ_MAX_RAW; ++s) {
+      mbar_init(&raw_full[s], 1);
+      mbar_init(&raw_empty[s], MMQ_PRODUCER_WARPS / 2);
+    }
+    *gave_up = 0;
+    fence_barrier_init();
+  }
+  decoder_fill_tables<TYPE>(s_tab);
+  if (warp == MMQ_PRODUCER_WARPS) {
+    tmem_alloc(tmem_slot, 512);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  pdl_trigger();   // the next kernel may become resident; it waits for this one before it touches anything
+  // What earlier kernels write: the activations (and the work list of a MoE step), and -- cleared, or read until now -- what the
+  // epilogue writes.  Everything else, decoding included, starts before they are done.
+  const bool moe = p.passes != nullptr;
+  if (moe) pdl_wait();
+  const int tiles = moe ? *p.n_passes * p.rt : p.rt * p.tt;
+  // Units: (tile, chunk) where CTAs share tiles, whole tiles where they do not -- there is no room for parts, or the last wave
+  // of whole tiles idles for less than sharing costs.  Every CTA in use has an equal contiguous range of them.
+  const int rest = tiles % (int)gridDim.x;
+  const bool split = p.part && rest != 0 && (unsigned)p.nc * (unsigned)((int)gridDim.x - rest) > (unsigned)p.waste * gridDim.x;
+  const int U = split ? tiles * p.nc : tiles, G = U < (int)gridDim.x ? U : (int)gridDim.x;
+  MmqPart q{};
+  const int cta = (int)blockIdx.x;
+  {
+    const int scale = split ? 1 : p.nc;
+    q.u = cta < G ? (int)((unsigned)(cta * U) / (unsigned)G) * scale : 0;
+    q.u1 = cta < G ? (int)((unsigned)((cta + 1) * U) / (unsigned)G) * scale : 0;
+  }
+  const int first_tile = (int)((unsigned)q.u / (unsigned)p.nc);
+  const int half_n = p.tn > 256 ? p.tn / 2 : 0;   // tokens of one instruction and of one activation box, where a tile takes two
+  bool ok = true;
+
+  if (warp < MMQ_PRODUCER_WARPS) {
+    // ---------------- producers and epilogue ----------------
+    // The work of a part, in order: two items per chunk (a half, 128 values, two stages) and one per block of corrections (one
+    // stage).  Group g takes the items g, g + 4, ... (counted over the whole life of the CTA); thread r of the group decodes
+    // row n0 + r.  Stage i goes to A slot i modulo their number.  The tile before is read out after every group has published
+    // its first item of the next one, so that the tensor core has eight stages of work while the accumulator goes to memory.
+    const int r = threadIdx.x & 127, g = threadIdx.x >> 7;
+    const DecodeCtx cx = decoder_context<TYPE>(s_tab, lane);
+    const int nunits = p.k / 32;
+    const uint32_t d_lane = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
+    const uint32_t a_lane = d_lane + (uint32_t)p.a_col0;
+    const uint32_t s_corr = smem_u32(smem + p.corr_off) + (uint32_t)(r * MMQ_CORR_ROW);
+    // (After a time-out the loops run on without waiting: every barrier still gets its arrivals, the result is invalid and the
+    // status word says so.)
+    auto wait = [&](uint64_t* bar, uint32_t parity) {
+      if (ok) ok = mbar_wait_bounded(bar, parity);
+      __syncwarp();
+    };
+    auto publish = [&](const uint32_t (&v)[32], int i) {   // wait until stage i's slot is free, store the row, signal the MMA warp
+      const int o = i - p.sa;   // the stage that had the slot before
+      if (o >= 0) wait(&empty[o & (MMQ_BARS - 1)], (uint32_t)(o >> 3) & 1u);
+      tc_fence_after();
+      tmem_st32(a_lane + (uint32_t)((i & (p.sa - 1)) * MMQ_A_COLS), v);
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&full[i & (MMQ_BARS - 1)]);
+    };
+    // Reads out part e, the pi-th of this CTA.  Kept short: this code runs two or three times in the life of a CTA, and fetching
+    // its instructions costs more than running them (unrolled over an accumulator held in 64 registers it took 10,000 clocks
+    // instead of 4,000, most of them for the first time through).  FINISH: the parts of e's tile are all in memory.
+    enum : int { MORE, FINAL, FINISH };
+    auto epilogue = [&](const MmqPart& e, int pi, int mode) {
+      const MmqTile et = mmq_tile(p, e.tile);
+      const int buf = p.nbuf == 2 ? pi & 1 : 0, use = p.nbuf == 2 ? pi >> 1 : pi;
+      const int n = et.n0 + r, nb = p.tn / 16;
+      const bool live = n < p.n;
+      const bool shared = e.c1 - e.c0 < p.nc;
+      // output rows (negative: none) and their weights, of the tokens this group reads: lanes 0..15 of each block of 16
+      auto out_row = [&](int b) {
+        const int t = 16 * b + (lane & 15);
+        int o = b < nb && t < et.rows ? et.x0 + t : -1;
+        if (moe && o >= 0) o = p.sorted[o];
+        return o < p.rows_out ? o : -1;
+      };
+      auto out_scale = [&](int o) { return p.row_scale && o >= 0 ? p.row_scale[o] : 1.f; };
+      int orow = out_row(g);
+      float scale = out_scale(orow);
+      if (mode != FINISH) {
+        wait(&accum[buf], (uint32_t)use & 1u);
+        tc_fence_after();
+        pdl_wait();
+      }
+      const uint32_t d = d_lane + (uint32_t)(buf * p.d_step);
+      int first = 0, last = 0, s_first = 0;
+      bool in_tmem = mode != FINISH;
+      const int slot4 = p.tn * 32;            // float4s of a partial tile
+      float4* part = reinterpret_cast<float4*>(p.part) + r;
+      if (shared) {
+        // The CTAs first .. last share the tile.  The last of them to arrive adds the parts in CTA order (deterministic).
+        const int ta = e.tile * p.nc;
+        first = (int)((unsigned)((ta + 1) * G - 1) / (unsigned)U);
+        last = (int)((unsigned)((ta + p.nc) * G - 1) / (unsigned)U);
+        s_first = 2 * first + ((unsigned)(first * U) / (unsigned)G >= (unsigned)ta ? 0 : 1);
+        if (mode != FINISH) {
+          if (mode == FINAL && e.c0 == 0) {   // the others did their parts first: if all are there, this one need not be published
+            if (threadIdx.x == 0) {
+              int seen;
+              asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(seen) : "l"(p.counter + e.tile) : "memory");
+              s_flag[0] = seen == last - first ? 2 : 0;
+            }
+            asm volatile("bar.sync 1, %0;" ::"n"(MMQ_PRODUCER_WARPS * 32) : "memory");
+            in_tmem = s_flag[0] == 2;
+          } else {
+            in_tmem = false;
+          }
+          if (!in_tmem) {
+            float4* out = part + (size_t)(2 * cta + (e.tile == first_tile ? 0 : 1)) * slot4;
+#pragma unroll 1
+            for (int b = g; b < nb; b += MMQ_GROUPS) {
+              uint32_t acc[16];
+              __syncwarp();
+              tmem_ld16(d + (uint32_t)(16 * b), acc);
+              tmem_ld_wait();
+#pragma unroll
+              for (int j = 0; j < 4; ++j)
+                __stcg(out + (4 * b + j) * 128, make_float4(__uint_as_float(acc[4 * j]), __uint_as_float(acc[4 * j + 1]),
+                                                            __uint_as_float(acc[4 * j + 2]), __uint_as_float(acc[4 * j + 3])));
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&drained[buf]);
+            asm volatile("bar.sync 1, %0;" ::"n"(MMQ_PRODUCER_WARPS * 32) : "memory");
+            if (threadIdx.x == 0) {
+              __threadfence();   // cumulative: covers what the barrier made visible to this thread
+              s_flag[mode == MORE ? 1 : 0] = atomicAdd(p.counter + e.tile, 1) == last - first ? 1 : 0;
+              __threadfence();
+            }
+            if (mode == MORE) return;
+            asm volatile("bar.sync 1, %0;" ::"n"(MMQ_PRODUCER_WARPS * 32) : "memory");
+            if (s_flag[0] == 0) return;
+          }
+        }
+      }
+      const bool plain = p.tp_world == 0 && p.dtype != DT_F32;
+#pragma unroll 1
+      for (int b = g; b < nb; b += MMQ_GROUPS) {
+        const int orow_next = out_row(b + MMQ_GROUPS);
+        uint32_t acc[16];
+        if (in_tmem) {
+          __syncwarp();
+          tmem_ld16(d + (uint32_t)(16 * b), acc);
+          tmem_ld_wait();
+        }
+        if (shared) {
+          if (!in_tmem) {   // (in tensor memory: only ever the part of the first CTA of the tile)
+#pragma unroll
+            for (int j = 0; j < 16; ++j) acc[j] = 0u;
+          }
+#pragma unroll 2
+          for (int c = in_tmem ? first + 1 : first; c <= last; ++c) {
+            const float4* in = part + (size_t)(c == first ? s_first : 2 * c) * slot4 + 4 * b * 128;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const float4 v = __ldcg(in + j * 128);
+              acc[4 * j] = __float_as_uint(__uint_as_float(acc[4 * j]) + v.x);
+              acc[4 * j + 1] = __float_as_uint(__uint_as_float(acc[4 * j + 1]) + v.y);
+              acc[4 * j + 2] = __float_as_uint(__uint_as_float(acc[4 * j + 2]) + v.z);
+              acc[4 * j + 3] = __float_as_uint(__uint_as_float(acc[4 * j + 3]) + v.w);
+            }
+          }
+        }
+        if (plain) {
+          uint16_t* y = static_cast<uint16_t*>(p.y) + n;
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            const int o = __shfl_sync(0xffffffffu, orow, j);
+            uint16_t v = mmq_bits16(p.dtype, __uint_as_float(acc[j]));
+            if (p.row_scale) {   // applied as the reference applies it: to the rounded value, rounded again
+              const float f = p.dtype == DT_F16 ? __half2float(__ushort_as_half(v)) : __bfloat162float(__ushort_as_bfloat16(v));
+              v = mmq_bits16(p.dtype, f * __shfl_sync(0xffffffffu, scale, j));
+            }
+            if (live && o >= 0) y[(int64_t)o * p.ldy] = v;
+          }
+        } else {
+#pragma unroll 1
+          for (int j = 0; j < 16; ++j) {
+            const int o = __shfl_sync(0xffffffffu, orow, j);
+            const float w = __shfl_sync(0xffffffffu, scale, j);
+            if (live && o >= 0) mmq_store(p, o, n, __uint_as_float(acc[0]), w);
+#pragma unroll
+            for (int k = 0; k < 15; ++k) acc[k] = acc[k + 1];   // (register indexes are static)
+          }
+        }
+        orow = orow_next;
+        scale = out_scale(orow);
+      }
+      if (in_tmem) {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&drained[buf]);
+      }
+    };
+
+    int t0 = 0, i0 = 0, pi = 0;  // first item and first stage of the block; parts so far
+    int rs0 = 0, nblk = 0;       // raw slot of the block's first chunk and its phase; blocks of corrections so far
+    uint32_t rph0 = 0;
+    MmqPart prev{}, head{};      // the part before, the CTA's first part
+    int mode = MORE;
+    constexpr int CI = Dec::CORR ? 1 : 0;
+    for (;;) {
+      const bool more = mode == MORE && mmq_next_part(p, q);
+      if (!more && mode == MORE) mode = FINAL;
+      const MmqTile qt = mmq_tile(p, q.tile);
+      const int n = qt.n0 + r;
+      const bool live = n < p.n;
+      const uint8_t* slot = sRaw + raw_slot(p.raw, r, qt.n0);
+      int cs = q.c0, ce = mmq_block_end(p, q, cs);
+      int m = (g - t0) & 3;      // this group's next item of the block
+      bool done = !more, read_out = pi > 0;
+      // On to the block that holds item m.  A group that is through with a block says so before it does anything else: the
+      // group that takes the corrections waits for it.
+      auto advance = [&]() {
+        while (!done && m >= 2 * (ce - cs) + CI) {
+          const int items = 2 * (ce - cs) + CI;
+          if constexpr (Dec::CORR) {
+            __syncwarp();
+            if (lane == 0 && m != items + 3) mbar_arrive(corr_full);   // (item items - 1 has arrived by itself)
+            ++nblk;
+          }
+          m -= items;
+          t0 += items;
+          i0 += 4 * (ce - cs) + CI;
+          rs0 += ce - cs;
+          if (rs0 >= p.raw_stages) {
+            const int laps = (int)((unsigned)rs0 / (unsigned)p.raw_stages);
+            rs0 -= laps * p.raw_stages;
+            rph0 ^= (uint32_t)laps & 1u;
+          }
+          cs = ce;
+          if (cs >= q.c1) done = true;
+          else ce = mmq_block_end(p, q, cs);
+        }
+      };
+      // With one accumulator and four slots the first items of groups two and three have no room before the tile is read out.
+      bool hold = read_out && p.nbuf == 1 && 2 * m >= p.sa;
+      advance();
+      for (;;) {
+        if (!done && !hold) {
+          // this block's corrections may be written, and its arrivals counted, once the block before has been taken out
+          if constexpr (Dec::CORR) wait(corr_free, ((uint32_t)nblk & 1u) ^ 1u);
+          if (!Dec::CORR || m < 2 * (ce - cs)) {
+            const int k = m >> 1, half = m & 1;
+            int rs = rs0 + k;
+            uint32_t rph = rph0;
+            while (rs >= p.raw_stages) { rs -= p.raw_stages; rph ^= 1u; }
+            wait(&raw_full[rs], rph);
+            const uint8_t* chunk = slot + rs * p.raw.bytes + (FAST ? 0u : raw_shift(p.raw, n, qt.row0, cs + k));
+            if constexpr (Dec::CORR) {
+              const uint2 cv = live ? Dec::corr(chunk, half, nunits - 8 * (cs + k)) : make_uint2(0u, 0u);
+              asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(s_corr + (uint32_t)(16 * ((cs + k) & (MMQ_CORR_CHUNKS - 1)) + 8 * half)), "r"(cv.x), "r"(cv.y) : "memory");
+            }
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              const int s2 = 2 * half + h;      // 64-value stage of the chunk
+              uint32_t v[32];
+              if constexpr (FAST) {
+                Stage64<TYPE, ab_t>::decode(chunk, s2, v);
+              } else {
+                const int u = 2 * s2;           // units (32 values) u, u + 1 of the chunk
+                const int left = nunits - 8 * (cs + k) - u;
+                uint32_t (&v0)[16] = *reinterpret_cast<uint32_t (*)[16]>(&v[0]);
+                uint32_t (&v1)[16] = *reinterpret_cast<uint32_t (*)[16]>(&v[16]);
+                uint32_t raw[Dec::RW];
+                if (live && left > 0) {
+                  Dec::load(chunk, u, raw);
+                  Dec::decode(chunk, u, raw, cx, v0);
+                } else {
+#pragma unroll
+                  for (int j = 0; j < 32; ++j) v[j] = 0;
+                }
+                if (live && left > 1) {
+                  if constexpr (!decoder_pair_load<TYPE>()) Dec::load(chunk, u + 1, raw);   // (one load serves both)
+                  Dec::decode(chunk, u + 1, raw, cx, v1);
+                } else {
+#pragma unroll
+                  for (int j = 0; j < 16; ++j) v1[j] = 0;
+                }
+              }
+              if (h == 1) {   // this warp is done reading the raw chunk: hand the slot back to the loader
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&raw_empty[rs]);
+              }
+              publish(v, i0 + 2 * m + h);
+            }
+          } else if constexpr (Dec::CORR) {
+            // the block's corrections: every warp's values are in, zeros for the chunks that other parts have
+            __syncwarp();
+            if (lane == 0) mbar_arrive(corr_full);
+            wait(corr_full, (uint32_t)nblk & 1u);
+            uint32_t v[32];
+#pragma unroll
+            for (int c = 0; c < MMQ_CORR_CHUNKS; ++c) {
+              const uint4 x = lds128s(s_corr + 16 * c);
+              const bool have = c >= (cs & (MMQ_CORR_CHUNKS - 1)) && c <= ((ce - 1) & (MMQ_CORR_CHUNKS - 1));
+              v[4 * c] = have ? x.x : 0u; v[4 * c + 1] = have ? x.y : 0u; v[4 * c + 2] = have ? x.z : 0u; v[4 * c + 3] = have ? x.w : 0u;
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(corr_free);
+            publish(v, i0 + 2 * m);
+          }
+          m += 4;
+          advance();
+        }
+        if (read_out) {
+          epilogue(prev, pi - 1, mode);
+          read_out = false;
+        }
+        if (done) break;
+        hold = false;
+      }
+      if (!more) {
+        if (mode == FINISH || head.c1 - head.c0 == p.nc || pi < 2) break;
+        asm volatile("bar.sync 1, %0;" ::"n"(MMQ_PRODUCER_WARPS * 32) : "memory");
+        if (s_flag[1] == 0) break;
+        mode = FINISH;           // the first part's tile fell to this CTA after all: once more, for it
+        prev = head;
+        continue;
+      }
+      if (pi == 0) head = q;
+      prev = q;
+      ++pi;
+    }
+  } else if (warp == MMQ_PRODUCER_WARPS) {
+    // ---------------- B loader: one TMA box (64 k x tn rows; two beyond 256) per stage ----------------
+    if (lane == 0) {
+      int i = 0, sb = 0;
+      pdl_wait();
+      while (ok && mmq_next_part(p, q)) {
+        const int x0 = mmq_tile(p, q.tile).x0;
+        for (int cs = q.c0, ce; ok && cs < q.c1; cs = ce) {
+          ce = mmq_block_end(p, q, cs);
+          const int nmain = 4 * (ce - cs), corr_col = p.kpad + cs / MMQ_CORR_CHUNKS * MMQ_BK;
+          for (int j = 0; j < nmain + p.corr; ++j, ++i) {
+            // B slot i % sb held stage i - sb: wait for that stage's commit
+            const int o = i - p.sb;
+            if (o >= 0 && !mbar_wait_bounded(&empty[o & (MMQ_BARS - 1)], (uint32_t)(o >> 3) & 1u)) { ok = false; break; }
+            uint64_t* fb = &full[i & (MMQ_BARS - 1)];
+            const int col = j < nmain ? cs * RAW_KC + j * MMQ_BK : corr_col;
+            mbar_expect_tx(fb, (uint32_t)b_stage);
+            raw_tma_box(sB + (size_t)sb * b_stage, &bmap, col, x0, fb);
+            if (half_n) raw_tma_box(sB + (size_t)sb * b_stage + half_n * (MMQ_BK * 2), &bmap, col, x0 + half_n, fb);
+            if (++sb == p.sb) sb = 0;
+          }
+        }
+      }
+    }
+  } else if (warp == MMQ_PRODUCER_WARPS + 2) {
+    // ---------------- raw-weight loader ----------------
+    int st = 0;
+    uint32_t sph = 0;
+    while (ok && mmq_next_part(p, q)) {
+      const MmqTile qt = mmq_tile(p, q.tile);
+      for (int c = q.c0; c < q.c1; ++c) {
+        if (!mbar_wait_bounded(&raw_empty[st], sph ^ 1u)) { ok = false; break; }
+        raw_issue(p.raw, &wmap, p.w, p.w_bytes, qt.row0, qt.n0, c, sRaw + (size_t)st * p.raw.bytes, &raw_full[st], 0u, lane);
+        __syncwarp();
+        if (++st == p.raw_stages) { st = 0; sph ^= 1u; }
+      }
+    }
+  } else {
+    // ---------------- MMA issuer ----------------
+    // One lane issues everything.  (Its loop is short: it shares its scheduler with four producer warps.)
+    if (elect_one()) {
+      int i = 0, sb = 0, pi = 0;
+      const uint64_t bd0 = umma_desc_sw128(smem_u32(sB));
+      const uint32_t b_step = (uint32_t)(b_stage >> 4), b_lo0 = (uint32_t)bd0, b_hi = (uint32_t)(bd0 >> 32);
+      uint32_t b_lo = b_lo0;
+      while (ok && mmq_next_part(p, q)) {
+        int end = i + 4 * (q.c1 - q.c0);
+        if (p.corr) end += (q.c1 - 1) / MMQ_CORR_CHUNKS - q.c0 / MMQ_CORR_CHUNKS + 1;
+        const int buf = p.nbuf == 2 ? pi & 1 : 0, use = p.nbuf == 2 ? pi >> 1 : pi;
+        ok = mbar_wait_bounded(&drained[buf], ((uint32_t)use & 1u) ^ 1u);
+        const uint32_t d = tmem_base + (uint32_t)(buf * p.d_step);
+        uint32_t accumulate = 0;
+        for (; ok && i < end; ++i) {
+          const int s = i & (MMQ_BARS - 1);
+          ok = mbar_wait_bounded(&full[s], (uint32_t)(i >> 3) & 1u);
+          tc_fence_after();
+          const uint32_t at = tmem_base + (uint32_t)(p.a_col0 + (i & (p.sa - 1)) * MMQ_A_COLS);
+          uint32_t dh = d, bh = b_lo;
+#pragma unroll 1
+          for (int h = half_n > 0 ? 1 : 0; h >= 0; --h) {
+#pragma unroll
+            for (int kk = 0; kk < MMQ_BK / 16; ++kk)  // 16 values = 8 columns of A, 32 bytes of B = +2 in the descriptor's 16-byte units
+              umma_f16_ts(dh, at + 8 * kk, bh + 2 * kk, b_hi, p.idesc, kk == 0 ? accumulate : 1u);
+            dh += (uint32_t)half_n;
+            bh += (uint32_t)(half_n * (MMQ_BK * 2) >> 4);
+          }
+          accumulate = 1;
+          umma_commit(&empty[s]);
+          b_lo += b_step;
+          if (++sb == p.sb) { sb = 0; b_lo = b_lo0; }
+        }
+        // committed in every case: the accumulator's barrier then completes once every tcgen05.mma issued so far has finished
+        umma_commit(&accum[buf]);
+        ++pi;
+      }
+    }
+    __syncwarp();
+  }
+  if (!ok) {   // (any lane)
+    atomicExch(p.status, E_TIMEOUT);
+    *gave_up = 1;
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (*gave_up) {
+    // A bounded wait ran out somewhere in this CTA (the result is invalid and the status word says so).  Before the tensor
+    // memory is released and the CTA retires, everything it started must have finished: the commit below covers the tensor
+    // pipe (bounded wait on a barrier nobody else uses any more), and the copies still in flight depend on nothing and land
+    // within microseconds, so a pause far longer than their latency covers them.  Nothing here can wait for ever.
+    if (warp == MMQ_PRODUCER_WARPS + 1) {
+      uint64_t* end = bars + 48;
+      if (lane == 0) mbar_init(end, 1);
+      __syncwarp();
+      if (elect_one()) umma_commit(end);
+      __syncwarp();
+      mbar_wait_bounded(end, 0);
+    }
+    drain_pause();
+    tc_fence_before();
+    __syncthreads();
+  }
+  if (warp == MMQ_PRODUCER_WARPS) tmem_dealloc(tmem_base, 512);
+  if (p.tp_world > 0) tp_finish(p.tp_epoch, p.tp_flag, p.tp_world, p.tp_slot, gridDim.x);
+}
+
+template <int TYPE, typename ab_t, bool FAST>
+static int mmq_launch_form(const MmqParams& p, const CUtensorMap& bmap, const CUtensorMap& wmap, int grid, size_t smem, cudaStream_t stream) {
+  auto kern = mmq_kernel<TYPE, ab_t, FAST>;
+  static bool configured[64] = {false};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (!configured[dev & 63]) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess) return E_CUDA;
+    configured[dev & 63] = true;
+  }
+  return launch_pdl(kern, dim3((unsigned)grid), dim3(MMQ_THREADS), smem, stream, bmap, wmap, p) == cudaSuccess ? E_OK : E_CUDA;
+}
+// ab: element type of the activation matrix (DT_F16, DT_BF16); fast: whole-stage decoder on dense boxes
+template <int TYPE> int mmq_launch(const MmqParams& p, const CUtensorMap& bmap, const CUtensorMap& wmap, int ab, bool fast, int grid, size_t smem,
+                                   cudaStream_t stream) {
+  if constexpr (Stage64<TYPE, __half>::FAST) {
+    if (fast) return ab == DT_F16 ? mmq_launch_form<TYPE, __half, true>(p, bmap, wmap, grid, smem, stream) : E_BAD_DTYPE;
+  }
+  if (fast) return E_BAD_SHAPE;
+  if constexpr (decoder_bf16<TYPE>()) {
+    if (ab == DT_BF16) return mmq_launch_form<TYPE, __nv_bfloat16, false>(p, bmap, wmap, grid, smem, stream);
+  }
+  return ab == DT_F16 ? mmq_launch_form<TYPE, __half, false>(p, bmap, wmap, grid, smem, stream) : E_BAD_DTYPE;
+}
+}  // namespace gguf_b200

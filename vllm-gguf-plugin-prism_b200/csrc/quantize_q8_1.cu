@@ -138,9 +138,12 @@ template <typename in_t>
 __global__ void __launch_bounds__(256) quantize_f16x8_kernel(const in_t* __restrict__ x, __half* __restrict__ xb, int64_t M, int64_t K,
                                                              int64_t kpad, int64_t ldb, int corr_mode, int perm,
                                                              const int32_t* __restrict__ gather_ids, int64_t gather_div,
-                                                             int64_t gather_limit, int act, int64_t x_ld) {
+                                                             int64_t gather_limit, int act, int64_t x_ld, int* __restrict__ zero,
+                                                             int64_t n_zero, const int32_t* __restrict__ n_used) {
   pdl_trigger();
   pdl_wait();
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_zero; i += (int64_t)gridDim.x * blockDim.x) zero[i] = 0;
+  if (n_used && n_used[1] < M) M = n_used[1];
   const int lane = threadIdx.x & 31, t = lane & 3;
   const int64_t nbr = kpad / 32;                                   // blocks per row
   const int64_t total = M * nbr;                                   // blocks in all
@@ -377,7 +380,8 @@ static int launch_mode(const void* x, int x_dtype, void* out, int64_t M, int64_t
 }
 
 static int launch_f16x8(const void* x, int x_dtype, void* out, int64_t M, int64_t K, int64_t ldb, int corr_mode, int perm,
-                        const int32_t* gid, int64_t gdiv, int64_t glim, cudaStream_t stream, int act, int64_t x_ld) {
+                        const int32_t* gid, int64_t gdiv, int64_t glim, cudaStream_t stream, int act, int64_t x_ld, int* zero, int64_t n_zero,
+                        const int32_t* n_used) {
   if (M <= 0 || K <= 0) return M < 0 || K < 0 ? E_BAD_SHAPE : E_OK;
   const int64_t kpad = round_up(K, 512);
   const int64_t total = M * (kpad / 32);
@@ -386,13 +390,13 @@ static int launch_f16x8(const void* x, int x_dtype, void* out, int64_t M, int64_
   __half* o = static_cast<__half*>(out);
   switch (x_dtype) {
     case DT_F32:
-      launch_pdl(quantize_f16x8_kernel<float>, dim3(blocks), dim3(256), 0, stream, (const float*)x, o, M, K, kpad, ldb, corr_mode, perm, gid, gdiv, glim, act, x_ld);
+      launch_pdl(quantize_f16x8_kernel<float>, dim3(blocks), dim3(256), 0, stream, (const float*)x, o, M, K, kpad, ldb, corr_mode, perm, gid, gdiv, glim, act, x_ld, zero, n_zero, n_used);
       break;
     case DT_F16:
-      launch_pdl(quantize_f16x8_kernel<__half>, dim3(blocks), dim3(256), 0, stream, (const __half*)x, o, M, K, kpad, ldb, corr_mode, perm, gid, gdiv, glim, act, x_ld);
+      launch_pdl(quantize_f16x8_kernel<__half>, dim3(blocks), dim3(256), 0, stream, (const __half*)x, o, M, K, kpad, ldb, corr_mode, perm, gid, gdiv, glim, act, x_ld, zero, n_zero, n_used);
       break;
     case DT_BF16:
-      launch_pdl(quantize_f16x8_kernel<__nv_bfloat16>, dim3(blocks), dim3(256), 0, stream, (const __nv_bfloat16*)x, o, M, K, kpad, ldb, corr_mode, perm, gid, gdiv, glim, act, x_ld);
+      launch_pdl(quantize_f16x8_kernel<__nv_bfloat16>, dim3(blocks), dim3(256), 0, stream, (const __nv_bfloat16*)x, o, M, K, kpad, ldb, corr_mode, perm, gid, gdiv, glim, act, x_ld, zero, n_zero, n_used);
       break;
     default:
       return E_BAD_DTYPE;
@@ -402,12 +406,14 @@ static int launch_f16x8(const void* x, int x_dtype, void* out, int64_t M, int64_
 
 int launch_quantize_q8_1(const void* x, int x_dtype, void* out, int64_t M, int64_t K, int mode, int sum_mode,
                          int64_t ldb, int corr_mode, const int32_t* gather_ids, int64_t gather_div, int64_t gather_limit,
-                         cudaStream_t stream, int perm, const Q8Tp* wait, int act, int64_t x_ld) {
+                         cudaStream_t stream, int perm, const Q8Tp* wait, int act, int64_t x_ld, int* zero, int64_t n_zero,
+                         const int32_t* n_used) {
   if (mode == Q8_MODE_F16) {
     // rows of x and of the output start on 16-byte boundaries when K and ldb are multiples of 8
     const bool aligned = K % 8 == 0 && ldb % 8 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
-    if (aligned) return launch_f16x8(x, x_dtype, out, M, K, ldb, corr_mode, perm, gather_ids, gather_div, gather_limit, stream, act, x_ld);
-    if (perm || act) return E_BAD_POINTER;
+    if (aligned) return launch_f16x8(x, x_dtype, out, M, K, ldb, corr_mode, perm, gather_ids, gather_div, gather_limit, stream, act, x_ld, zero, n_zero, n_used);
+    if (perm || act || n_used) return E_BAD_POINTER;
+    if (n_zero > 0 && launch_zero(zero, n_zero, stream)) return E_CUDA;
   } else if (act) {
     return E_BAD_SHAPE;
   }

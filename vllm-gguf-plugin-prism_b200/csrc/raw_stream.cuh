@@ -35,6 +35,7 @@ struct RawPlan {
   int nrows, nfull;        // rows of a matrix, and how many of them the map covers
   int64_t pitch;           // bytes between weight rows
   int64_t row_bytes;       // bytes of a row that hold values
+  int64_t gap;             // rows form: bytes between one matrix of nrows rows and the next
 };
 
 __device__ __forceinline__ void raw_tma_box(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
@@ -44,23 +45,27 @@ __device__ __forceinline__ void raw_tma_box(void* dst, const CUtensorMap* map, i
       : "memory");
 }
 
-// offset, inside a stage, of the chunk c of row r of the tile that starts at row n0 of the matrix (whose first row is row
-// `row0` of all matrices)
-__device__ __forceinline__ uint32_t raw_offset(const RawPlan& p, int r, int n0, int row0, int c) {
-  if (p.mode == 1) return (uint32_t)(r * p.slot);
+// Offset, inside a stage, of row r of the tile that starts at row n0 of the matrix (whose first row is row `row0` of all
+// matrices): where its slot starts, and by how much its chunk c is displaced in it.
+__device__ __forceinline__ uint32_t raw_slot(const RawPlan& p, int r, int n0) {
+  if (p.mode != 2) return (uint32_t)(r * p.slot);
   const int n = n0 + r;
-  const uint32_t rem = ((uint32_t)(row0 + n) * (uint32_t)p.pitch + (uint32_t)c * (uint32_t)p.rbc) & 15u;
-  if (p.mode == 0) return (uint32_t)(r * p.slot) + rem;
   const int s = n >= p.nfull && n < p.nrows ? RAW_ROWS + (n - p.nfull) : ((r & ((1 << p.cl2) - 1)) << (7 - p.cl2)) | (r >> p.cl2);
-  return (uint32_t)(s * p.slot) + rem;
+  return (uint32_t)(s * p.slot);
+}
+__device__ __forceinline__ uint32_t raw_shift(const RawPlan& p, int n, int row0, int c) {
+  if (p.mode == 1) return 0u;
+  uint32_t at = (uint32_t)(row0 + n) * (uint32_t)p.pitch + (uint32_t)c * (uint32_t)p.rbc;
+  if (p.gap != 0) at += ((uint32_t)row0 / (uint32_t)p.nrows) * (uint32_t)p.gap;
+  return at & 15u;
 }
 
 // One row's chunk by a bulk copy into `dst`, from its address rounded down to 16 bytes; the bytes of the buffer's ragged end
 // with plain loads.  Split in two so that the byte count is announced before the copy starts.
 struct RawCopy { int64_t beg; uint32_t bytes; };
-__device__ __forceinline__ RawCopy raw_row_copy(const RawPlan& p, const uint8_t* w, int64_t w_bytes, int64_t n, int c, uint8_t* dst) {
-  const int64_t beg = n * p.pitch + (int64_t)c * p.rbc;
-  const int64_t row_end = n * p.pitch + p.row_bytes;
+__device__ __forceinline__ RawCopy raw_row_copy(const RawPlan& p, const uint8_t* w, int64_t w_bytes, int64_t row, int c, uint8_t* dst) {
+  const int64_t beg = row + (int64_t)c * p.rbc;
+  const int64_t row_end = row + p.row_bytes;
   const int64_t end = beg + p.rbc < row_end ? beg + p.rbc : row_end;
   const int64_t safe = w_bytes & ~int64_t(15), a0 = beg & ~int64_t(15);
   int64_t a1 = (end + 15) & ~int64_t(15);
@@ -88,7 +93,7 @@ __device__ __forceinline__ void raw_issue(const RawPlan& p, const CUtensorMap* m
     const bool tail = n0 + RAW_ROWS > p.nfull && p.nfull < p.nrows;
     if (tail) {
       const int n = p.nfull + lane;
-      if (n < p.nrows) rc = raw_row_copy(p, w, w_bytes, (int64_t)row0 + n, c, stage + (size_t)(RAW_ROWS + lane) * p.slot);
+      if (n < p.nrows) rc = raw_row_copy(p, w, w_bytes, ((int64_t)row0 + n) * p.pitch, c, stage + (size_t)(RAW_ROWS + lane) * p.slot);
       uint32_t sum = rc.bytes;
 #pragma unroll
       for (int m = 1; m < 8; m <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, m);   // (the tail has at most seven rows: lanes 0..7)
@@ -110,10 +115,12 @@ __device__ __forceinline__ void raw_issue(const RawPlan& p, const CUtensorMap* m
   }
   RawCopy rc[4];
   uint32_t total = 0;
+  int64_t row = ((int64_t)row0 + n0 + lane) * p.pitch;
+  if (p.gap != 0) row += (int64_t)((unsigned)row0 / (unsigned)p.nrows) * p.gap;
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
     const int r = lane + 32 * q;
-    rc[q] = n0 + r < p.nrows ? raw_row_copy(p, w, w_bytes, (int64_t)row0 + n0 + r, c, stage + (size_t)r * p.slot) : RawCopy{0, 0u};
+    rc[q] = n0 + r < p.nrows ? raw_row_copy(p, w, w_bytes, row + 32 * q * p.pitch, c, stage + (size_t)r * p.slot) : RawCopy{0, 0u};
     total += rc[q].bytes;
   }
 #pragma unroll
@@ -139,8 +146,14 @@ inline int raw_type_align(int type) {
   return 2;
 }
 
-// Host: the plan and (dense, class) the tensor map of a matrix of n_rows rows, `copies` such matrices back to back (experts).
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+EncodeTiledFn tensor_map_encoder();
+
+// Host: whether a matrix takes the dense form; the plan and (dense, class) the tensor map of a matrix of n_rows rows, `copies` such matrices (experts), `gap` bytes apart.
 // False when the layout is outside what the decoders can read.
-bool plan_raw(int type, const void* w, int64_t n_rows, int64_t copies, int64_t K, int64_t pitch, RawPlan& p, CUtensorMap& map);
+bool raw_dense(int type, int64_t K, int64_t pitch);
+bool plan_raw(int type, const void* w, int64_t n_rows, int64_t copies, int64_t K, int64_t pitch, RawPlan& p, CUtensorMap& map, int64_t gap = 0);
 
 }  // namespace gguf_b200

@@ -26,56 +26,6 @@ namespace gguf_b200 {
   X(T_IQ2_S) X(T_IQ3_XXS) X(T_IQ3_S) X(T_IQ1_S) X(T_IQ1_M) X(T_IQ4_NL) X(T_IQ4_XS)
 SM_TYPES(SM_EXTERN)
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-static EncodeTiledFn encode_fn() {
-  static EncodeTiledFn fn = [] {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    return cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess
-               ? reinterpret_cast<EncodeTiledFn>(p)
-               : nullptr;
-  }();
-  return fn;
-}
-
-bool plan_raw(int type, const void* w, int64_t n_rows, int64_t copies, int64_t K, int64_t pitch, RawPlan& p, CUtensorMap& map) {
-  const int qk = block_size(type), ts = type_size(type);
-  p = RawPlan{};
-  p.pitch = pitch;
-  p.row_bytes = K / qk * ts;
-  p.rbc = RAW_KC / qk * ts;
-  p.nrows = p.nfull = (int)n_rows;
-  if (pitch % raw_type_align(type) != 0 || pitch < p.row_bytes) return false;
-  const int s16 = (p.rbc + 30) / 16 + 1;
-  p.slot = (s16 % 2 ? s16 : s16 + 1) * 16;
-  EncodeTiledFn enc = encode_fn();
-  const cuuint32_t estr[2] = {1, 1};
-  auto encode = [&](int64_t row, int64_t rows, int box0, int box1) {
-    const cuuint64_t wd[2] = {(cuuint64_t)(row / 4), (cuuint64_t)rows};
-    const cuuint64_t ws[1] = {(cuuint64_t)row};
-    const cuuint32_t wb[2] = {(cuuint32_t)(box0 / 4), (cuuint32_t)box1};
-    return enc && enc(&map, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<void*>(w), wd, ws, wb, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                      CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-  };
-  int cl = 0;
-  while (((pitch << cl) & 15) != 0) ++cl;
-  if (p.rbc % 16 == 0 && cl == 0 && encode(pitch, n_rows * copies, p.rbc, RAW_ROWS)) {
-    p.mode = 1;
-    p.slot = p.rbc;
-  } else {
-    const int64_t covered = n_rows >> cl << cl;
-    if (covered > 0 && (covered == n_rows || copies == 1) && encode(pitch << cl, (covered >> cl) * copies, p.slot, RAW_ROWS >> cl)) {
-      p.mode = 2;
-      p.cl2 = cl;
-      p.nfull = (int)covered;
-    }
-  }
-  p.bytes = (int)round_up((int64_t)(RAW_ROWS + (p.nfull < p.nrows ? RAW_EXTRA : 0)) * p.slot, 128);
-  return true;
-}
-
 // Column tiles per CTA pass; the kernel is compiled for 1, 2 and 4.
 static int sm_t(int tiles) { return tiles <= 1 ? 1 : tiles <= 2 ? 2 : 4; }
 int smallm_max_tokens() { return 32; }

@@ -237,6 +237,7 @@ __global__ void __launch_bounds__(SM_THREADS, 2) smallm_kernel(const __grid_cons
       nt = pi.z;
     }
     const int n0 = r * RAW_ROWS;
+    const uint32_t slot_lo = raw_slot(p.raw, r_lo, n0), slot_hi = raw_slot(p.raw, r_hi, n0);
     float acc[T][4];
 #pragma unroll
     for (int i = 0; i < T; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
@@ -246,7 +247,7 @@ __global__ void __launch_bounds__(SM_THREADS, 2) smallm_kernel(const __grid_cons
         ok = false;   // keep the barrier protocol of the CTA going; the result is invalid and the status says so
       }
       const uint32_t base = sm_fresh(ring_s + (uint32_t)(st * p.stage_bytes));
-      const uint32_t ra = base + raw_offset(p.raw, r_lo, n0, row0, c), rb = base + raw_offset(p.raw, r_hi, n0, row0, c);
+      const uint32_t ra = base + slot_lo + raw_shift(p.raw, n0 + r_lo, row0, c), rb = base + slot_hi + raw_shift(p.raw, n0 + r_hi, row0, c);
       const uint32_t xt = base + (uint32_t)p.raw.bytes, xb = xt + 8u * lane, xd = xt + SM_CODE_BYTES + 16u * t;
       const int left = PARTIAL ? p.nblk - 8 * c : 8;
       if (ok) {

@@ -163,7 +163,7 @@ Tensor ggml_moe_a8(const Tensor& X, const Tensor& W, const Tensor& sorted_token_
               "ggml_moe_a8: sorted_token_ids/expert_ids were not built with block size ggml_moe_get_block_size(type)");
   const int code = dtype_code(X.scalar_type(), "ggml_moe_a8");
   Tensor Y = new_tensor({tokens * top_k, row}, X.scalar_type(), X.device());  // zeroed by the C-ABI call
-  const int64_t ws_bytes = gguf_b200_workspace_bytes(GGUF_B200_OP_MOE, (int)type, n_sorted, row, K);
+  const int64_t ws_bytes = gguf_b200_scratch_bytes(GGUF_B200_OP_MOE, (int)type, n_sorted, row, K);
   const Scratch ws(ws_bytes);
   check_rc(gguf_b200_moe_a8(X.data_ptr(), W.data_ptr(), Y.data_ptr(), ws.get(), ws_bytes,
                             static_cast<const int32_t*>(sorted_token_ids.data_ptr()), static_cast<const int32_t*>(expert_ids.data_ptr()),
@@ -310,7 +310,7 @@ int linear_op(int64_t type, int64_t M, int64_t N, ScalarType dt) {
   const int64_t most = im ? (N > 5120 ? 8 : 16) : (N > 5120 ? 2 : 6);
   if (M <= most) return GGUF_B200_OP_GEMV;
   if (!im) return GGUF_B200_OP_MMQ;
-  const bool fused = (type == 16 || type == 20 || type == 23) && (dt == ScalarType::Half || dt == ScalarType::BFloat16);
+  const bool fused = dt == ScalarType::Half || dt == ScalarType::BFloat16;
   return fused ? GGUF_B200_OP_DEQUANT_MATMUL : -1;
 }
 

@@ -26,7 +26,7 @@ OUT = PKG / "vllm_gguf_plugin"
 OBJ = PKG / "build"
 CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-CU_FILES = ["capi.cu", "quantize_q8_1.cu", "dequantize.cu", "gemv.cu", "gemv1.cu", "smallm.cu", "smallm_inst_a.cu", "smallm_inst_b.cu", "smallm_inst_c.cu", "mmq.cu", "noalloc.cu", "tp.cu", "moe_fused.cu"]
+CU_FILES = ["capi.cu", "quantize_q8_1.cu", "dequantize.cu", "gemv.cu", "gemv1.cu", "smallm.cu", "smallm_inst_a.cu", "smallm_inst_b.cu", "smallm_inst_c.cu", "raw_stream.cu", "mmq.cu", "mmq_inst_a.cu", "mmq_inst_b.cu", "mmq_inst_c.cu", "mmq_inst_d.cu", "noalloc.cu", "tp.cu", "moe_fused.cu"]
 FAST_MATH = {"quantize_q8_1.cu", "gemv1.cu"}
 
 

@@ -120,7 +120,9 @@ def dequantize_rows(W: torch.Tensor, row_ids: torch.Tensor, qtype: int, dtype=to
 def _matmul(fn_name: str, op: int, W: torch.Tensor, X: torch.Tensor, qtype: int, N: int) -> torch.Tensor:
     M, K = X.shape
     Y = torch.empty((M, N), dtype=X.dtype, device=X.device)
-    nbytes = lib().gguf_b200_workspace_bytes(op, qtype, M, N, K)
+    # (the GEMV keeps the smaller size: the passes of one and two vectors, and the comparison with the workspace-free entry point)
+    size = lib().gguf_b200_workspace_bytes if op == OP_GEMV else lib().gguf_b200_scratch_bytes
+    nbytes = size(op, qtype, M, N, K)
     ws = _ws(X, nbytes)
     fn = getattr(lib(), fn_name)
     _check(fn(W.data_ptr(), X.data_ptr(), Y.data_ptr(), ws.data_ptr(), nbytes, qtype, _DT[X.dtype], M, N, K, _stream(X)), fn_name)

@@ -94,7 +94,8 @@ DEQUANT_ONLY_SIZES: dict = {}
 _CUDA_DEQUANT_TYPES = _CUDA_GEMV_QUANT_TYPES | frozenset(DEQUANT_ONLY_SIZES)
 _CUDA_GEMM_QUANT_TYPES = frozenset({GGML_TYPE_Q4_0, GGML_TYPE_Q4_1, GGML_TYPE_Q5_0, GGML_TYPE_Q5_1, GGML_TYPE_Q8_0,
                                     GGML_TYPE_Q2_K, GGML_TYPE_Q3_K, GGML_TYPE_Q4_K, GGML_TYPE_Q5_K, GGML_TYPE_Q6_K})
-_DEQUANT_MATMUL_TYPES = frozenset({GGML_TYPE_IQ2_XXS, GGML_TYPE_IQ4_NL, GGML_TYPE_IQ4_XS})
+_DEQUANT_MATMUL_TYPES = frozenset({GGML_TYPE_IQ2_XXS, GGML_TYPE_IQ2_XS, GGML_TYPE_IQ2_S, GGML_TYPE_IQ3_XXS, GGML_TYPE_IQ3_S, GGML_TYPE_IQ1_S,
+                                   GGML_TYPE_IQ1_M, GGML_TYPE_IQ4_NL, GGML_TYPE_IQ4_XS})
 
 
 def _require(quant_type: int, allowed, op: str) -> None:
@@ -179,7 +180,7 @@ def ggml_mul_mat_a8(W: torch.Tensor, X: torch.Tensor, quant_type: int, row: int)
 
 
 def ggml_dequant_matmul(W: torch.Tensor, X: torch.Tensor, quant_type: int, row: int) -> torch.Tensor:
-    """x @ dequantize(W).T in one kernel, unquantized fp16/bf16 activations (IQ2_XXS, IQ4_XS)."""
+    """x @ dequantize(W).T in one kernel, unquantized fp16/bf16 activations (the code-book types)."""
     _require(quant_type, _DEQUANT_MATMUL_TYPES, "ggml_dequant_matmul")
     y = _mul_mat(W, X, quant_type, row, _OP_DEQUANT_MATMUL)
     return torch.ops._C_gguf.dequant_matmul(W, X, quant_type, row) if y is None else y
