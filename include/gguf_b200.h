@@ -91,6 +91,15 @@ int64_t gguf_b200_scratch_bytes(int op, int type, int64_t M, int64_t N, int64_t 
 int gguf_b200_mul_mat_vec_a8(const void* W, const void* X, void* Y, void* workspace, int64_t workspace_bytes,
                              int type, int dtype, int64_t M, int64_t N, int64_t K, void* stream);
 
+/* The dense products (op: GGUF_B200_OP_GEMV, _MMQ or _DEQUANT_MATMUL) on rows that do not lie back to back: weight rows
+ * `pitch` bytes apart (the last one, too, followed by the bytes up to the next), results ldy elements apart.  For the
+ * differently quantized parts of a merged projection, which are stored padded to the widest row and write their columns of
+ * one result.  The workspace is gguf_b200_scratch_bytes(op, ...) long.  Returns GGUF_B200_E_SHAPE for a pitch that the
+ * format's blocks cannot be read at, GGUF_B200_E_TOO_LARGE for sizes that only the packed entry points serve.
+ * Replaces: the per-shard copies, products and concatenation of quantization/linear.py:246-262. */
+int gguf_b200_mul_mat_strided(const void* W, const void* X, void* Y, void* workspace, int64_t workspace_bytes, int op, int type,
+                              int dtype, int64_t M, int64_t N, int64_t K, int64_t pitch, int64_t ldy, void* stream);
+
 /* The two halves of gguf_b200_mul_mat_vec_a8, for callers that multiply the same activations
  * by several weight matrices (q/k/v, gate/up): quantize once into `workspace`, then run any
  * number of GEMVs on it.

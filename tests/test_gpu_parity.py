@@ -965,3 +965,25 @@ def test_moe_experts_with_a_gap_between_them(name, pad):
     spread.copy_(w)
     assert torch.equal(capi.moe_a8(x, spread, s, e, n, t, N, top_k, T), capi.moe_a8(x, w, s, e, n, t, N, top_k, T))
     assert capi.last_status() == 0
+
+
+@pytest.mark.parametrize("types", [("Q4_K", "Q4_K", "Q6_K"), ("Q6_K", "Q8_0", "Q4_0"), ("IQ2_XXS", "IQ4_XS", "Q5_K"), ("Q4_K", "Q3_K", "Q3_K")])
+@pytest.mark.parametrize("K", [768, 4096])
+def test_merged_shards_of_several_types(types, K):
+    """A merged projection multiplied where its shards lie against one product per shard."""
+    from vllm_gguf_plugin.quantization.linear import GGUFLinearMethod, _fused_mul_mat_gguf
+
+    method, layer, rows = GGUFLinearMethod(None), torch.nn.Module(), [264, 136, 72]
+    method.create_weights(layer, K, rows, K, sum(rows), torch.float16)
+    parts = [torch.from_numpy(synth.make_weight(TYPES[n], r, K, seed=r)).to(DEV) for n, r in zip(types, rows)]
+    for sid, n, w in zip("qkv", types, parts):
+        layer.weight.weight_loader(layer.weight, w, sid)
+        layer.weight_type.weight_loader(layer.weight_type, torch.tensor(TYPES[n]), sid)
+    method.process_weights_after_loading(layer)
+    for M in (1, 2, 3, 7, 16, 17, 200):
+        for dtype, tol in ((torch.float16, 3e-4), (torch.bfloat16, 3e-3)):
+            x = dev_x(M, K, seed=M).to(dtype)
+            want = torch.cat([_fused_mul_mat_gguf(x, w, TYPES[n]) for n, w in zip(types, parts)], dim=1)
+            assert rel_l2(method.apply(layer, x).float().cpu(), want.float().cpu()) <= tol, (M, dtype)
+    torch.cuda.synchronize()
+    assert capi.last_status() == 0

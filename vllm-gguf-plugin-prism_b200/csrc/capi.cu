@@ -7,6 +7,7 @@
 
 #include "common.cuh"
 #include "kernels.h"
+#include "raw_stream.cuh"
 
 using namespace gguf_b200;
 
@@ -487,6 +488,42 @@ int gguf_b200_dequant_matmul(const void* W, const void* X, void* Y, void* ws, in
   // (the workspace is optional: room for the parts of shared tiles)
   return tiled_dense(false, W, X, Y, ws, ws_bytes, type, dtype, M, N, K, K / block_size(type) * type_size(type), N, nullptr, st,
                      static_cast<cudaStream_t>(stream));
+}
+
+int gguf_b200_mul_mat_strided(const void* W, const void* X, void* Y, void* ws, int64_t ws_bytes, int op, int type, int dtype, int64_t M,
+                              int64_t N, int64_t K, int64_t pitch, int64_t ldy, void* stream) {
+  int rc = check_common(W, X, Y, type, dtype, M, N, K);
+  if (rc || M == 0 || N == 0) return rc;
+  const int64_t row_bytes = K / block_size(type) * type_size(type);
+  if (pitch < row_bytes || ldy < N || pitch % raw_type_align(type) != 0) return E_BAD_SHAPE;
+  if (ws_bytes < gguf_b200_scratch_bytes(op, type, M, N, K)) return E_WORKSPACE;
+  if (ws_bytes > 0 && (!ws || !aligned16(ws))) return E_BAD_POINTER;
+  int* st = status_ptr();
+  if (!st) return E_CUDA;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (op == GGUF_B200_OP_DEQUANT_MATMUL) {
+    if (!is_dequant_matmul_type(type)) return E_BAD_TYPE;
+    if (dtype == DT_F32) return E_BAD_DTYPE;
+    if (K % 64 != 0) return E_BAD_SHAPE;
+    return tiled_dense(false, W, X, Y, ws, ws_bytes, type, dtype, M, N, K, pitch, ldy, nullptr, st, s);
+  }
+  if (op != GGUF_B200_OP_GEMV && op != GGUF_B200_OP_MMQ) return E_BAD_SHAPE;
+  if (op == GGUF_B200_OP_MMQ && !is_mmq_type(type)) return E_BAD_TYPE;
+  const int sum_mode = op == GGUF_B200_OP_GEMV ? gemv_sum_mode(type) : type == T_Q5_0 ? 1 : 0;
+  if (M >= small_min_tokens() && (op == GGUF_B200_OP_GEMV || M <= mmq_small_max_tokens())) {
+    if (!small_fits(N, K)) return E_TOO_LARGE;
+    return small_dense(W, X, Y, ws, type, dtype, sum_mode, M, N, K, pitch, ldy, st, s);
+  }
+  if (op == GGUF_B200_OP_MMQ && M > 2) return tiled_dense(true, W, X, Y, ws, ws_bytes, type, dtype, M, N, K, pitch, ldy, nullptr, st, s);
+  // one or two vectors; a single one of a short row is quantized by the GEMV kernel itself
+  if (M > 2) return E_TOO_LARGE;
+  rc = 1;
+  if (op == GGUF_B200_OP_GEMV) rc = launch_gemv_fused(W, X, Y, type, dtype, M, N, K, sum_mode, st, s, pitch);
+  if (rc <= 0) return rc;
+  rc = launch_quantize_q8_1(X, dtype, ws, M, K, Q8_MODE_SOA, sum_mode, 0, CORR_NONE, nullptr, 1, 0, s);
+  if (rc) return rc;
+  rc = launch_gemv1(W, ws, Y, type, dtype, N, K, st, s, nullptr, (int)M, nullptr, 0, 0, nullptr, 0, pitch, ldy);
+  return rc == 1 ? E_TOO_LARGE : rc;   // rows too long for the kernels that take a pitch
 }
 
 int gguf_b200_moe_a8(const void* X, const void* W, void* Y, void* ws, int64_t ws_bytes, const int32_t* sorted_token_ids,

@@ -681,6 +681,8 @@ struct G1Params {
   void* y;
   int64_t n, k;
   int bpr;               // blocks per row
+  int packed;            // 1: rows lie back to back
+  int64_t pitch, ldy;    // bytes between rows, elements between the vectors' results
   int ks, rl;            // K-slices per row, row lanes per CTA (ks * rl <= 8)
   int slice_q, slice_r;  // slice i holds slice_q + (i < slice_r) blocks, so no slice is ever empty
   int rows_per_item;     // <= G1_R
@@ -720,7 +722,7 @@ template <typename out_t>
 __device__ __forceinline__ void store_result(const G1Params& p, int64_t row, float v, int m, unsigned tag) {
   if (p.world == 0) {
     m = p.topk_ids ? (int)blockIdx.y : m + p.vec0;   // MoE decode: one output row of y per (token, expert) pair
-    static_cast<out_t*>(p.y)[(int64_t)m * p.n + row] = from_float<out_t>(v);
+    static_cast<out_t*>(p.y)[(int64_t)m * p.ldy + row] = from_float<out_t>(v);
     return;
   }
   const out_t o = from_float<out_t>(v);
@@ -803,10 +805,10 @@ __global__ void __launch_bounds__(G1_WARPS * 32, 2) gemv1_kernel(const G1Params 
   const int nblk = active ? p.slice_q + (ks_i < p.slice_r ? 1 : 0) : 0;
   const int units = nblk * UPB;
   const int R = p.rows_per_item;
-  const int64_t row_bytes = (int64_t)p.bpr * TS;
+  const int64_t row_bytes = p.pitch;
   const int64_t w_safe = p.w_bytes & ~int64_t(15);
   const uint32_t slice_bytes = (uint32_t)nblk * TS;
-  const bool contiguous = p.ks == 1;
+  const bool contiguous = p.ks == 1 && p.packed;
   const bool staged = p.ks > 1 || p.world > 0;   // results meet in shared memory before they are stored
 
   // ---- which rows: row lane wl (= the ks warps of a CTA that work on the same rows) owns the
@@ -1174,11 +1176,12 @@ static int launch_g1(G1Params p, cudaStream_t stream) {
   p.partial_bytes = (ks > 1 || p.world > 0) ? G1_BATCH * 8 * G1_R * MV * 4 : 0;
   const int room2 = (int)(((size_t)113 * 1024 - tables - (size_t)p.partial_bytes - (size_t)G1_WARPS * 8 * 16) / (2 * G1_WARPS)) - 48;
   const int item_cap = item_env < room2 ? item_env : room2;
-  while (R > 1 && (int64_t)R * (ks == 1 ? slice_bytes : (int)round_up(slice_bytes + 32, 16)) > item_cap) --R;
+  const bool contiguous = ks == 1 && p.packed;   // an item is one run of bytes
+  while (R > 1 && (int64_t)R * (contiguous ? slice_bytes : (int)round_up(slice_bytes + 32, 16)) > item_cap) --R;
   p.rows_per_item = R;
   p.inv_r = R == 1 ? 0u : (unsigned)(((1ull << 32) + R - 1) / R);
-  p.slot_bytes = ks == 1 ? slice_bytes : (int)round_up(slice_bytes + 32, 16);
-  p.stage_bytes = ks == 1 ? (int)round_up((int64_t)R * slice_bytes + 32, 16) : R * p.slot_bytes;
+  p.slot_bytes = contiguous ? slice_bytes : (int)round_up(slice_bytes + 32, 16);
+  p.stage_bytes = contiguous ? (int)round_up((int64_t)R * slice_bytes + 32, 16) : R * p.slot_bytes;
   const int kpad = (int)round_up(p.k, 512);
   p.x_bytes = p.x_raw ? (int)round_up((int64_t)MV * (kpad + kpad / 4), 128) : 0;
   p.x_alias = (p.x_raw && p.x_bytes <= p.stage_bytes) ? 1 : 0;
@@ -1269,7 +1272,7 @@ static int launch_g1_out(const G1Params& p, int out_dtype, int mv, cudaStream_t 
 // Returns E_OK, a negative error, or 1 when the shape is outside this kernel's reach.
 int launch_gemv1(const void* w, const void* xq_soa, void* y, int type, int out_dtype, int64_t N, int64_t K, int* status,
                  cudaStream_t stream, const GemvTp* tp, int vectors, const GemvMoe* moe, int vec0, int total_vecs,
-                 const void* x_raw, int x_sum_mode) {
+                 const void* x_raw, int x_sum_mode, int64_t pitch, int64_t ldy) {
   G1Params p{};
   p.x_raw = x_raw;
   p.x_sum_mode = x_sum_mode;
@@ -1297,7 +1300,11 @@ int launch_gemv1(const void* w, const void* xq_soa, void* y, int type, int out_d
   }
   p.w = static_cast<const uint8_t*>(w);
   p.bpr = (int)(K / block_size(type));
-  p.w_bytes = N * p.bpr * type_size(type);
+  const int64_t row_bytes = (int64_t)p.bpr * type_size(type);
+  p.packed = pitch == 0 || pitch == row_bytes;
+  p.pitch = p.packed ? row_bytes : pitch;
+  p.ldy = ldy > 0 ? ldy : N;
+  p.w_bytes = (N - 1) * p.pitch + row_bytes;
   p.xq = static_cast<const uint8_t*>(xq_soa);
   p.y = y;
   p.n = N;

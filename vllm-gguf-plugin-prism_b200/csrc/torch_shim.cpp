@@ -330,6 +330,55 @@ PyObject* py_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
+// linear_runs(x, W, runs): a layer whose rows are of several types, stacked in W and padded to its width.  runs: a flat tuple of
+// (type, first row, rows, bytes of a row, rows that decide the routing) per run.  Every run is multiplied where it lies, into its columns of one result.
+PyObject* py_linear_runs(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  TORCH_CHECK(n == 3 && PyTuple_Check(a[2]) && PyTuple_GET_SIZE(a[2]) % 5 == 0, "linear_runs takes x, W and a tuple of runs");
+  const Tensor *X = plain_cuda(a[0]), *W = plain_cuda(a[1]);
+  if (!W || !X || X->dim() != 2 || W->dim() != 2 || X->size(0) == 0 || !modes_off() || !X->is_contiguous() || !W->is_contiguous() ||
+      W->scalar_type() != ScalarType::Byte)
+    Py_RETURN_NONE;
+  const ScalarType dt = X->scalar_type();
+  if (dt != ScalarType::Float && dt != ScalarType::Half && dt != ScalarType::BFloat16) Py_RETURN_NONE;
+  struct Run { int type, op; int64_t row, rows, ws; };
+  c10::SmallVector<Run, 4> runs;
+  const int64_t M = X->size(0), K = X->size(1), pitch = W->size(1);
+  int64_t N = 0, most = 0;
+  for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(a[2]); i += 5) {
+    long v[5];
+    for (int j = 0; j < 5; ++j) v[j] = PyLong_AsLong(PyTuple_GET_ITEM(a[2], i + j));
+    if (PyErr_Occurred()) return nullptr;
+    const int ts = gguf_b200_type_size((int)v[0]);
+    if (ts == 0 || v[3] % ts != 0 || v[3] / ts * gguf_b200_block_size((int)v[0]) != K || v[1] < 0 || v[1] + v[2] > W->size(0) || v[1] * pitch % 16 != 0)
+      Py_RETURN_NONE;
+    const int op = linear_op(v[0], M, v[4], dt);
+    if (op < 0) Py_RETURN_NONE;
+    const int64_t ws = gguf_b200_scratch_bytes(op, (int)v[0], M, v[2], K);
+    most = ws > most ? ws : most;
+    runs.push_back({(int)v[0], op, v[1], v[2], ws});
+    N += v[2];
+  }
+  if (N == 0) Py_RETURN_NONE;
+  const c10::cuda::CUDAGuard guard(X->device());
+  Tensor Y = new_tensor({M, N}, dt, X->device());
+  const Scratch ws(most);
+  const int code = dtype_code(dt, "linear_runs");
+  void* s = current_stream(X->get_device());
+  int64_t col = 0;
+  for (const Run& r : runs) {
+    uint8_t* y = static_cast<uint8_t*>(Y.data_ptr()) + col * Y.element_size();
+    if (reinterpret_cast<uintptr_t>(y) % 16 != 0) Py_RETURN_NONE;
+    const int rc = gguf_b200_mul_mat_strided(static_cast<const uint8_t*>(W->data_ptr()) + r.row * pitch, X->data_ptr(), y, ws.get(), most, r.op, r.type,
+                                             code, M, r.rows, K, pitch, N, s);
+    if (rc == GGUF_B200_E_SHAPE || rc == GGUF_B200_E_TOO_LARGE) Py_RETURN_NONE;   // a layout that only copies can serve
+    check_rc(rc, "linear_runs");
+    col += r.rows;
+  }
+  return THPVariable_Wrap(std::move(Y));
+  END_HANDLE_TH_ERRORS
+}
+
 // moe(x, W13, W2, topk_weights, topk_ids, type13, type2, act): the whole expert step
 PyObject* py_moe(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
@@ -348,6 +397,7 @@ PyMethodDef methods[] = {
     {"moe", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(&py_moe)), METH_FASTCALL, nullptr},
     {"mul_mat", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(&py_mul_mat)), METH_FASTCALL, nullptr},
     {"embed", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(&py_embed)), METH_FASTCALL, nullptr},
+    {"linear_runs", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(&py_linear_runs)), METH_FASTCALL, nullptr},
     {"linear", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(&py_linear)), METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr},
 };

@@ -16,7 +16,7 @@ import torch
 from torch.compiler import is_compiling
 
 from .. import ops
-from .._C_gguf import linear as _native_linear
+from .._C_gguf import linear as _native_linear, linear_runs as _native_runs
 from .utils import (
     DEQUANT_TYPES,
     IMATRIX_QUANT_TYPES,
@@ -136,6 +136,7 @@ class GGUFLinearMethod(LinearMethodBase):
         weight = torch.nn.Parameter(torch.empty(0, dtype=torch.uint8), requires_grad=False)
         weight.shard_id = []
         weight.gguf_one_type = None
+        weight.gguf_runs = ()
         weight.shard_offset_map = {}
         weight.output_partition_sizes = list(output_partition_sizes)
         weight.input_size_per_partition = input_size_per_partition
@@ -212,6 +213,16 @@ class GGUFLinearMethod(LinearMethodBase):
         types = {wtype.shard_weight_type.get(i, wtype.weight_type) for i in w.shard_id}
         same_width = len({o[2] for o in w.shard_offset_map.values()}) == 1
         w.gguf_one_type = types.pop() if len(types) == 1 and same_width else None
+        # ... and else the runs of rows of one type: (type, first row, rows, bytes of a row, rows of a shard as the batch-size
+        # rule counts them) of each, in one flat tuple
+        runs: list[list[int]] = []
+        for i in w.shard_id:
+            (start, end, width), t = w.shard_offset_map[i], int(wtype.shard_weight_type.get(i, wtype.weight_type))
+            if runs and runs[-1][0] == t and runs[-1][3] == width and (runs[-1][4] > 5120) == (end - start > 5120):
+                runs[-1][2] += end - start
+            else:
+                runs.append([t, start, end - start, width, end - start])
+        w.gguf_runs = tuple(v for r in runs for v in r)
 
     def apply(self, layer: torch.nn.Module, x: torch.Tensor, bias: torch.Tensor | None = None) -> torch.Tensor:
         if self.layout is not None:
@@ -221,10 +232,9 @@ class GGUFLinearMethod(LinearMethodBase):
             # the layers in between (custom op, operator dispatch), which cost more than a decode GEMV runs for.
             weight = layer.weight
             one_type = weight.gguf_one_type if weight.shard_id else layer.weight_type.weight_type
-            if one_type is not None:
-                out = _native_linear(x, weight, one_type)
-                if out is not None:
-                    return out if bias is None else out.add_(bias)
+            out = _native_linear(x, weight, one_type) if one_type is not None else _native_runs(x, weight, weight.gguf_runs)
+            if out is not None:
+                return out if bias is None else out.add_(bias)
         shard_id = layer.weight.shard_id
         if shard_id:
             shard_id = ["q", "k", "v"] if "q" in shard_id else shard_id
