@@ -135,6 +135,8 @@ __global__ void __launch_bounds__(256) dequantize_kernel(const uint8_t* __restri
     for (int i = threadIdx.x; i < 128; i += blockDim.x) s_signs[i] = d_ksigns_iq2xs[i];
     __syncthreads();
   }
+  pdl_trigger();
+  pdl_wait();   // (whatever wrote the weights, the row numbers or read the output before)
   constexpr int TS = BlockTraits<TYPE>::TS;
   const int lane = threadIdx.x & 31;
   const int64_t chunks = (n_elems + 255) / 256;  // 256 outputs per warp step
@@ -150,8 +152,9 @@ __global__ void __launch_bounds__(256) dequantize_kernel(const uint8_t* __restri
     const uint8_t* w = w_all;
     int64_t c = cg;
     if (rg.ids) {
-      const int64_t r = cg / rg.chunks_per_row, id = rg.ids[r];
-      c = cg - r * rg.chunks_per_row;
+      const unsigned r = (unsigned)cg / (unsigned)rg.chunks_per_row;   // (a 64-bit division costs as much as the decoding)
+      const int64_t id = rg.ids[r];
+      c = (int64_t)((unsigned)cg - r * (unsigned)rg.chunks_per_row);
       if (id < 0 || id >= rg.weight_rows) {   // no such row: zeros (index_select would have refused)
 #pragma unroll
         for (int j = 0; j < 8; ++j) { h[j] = __float2half_rn(0.f); f[j] = 0.f; }
@@ -207,23 +210,6 @@ __global__ void __launch_bounds__(256) dequantize_kernel(const uint8_t* __restri
         const uint32_t ws = (i ? q.y : q.x) >> (4 * hi);
         put4(h, 4 * i, q4k_value2<Q4K_CONTRACT>(d12, ints_h2(ws & 0x000F000Fu, 1024.f), m12),
              q4k_value2<Q4K_CONTRACT>(d12, ints_h2((ws >> 8) & 0x000F000Fu, 1024.f), m12));
-      }
-      store_from_half(y + o, h);
-    } else if (TYPE == T_Q6_K) {  // dequantize_block_q6_K
-      const uint8_t* blk = w + c * TS;
-      const int ip = lane >> 4, off = (lane & 15) * 8, qd = off >> 5, l0 = off & 31;
-      const uint2 ql = ldg_8_a2(blk + 64 * ip + 32 * (qd & 1) + l0);
-      const uint2 qh = ldg_8_a2(blk + 128 + 32 * ip + l0);
-      const int sc = (int)(int8_t)__ldg(blk + 192 + 8 * ip + 2 * qd + (l0 >> 4));
-      const __half d = __ushort_as_half((unsigned short)ldg_u16(blk + 208));
-      // (The pair form used for the 4- and 8-bit types above gained nothing here -- 99.4 vs 98.1 us on
-      //  37888x3584 -- and a product of a negative scale with a zero code comes out as -0 where the
-      //  reference's integer product gives +0, so the integer form stays.)
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const int lo = (byte_of(ql, j) >> (4 * (qd >> 1))) & 0xF;
-        const int hb = (byte_of(qh, j) >> (2 * qd)) & 3;
-        h[j] = hmul_rn(d, __int2half_rn(sc * ((lo | (hb << 4)) - 32)));
       }
       store_from_half(y + o, h);
     } else if (TYPE == T_IQ2_XXS) {  // dequantize_block_iq2_xxs (fp32)
@@ -405,19 +391,93 @@ __global__ void __launch_bounds__(256) dequantize_kernel(const uint8_t* __restri
   }
 }
 
+// Q6_K.  Eight lanes per super-block: lane (ip, i) has the bytes 8i .. 8i + 7 of both 32-byte rows of ql and of the row of qh of
+// half ip, which hold 32 values -- eight in each of the half's four quarters, one 16-byte store each.  (With eight values per
+// lane all 24 bytes were fetched, two at a time, for every eight values: 32 instructions per value, and 9.0 us for 1024 rows of
+// 4096 to bf16, of which 1.8 us is memory traffic; 37888 x 3584 took 98 us.)  A product of scale and code is exact or rounds
+// once, as the reference's conversion of the integer product does; adding +0 gives zero products the sign that conversion gives.
+__device__ __forceinline__ void q6_store(__half* y, const __half2 (&v)[4]) {
+  uint4 o;
+  o.x = *reinterpret_cast<const uint32_t*>(&v[0]); o.y = *reinterpret_cast<const uint32_t*>(&v[1]);
+  o.z = *reinterpret_cast<const uint32_t*>(&v[2]); o.w = *reinterpret_cast<const uint32_t*>(&v[3]);
+  *reinterpret_cast<uint4*>(y) = o;
+}
+__device__ __forceinline__ void q6_store(__nv_bfloat16* y, const __half2 (&v)[4]) {
+  uint32_t o[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 f = __half22float2(v[i]);
+    const __nv_bfloat162 b = __floats2bfloat162_rn(f.x, f.y);
+    o[i] = *reinterpret_cast<const uint32_t*>(&b);
+  }
+  *reinterpret_cast<uint4*>(y) = make_uint4(o[0], o[1], o[2], o[3]);
+}
+__device__ __forceinline__ void q6_store(float* y, const __half2 (&v)[4]) {
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const float2 a = __half22float2(v[2 * i]), b = __half22float2(v[2 * i + 1]);
+    reinterpret_cast<float4*>(y)[i] = make_float4(a.x, a.y, b.x, b.y);
+  }
+}
+template <typename out_t>
+__global__ void __launch_bounds__(256) dequantize_q6k_kernel(const uint8_t* __restrict__ w_all, out_t* __restrict__ y, int64_t blocks, RowGather rg) {
+  pdl_trigger();
+  pdl_wait();
+  const int lane = threadIdx.x & 31, ip = (lane >> 2) & 1, l0 = 8 * (lane & 3);
+  const int64_t step = (int64_t)gridDim.x * 32;
+  for (int64_t cg = (int64_t)blockIdx.x * 32 + (threadIdx.x >> 3); cg < blocks; cg += step) {
+    const uint8_t* blk = w_all + cg * 210;
+    out_t* out = y + cg * 256 + 128 * ip + l0;
+    if (rg.ids) {
+      const unsigned r = (unsigned)cg / (unsigned)rg.chunks_per_row;
+      const int64_t id = rg.ids[r];
+      if (id < 0 || id >= rg.weight_rows) {   // no such row: zeros
+        const __half2 z[4] = {};
+#pragma unroll
+        for (int q = 0; q < 4; ++q) q6_store(out + 32 * q, z);
+        continue;
+      }
+      blk = w_all + id * rg.row_bytes + (int64_t)((unsigned)cg - r * (unsigned)rg.chunks_per_row) * 210;
+    }
+    const uint2 la = ldg_8_a2(blk + 64 * ip + l0), lb = ldg_8_a2(blk + 64 * ip + 32 + l0), hb = ldg_8_a2(blk + 128 + 32 * ip + l0);
+    int sc[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) sc[q] = (int)(int8_t)__ldg(blk + 192 + 8 * ip + 2 * q + (l0 >> 4));
+    const __half2 d2 = __half2half2(__ushort_as_half((unsigned short)ldg_u16(blk + 208)));
+    const __half2 zero = __floats2half2_rn(0.f, 0.f), off = __floats2half2_rn(1056.f, 1056.f);   // 1024 + 32
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const __half2 s2 = __half2half2(__int2half_rn(sc[q]));
+      __half2 v[4];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const uint32_t l = q & 1 ? (i ? lb.y : lb.x) : (i ? la.y : la.x), h = i ? hb.y : hb.x;
+        const uint32_t c = ((q < 2 ? l : l >> 4) & 0x0F0F0F0Fu) | ((q == 0 ? h << 4 : q == 1 ? h << 2 : q == 2 ? h : h >> 2) & 0x30303030u);
+        const __half2 a = __hsub2_rn(u32_h2(__byte_perm(c, 0x64646464u, 0x4140)), off), b = __hsub2_rn(u32_h2(__byte_perm(c, 0x64646464u, 0x4342)), off);
+        v[2 * i] = __hmul2_rn(d2, __hfma2(s2, a, zero));
+        v[2 * i + 1] = __hmul2_rn(d2, __hfma2(s2, b, zero));
+      }
+      q6_store(out + 32 * q, v);
+    }
+  }
+}
+
 template <int TYPE, typename out_t>
 static int launch_t(const void* w, void* out, int64_t n, int q4k_contract, cudaStream_t s, const RowGather& rg) {
   const int64_t chunks = (n + 255) / 256;
+  if constexpr (TYPE == T_Q6_K) {
+    const int64_t want = (chunks + 31) / 32, most = 148 * 16;
+    return launch_pdl(dequantize_q6k_kernel<out_t>, dim3((unsigned)(want < most ? want : most)), dim3(256), 0, s, (const uint8_t*)w, (out_t*)out, chunks, rg) ==
+           cudaSuccess ? E_OK : E_CUDA;
+  }
   int64_t ctas = (chunks + 7) / 8;
   const int64_t cap = 148 * 32;  // four rounds of the 8 resident CTAs per SM measured best (148*8: -5 %, one CTA per 8 chunks: -25 %)
   if (ctas > cap) ctas = cap;
   if (ctas < 1) ctas = 1;
   constexpr bool fusible = TYPE == T_Q4_K || TYPE == T_Q5_K || TYPE == T_Q2_K || TYPE == T_Q4_1 || TYPE == T_Q5_1;
   if (fusible && q4k_contract)
-    dequantize_kernel<TYPE, out_t, true><<<(int)ctas, 256, 0, s>>>((const uint8_t*)w, (out_t*)out, n, rg);
-  else
-    dequantize_kernel<TYPE, out_t, false><<<(int)ctas, 256, 0, s>>>((const uint8_t*)w, (out_t*)out, n, rg);
-  return cudaGetLastError() == cudaSuccess ? E_OK : E_CUDA;
+    return launch_pdl(dequantize_kernel<TYPE, out_t, fusible>, dim3((unsigned)ctas), dim3(256), 0, s, (const uint8_t*)w, (out_t*)out, n, rg) == cudaSuccess ? E_OK : E_CUDA;
+  return launch_pdl(dequantize_kernel<TYPE, out_t, false>, dim3((unsigned)ctas), dim3(256), 0, s, (const uint8_t*)w, (out_t*)out, n, rg) == cudaSuccess ? E_OK : E_CUDA;
 }
 
 template <int TYPE>

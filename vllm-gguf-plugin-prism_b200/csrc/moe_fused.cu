@@ -30,7 +30,7 @@ __global__ void __launch_bounds__(1024) moe_plan_kernel(const int32_t* __restric
   for (int e = lane; e < n_experts; e += 32) s_cnt[warp][e] = 0;
   pdl_wait();
   __syncthreads();
-  const int run = ((slots + 31) / 32 + 31) / 32 * 32, s0 = warp * run, s1 = min(slots, s0 + run);
+  const int run = ((slots + 31) / 32 + 31) / 32 * 32, s0 = warp * run, s1 = min(slots, s0 + run), warps = (slots + run - 1) / run;   // warps that have slots
   for (int s = s0; s < s1; s += 32) {
     const int e = s + lane < s1 ? topk_ids[s + lane] : -1;
     const unsigned same = __match_any_sync(0xffffffffu, e);
@@ -40,10 +40,15 @@ __global__ void __launch_bounds__(1024) moe_plan_kernel(const int32_t* __restric
   __syncthreads();
   for (int e = threadIdx.x; e < n_experts; e += blockDim.x) {   // per expert: prefix over the warps
     int c = 0;
-    for (int w = 0; w < 32; ++w) {
-      const int v = s_cnt[w][e];
-      s_cnt[w][e] = c;
-      c += v;
+    for (int w0 = 0; w0 < warps; w0 += 8) {   // (eight loads in flight)
+      int v[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = s_cnt[w0 + i][e];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        s_cnt[w0 + i][e] = c;
+        c += v[i];
+      }
     }
     s_tot[e] = c;
   }
@@ -144,27 +149,48 @@ int launch_moe_blocks(const int32_t* expert_ids, const int32_t* n_post_pad, int6
                     static_cast<int4*>(passes), n_passes) == cudaSuccess ? E_OK : E_CUDA;
 }
 
+// Eight columns per thread.  (One column per thread, with a 64-bit division for it, took 10.4 us for 256 tokens of 2048
+// columns and eight experts, 278 instructions a column; the traffic is worth 1.5 us.)
 template <typename T>
 __global__ void __launch_bounds__(256) moe_sum_kernel(const T* __restrict__ y, T* __restrict__ out, const int32_t* __restrict__ topk_ids,
                                                       int n_experts, int64_t tokens, int top_k, int64_t h) {
   pdl_trigger();
   pdl_wait();
-  const int64_t total = tokens * h;
+  constexpr int W = sizeof(T) / 2;               // 16-byte words of eight values
+  const unsigned per_row = (unsigned)(h / 8);
+  const int64_t total = tokens * per_row;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t t = i / h, c = i - t * h;
-    float s = 0.f;
-    for (int j = 0; j < top_k; ++j) {
-      const int e = topk_ids[t * top_k + j];
-      if (e >= 0 && e < n_experts) s += to_float<T>(y[(t * top_k + j) * h + c]);   // a slot without a valid expert contributes nothing
+    const unsigned t = (unsigned)i / per_row;
+    const int64_t c = 8 * (int64_t)((unsigned)i - t * per_row);
+    const int32_t* ids = topk_ids + (int64_t)t * top_k;
+    const T* in = y + (int64_t)t * top_k * h + c;
+    float s[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) s[k] = 0.f;
+#pragma unroll 4
+    for (int j = 0; j < top_k; ++j, in += h) {
+      const int e = __ldg(ids + j);
+      if (e < 0 || e >= n_experts) continue;     // a slot without a valid expert contributes nothing
+      uint4 v[W];
+#pragma unroll
+      for (int k = 0; k < W; ++k) v[k] = reinterpret_cast<const uint4*>(in)[k];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) s[k] += to_float<T>(reinterpret_cast<const T*>(v)[k]);
     }
-    out[i] = from_float<T>(s);
+    uint4 o[W];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) reinterpret_cast<T*>(o)[k] = from_float<T>(s[k]);
+#pragma unroll
+    for (int k = 0; k < W; ++k) reinterpret_cast<uint4*>(out + (int64_t)t * h + c)[k] = o[k];
   }
 }
 
 int launch_moe_sum(const void* y, void* out, const int32_t* topk_ids, int n_experts, int64_t tokens, int64_t top_k, int64_t h,
                    int dtype, cudaStream_t stream) {
-  const int64_t total = tokens * h;
+  if (h % 8 != 0) return E_BAD_SHAPE;
+  const int64_t total = tokens * (h / 8);
   if (total == 0) return E_OK;
+  if (total >= (int64_t)1 << 32) return E_TOO_LARGE;
   const unsigned grid = (unsigned)((total + 255) / 256 > 148 * 8 ? 148 * 8 : (total + 255) / 256);
   cudaError_t e;
   switch (dtype) {
