@@ -53,6 +53,24 @@ template <int N> __device__ __forceinline__ void slw(uint32_t a, uint32_t (&w)[N
 }
 __device__ __forceinline__ uint32_t slw1(uint32_t a) { uint32_t w[1]; slw<1>(a, w); return w[0]; }
 
+// ... from a + off, `a` a multiple of four.  KNOWN: so is the row's start, and off, a constant where this is called, says how
+// the words lie -- no address arithmetic, no second load where they are aligned.
+template <bool KNOWN, int N> __device__ __forceinline__ void slwo(uint32_t a, int off, uint32_t (&w)[N]) {
+  if constexpr (!KNOWN) {
+    slw<N>(a + off, w);
+  } else if ((off & 3) == 0) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) w[i] = sl32(a + off + 4 * i);
+  } else {
+    uint32_t r[N + 1];
+#pragma unroll
+    for (int i = 0; i <= N; ++i) r[i] = sl32(a + (off & ~3) + 4 * i);
+#pragma unroll
+    for (int i = 0; i < N; ++i) w[i] = __byte_perm(r[i], r[i + 1], 0x5432);   // (offsets are even)
+  }
+}
+template <bool KNOWN> __device__ __forceinline__ uint32_t slwo1(uint32_t a, int off) { uint32_t w[1]; slwo<KNOWN, 1>(a, off, w); return w[0]; }
+
 struct SmBlk {
   uint32_t w0, w1;     // codes
   uint32_t v0, v1;     // KIND 4: minima
@@ -86,6 +104,10 @@ __device__ __forceinline__ uint32_t sm_spread4(uint32_t x) { return ((x & 0xFu) 
 // U8: the codes are unsigned bytes.  MINS: mins(rp, row, t, nb, a) gives the minima of the blocks t and t + 4 (0 for blocks
 // from nb on) and returns the row's factor.
 template <int TYPE> struct SmDec;
+// the formats of 32-value blocks: rows of whole chunks of which start on 16-byte boundaries (block<KNOWN>)
+template <int TYPE> __host__ __device__ constexpr bool sm_can_be_whole() {
+  return TYPE == T_Q4_0 || TYPE == T_Q4_1 || TYPE == T_Q5_0 || TYPE == T_Q5_1 || TYPE == T_Q8_0 || TYPE == T_IQ4_NL;
+}
 
 template <> struct SmDec<T_Q4_0> {
   static constexpr int ORDER = 0, KIND = 0;
@@ -97,8 +119,8 @@ template <> struct SmDec<T_Q4_0> {
     a[1] = t + 4 < nb ? slh(rp + 18 * (t + 4)) : 0.f;
     return -8.f;
   }
-  static __device__ __forceinline__ void block(uint32_t rp, const Row&, int j, int t, uint32_t, SmBlk& b) {
-    const uint32_t q = slw1(rp + 18 * j + 2 + 4 * t);
+  template <bool KNOWN> static __device__ __forceinline__ void block(uint32_t rp, const Row&, int j, int t, uint32_t, SmBlk& b) {
+    const uint32_t q = slwo1<KNOWN>(rp + 4 * t, 18 * j + 2);
     b.w0 = q & 0x0F0F0F0Fu;
     b.w1 = (q >> 4) & 0x0F0F0F0Fu;
     b.s = slh(rp + 18 * j);
@@ -109,7 +131,7 @@ template <> struct SmDec<T_Q4_1> {
   static constexpr bool U8 = true, MINS = false;
   using Row = SmNone;
   static __device__ __forceinline__ void head(uint32_t, Row&) {}
-  static __device__ __forceinline__ void block(uint32_t rp, const Row&, int j, int t, uint32_t, SmBlk& b) {
+  template <bool KNOWN> static __device__ __forceinline__ void block(uint32_t rp, const Row&, int j, int t, uint32_t, SmBlk& b) {
     const uint32_t q = sl32(rp + 20 * j + 4 + 4 * t);
     b.w0 = q & 0x0F0F0F0Fu;
     b.w1 = (q >> 4) & 0x0F0F0F0Fu;
@@ -126,8 +148,8 @@ template <> struct SmDec<T_Q5_0> {
     a[1] = t + 4 < nb ? slh(rp + 22 * (t + 4)) : 0.f;
     return -16.f;
   }
-  static __device__ __forceinline__ void block(uint32_t rp, const Row&, int j, int t, uint32_t, SmBlk& b) {
-    const uint32_t qh = slw1(rp + 22 * j + 2), q = slw1(rp + 22 * j + 6 + 4 * t);
+  template <bool KNOWN> static __device__ __forceinline__ void block(uint32_t rp, const Row&, int j, int t, uint32_t, SmBlk& b) {
+    const uint32_t qh = slwo1<KNOWN>(rp, 22 * j + 2), q = slwo1<KNOWN>(rp + 4 * t, 22 * j + 6);
     b.w0 = (q & 0x0F0F0F0Fu) | sm_spread4(qh >> (4 * t));
     b.w1 = ((q >> 4) & 0x0F0F0F0Fu) | sm_spread4(qh >> (16 + 4 * t));
     b.s = slh(rp + 22 * j);
@@ -138,7 +160,7 @@ template <> struct SmDec<T_Q5_1> {
   static constexpr bool U8 = true, MINS = false;
   using Row = SmNone;
   static __device__ __forceinline__ void head(uint32_t, Row&) {}
-  static __device__ __forceinline__ void block(uint32_t rp, const Row&, int j, int t, uint32_t, SmBlk& b) {
+  template <bool KNOWN> static __device__ __forceinline__ void block(uint32_t rp, const Row&, int j, int t, uint32_t, SmBlk& b) {
     const uint2 h = sl64(rp + 24 * j);
     const uint32_t q = sl32(rp + 24 * j + 8 + 4 * t);
     b.w0 = (q & 0x0F0F0F0Fu) | sm_spread4(h.y >> (4 * t));
@@ -151,9 +173,9 @@ template <> struct SmDec<T_Q8_0> {
   static constexpr bool U8 = false, MINS = false;
   using Row = SmNone;
   static __device__ __forceinline__ void head(uint32_t, Row&) {}
-  static __device__ __forceinline__ void block(uint32_t rp, const Row&, int j, int t, uint32_t, SmBlk& b) {
+  template <bool KNOWN> static __device__ __forceinline__ void block(uint32_t rp, const Row&, int j, int t, uint32_t, SmBlk& b) {
     uint32_t w[2];
-    slw<2>(rp + 34 * j + 2 + 8 * t, w);
+    slwo<KNOWN, 2>(rp + 8 * t, 34 * j + 2, w);
     b.w0 = w[0];
     b.w1 = w[1];
     b.s = slh(rp + 34 * j);
@@ -301,8 +323,8 @@ template <> struct SmDec<T_IQ4_NL> {
   static constexpr bool U8 = false, MINS = false;
   using Row = SmNone;
   static __device__ __forceinline__ void head(uint32_t, Row&) {}
-  static __device__ __forceinline__ void block(uint32_t rp, const Row&, int j, int t, uint32_t, SmBlk& b) {
-    sm_iq4_words(slw1(rp + 18 * j + 2 + 4 * t), b.w0, b.w1);
+  template <bool KNOWN> static __device__ __forceinline__ void block(uint32_t rp, const Row&, int j, int t, uint32_t, SmBlk& b) {
+    sm_iq4_words(slwo1<KNOWN>(rp + 4 * t, 18 * j + 2), b.w0, b.w1);
     b.s = slh(rp + 18 * j);
   }
 };
