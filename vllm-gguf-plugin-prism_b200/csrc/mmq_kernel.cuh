@@ -384,7 +384,7 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_consta
           }
         }
       }
-      const bool plain = p.tp_world == 0 && p.dtype != DT_F32;
+      const bool plain = p.tp_world == 0 && p.dtype != DT_F32, rows = plain && !moe && !p.row_scale;
 #pragma unroll 1
       for (int b = g; b < nb; b += MMQ_GROUPS) {
         const int orow_next = out_row(b + MMQ_GROUPS);
@@ -412,7 +412,31 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_consta
             }
           }
         }
-        if (plain) {
+        if (rows) {   // consecutive rows: 5 instructions a value (20 through the row numbers, a tenth of all the kernel issued at 512 tokens)
+          uint32_t h[8];
+          if (p.dtype == DT_F16) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) h[j] = pack2<__half>(__uint_as_float(acc[2 * j]), __uint_as_float(acc[2 * j + 1]));
+          } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) h[j] = pack2<__nv_bfloat16>(__uint_as_float(acc[2 * j]), __uint_as_float(acc[2 * j + 1]));
+          }
+          const int left = live ? et.rows - 16 * b : 0;
+          uint16_t* y = static_cast<uint16_t*>(p.y) + (int64_t)(et.x0 + 16 * b) * p.ldy + n;
+          if (left >= 16) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j, y += p.ldy) *y = (uint16_t)(j & 1 ? h[j >> 1] >> 16 : h[j >> 1]);
+          } else {
+#pragma unroll 1
+            for (int j = 0; j < left; ++j, y += p.ldy) {
+              *y = (uint16_t)h[0];
+              h[0] = __funnelshift_r(h[0], h[1], 16);
+#pragma unroll
+              for (int i = 1; i < 7; ++i) h[i] = __funnelshift_r(h[i], h[i + 1], 16);
+              h[7] >>= 16;
+            }
+          }
+        } else if (plain) {
           uint16_t* y = static_cast<uint16_t*>(p.y) + n;
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
