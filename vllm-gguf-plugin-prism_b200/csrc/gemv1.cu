@@ -674,6 +674,9 @@ template <> struct G1<T_Q5_K> {
 constexpr int G1_R = 4;
 constexpr int G1_MAX_WORLD = 8;
 
+// what divides the bytes of a block, and with it every distance between rows: known when the kernel is compiled
+__host__ __device__ constexpr int g1_align(int block_bytes) { return block_bytes % 16 == 0 ? 16 : block_bytes % 8 == 0 ? 8 : block_bytes % 4 == 0 ? 4 : 2; }
+
 struct G1Params {
   const uint8_t* w;
   int64_t w_bytes;
@@ -682,7 +685,8 @@ struct G1Params {
   int64_t n, k;
   int bpr;               // blocks per row
   int packed;            // 1: rows lie back to back
-  int64_t pitch, ldy;    // bytes between rows, elements between the vectors' results
+  int pitch;             // units of g1_align bytes between rows (32 bits: a row's address is one wide product)
+  int64_t ldy;           // elements between the vectors' results
   int ks, rl;            // K-slices per row, row lanes per CTA (ks * rl <= 8)
   int slice_q, slice_r;  // slice i holds slice_q + (i < slice_r) blocks, so no slice is ever empty
   int rows_per_item;     // <= G1_R
@@ -805,7 +809,7 @@ __global__ void __launch_bounds__(G1_WARPS * 32, 2) gemv1_kernel(const G1Params 
   const int nblk = active ? p.slice_q + (ks_i < p.slice_r ? 1 : 0) : 0;
   const int units = nblk * UPB;
   const int R = p.rows_per_item;
-  const int64_t row_bytes = p.pitch;
+  const int row_bytes = p.pitch * g1_align(TS);
   const int64_t w_safe = p.w_bytes & ~int64_t(15);
   const uint32_t slice_bytes = (uint32_t)nblk * TS;
   const bool contiguous = p.ks == 1 && p.packed;
@@ -1302,9 +1306,12 @@ int launch_gemv1(const void* w, const void* xq_soa, void* y, int type, int out_d
   p.bpr = (int)(K / block_size(type));
   const int64_t row_bytes = (int64_t)p.bpr * type_size(type);
   p.packed = pitch == 0 || pitch == row_bytes;
-  p.pitch = p.packed ? row_bytes : pitch;
+  if (pitch > 0x7ffffffll) return E_TOO_LARGE;
+  const int64_t step = p.packed ? row_bytes : pitch;
+  if (step % g1_align(type_size(type)) != 0) return 1;
+  p.pitch = (int)(step / g1_align(type_size(type)));
   p.ldy = ldy > 0 ? ldy : N;
-  p.w_bytes = (N - 1) * p.pitch + row_bytes;
+  p.w_bytes = (N - 1) * step + row_bytes;
   p.xq = static_cast<const uint8_t*>(xq_soa);
   p.y = y;
   p.n = N;

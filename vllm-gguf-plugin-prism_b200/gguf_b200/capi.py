@@ -163,7 +163,7 @@ def moe_a8(X, W, sorted_ids, expert_ids, n_post_pad, qtype, N, top_k, tokens):
     K = X.shape[1]
     Y = torch.empty((tokens * top_k, N), dtype=X.dtype, device=X.device)
     n_sorted = sorted_ids.numel()
-    nbytes = lib().gguf_b200_workspace_bytes(OP_MOE, qtype, n_sorted, N, K)
+    nbytes = lib().gguf_b200_scratch_bytes(OP_MOE, qtype, n_sorted, N, K)
     ws = _ws(X, nbytes)
     _check(lib().gguf_b200_moe_a8(X.data_ptr(), W.data_ptr(), Y.data_ptr(), ws.data_ptr(), nbytes, sorted_ids.data_ptr(),
                                   expert_ids.data_ptr(), n_post_pad.data_ptr(), n_sorted, W.stride(0), W.shape[0], qtype,
@@ -282,7 +282,7 @@ def matmul_tp(op, W_local, X, y_ptrs, flag_ptrs, epochs_local, slot, qtype, rank
     world = len(y_ptrs)
     M, K = X.shape
     n_local = W_local.shape[0]
-    nbytes = lib().gguf_b200_workspace_bytes(op, qtype, M, n_local, K)
+    nbytes = lib().gguf_b200_scratch_bytes(op, qtype, M, n_local, K)
     ws = _ws(X, nbytes)
     k1, ya = _ptr_array(y_ptrs)
     k2, fa = _ptr_array(flag_ptrs)
