@@ -37,8 +37,8 @@
 // clocks because a B slot came back 745 clocks after its MMA and refilling it took 1,050 more, over a ring of four.
 // tcgen05.mma itself takes max(61, tn / 2) clocks per 16 values, so at 128 tokens or less a stage need not take more than 256;
 // it takes about 350 with the whole-stage decoders, 600 to 1,000 with the others, which is what bounds those.
-// Measured, before -> after: IQ3_S 8192 x 28672, 300 tokens 291 -> 149 us; Q6_K 37888 x 3584, 1999 tokens 668 -> 587 us;
-// IQ2_XXS 28672 x 8192, 128 tokens 108 -> 95 us; a MoE step of 256 tokens (64 experts, Q4_0) 222 -> 172 us.
+// Measured, before -> after: IQ3_S 8192 x 28672, 300 tokens 291 -> 134 us; Q6_K 37888 x 3584, 1999 tokens 668 -> 567 us;
+// IQ2_XXS 28672 x 8192, 128 tokens 108 -> 95 us; a MoE step of 256 tokens (64 experts, Q4_0) 222 -> 169 us.
 #include "mmq_kernel.cuh"
 
 namespace gguf_b200 {
