@@ -1,0 +1,223 @@
+// The functions of an eager call: plain Python functions over the C-ABI of libgguf_b200, the same bodies as the registered
+// operators (op_calls.h).  A decode GEMV runs for 3 to 8 us on the device, and the dispatcher with its boxed arguments
+// costs more host time than that per call (a 3072 x 1024 matrix, one token: 12.6 us per call through two registered
+// operators, of which the kernel is 3.3).  They answer None whenever the tensors are not plain CUDA tensors (tracing, fake
+// tensors, dispatch modes), and the caller then takes the registered operator.
+//
+// They take tensors apart that Python holds, with torch's own C++ interface, so this module is tied to one Python and to
+// the torch it was built against; it refuses to load next to another one, and calls then go through the operators
+// (native.py).
+#include <Python.h>
+
+#include <ATen/core/Tensor.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
+#include <c10/cuda/CUDACachingAllocator.h>
+#include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Dtype.h>
+#include <torch/csrc/DynamicTypes.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/python_variable.h>
+#include <torch/headeronly/version.h>
+
+#include "op_calls.h"
+
+using at::ScalarType;
+using at::Tensor;
+
+namespace {
+
+struct Eager {
+  using Tensor = at::Tensor;
+  using Guard = c10::cuda::CUDAGuard;
+  static c10::DeviceIndex device(const Tensor& t) { return t.get_device(); }
+  static void* stream(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(device(t)).stream(); }
+  static Tensor empty(const Tensor& like, at::IntArrayRef sizes, ScalarType t) { return at::detail::empty_cuda(sizes, t, like.device(), std::nullopt); }
+  // scratch memory of one call, given back to the stream's pool when the call returns
+  struct Scratch {
+    c10::DataPtr p;
+    Scratch(const Tensor&, int64_t bytes) : p(c10::cuda::CUDACachingAllocator::get()->allocate((size_t)(bytes > 0 ? bytes : 1))) {}
+    void* get() const { return p.get(); }
+  };
+};
+using Op = gguf_ops::Calls<Eager>;
+
+// Nothing between Python and the kernel wants to see the call: no tracing, functionalization or
+// dispatch mode, no tensor subclass.
+bool modes_off() {
+  if (c10::impl::TorchDispatchModeTLS::any_modes_set()) return false;
+  const auto inc = c10::impl::tls_local_dispatch_key_set().included_;
+  return !inc.has_any(c10::DispatchKeySet({c10::DispatchKey::Python, c10::DispatchKey::Functionalize, c10::DispatchKey::FuncTorchDynamicLayerFrontMode}));
+}
+const Tensor* plain_cuda(PyObject* o) {
+  if (!THPVariable_Check(o)) return nullptr;
+  const Tensor& t = THPVariable_Unpack(o);
+  if (!t.defined() || !t.is_cuda()) return nullptr;
+  const c10::DispatchKeySet odd({c10::DispatchKey::Python, c10::DispatchKey::PythonTLSSnapshot, c10::DispatchKey::Functionalize,
+                                 c10::DispatchKey::FuncTorchBatched, c10::DispatchKey::FuncTorchGradWrapper});
+  return t.key_set().has_any(odd) ? nullptr : &t;
+}
+
+// mul_mat(W, X, type, row, op): the three dense products
+PyObject* py_mul_mat(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  TORCH_CHECK(n == 5, "mul_mat takes 5 arguments");
+  const Tensor *W = plain_cuda(a[0]), *X = plain_cuda(a[1]);
+  if (!W || !X || !modes_off()) Py_RETURN_NONE;
+  const long type = PyLong_AsLong(a[2]), row = PyLong_AsLong(a[3]), op = PyLong_AsLong(a[4]);
+  if (PyErr_Occurred()) return nullptr;
+  TORCH_CHECK(op == GGUF_B200_OP_GEMV || op == GGUF_B200_OP_MMQ || op == GGUF_B200_OP_DEQUANT_MATMUL, "mul_mat: unknown op");
+  static const char* const names[] = {"ggml_mul_mat_vec_a8", "ggml_mul_mat_a8", "", "", "dequant_matmul"};
+  return THPVariable_Wrap(Op::mul_mat(*W, *X, type, row, (int)op, names[op]));
+  END_HANDLE_TH_ERRORS
+}
+
+// embed(ids, W, type, hidden, dtype): the embedding look-up, result shaped [*ids.shape, hidden]
+PyObject* py_embed(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  TORCH_CHECK(n == 5, "embed takes 5 arguments");
+  const Tensor *ids = plain_cuda(a[0]), *W = plain_cuda(a[1]);
+  if (!ids || !W || !modes_off() || ids->scalar_type() != ScalarType::Long || !ids->is_contiguous() || W->dim() != 2) Py_RETURN_NONE;
+  const long type = PyLong_AsLong(a[2]), hidden = PyLong_AsLong(a[3]);
+  if (PyErr_Occurred()) return nullptr;
+  const ScalarType dt = THPDtype_Check(a[4]) ? reinterpret_cast<THPDtype*>(a[4])->scalar_type : ScalarType::Half;
+  const c10::cuda::CUDAGuard guard(W->device());
+  const int64_t K = Op::check_weight(*W, type, "embed");
+  if (K != hidden || K % 256 != 0 || ids->device() != W->device()) Py_RETURN_NONE;
+  const int code = gguf_ops::dtype_code(dt, "embed");
+  c10::SmallVector<int64_t, 4> shape(ids->sizes().begin(), ids->sizes().end());
+  shape.push_back(hidden);
+  Tensor out = Eager::empty(*W, shape, dt);
+  Op::rows_into(*W, *ids, type, K, out, code);
+  return THPVariable_Wrap(std::move(out));
+  END_HANDLE_TH_ERRORS
+}
+
+// The batch-size rule of the linear dispatcher (quantization/linear.py `_fused_mul_mat_gguf`): the
+// operation that serves M rows against N weight rows of `type`, or -1 where only Python does.
+bool imatrix_type(int64_t t) { return t == 16 || t == 17 || t == 18 || t == 19 || t == 20 || t == 21 || t == 22 || t == 23 || t == 29; }
+int linear_op(int64_t type, int64_t M, int64_t N, ScalarType dt) {
+  const bool im = imatrix_type(type);
+  const int64_t most = im ? (N > 5120 ? 8 : 16) : (N > 5120 ? 2 : 6);
+  if (M <= most) return GGUF_B200_OP_GEMV;
+  if (!im) return GGUF_B200_OP_MMQ;
+  const bool fused = dt == ScalarType::Half || dt == ScalarType::BFloat16;
+  return fused ? GGUF_B200_OP_DEQUANT_MATMUL : -1;
+}
+
+// linear(x, W, type): one layer's product, routed as the dispatcher routes it
+PyObject* py_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  TORCH_CHECK(n == 3, "linear takes 3 arguments");
+  const Tensor *X = plain_cuda(a[0]), *W = plain_cuda(a[1]);
+  if (!W || !X || X->dim() != 2 || W->dim() != 2 || X->size(0) == 0 || !modes_off()) Py_RETURN_NONE;
+  const long type = PyLong_AsLong(a[2]);
+  if (PyErr_Occurred()) return nullptr;
+  if (gguf_b200_type_size((int)type) == 0) Py_RETURN_NONE;
+  const int64_t N = W->size(0);
+  const int op = linear_op(type, X->size(0), N, X->scalar_type());
+  if (op < 0) Py_RETURN_NONE;
+  return THPVariable_Wrap(Op::mul_mat(*W, *X, type, N, op, "linear"));
+  END_HANDLE_TH_ERRORS
+}
+
+// linear_runs(x, W, runs): a layer whose rows are of several types, stacked in W and padded to its width.  runs: a flat tuple of
+// (type, first row, rows, bytes of a row, rows that decide the routing) per run.  Every run is multiplied where it lies, into its columns of one result.
+PyObject* py_linear_runs(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  TORCH_CHECK(n == 3 && PyTuple_Check(a[2]) && PyTuple_GET_SIZE(a[2]) % 5 == 0, "linear_runs takes x, W and a tuple of runs");
+  const Tensor *X = plain_cuda(a[0]), *W = plain_cuda(a[1]);
+  if (!W || !X || X->dim() != 2 || W->dim() != 2 || X->size(0) == 0 || !modes_off() || !X->is_contiguous() || !W->is_contiguous() ||
+      W->scalar_type() != ScalarType::Byte)
+    Py_RETURN_NONE;
+  const ScalarType dt = X->scalar_type();
+  if (dt != ScalarType::Float && dt != ScalarType::Half && dt != ScalarType::BFloat16) Py_RETURN_NONE;
+  struct Run { int type, op; int64_t row, rows, ws; };
+  c10::SmallVector<Run, 4> runs;
+  const int64_t M = X->size(0), K = X->size(1), pitch = W->size(1);
+  int64_t N = 0, most = 0;
+  for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(a[2]); i += 5) {
+    long v[5];
+    for (int j = 0; j < 5; ++j) v[j] = PyLong_AsLong(PyTuple_GET_ITEM(a[2], i + j));
+    if (PyErr_Occurred()) return nullptr;
+    const int ts = gguf_b200_type_size((int)v[0]);
+    if (ts == 0 || v[3] % ts != 0 || v[3] / ts * gguf_b200_block_size((int)v[0]) != K || v[1] < 0 || v[1] + v[2] > W->size(0) || v[1] * pitch % 16 != 0)
+      Py_RETURN_NONE;
+    const int op = linear_op(v[0], M, v[4], dt);
+    if (op < 0) Py_RETURN_NONE;
+    const int64_t ws = gguf_b200_scratch_bytes(op, (int)v[0], M, v[2], K);
+    most = ws > most ? ws : most;
+    runs.push_back({(int)v[0], op, v[1], v[2], ws});
+    N += v[2];
+  }
+  if (N == 0) Py_RETURN_NONE;
+  const c10::cuda::CUDAGuard guard(X->device());
+  Tensor Y = Eager::empty(*X, {M, N}, dt);
+  const Eager::Scratch ws(*X, most);
+  const int code = gguf_ops::dtype_code(dt, "linear_runs");
+  void* s = Eager::stream(*X);
+  int64_t col = 0;
+  for (const Run& r : runs) {
+    uint8_t* y = static_cast<uint8_t*>(Y.data_ptr()) + col * Y.element_size();
+    if (reinterpret_cast<uintptr_t>(y) % 16 != 0) Py_RETURN_NONE;
+    const int rc = gguf_b200_mul_mat_strided(static_cast<const uint8_t*>(W->data_ptr()) + r.row * pitch, X->data_ptr(), y, ws.get(), most, r.op, r.type,
+                                             code, M, r.rows, K, pitch, N, s);
+    if (rc == GGUF_B200_E_SHAPE || rc == GGUF_B200_E_TOO_LARGE) Py_RETURN_NONE;   // a layout that only copies can serve
+    gguf_ops::check_rc(rc, "linear_runs");
+    col += r.rows;
+  }
+  return THPVariable_Wrap(std::move(Y));
+  END_HANDLE_TH_ERRORS
+}
+
+// moe(x, W13, W2, topk_weights, topk_ids, type13, type2, act): the whole expert step
+PyObject* py_moe(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  TORCH_CHECK(n == 8, "moe takes 8 arguments");
+  const Tensor* t[5];
+  for (int i = 0; i < 5; ++i)
+    if (!(t[i] = plain_cuda(a[i]))) Py_RETURN_NONE;
+  if (!modes_off()) Py_RETURN_NONE;
+  const long type13 = PyLong_AsLong(a[5]), type2 = PyLong_AsLong(a[6]), act = PyLong_AsLong(a[7]);
+  if (PyErr_Occurred()) return nullptr;
+  return THPVariable_Wrap(Op::fused_moe(*t[0], *t[1], *t[2], *t[3], *t[4], type13, type2, act));
+  END_HANDLE_TH_ERRORS
+}
+
+PyMethodDef methods[] = {
+    {"moe", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(&py_moe)), METH_FASTCALL, nullptr},
+    {"mul_mat", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(&py_mul_mat)), METH_FASTCALL, nullptr},
+    {"embed", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(&py_embed)), METH_FASTCALL, nullptr},
+    {"linear_runs", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(&py_linear_runs)), METH_FASTCALL, nullptr},
+    {"linear", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(&py_linear)), METH_FASTCALL, nullptr},
+    {nullptr, nullptr, 0, nullptr},
+};
+PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_eager", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+extern "C" PyObject* PyInit__eager(void) {
+  // (the file's name says which Python; the symbols alone do not say which torch)
+  PyObject* torch = PyImport_ImportModule("torch");
+  if (!torch) return nullptr;
+  PyObject* version = PyObject_GetAttrString(torch, "__version__");
+  Py_DECREF(torch);
+  if (!version) return nullptr;
+  PyObject* text = PyObject_Str(version);
+  Py_DECREF(version);
+  const char* have = text ? PyUnicode_AsUTF8(text) : nullptr;
+  if (!have) {
+    Py_XDECREF(text);
+    return nullptr;
+  }
+  const std::string built = TORCH_VERSION, run = std::string(have).substr(0, std::string(have).find('+'));
+  Py_DECREF(text);
+  if (run != built) {
+    PyErr_Format(PyExc_ImportError, "built for torch %s, this is %s", built.c_str(), run.c_str());
+    return nullptr;
+  }
+  return PyModule_Create(&module_def);
+}

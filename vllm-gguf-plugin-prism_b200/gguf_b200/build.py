@@ -2,7 +2,8 @@
 
 Outputs, next to the Python package they serve (git-ignored, shipped with the tree):
   vllm_gguf_plugin/libgguf_b200.so   the C-ABI kernel library (include/gguf_b200.h)
-  vllm_gguf_plugin/_C_gguf.abi3.so   torch library `_C_gguf` and the module's eager functions, calling the C-ABI
+  vllm_gguf_plugin/_C_gguf.abi3.so   torch library `_C_gguf` (torch's stable ABI, any Python), calling the C-ABI
+  vllm_gguf_plugin/_eager<suffix>    the functions eager calls go through (this Python, this torch)
 
 quantize_q8_1.cu and gemv1.cu (the decode GEMV that quantizes its activations itself) are
 compiled with --use_fast_math: the two fp32 divisions of the q8_1 quantization must be the same
@@ -75,24 +76,29 @@ def build_kernels(force: bool = False, verbose: bool = False) -> Path:
     return so
 
 
-def build_torch_shim(force: bool = False) -> Path:
+def _cxx(src: Path, so: Path, force: bool, flags, libs) -> Path:
     import torch
 
     troot = Path(torch.__file__).parent
-    so = OUT / "_C_gguf.abi3.so"
-    src = CSRC / "torch_shim.cpp"
-    if not force and not _stale(so, [src, PKG.parent / "include" / "gguf_b200.h"]):
-        return so
-    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-DUSE_CUDA", str(src), "-o", str(so),
-           f"-I{troot / 'include'}", f"-I{sysconfig.get_paths()['include']}", f"-I{CUDA}/include",
-           f"-L{OUT}", "-lgguf_b200", f"-L{troot / 'lib'}", "-ltorch_python", "-ltorch", "-ltorch_cuda", "-ltorch_cpu", "-lc10_cuda", "-lc10",
-           "-Wl,-rpath,$ORIGIN", f"-Wl,-rpath,{troot / 'lib'}"]
-    subprocess.check_call(cmd)
+    if force or _stale(so, [*_includes(src), PKG.parent / "include" / "gguf_b200.h"]):
+        subprocess.check_call(
+            ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-DUSE_CUDA", *flags, str(src), "-o", str(so), f"-I{troot / 'include'}",
+             f"-I{sysconfig.get_paths()['include']}", f"-I{CUDA}/include", f"-L{OUT}", "-lgguf_b200", f"-L{troot / 'lib'}",
+             *(f"-l{n}" for n in libs), "-Wl,-rpath,$ORIGIN", f"-Wl,-rpath,{troot / 'lib'}"])
     return so
 
 
+def build_torch_shim(force: bool = False) -> Path:
+    return _cxx(CSRC / "torch_shim.cpp", OUT / "_C_gguf.abi3.so", force, ["-DPy_LIMITED_API=0x03090000"], ["torch", "torch_cpu", "c10"])
+
+
+def build_eager(force: bool = False) -> Path:
+    return _cxx(CSRC / "eager.cpp", OUT / ("_eager" + sysconfig.get_config_var("EXT_SUFFIX")), force, [],
+                ["torch_python", "torch", "torch_cuda", "torch_cpu", "c10_cuda", "c10"])
+
+
 def build_all(force: bool = False, verbose: bool = False):
-    return build_kernels(force, verbose), build_torch_shim(force)
+    return build_kernels(force, verbose), build_torch_shim(force), build_eager(force)
 
 
 if __name__ == "__main__":

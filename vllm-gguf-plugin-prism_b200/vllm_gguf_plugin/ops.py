@@ -61,6 +61,8 @@ except ImportError as exc:  # no silent fallback: the CUDA extension IS the prod
         "`python vllm-gguf-plugin-prism_b200/gguf_b200/build.py` from the repository root"
     ) from exc
 
+from . import native  # noqa: E402
+
 _CUDA_AVAILABLE = True
 _CUDA_ENABLED = True
 _OP_GEMV, _OP_MMQ, _OP_DEQUANT_MATMUL = 0, 1, 4   # GGUF_B200_OP_* of include/gguf_b200.h
@@ -159,7 +161,7 @@ def _ggml_moe_a8_vec_fake(X, W, topk_ids, top_k, quant_type, row, tokens):
 def _mul_mat(W, X, quant_type, row, op):
     """An eager product without the dispatcher's overhead; None while compiling or tracing, and for anything that is not
     a plain CUDA tensor."""
-    return None if is_compiling() else _C_gguf.mul_mat(W, X, quant_type, row, op)
+    return None if is_compiling() else native.mul_mat(W, X, quant_type, row, op)
 
 
 def ggml_dequantize(W: torch.Tensor, quant_type: int, m: int, n: int, dtype: torch.dtype | None) -> torch.Tensor:
@@ -225,7 +227,7 @@ def ggml_fused_moe(X: torch.Tensor, W13: torch.Tensor, W2: torch.Tensor, topk_we
     if topk_ids.dtype != torch.int32 or not topk_ids.is_contiguous():
         topk_ids = topk_ids.to(torch.int32).contiguous()
     act = MOE_ACTIVATIONS[activation]
-    y = None if is_compiling() else _C_gguf.moe(X, W13, W2, topk_weights, topk_ids, quant_type, quant_type2, act)
+    y = None if is_compiling() else native.moe(X, W13, W2, topk_weights, topk_ids, quant_type, quant_type2, act)
     return torch.ops._C_gguf.fused_moe(X, W13, W2, topk_weights, topk_ids, quant_type, quant_type2, act) if y is None else y
 
 

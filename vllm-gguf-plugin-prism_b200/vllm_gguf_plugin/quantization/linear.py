@@ -15,8 +15,7 @@ from __future__ import annotations
 import torch
 from torch.compiler import is_compiling
 
-from .. import ops
-from .._C_gguf import linear as _native_linear, linear_runs as _native_runs
+from .. import native, ops
 from .utils import (
     DEQUANT_TYPES,
     IMATRIX_QUANT_TYPES,
@@ -232,7 +231,7 @@ class GGUFLinearMethod(LinearMethodBase):
             # the layers in between (custom op, operator dispatch), which cost more than a decode GEMV runs for.
             weight = layer.weight
             one_type = weight.gguf_one_type if weight.shard_id else layer.weight_type.weight_type
-            out = _native_linear(x, weight, one_type) if one_type is not None else _native_runs(x, weight, weight.gguf_runs)
+            out = native.linear(x, weight, one_type) if one_type is not None else native.linear_runs(x, weight, weight.gguf_runs)
             if out is not None:
                 return out if bias is None else out.add_(bias)
         shard_id = layer.weight.shard_id

@@ -11,8 +11,7 @@ from __future__ import annotations
 import torch
 from torch.compiler import is_compiling
 
-from .. import ops
-from .._C_gguf import embed as _native_embed
+from .. import native, ops
 from .utils import DEQUANT_TYPES, UNQUANTIZED_TYPES, quant_sizes
 
 
@@ -21,7 +20,7 @@ def _apply_gguf_embedding(x: torch.Tensor, weight: torch.Tensor, weight_type: in
     if weight_type in UNQUANTIZED_TYPES:
         return torch.embedding(weight, x)
     if weight_type in DEQUANT_TYPES:
-        out = None if is_compiling() else _native_embed(x, weight, weight_type, hidden_size, dtype)
+        out = None if is_compiling() else native.embed(x, weight, weight_type, hidden_size, dtype)
         if out is not None:
             return out
         block_size, type_size = quant_sizes(weight_type)
