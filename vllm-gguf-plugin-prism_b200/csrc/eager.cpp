@@ -45,6 +45,22 @@ struct Eager {
 };
 using Op = gguf_ops::Calls<Eager>;
 
+// Allocation and launches run without the GIL, as an operator's do: cudaMalloc takes a lock and may wait for the device, and
+// a launch waits as soon as a thousand are queued (a thread that launches into a full queue held all others for the 0.6 s it
+// took to drain).  What is used meanwhile belongs to this call: handles of the tensors, taken while the GIL was held.
+struct NoGil {
+  PyThreadState* state = PyEval_SaveThread();
+  ~NoGil() { PyEval_RestoreThread(state); }
+};
+template <class F> Tensor without_gil(F&& body) {
+  Tensor out;
+  {
+    const NoGil release;
+    out = body();
+  }
+  return out;
+}
+
 // Nothing between Python and the kernel wants to see the call: no tracing, functionalization or
 // dispatch mode, no tensor subclass.
 bool modes_off() {
@@ -71,7 +87,8 @@ PyObject* py_mul_mat(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (PyErr_Occurred()) return nullptr;
   TORCH_CHECK(op == GGUF_B200_OP_GEMV || op == GGUF_B200_OP_MMQ || op == GGUF_B200_OP_DEQUANT_MATMUL, "mul_mat: unknown op");
   static const char* const names[] = {"ggml_mul_mat_vec_a8", "ggml_mul_mat_a8", "", "", "dequant_matmul"};
-  return THPVariable_Wrap(Op::mul_mat(*W, *X, type, row, (int)op, names[op]));
+  const Tensor w = *W, x = *X;
+  return THPVariable_Wrap(without_gil([&] { return Op::mul_mat(w, x, type, row, (int)op, names[op]); }));
   END_HANDLE_TH_ERRORS
 }
 
@@ -84,15 +101,18 @@ PyObject* py_embed(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const long type = PyLong_AsLong(a[2]), hidden = PyLong_AsLong(a[3]);
   if (PyErr_Occurred()) return nullptr;
   const ScalarType dt = THPDtype_Check(a[4]) ? reinterpret_cast<THPDtype*>(a[4])->scalar_type : ScalarType::Half;
-  const c10::cuda::CUDAGuard guard(W->device());
   const int64_t K = Op::check_weight(*W, type, "embed");
   if (K != hidden || K % 256 != 0 || ids->device() != W->device()) Py_RETURN_NONE;
   const int code = gguf_ops::dtype_code(dt, "embed");
   c10::SmallVector<int64_t, 4> shape(ids->sizes().begin(), ids->sizes().end());
   shape.push_back(hidden);
-  Tensor out = Eager::empty(*W, shape, dt);
-  Op::rows_into(*W, *ids, type, K, out, code);
-  return THPVariable_Wrap(std::move(out));
+  const Tensor w = *W, rows = *ids;
+  return THPVariable_Wrap(without_gil([&] {
+    const Eager::Guard guard(Eager::device(w));
+    Tensor out = Eager::empty(w, shape, dt);
+    Op::rows_into(w, rows, type, K, out, code);
+    return out;
+  }));
   END_HANDLE_TH_ERRORS
 }
 
@@ -120,7 +140,8 @@ PyObject* py_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const int64_t N = W->size(0);
   const int op = linear_op(type, X->size(0), N, X->scalar_type());
   if (op < 0) Py_RETURN_NONE;
-  return THPVariable_Wrap(Op::mul_mat(*W, *X, type, N, op, "linear"));
+  const Tensor w = *W, x = *X;
+  return THPVariable_Wrap(without_gil([&] { return Op::mul_mat(w, x, type, N, op, "linear"); }));
   END_HANDLE_TH_ERRORS
 }
 
@@ -154,22 +175,27 @@ PyObject* py_linear_runs(PyObject*, PyObject* const* a, Py_ssize_t n) {
     N += v[2];
   }
   if (N == 0) Py_RETURN_NONE;
-  const c10::cuda::CUDAGuard guard(X->device());
-  Tensor Y = Eager::empty(*X, {M, N}, dt);
-  const Eager::Scratch ws(*X, most);
+  const Tensor w = *W, x = *X;
   const int code = gguf_ops::dtype_code(dt, "linear_runs");
-  void* s = Eager::stream(*X);
-  int64_t col = 0;
-  for (const Run& r : runs) {
-    uint8_t* y = static_cast<uint8_t*>(Y.data_ptr()) + col * Y.element_size();
-    if (reinterpret_cast<uintptr_t>(y) % 16 != 0) Py_RETURN_NONE;
-    const int rc = gguf_b200_mul_mat_strided(static_cast<const uint8_t*>(W->data_ptr()) + r.row * pitch, X->data_ptr(), y, ws.get(), most, r.op, r.type,
-                                             code, M, r.rows, K, pitch, N, s);
-    if (rc == GGUF_B200_E_SHAPE || rc == GGUF_B200_E_TOO_LARGE) Py_RETURN_NONE;   // a layout that only copies can serve
-    gguf_ops::check_rc(rc, "linear_runs");
-    col += r.rows;
-  }
-  return THPVariable_Wrap(std::move(Y));
+  Tensor out = without_gil([&]() -> Tensor {   // undefined: a layout that only copies can serve
+    const Eager::Guard guard(Eager::device(x));
+    Tensor Y = Eager::empty(x, {M, N}, dt);
+    const Eager::Scratch ws(x, most);
+    void* s = Eager::stream(x);
+    int64_t col = 0;
+    for (const Run& r : runs) {
+      uint8_t* y = static_cast<uint8_t*>(Y.data_ptr()) + col * Y.element_size();
+      if (reinterpret_cast<uintptr_t>(y) % 16 != 0) return Tensor();
+      const int rc = gguf_b200_mul_mat_strided(static_cast<const uint8_t*>(w.data_ptr()) + r.row * pitch, x.data_ptr(), y, ws.get(), most, r.op, r.type,
+                                               code, M, r.rows, K, pitch, N, s);
+      if (rc == GGUF_B200_E_SHAPE || rc == GGUF_B200_E_TOO_LARGE) return Tensor();
+      gguf_ops::check_rc(rc, "linear_runs");
+      col += r.rows;
+    }
+    return Y;
+  });
+  if (!out.defined()) Py_RETURN_NONE;
+  return THPVariable_Wrap(std::move(out));
   END_HANDLE_TH_ERRORS
 }
 
@@ -177,13 +203,16 @@ PyObject* py_linear_runs(PyObject*, PyObject* const* a, Py_ssize_t n) {
 PyObject* py_moe(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   TORCH_CHECK(n == 8, "moe takes 8 arguments");
-  const Tensor* t[5];
-  for (int i = 0; i < 5; ++i)
-    if (!(t[i] = plain_cuda(a[i]))) Py_RETURN_NONE;
+  Tensor t[5];
+  for (int i = 0; i < 5; ++i) {
+    const Tensor* p = plain_cuda(a[i]);
+    if (!p) Py_RETURN_NONE;
+    t[i] = *p;
+  }
   if (!modes_off()) Py_RETURN_NONE;
   const long type13 = PyLong_AsLong(a[5]), type2 = PyLong_AsLong(a[6]), act = PyLong_AsLong(a[7]);
   if (PyErr_Occurred()) return nullptr;
-  return THPVariable_Wrap(Op::fused_moe(*t[0], *t[1], *t[2], *t[3], *t[4], type13, type2, act));
+  return THPVariable_Wrap(without_gil([&] { return Op::fused_moe(t[0], t[1], t[2], t[3], t[4], type13, type2, act); }));
   END_HANDLE_TH_ERRORS
 }
 
