@@ -14,6 +14,12 @@
  * 18 (IQ3_XXS), 19 (IQ1_S), 21 (IQ3_S), 22 (IQ2_S), 29 (IQ1_M) -- all nineteen block types of the reference's dispatch.
  * Weights W are raw GGUF blocks, row-major `uint8 [N][K/QK*type_size]`, base 16-byte aligned.
  * Activations X are `[M][K]` contiguous in `dtype`; outputs Y are `[M][N]` in the same dtype.
+ *
+ * Stream order: X, Y and the workspace follow the stream as usual.  Weights may be read ahead of it: gguf_b200_mul_mat_vec_a8
+ * with one vector, gguf_b200_gemv_prepared and gguf_b200_dequant_matmul (plain, strided or tensor-parallel) start on W while the
+ * kernel ahead of them in the stream is still finishing.  A host that writes weights on the device (loading, merging an
+ * adapter) queues any other kernel behind the writes, or synchronises, before it uses them; where W comes straight out of a
+ * kernel, it calls gguf_b200_mul_mat_strided with GGUF_B200_W_IN_FLIGHT.  All other entry points read W in stream order.
  */
 #ifndef GGUF_B200_H
 #define GGUF_B200_H
@@ -40,6 +46,9 @@ enum {
 
 enum { GGUF_B200_OP_GEMV = 0, GGUF_B200_OP_MMQ = 1, GGUF_B200_OP_MOE = 2, GGUF_B200_OP_MOE_VEC = 3,
        GGUF_B200_OP_DEQUANT_MATMUL = 4 };
+/* added to the op of gguf_b200_mul_mat_strided: W may be written by the work directly ahead in the stream; no byte of it is
+ * read before that is complete */
+enum { GGUF_B200_W_IN_FLIGHT = 0x100 };
 
 const char* gguf_b200_error_string(int code);
 const char* gguf_b200_version(void);

@@ -138,3 +138,13 @@ def test_ops_module_fails_loudly_without_extension(tmp_path, monkeypatch):
         for k in [k for k in sys.modules if k.split(".")[0] == "vllm_gguf_plugin"]:
             del sys.modules[k]
         sys.modules.update(saved)
+
+
+def test_quantizers_let_the_product_start_only_behind_their_own_wait():
+    """A product reads weights as soon as it starts, so the quantizer ahead of it must not release it (pdl_trigger) before the
+    work ahead of the call -- a kernel that wrote those weights, for one -- is complete (pdl_wait)."""
+    src = (ROOT / "vllm-gguf-plugin-prism_b200" / "csrc" / "quantize_q8_1.cu").read_text()
+    kernels = re.split(r"^__global__", src, flags=re.M)[1:]
+    assert len(kernels) == 3
+    for k in kernels:
+        assert 0 < k.index("pdl_wait();") < k.index("pdl_trigger();")

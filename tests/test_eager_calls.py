@@ -78,3 +78,66 @@ def test_other_threads_run_while_a_call_waits_for_the_launch_queue(native_libs, 
     seen = [t0, *(t for t in ticks if t0 <= t <= t1), t1]
     assert t1 - t0 > 0.2, "the queue never filled up"
     assert max(b - a for a, b in zip(seen, seen[1:])) < 0.5 * (t1 - t0)
+
+
+# (operation, tokens, K): the one-launch and the two-launch GEMV, two vectors, the small-batch kernel, the tiled one, the GEMM
+# on plain activations with whole tiles and with shared ones, the GEMV per routed expert
+IN_FLIGHT = [("vec", "Q4_K", 1, 1024), ("vec", "Q6_K", 1, 8192), ("vec", "Q8_0", 2, 1024), ("vec", "IQ4_XS", 5, 1024), ("mmq", "Q4_K", 8, 1024),
+             ("mmq", "Q6_K", 40, 2048), ("dqmm", "IQ2_XXS", 300, 1024), ("dqmm", "IQ4_XS", 20, 4096), ("moe_vec", "Q4_0", 3, 1024)]
+
+
+@pytest.mark.parametrize("eager", [True, False])
+@pytest.mark.parametrize("case", IN_FLIGHT)
+def test_products_of_weights_that_a_kernel_has_just_written(native_libs, case, eager):
+    """Weights that come straight out of a kernel are read behind it, through the functions and through the operators."""
+    from helpers import TYPES
+    from vllm_gguf_plugin import ops
+
+    kind, name, M, K = case
+    t, N, E = TYPES[name], 4096, 4 if kind == "moe_vec" else 1
+    ws = [weight(t, N * E, K, seed=s) for s in (1, 2)]
+    x = torch.randn(M, K, device=DEV).half()
+    ids = torch.arange(M * 2, device=DEV, dtype=torch.int32).view(M, 2) % E
+    op = torch.ops._C_gguf
+
+    def product(w):
+        if kind == "moe_vec":
+            return ops.ggml_moe_a8_vec(x, w.view(E, N, -1), ids, 2, t, N, M)
+        if eager:
+            return {"vec": ops.ggml_mul_mat_vec_a8, "mmq": ops.ggml_mul_mat_a8, "dqmm": ops.ggml_dequant_matmul}[kind](w, x, t, N)
+        return {"vec": op.ggml_mul_mat_vec_a8, "mmq": op.ggml_mul_mat_a8, "dqmm": op.dequant_matmul}[kind](w, x, t, N)
+
+    want = []
+    for w in ws:
+        torch.cuda.synchronize()
+        want.append(product(w))
+    buf = torch.empty_like(ws[0])
+    torch.cuda.synchronize()
+    got = []
+    for i in range(40):
+        buf.copy_(ws[i & 1])
+        got.append(product(buf))
+    torch.cuda.synchronize()
+    assert capi.last_status() == 0
+    assert all(torch.equal(y, want[i & 1]) for i, y in enumerate(got))
+
+
+def test_first_product_behind_loading_reads_the_loaded_weights(native_libs):
+    """A layer's products may read its weights ahead of the stream, so loading puts a kernel of its own behind the writes."""
+    from vllm_gguf_plugin.quantization.linear import GGUFLinearMethod
+
+    files = [weight(12, 8192, 1024, seed=s) for s in (1, 2)]
+    x = torch.randn(1, 1024, device=DEV).half()
+    want = [capi.mul_mat_vec_a8(w, x, 12, 8192) for w in files]
+    torch.cuda.synchronize()
+    got = []
+    for i in range(40):
+        w, method, layer = files[i & 1], GGUFLinearMethod(None), torch.nn.Module()
+        method.create_weights(layer, 1024, [8192], 1024, 8192, torch.float16)
+        for sid, part in ((None, w),) if i % 4 < 2 else ((0, w[:4096]), (1, w[4096:])):
+            layer.weight.weight_loader(layer.weight, part.clone(), sid)
+            layer.weight_type.weight_loader(layer.weight_type, torch.tensor(12), sid)
+        method.process_weights_after_loading(layer)
+        got.append(method.apply(layer, x))
+    torch.cuda.synchronize()
+    assert all(torch.equal(y, want[i & 1]) for i, y in enumerate(got))

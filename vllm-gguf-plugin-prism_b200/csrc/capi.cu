@@ -105,7 +105,7 @@ static int64_t mmq_b_bytes(int type, int64_t M, int64_t K) { return round_up(M *
 
 // The tensor-core GEMM on q8_1 activations (quantize != 0) or on the activations as they are.
 static int tiled_dense(bool quantize, const void* W, const void* X, void* Y, void* ws, int64_t ws_bytes, int type, int dtype, int64_t M, int64_t N,
-                       int64_t K, int64_t pitch, int64_t ldy, const MmqTp* tp, int* st, cudaStream_t s) {
+                       int64_t K, int64_t pitch, int64_t ldy, const MmqTp* tp, int* st, cudaStream_t s, bool w_in_flight = false) {
   MmqArgs a{};
   a.w = W; a.y = Y;
   a.type = type; a.out_dtype = dtype;
@@ -130,6 +130,7 @@ static int tiled_dense(bool quantize, const void* W, const void* X, void* Y, voi
                                         a.counter ? share.n_counters : 0);
     if (rc) return rc;
   } else {
+    a.w_in_flight = w_in_flight;
     a.b = X; a.b_dtype = dtype; a.ldb = K;
     a.corr_mode = CORR_NONE;
     a.zero_counters = share.n_counters;
@@ -492,6 +493,8 @@ int gguf_b200_dequant_matmul(const void* W, const void* X, void* Y, void* ws, in
 
 int gguf_b200_mul_mat_strided(const void* W, const void* X, void* Y, void* ws, int64_t ws_bytes, int op, int type, int dtype, int64_t M,
                               int64_t N, int64_t K, int64_t pitch, int64_t ldy, void* stream) {
+  const bool in_flight = (op & GGUF_B200_W_IN_FLIGHT) != 0;
+  op &= ~GGUF_B200_W_IN_FLIGHT;
   int rc = check_common(W, X, Y, type, dtype, M, N, K);
   if (rc || M == 0 || N == 0) return rc;
   const int64_t row_bytes = K / block_size(type) * type_size(type);
@@ -505,7 +508,7 @@ int gguf_b200_mul_mat_strided(const void* W, const void* X, void* Y, void* ws, i
     if (!is_dequant_matmul_type(type)) return E_BAD_TYPE;
     if (dtype == DT_F32) return E_BAD_DTYPE;
     if (K % 64 != 0) return E_BAD_SHAPE;
-    return tiled_dense(false, W, X, Y, ws, ws_bytes, type, dtype, M, N, K, pitch, ldy, nullptr, st, s);
+    return tiled_dense(false, W, X, Y, ws, ws_bytes, type, dtype, M, N, K, pitch, ldy, nullptr, st, s, in_flight);
   }
   if (op != GGUF_B200_OP_GEMV && op != GGUF_B200_OP_MMQ) return E_BAD_SHAPE;
   if (op == GGUF_B200_OP_MMQ && !is_mmq_type(type)) return E_BAD_TYPE;
@@ -518,7 +521,7 @@ int gguf_b200_mul_mat_strided(const void* W, const void* X, void* Y, void* ws, i
   // one or two vectors; a single one of a short row is quantized by the GEMV kernel itself
   if (M > 2) return E_TOO_LARGE;
   rc = 1;
-  if (op == GGUF_B200_OP_GEMV) rc = launch_gemv_fused(W, X, Y, type, dtype, M, N, K, sum_mode, st, s, pitch);
+  if (op == GGUF_B200_OP_GEMV) rc = launch_gemv_fused(W, X, Y, type, dtype, M, N, K, sum_mode, st, s, pitch, in_flight);
   if (rc <= 0) return rc;
   rc = launch_quantize_q8_1(X, dtype, ws, M, K, Q8_MODE_SOA, sum_mode, 0, CORR_NONE, nullptr, 1, 0, s);
   if (rc) return rc;

@@ -88,7 +88,7 @@ PyObject* py_mul_mat(PyObject*, PyObject* const* a, Py_ssize_t n) {
   TORCH_CHECK(op == GGUF_B200_OP_GEMV || op == GGUF_B200_OP_MMQ || op == GGUF_B200_OP_DEQUANT_MATMUL, "mul_mat: unknown op");
   static const char* const names[] = {"ggml_mul_mat_vec_a8", "ggml_mul_mat_a8", "", "", "dequant_matmul"};
   const Tensor w = *W, x = *X;
-  return THPVariable_Wrap(without_gil([&] { return Op::mul_mat(w, x, type, row, (int)op, names[op]); }));
+  return THPVariable_Wrap(without_gil([&] { return Op::mul_mat(w, x, type, row, (int)op, names[op], false); }));
   END_HANDLE_TH_ERRORS
 }
 
@@ -141,7 +141,7 @@ PyObject* py_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const int op = linear_op(type, X->size(0), N, X->scalar_type());
   if (op < 0) Py_RETURN_NONE;
   const Tensor w = *W, x = *X;
-  return THPVariable_Wrap(without_gil([&] { return Op::mul_mat(w, x, type, N, op, "linear"); }));
+  return THPVariable_Wrap(without_gil([&] { return Op::mul_mat(w, x, type, N, op, "linear", true); }));
   END_HANDLE_TH_ERRORS
 }
 

@@ -685,6 +685,7 @@ struct G1Params {
   int64_t n, k;
   int bpr;               // blocks per row
   int packed;            // 1: rows lie back to back
+  int w_wait;            // 1: the weights may still be written when the kernel starts
   int pitch;             // units of g1_align bytes between rows (32 bits: a row's address is one wide product)
   int64_t ldy;           // elements between the vectors' results
   int ks, rl;            // K-slices per row, row lanes per CTA (ks * rl <= 8)
@@ -876,6 +877,7 @@ __global__ void __launch_bounds__(G1_WARPS * 32, 2) gemv1_kernel(const G1Params 
   // activations are in registers.  (Filling every stage at once was slower: the memory system
   // serves what is outstanding interleaved, so every warp's FIRST item arrived later and the first
   // dot products with it -- 14336x4096 Q4_K 8.6 us against 8.0 us.)
+  if (p.w_wait) pdl_wait();   // (the weights may still be written)
   int p_it = 0, p_st = 0;
   for (int s = 0; s < p.stages - 1; ++s) {
     if (p_it < my_iters) {
@@ -905,7 +907,7 @@ __global__ void __launch_bounds__(G1_WARPS * 32, 2) gemv1_kernel(const G1Params 
       tab_s[i] = make_uint2(lo, hi);
     }
   }
-  // The weight copies above touch nothing another kernel writes; everything below does.
+  // The copies above read nothing but weights; everything below reads or writes what earlier kernels may use.
   pdl_wait();
   const unsigned tag = p.world > 0 ? (sizeof(out_t) == 2 ? (p.epoch[p.slot] & 0xFFFFu) : p.epoch[p.slot]) : 0u;
   // this lane's units (block offset inside the slice, sub-unit) and their activations
@@ -1276,8 +1278,9 @@ static int launch_g1_out(const G1Params& p, int out_dtype, int mv, cudaStream_t 
 // Returns E_OK, a negative error, or 1 when the shape is outside this kernel's reach.
 int launch_gemv1(const void* w, const void* xq_soa, void* y, int type, int out_dtype, int64_t N, int64_t K, int* status,
                  cudaStream_t stream, const GemvTp* tp, int vectors, const GemvMoe* moe, int vec0, int total_vecs,
-                 const void* x_raw, int x_sum_mode, int64_t pitch, int64_t ldy) {
+                 const void* x_raw, int x_sum_mode, int64_t pitch, int64_t ldy, bool w_in_flight) {
   G1Params p{};
+  p.w_wait = w_in_flight ? 1 : 0;
   p.x_raw = x_raw;
   p.x_sum_mode = x_sum_mode;
   if (vectors != 1 && (vectors != 2 || tp || moe)) return 1;

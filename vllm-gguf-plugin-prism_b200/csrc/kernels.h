@@ -54,7 +54,7 @@ int launch_gemv(const void* w, const void* xq_soa, void* y, int type, int out_dt
 // The whole decode op for M <= 2 vectors in ONE launch (activations quantized inside the GEMV kernel);
 // returns 1 when the shape needs the two-kernel route.
 int launch_gemv_fused(const void* w, const void* x, void* y, int type, int dtype, int64_t M, int64_t N, int64_t K, int sum_mode,
-                      int* status, cudaStream_t stream, int64_t pitch = 0);
+                      int* status, cudaStream_t stream, int64_t pitch = 0, bool w_in_flight = false);
 // One- and two-vector specialisation (gemv1.cu): activations in registers.  Returns 1 when the
 // shape is outside its reach (the caller then uses the general kernel).
 // Tensor-parallel output of the single-vector kernel: every result is sent to all `world` ranks
@@ -74,7 +74,8 @@ struct GemvMoe {
 int launch_gemv1(const void* w, const void* xq_soa, void* y, int type, int out_dtype, int64_t N, int64_t K, int* status,
                  cudaStream_t stream, const GemvTp* tp = nullptr, int vectors = 1, const GemvMoe* moe = nullptr,
                  int vec0 = 0, int total_vecs = 0,    // vec0 / total_vecs: the `vectors` handled are vec0.. of total_vecs in the scratch
-                 const void* x_raw = nullptr, int x_sum_mode = 0, int64_t pitch = 0, int64_t ldy = 0);   // 0: rows back to back, ldy = N
+                 const void* x_raw = nullptr, int x_sum_mode = 0, int64_t pitch = 0, int64_t ldy = 0,    // 0: rows back to back, ldy = N
+                 bool w_in_flight = false);   // the work ahead may still write w: no byte of it is read before that is complete
 // x_raw != null (element type = out_dtype): the activations [vectors or tokens][K] are NOT quantized yet and xq_soa is
 // ignored -- every CTA quantizes what it needs in shared memory (one launch per GEMV); returns 1 if that does not fit.
 // 1 when the q8_1 scratch of this type's GEMV must hold d * sum(q) instead of the fp16 sum of the inputs
@@ -124,6 +125,7 @@ struct MmqArgs {
   const float* row_scale;   // MoE: output row r is multiplied by row_scale[r] (routing weights); null: no scaling
   int* status;
   const MmqTp* tp;          // null: plain output y
+  bool w_in_flight;         // no quantizer is ahead and earlier work may still write w (see pdl_wait)
   // Optional: room for tiles that several CTAs share (mmq_share_bytes).  `counter` must be zero when the kernel starts.
   int* counter;
   int64_t zero_counters;    // > 0: so many words of it are cleared here first

@@ -182,6 +182,7 @@ int launch_mmq(const MmqArgs& a, cudaStream_t stream) {
   p.nbuf = p.tn <= 128 ? 2 : 1;
   p.d_step = 128;
   p.status = a.status;
+  p.w_wait = a.w_in_flight ? 1 : 0;
   p.passes = static_cast<const int4*>(a.passes);
   p.n_passes = a.n_passes;
   p.sorted = a.sorted;

@@ -41,6 +41,7 @@ struct MmqParams {
   int raw_off, aux_off, corr_off;   // shared memory behind the B ring
   uint32_t idesc;
   float* part;            // partial tiles, two slots of 128 x tn per CTA; null: every tile is one CTA's
+  int w_wait;             // the weights may still be written when the kernel starts
   int waste;              // idle chunks of a CTA up to which whole tiles are dealt out all the same
   int* counter;           // arrivals per tile, zero at the start
   int* status;
@@ -260,7 +261,7 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_consta
   const uint32_t tmem_base = *tmem_slot;
   pdl_trigger();   // the next kernel may become resident; it waits for this one before it touches anything
   // What earlier kernels write: the activations (and the work list of a MoE step), and -- cleared, or read until now -- what the
-  // epilogue writes.  Everything else, decoding included, starts before they are done.
+  // epilogue writes.  Everything else, decoding included, starts before they are done (the weights: see pdl_wait).
   const bool moe = p.passes != nullptr;
   if (moe) pdl_wait();
   const int tiles = moe ? *p.n_passes * p.rt : p.rt * p.tt;
@@ -623,6 +624,7 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_consta
     }
   } else if (warp == MMQ_PRODUCER_WARPS + 2) {
     // ---------------- raw-weight loader ----------------
+    if (p.w_wait) pdl_wait();
     int st = 0;
     uint32_t sph = 0;
     while (ok && mmq_next_part(p, q)) {

@@ -81,8 +81,10 @@ template <class A> struct Calls {
     return out;
   }
 
-  // the three dense products (op: GGUF_B200_OP_GEMV, _MMQ, _DEQUANT_MATMUL)
-  static Tensor mul_mat(const Tensor& W, const Tensor& X, int64_t type, int64_t row, int op, const char* name) {
+  // The three dense products (op: GGUF_B200_OP_GEMV, _MMQ, _DEQUANT_MATMUL).  settled: W is a loaded layer's weight, complete
+  // since its loading; any other tensor may come straight out of a kernel, and the calls that read weights ahead of the
+  // stream are told so.
+  static Tensor mul_mat(const Tensor& W, const Tensor& X, int64_t type, int64_t row, int op, const char* name, bool settled) {
     const typename A::Guard guard(A::device(X));
     const int64_t K = check_weight(W, type, name);
     STD_TORCH_CHECK(X.dim() == 2 && X.is_contiguous(), name, ": X must be a contiguous [tokens, K] tensor");
@@ -95,8 +97,13 @@ template <class A> struct Calls {
     const int64_t ws_bytes = gguf_b200_scratch_bytes(op, (int)type, M, row, K);
     const typename A::Scratch ws(X, ws_bytes);
     void* s = A::stream(X);
-    int rc;
-    if (op == GGUF_B200_OP_GEMV)
+    int rc = GGUF_B200_E_TOO_LARGE;
+    if (!settled && (op == GGUF_B200_OP_DEQUANT_MATMUL || (op == GGUF_B200_OP_GEMV && M == 1)))
+      rc = gguf_b200_mul_mat_strided(W.data_ptr(), X.data_ptr(), Y.data_ptr(), ws.get(), ws_bytes, op | GGUF_B200_W_IN_FLIGHT, (int)type, code, M, row,
+                                     K, W.size(W.dim() - 1), row, s);
+    if (rc != GGUF_B200_E_TOO_LARGE)
+      ;   // (rows too long for that form go through a quantizer, which keeps the order)
+    else if (op == GGUF_B200_OP_GEMV)
       rc = gguf_b200_mul_mat_vec_a8(W.data_ptr(), X.data_ptr(), Y.data_ptr(), ws.get(), ws_bytes, (int)type, code, M, row, K, s);
     else if (op == GGUF_B200_OP_MMQ)
       rc = gguf_b200_mul_mat_a8(W.data_ptr(), X.data_ptr(), Y.data_ptr(), ws.get(), ws_bytes, (int)type, code, M, row, K, s);

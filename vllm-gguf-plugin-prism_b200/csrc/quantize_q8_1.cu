@@ -30,8 +30,8 @@ __global__ void __launch_bounds__(256) quantize_q8_1_kernel(const in_t* __restri
                                                             int64_t M, int64_t K, int64_t kpad, int sum_mode,
                                                             int64_t ldb, int corr_mode, const int32_t* __restrict__ gather_ids,
                                                             int64_t gather_div, int64_t gather_limit, Q8Tp tp) {
-  pdl_trigger();  // the consumer kernel may start its weight prefetch now; it waits for this grid before reading
   pdl_wait();     // the activations (and the scratch we overwrite) belong to earlier kernels
+  pdl_trigger();  // not before: the product behind this kernel reads weights as soon as it starts (see pdl_wait)
   // tensor-parallel decode: this launch's number for the GEMV behind it, and the tag of the
   // gathered vector (written by all ranks' GEMV kernels into this rank's memory) that is added to x
   if (MODE == Q8_MODE_SOA && tp.bump && blockIdx.x == 0 && threadIdx.x == 0) *tp.bump += 1u;
@@ -140,8 +140,8 @@ __global__ void __launch_bounds__(256) quantize_f16x8_kernel(const in_t* __restr
                                                              const int32_t* __restrict__ gather_ids, int64_t gather_div,
                                                              int64_t gather_limit, int act, int64_t x_ld, int* __restrict__ zero,
                                                              int64_t n_zero, const int32_t* __restrict__ n_used) {
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();   // (after the wait: see quantize_q8_1_kernel)
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_zero; i += (int64_t)gridDim.x * blockDim.x) zero[i] = 0;
   if (n_used && n_used[1] < M) M = n_used[1];
   const int lane = threadIdx.x & 31, t = lane & 3;
@@ -248,8 +248,8 @@ __global__ void __launch_bounds__(256) quantize_frag_kernel(const in_t* __restri
                                                             int tiles, int nc, int order, int with_sum, int sum_mode, const int32_t* __restrict__ sorted,
                                                             const int32_t* __restrict__ n_used, int x_div, int act, int64_t x_ld,
                                                             int* __restrict__ counters, int n_counters) {
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();   // (after the wait: see quantize_q8_1_kernel)
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_counters; i += gridDim.x * blockDim.x) counters[i] = 0;
   const int used = n_used ? n_used[1] : tiles;                    // column tiles in use

@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(SM_THREADS, 2) smallm_kernel(const __grid_cons
   const bool moe = p.passes != nullptr;
   const bool producer = warp == SM_WARPS;
   pdl_trigger();   // the next kernel may become resident; it waits for this one before it touches anything
-  if (moe || !producer) pdl_wait();   // (the producer of a dense product first asks for weights, which no kernel writes)
+  if (moe || !producer) pdl_wait();   // (the producer of a dense product first asks for weights: see pdl_wait)
   // units: chunk by chunk, row tile by row tile, pass by pass; CTA i owns the units [i * U / G, (i + 1) * U / G)
   // (the host sees to it that U * G fits 31 bits: everything here is 32-bit arithmetic, and divisions are few -- a 64-bit
   // division costs as much as a block of the product)

@@ -42,9 +42,9 @@ using torch::headeronly::ScalarType;
 
 Tensor ggml_dequantize(Tensor W, int64_t type, int64_t m, int64_t n, std::optional<ScalarType> dtype) { return Op::dequantize(W, type, m, n, dtype); }
 Tensor dequantize_rows(Tensor W, Tensor ids, int64_t type, std::optional<ScalarType> dtype) { return Op::dequantize_rows(W, ids, type, dtype); }
-Tensor ggml_mul_mat_vec_a8(Tensor W, Tensor X, int64_t type, int64_t row) { return Op::mul_mat(W, X, type, row, GGUF_B200_OP_GEMV, "ggml_mul_mat_vec_a8"); }
-Tensor ggml_mul_mat_a8(Tensor W, Tensor X, int64_t type, int64_t row) { return Op::mul_mat(W, X, type, row, GGUF_B200_OP_MMQ, "ggml_mul_mat_a8"); }
-Tensor dequant_matmul(Tensor W, Tensor X, int64_t type, int64_t row) { return Op::mul_mat(W, X, type, row, GGUF_B200_OP_DEQUANT_MATMUL, "dequant_matmul"); }
+Tensor ggml_mul_mat_vec_a8(Tensor W, Tensor X, int64_t type, int64_t row) { return Op::mul_mat(W, X, type, row, GGUF_B200_OP_GEMV, "ggml_mul_mat_vec_a8", false); }
+Tensor ggml_mul_mat_a8(Tensor W, Tensor X, int64_t type, int64_t row) { return Op::mul_mat(W, X, type, row, GGUF_B200_OP_MMQ, "ggml_mul_mat_a8", false); }
+Tensor dequant_matmul(Tensor W, Tensor X, int64_t type, int64_t row) { return Op::mul_mat(W, X, type, row, GGUF_B200_OP_DEQUANT_MATMUL, "dequant_matmul", false); }
 Tensor ggml_moe_a8(Tensor X, Tensor W, Tensor sorted_token_ids, Tensor expert_ids, Tensor num_tokens_post_padded, int64_t type, int64_t row,
                    int64_t top_k, int64_t tokens) {
   return Op::moe_a8(X, W, sorted_token_ids, expert_ids, num_tokens_post_padded, type, row, top_k, tokens);

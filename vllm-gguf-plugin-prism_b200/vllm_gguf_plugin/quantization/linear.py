@@ -97,6 +97,14 @@ if _HAVE_VLLM:
         fused_mul_mat_gguf = getattr(getattr(torch.ops, "vllm", None), "_fused_mul_mat_gguf", _fused_mul_mat_gguf)
 
 
+def _weights_complete(w: torch.Tensor) -> None:
+    """Puts an ordinary kernel behind whatever still writes a layer's weights.  A decode product starts on them while the
+    kernel ahead of it in the stream is finishing; with this one ahead, which starts when the writes are complete and visible,
+    it never starts too soon.  (Whoever rewrites weights in place later calls process_weights_after_loading again.)"""
+    if w.is_cuda:
+        torch.empty(1, dtype=torch.int32, device=w.device).fill_(1)
+
+
 class GGUFWeightType(torch.nn.Parameter):
     """Scalar parameter carrying the GGML type id of a layer (and of each merged shard)."""
 
@@ -190,7 +198,7 @@ class GGUFLinearMethod(LinearMethodBase):
         w = layer.weight
         shards = getattr(w, "_shards", None)
         if not shards:
-            return
+            return _weights_complete(w)
         if None in shards:
             data = shards[None].contiguous()
         else:
@@ -222,6 +230,7 @@ class GGUFLinearMethod(LinearMethodBase):
             else:
                 runs.append([t, start, end - start, width, end - start])
         w.gguf_runs = tuple(v for r in runs for v in r)
+        _weights_complete(w)
 
     def apply(self, layer: torch.nn.Module, x: torch.Tensor, bias: torch.Tensor | None = None) -> torch.Tensor:
         if self.layout is not None:
