@@ -141,3 +141,25 @@ def test_first_product_behind_loading_reads_the_loaded_weights(native_libs):
         got.append(method.apply(layer, x))
     torch.cuda.synchronize()
     assert all(torch.equal(y, want[i & 1]) for i, y in enumerate(got))
+
+
+@pytest.mark.parametrize("types", [("Q4_K", "Q4_K", "Q6_K"), ("Q5_K", "Q5_K", "Q6_K"), ("Q3_K", "Q3_K", "Q5_K"), ("IQ3_S", "IQ3_S", "IQ4_XS"),
+                                   ("IQ4_XS", "IQ4_XS", "Q5_K"), ("Q8_0", "Q4_1", "Q6_K")])
+@pytest.mark.parametrize("K", [768, 2560, 3072, 3584, 5120])
+def test_merged_shards_are_multiplied_where_they_lie(native_libs, types, K):
+    """Whatever the hidden size, no shard is copied: `linear_runs` answers, and with what the shards' own products give."""
+    from helpers import TYPES, rel_l2
+    from vllm_gguf_plugin import native
+    from vllm_gguf_plugin.quantization.linear import _fused_mul_mat_gguf
+
+    ids = [TYPES[n] for n in types]
+    method, layer, parts = merged_layer(ids, [264, 136, 72], K)
+    for M in (1, 2, 3, 8, 17, 130):
+        x = (torch.randn(M, K, device=DEV) / 8).half()
+        y = native.linear_runs(x, layer.weight, layer.weight.gguf_runs)
+        assert y is not None, (types, K, M)
+        want = torch.cat([_fused_mul_mat_gguf(x, w, t) for t, w in zip(ids, parts)], dim=1)
+        assert rel_l2(y.float().cpu(), want.float().cpu()) <= 3e-4, (types, K, M)    # (shared tiles add fp32 sums in another order)
+        assert torch.equal(method.apply(layer, x), y)
+    torch.cuda.synchronize()
+    assert capi.last_status() == 0

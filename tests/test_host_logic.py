@@ -105,6 +105,24 @@ def test_linear_method_mixed_type_shards_call_per_shard(recorded_ops):
     assert calls == ["ggml_mul_mat_a8", "ggml_mul_mat_a8"] and tuple(y.shape) == (9, 16)
 
 
+@pytest.mark.parametrize("K", [256, 2560, 3072, 3584, 4096, 5120])
+def test_shards_of_several_types_lie_whole_16_byte_units_apart(recorded_ops, K):
+    """Q6_K rows are 210 bytes per 256 values; the formats beside them are read in units of up to 16 bytes."""
+    _, linear = recorded_ops
+    m, layer, shards = linear.GGUFLinearMethod(None), torch.nn.Module(), {}
+    m.create_weights(layer, K, [16, 8, 8], K, 32, torch.float16)
+    for sid, rows, t in (("q", 16, 12), ("k", 8, 12), ("v", 8, 14)):
+        shards[sid] = torch.randint(0, 255, (rows, K // 256 * synth.QUANT_SIZES[t][1]), dtype=torch.uint8)
+        layer.weight.weight_loader(layer.weight, shards[sid], sid)
+        layer.weight_type.weight_loader(layer.weight_type, torch.tensor(t), sid)
+    m.process_weights_after_loading(layer)
+    w = layer.weight.data
+    assert tuple(w.shape) == (32, K // 256 * 210) and w.stride(0) % 16 == 0 and w.stride(1) == 1
+    assert w.untyped_storage().nbytes() >= 32 * w.stride(0)
+    for sid, (start, end, width) in layer.weight.shard_offset_map.items():
+        assert torch.equal(w[start:end, :width], shards[sid])
+
+
 def _strict_set_weight_attrs(weight, attrs):
     """vLLM's set_weight_attrs: refuses to overwrite an attribute that is already there."""
     for k, v in (attrs or {}).items():

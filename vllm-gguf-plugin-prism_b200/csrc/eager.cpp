@@ -145,20 +145,22 @@ PyObject* py_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
-// linear_runs(x, W, runs): a layer whose rows are of several types, stacked in W and padded to its width.  runs: a flat tuple of
-// (type, first row, rows, bytes of a row, rows that decide the routing) per run.  Every run is multiplied where it lies, into its columns of one result.
+// linear_runs(x, W, runs): a layer whose rows are of several types, stacked in W a stride apart.  runs: a flat tuple of (type, first
+// row, rows, bytes of a row, rows that decide the routing) per run.  Every run is multiplied where it lies, into its columns of one result.
 PyObject* py_linear_runs(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   TORCH_CHECK(n == 3 && PyTuple_Check(a[2]) && PyTuple_GET_SIZE(a[2]) % 5 == 0, "linear_runs takes x, W and a tuple of runs");
   const Tensor *X = plain_cuda(a[0]), *W = plain_cuda(a[1]);
-  if (!W || !X || X->dim() != 2 || W->dim() != 2 || X->size(0) == 0 || !modes_off() || !X->is_contiguous() || !W->is_contiguous() ||
-      W->scalar_type() != ScalarType::Byte)
+  if (!W || !X || X->dim() != 2 || W->dim() != 2 || X->size(0) == 0 || !modes_off() || !X->is_contiguous() || W->scalar_type() != ScalarType::Byte ||
+      W->stride(1) != 1 || W->stride(0) < W->size(1))
     Py_RETURN_NONE;
+  // (every row is followed by the bytes up to the next, the last one, too)
+  if ((int64_t)W->storage().nbytes() < W->storage_offset() + W->size(0) * W->stride(0)) Py_RETURN_NONE;
   const ScalarType dt = X->scalar_type();
   if (dt != ScalarType::Float && dt != ScalarType::Half && dt != ScalarType::BFloat16) Py_RETURN_NONE;
   struct Run { int type, op; int64_t row, rows, ws; };
   c10::SmallVector<Run, 4> runs;
-  const int64_t M = X->size(0), K = X->size(1), pitch = W->size(1);
+  const int64_t M = X->size(0), K = X->size(1), pitch = W->stride(0);
   int64_t N = 0, most = 0;
   for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(a[2]); i += 5) {
     long v[5];

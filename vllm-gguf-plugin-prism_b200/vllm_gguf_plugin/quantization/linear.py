@@ -194,7 +194,11 @@ class GGUFLinearMethod(LinearMethodBase):
 
     def process_weights_after_loading(self, layer: torch.nn.Module):
         """Materializes ``layer.weight``: a single tensor, or merged shards stacked along the
-        output dim and padded to the widest byte row (reference: linear.py:154-219)."""
+        output dim and padded to the widest byte row (reference: linear.py:154-219).
+
+        Shards of several types lie a multiple of 16 bytes apart, whatever the widest row is: the
+        kernels that multiply them in place read headers of 16 bytes (210 bytes of Q6_K per 256 values are a
+        multiple of 16 only where K is one of 2048)."""
         w = layer.weight
         shards = getattr(w, "_shards", None)
         if not shards:
@@ -205,7 +209,10 @@ class GGUFLinearMethod(LinearMethodBase):
             order = [k for k in ("q", "k", "v") if k in shards] or sorted(shards)
             width = max(shards[k].shape[1] for k in order)
             rows = sum(shards[k].shape[0] for k in order)
-            data = torch.zeros(rows, width, dtype=torch.uint8, device=shards[order[0]].device)
+            wt = layer.weight_type
+            mixed = len({wt.shard_weight_type.get(k, wt.weight_type) for k in order}) > 1
+            pitch = (width + 15) // 16 * 16 if mixed else width
+            data = torch.zeros(rows, pitch, dtype=torch.uint8, device=shards[order[0]].device)[:, :width]
             start = 0
             for k in order:
                 s = shards[k]
