@@ -163,3 +163,52 @@ def test_merged_shards_are_multiplied_where_they_lie(native_libs, types, K):
         assert torch.equal(method.apply(layer, x), y)
     torch.cuda.synchronize()
     assert capi.last_status() == 0
+
+
+# rows of the three shards: columns on and off 16-byte boundaries, a shard of one row
+@pytest.mark.parametrize("rows", [[264, 136, 72], [33, 1, 30]])
+@pytest.mark.parametrize("types", [("Q4_K", "Q4_K", "Q6_K"), ("IQ3_S", "IQ3_S", "IQ4_XS"), ("Q4_K", "Q4_K", "Q4_K")])
+def test_compiled_layer_equals_the_eager_one(native_libs, types, rows):
+    """One operator in the compiled graph, with the eager call's bits; fp32 activations and other batches as well."""
+    from helpers import TYPES
+
+    ids, graphs = [TYPES[n] for n in types], []
+    method, layer, _ = merged_layer(ids, rows, 1024)
+
+    def backend(gm, inputs):
+        graphs.append([str(n.target) for n in gm.graph.nodes if n.op == "call_function"])
+        return gm.forward
+
+    torch._dynamo.reset()
+    compiled = torch.compile(lambda x: method.apply(layer, x), backend=backend, fullgraph=True)
+    for M, dtype in ((1, torch.float16), (2, torch.bfloat16), (9, torch.float16), (40, torch.float32)):
+        if dtype == torch.float32 and types[0].startswith("IQ"):
+            continue
+        x = (torch.randn(M, 1024, device=DEV) / 8).to(dtype)
+        assert torch.equal(compiled(x), method.apply(layer, x)), (M, dtype)
+    assert graphs and all(g == ["_C_gguf.linear_runs"] or g == ["_C_gguf.linear_runs.default"] for g in graphs), graphs
+    torch.cuda.synchronize()
+    assert capi.last_status() == 0
+
+
+def test_layer_copies_only_what_the_kernels_cannot_read_in_place(native_libs):
+    """Rows a distance apart that Q4_K cannot be read at, and rows too long for the GEMV that takes a distance."""
+    from helpers import TYPES, rel_l2
+
+    op = torch.ops._C_gguf.linear_runs
+    for K, names, pad in ((768, ("Q4_K", "Q6_K"), 6), (40960, ("Q4_K", "Q8_0"), 0)):
+        ids = [TYPES[n] for n in names]
+        parts = [weight(t, 24, K, seed=t) for t in ids]
+        width = max(p.shape[1] for p in parts)
+        buf = torch.zeros(48, width + pad, dtype=torch.uint8, device=DEV)
+        W = buf[:, :width]
+        runs = []
+        for i, (t, p) in enumerate(zip(ids, parts)):
+            W[24 * i:24 * i + 24, :p.shape[1]] = p
+            runs += [t, 24 * i, 24, p.shape[1], 24]
+        for M in (1, 2, 5, 30):
+            x = (torch.randn(M, K, device=DEV) / 8).half()
+            want = torch.cat([op(x, p, [t, 0, 24, p.shape[1], 24]) for t, p in zip(ids, parts)], dim=1)
+            assert rel_l2(op(x, W, runs).float().cpu(), want.float().cpu()) <= 3e-4, (K, M)
+    torch.cuda.synchronize()
+    assert capi.last_status() == 0

@@ -203,3 +203,28 @@ def test_moe_loader_honours_expert_and_shard_ids(recorded_ops, monkeypatch, size
     assert torch.equal(layer.w2_weight.data, w2[:, :, rank * b:(rank + 1) * b])
     layer.w13_weight_type.weight_loader(layer.w13_weight_type, torch.tensor(2), "x", shard_id="w1", expert_id=0)
     assert layer.w13_weight_type.weight_type == 2
+
+
+@pytest.mark.parametrize("types", [(12, 12, 14), (12, 12, 12), (2, 23, 14)])
+def test_traced_layer_is_one_operator(native_libs, types):
+    """A traced merged layer multiplies its shards in place too: no copy of a shard, no concatenation in the graph."""
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    from torch.fx.experimental.proxy_tensor import make_fx
+    from vllm_gguf_plugin.quantization.linear import GGUFLinearMethod
+
+    K, rows = 512, [16, 8, 8]
+    with FakeTensorMode(allow_non_fake_inputs=True):
+        method, layer = GGUFLinearMethod(None), torch.nn.Module()
+        method.create_weights(layer, K, rows, K, 32, torch.float16)
+        for sid, n, t in zip("qkv", rows, types):
+            bs, ts = synth.QUANT_SIZES[t]
+            layer.weight.weight_loader(layer.weight, torch.zeros(n, K // bs * ts, dtype=torch.uint8, device="cuda"), sid)
+            layer.weight_type.weight_loader(layer.weight_type, t, sid)
+        method.process_weights_after_loading(layer)
+        for dtype in (torch.float16, torch.float32):
+            x = torch.zeros(3, K, dtype=dtype, device="cuda")
+            graph = make_fx(lambda x: method.apply(layer, x))(x).graph
+            calls = [str(n.target) for n in graph.nodes if n.op == "call_function"]
+            if dtype == torch.float16 or 23 not in types:
+                assert calls == ["_C_gguf.linear_runs.default"], calls
+            assert method.apply(layer, x).shape == (3, 32)

@@ -36,6 +36,10 @@ struct Eager {
   static c10::DeviceIndex device(const Tensor& t) { return t.get_device(); }
   static void* stream(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(device(t)).stream(); }
   static Tensor empty(const Tensor& like, at::IntArrayRef sizes, ScalarType t) { return at::detail::empty_cuda(sizes, t, like.device(), std::nullopt); }
+  static bool has_room(const Tensor& t, int64_t bytes) { return (int64_t)t.storage().nbytes() - t.storage_offset() >= bytes; }
+  static Tensor block(const Tensor& t, int64_t row, int64_t rows, int64_t col, int64_t cols) { return t.narrow(0, row, rows).narrow(1, col, cols); }
+  static Tensor packed(const Tensor& t) { return t.contiguous(); }
+  static void copy(Tensor to, const Tensor& from) { to.copy_(from); }
   // scratch memory of one call, given back to the stream's pool when the call returns
   struct Scratch {
     c10::DataPtr p;
@@ -116,18 +120,6 @@ PyObject* py_embed(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
-// The batch-size rule of the linear dispatcher (quantization/linear.py `_fused_mul_mat_gguf`): the
-// operation that serves M rows against N weight rows of `type`, or -1 where only Python does.
-bool imatrix_type(int64_t t) { return t == 16 || t == 17 || t == 18 || t == 19 || t == 20 || t == 21 || t == 22 || t == 23 || t == 29; }
-int linear_op(int64_t type, int64_t M, int64_t N, ScalarType dt) {
-  const bool im = imatrix_type(type);
-  const int64_t most = im ? (N > 5120 ? 8 : 16) : (N > 5120 ? 2 : 6);
-  if (M <= most) return GGUF_B200_OP_GEMV;
-  if (!im) return GGUF_B200_OP_MMQ;
-  const bool fused = dt == ScalarType::Half || dt == ScalarType::BFloat16;
-  return fused ? GGUF_B200_OP_DEQUANT_MATMUL : -1;
-}
-
 // linear(x, W, type): one layer's product, routed as the dispatcher routes it
 PyObject* py_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
@@ -138,66 +130,26 @@ PyObject* py_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (PyErr_Occurred()) return nullptr;
   if (gguf_b200_type_size((int)type) == 0) Py_RETURN_NONE;
   const int64_t N = W->size(0);
-  const int op = linear_op(type, X->size(0), N, X->scalar_type());
+  const int op = gguf_ops::linear_op(type, X->size(0), N, X->scalar_type());
   if (op < 0) Py_RETURN_NONE;
   const Tensor w = *W, x = *X;
   return THPVariable_Wrap(without_gil([&] { return Op::mul_mat(w, x, type, N, op, "linear", true); }));
   END_HANDLE_TH_ERRORS
 }
 
-// linear_runs(x, W, runs): a layer whose rows are of several types, stacked in W a stride apart.  runs: a flat tuple of (type, first
-// row, rows, bytes of a row, rows that decide the routing) per run.  Every run is multiplied where it lies, into its columns of one result.
+// linear_runs(x, W, runs): Op::linear_runs with the runs in a tuple
 PyObject* py_linear_runs(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   TORCH_CHECK(n == 3 && PyTuple_Check(a[2]) && PyTuple_GET_SIZE(a[2]) % 5 == 0, "linear_runs takes x, W and a tuple of runs");
   const Tensor *X = plain_cuda(a[0]), *W = plain_cuda(a[1]);
-  if (!W || !X || X->dim() != 2 || W->dim() != 2 || X->size(0) == 0 || !modes_off() || !X->is_contiguous() || W->scalar_type() != ScalarType::Byte ||
-      W->stride(1) != 1 || W->stride(0) < W->size(1))
-    Py_RETURN_NONE;
-  // (every row is followed by the bytes up to the next, the last one, too)
-  if ((int64_t)W->storage().nbytes() < W->storage_offset() + W->size(0) * W->stride(0)) Py_RETURN_NONE;
-  const ScalarType dt = X->scalar_type();
-  if (dt != ScalarType::Float && dt != ScalarType::Half && dt != ScalarType::BFloat16) Py_RETURN_NONE;
-  struct Run { int type, op; int64_t row, rows, ws; };
-  c10::SmallVector<Run, 4> runs;
-  const int64_t M = X->size(0), K = X->size(1), pitch = W->stride(0);
-  int64_t N = 0, most = 0;
-  for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(a[2]); i += 5) {
-    long v[5];
-    for (int j = 0; j < 5; ++j) v[j] = PyLong_AsLong(PyTuple_GET_ITEM(a[2], i + j));
-    if (PyErr_Occurred()) return nullptr;
-    const int ts = gguf_b200_type_size((int)v[0]);
-    if (ts == 0 || v[3] % ts != 0 || v[3] / ts * gguf_b200_block_size((int)v[0]) != K || v[1] < 0 || v[1] + v[2] > W->size(0) || v[1] * pitch % 16 != 0)
-      Py_RETURN_NONE;
-    const int op = linear_op(v[0], M, v[4], dt);
-    if (op < 0) Py_RETURN_NONE;
-    const int64_t ws = gguf_b200_scratch_bytes(op, (int)v[0], M, v[2], K);
-    most = ws > most ? ws : most;
-    runs.push_back({(int)v[0], op, v[1], v[2], ws});
-    N += v[2];
-  }
-  if (N == 0) Py_RETURN_NONE;
+  if (!W || !X || X->dim() != 2 || X->size(0) == 0 || !modes_off()) Py_RETURN_NONE;
+  c10::SmallVector<int64_t, 15> runs(PyTuple_GET_SIZE(a[2]));
+  for (size_t i = 0; i < runs.size(); ++i) runs[i] = PyLong_AsLongLong(PyTuple_GET_ITEM(a[2], i));
+  if (PyErr_Occurred()) return nullptr;
+  for (size_t i = 0; i < runs.size(); i += 5)
+    if (gguf_b200_type_size((int)runs[i]) == 0 || gguf_ops::linear_op(runs[i], X->size(0), runs[i + 4], X->scalar_type()) < 0) Py_RETURN_NONE;
   const Tensor w = *W, x = *X;
-  const int code = gguf_ops::dtype_code(dt, "linear_runs");
-  Tensor out = without_gil([&]() -> Tensor {   // undefined: a layout that only copies can serve
-    const Eager::Guard guard(Eager::device(x));
-    Tensor Y = Eager::empty(x, {M, N}, dt);
-    const Eager::Scratch ws(x, most);
-    void* s = Eager::stream(x);
-    int64_t col = 0;
-    for (const Run& r : runs) {
-      uint8_t* y = static_cast<uint8_t*>(Y.data_ptr()) + col * Y.element_size();
-      if (reinterpret_cast<uintptr_t>(y) % 16 != 0) return Tensor();
-      const int rc = gguf_b200_mul_mat_strided(static_cast<const uint8_t*>(w.data_ptr()) + r.row * pitch, x.data_ptr(), y, ws.get(), most, r.op, r.type,
-                                               code, M, r.rows, K, pitch, N, s);
-      if (rc == GGUF_B200_E_SHAPE || rc == GGUF_B200_E_TOO_LARGE) return Tensor();
-      gguf_ops::check_rc(rc, "linear_runs");
-      col += r.rows;
-    }
-    return Y;
-  });
-  if (!out.defined()) Py_RETURN_NONE;
-  return THPVariable_Wrap(std::move(out));
+  return THPVariable_Wrap(without_gil([&] { return Op::linear_runs(x, w, runs.data(), runs.size()); }));
   END_HANDLE_TH_ERRORS
 }
 

@@ -32,6 +32,18 @@ inline int dtype_code(ScalarType t, const char* what) {
 
 inline void check_rc(int rc, const char* op) { STD_TORCH_CHECK(rc == GGUF_B200_OK, op, " failed: ", gguf_b200_error_string(rc)); }
 
+// The batch-size rule of the linear dispatcher (quantization/linear.py `_fused_mul_mat_gguf`): the
+// operation that serves M rows against N weight rows of `type`, or -1 where only Python does.
+inline bool imatrix_type(int64_t t) { return t == 16 || t == 17 || t == 18 || t == 19 || t == 20 || t == 21 || t == 22 || t == 23 || t == 29; }
+inline int linear_op(int64_t type, int64_t M, int64_t N, ScalarType dt) {
+  const bool im = imatrix_type(type);
+  const int64_t most = im ? (N > 5120 ? 8 : 16) : (N > 5120 ? 2 : 6);
+  if (M <= most) return GGUF_B200_OP_GEMV;
+  if (!im) return GGUF_B200_OP_MMQ;
+  const bool fused = dt == ScalarType::Half || dt == ScalarType::BFloat16;
+  return fused ? GGUF_B200_OP_DEQUANT_MATMUL : -1;
+}
+
 template <class A> struct Calls {
   using Tensor = typename A::Tensor;
 
@@ -110,6 +122,62 @@ template <class A> struct Calls {
     else
       rc = gguf_b200_dequant_matmul(W.data_ptr(), X.data_ptr(), Y.data_ptr(), ws.get(), ws_bytes, (int)type, code, M, row, K, s);
     check_rc(rc, name);
+    return Y;
+  }
+
+  // A loaded layer's product.  Its rows may be of several types, stacked in W [rows, bytes of the widest] a stride apart; runs: (type,
+  // first row, rows, bytes of a row, rows that decide the routing) of each run of one type.  Every run is multiplied where it lies, into
+  // its columns of one result.  What the kernels cannot do in place -- columns off a 16-byte boundary, a row distance that the
+  // format cannot be read at, rows too long for them -- is multiplied into, or as, a copy.
+  static Tensor linear_runs(const Tensor& X, const Tensor& W, const int64_t* runs, size_t n) {
+    const char* name = "linear_runs";
+    const typename A::Guard guard(A::device(X));
+    STD_TORCH_CHECK(n > 0 && n % 5 == 0, name, ": five numbers per run");
+    STD_TORCH_CHECK(W.scalar_type() == ScalarType::Byte && W.dim() == 2 && W.stride(1) == 1, name, ": W must be uint8 rows of raw GGUF blocks");
+    STD_TORCH_CHECK(X.dim() == 2 && X.is_contiguous(), name, ": X must be a contiguous [tokens, K] tensor");
+    const ScalarType dt = X.scalar_type();
+    const int code = dtype_code(dt, name);
+    const int64_t M = X.size(0), K = X.size(1), pitch = W.stride(0), esz = dt == ScalarType::Float ? 4 : 2;
+    int64_t N = 0, ws_bytes = 0;
+    for (size_t i = 0; i < n; i += 5) {
+      const int64_t *r = runs + i, ts = gguf_b200_type_size((int)r[0]);
+      STD_TORCH_CHECK(ts > 0, name, ": unsupported GGML quantization type ", std::to_string(r[0]));
+      STD_TORCH_CHECK(r[1] >= 0 && r[2] >= 0 && r[1] + r[2] <= W.size(0) && r[3] <= W.size(1) && r[3] % ts == 0 && r[3] / ts * gguf_b200_block_size((int)r[0]) == K,
+                      name, ": a run does not match X and W");
+      const int op = linear_op(r[0], M, r[4], dt);
+      STD_TORCH_CHECK(op >= 0, name, ": no kernel for this type, batch and dtype");
+      const int64_t ws = M > 0 ? gguf_b200_scratch_bytes(op, (int)r[0], M, r[2], K) : 0;
+      ws_bytes = ws > ws_bytes ? ws : ws_bytes;
+      N += r[2];
+    }
+    Tensor Y = A::empty(X, {M, N}, dt);
+    if (M == 0 || N == 0) return Y;
+    const typename A::Scratch ws(X, ws_bytes);
+    void* s = A::stream(X);
+    // (every row is followed by the bytes up to the next, the last one, too)
+    const bool in_place = pitch >= W.size(1) && A::has_room(W, W.size(0) * pitch);
+    int64_t col = 0;
+    for (size_t i = 0; i < n; i += 5) {
+      const int64_t *r = runs + i, rows = r[2];
+      if (rows == 0) continue;
+      const int type = (int)r[0], op = linear_op(r[0], M, r[4], dt);
+      uint8_t* y = static_cast<uint8_t*>(Y.data_ptr()) + col * esz;
+      const uint8_t* w = static_cast<const uint8_t*>(W.data_ptr()) + r[1] * pitch;
+      const bool direct = reinterpret_cast<uintptr_t>(y) % 16 == 0;
+      std::optional<Tensor> part;
+      if (!direct) part = A::empty(X, {M, rows}, dt);
+      int rc = GGUF_B200_E_SHAPE;
+      if (in_place && reinterpret_cast<uintptr_t>(w) % 16 == 0)
+        rc = gguf_b200_mul_mat_strided(w, X.data_ptr(), direct ? y : part->data_ptr(), ws.get(), ws_bytes, op, type, code, M, rows, K, pitch,
+                                       direct ? N : rows, s);
+      if (rc == GGUF_B200_E_SHAPE || rc == GGUF_B200_E_TOO_LARGE) {
+        part = mul_mat(A::packed(A::block(W, r[1], rows, 0, r[3])), X, type, rows, op, name, false);
+        rc = GGUF_B200_OK;
+      }
+      check_rc(rc, name);
+      if (part) A::copy(A::block(Y, 0, M, col, rows), *part);
+      col += rows;
+    }
     return Y;
   }
 

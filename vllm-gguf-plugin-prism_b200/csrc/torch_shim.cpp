@@ -2,7 +2,7 @@
 // reference's binding file (vllm_gguf_plugin/csrc/torch_bindings.cpp:22-53), registered the same
 // way (stable ABI, ops on the CUDA key, ggml_moe_get_block_size as CompositeExplicitAutograd), so
 // `vllm_gguf_plugin.ops` finds `torch.ops._C_gguf.*` unchanged, plus dequant_matmul (the fused route
-// of the IQ types), dequantize_rows and fused_moe.  The bodies are in op_calls.h.
+// of the IQ types), dequantize_rows, fused_moe and linear_runs.  The bodies are in op_calls.h.
 //
 // This file uses nothing of torch but its stable ABI and nothing of Python but the module
 // entry: the library runs under every torch that has that ABI, whatever the Python version.
@@ -13,6 +13,8 @@
 #include <torch/csrc/stable/library.h>
 #include <torch/csrc/stable/ops.h>
 #include <torch/csrc/stable/tensor.h>
+
+#include <vector>
 
 #include "op_calls.h"
 
@@ -30,6 +32,18 @@ struct Stable {
   static Tensor empty(const Tensor& like, std::initializer_list<int64_t> sizes, torch::headeronly::ScalarType t) {
     return torch::stable::new_empty(like, sizes, t);
   }
+  static bool has_room(const Tensor& t, int64_t bytes) {
+    int64_t size = 0, offset = 0;
+    TORCH_ERROR_CODE_CHECK(aoti_torch_get_storage_size(t.get(), &size));
+    TORCH_ERROR_CODE_CHECK(aoti_torch_get_storage_offset(t.get(), &offset));
+    return size - offset >= bytes;
+  }
+  static Tensor block(Tensor t, int64_t row, int64_t rows, int64_t col, int64_t cols) {
+    Tensor r = torch::stable::narrow(t, 0, row, rows);
+    return torch::stable::narrow(r, 1, col, cols);
+  }
+  static Tensor packed(const Tensor& t) { return torch::stable::contiguous(t); }
+  static void copy(Tensor to, const Tensor& from) { torch::stable::copy_(to, from); }
   struct Scratch {
     Tensor t;
     Scratch(const Tensor& like, int64_t bytes) : t(empty(like, {bytes > 0 ? bytes : 1}, torch::headeronly::ScalarType::Byte)) {}
@@ -55,6 +69,7 @@ Tensor ggml_moe_a8_vec(Tensor X, Tensor W, Tensor topk_ids, int64_t top_k, int64
 Tensor fused_moe(Tensor X, Tensor W13, Tensor W2, Tensor topk_weights, Tensor topk_ids, int64_t type13, int64_t type2, int64_t act) {
   return Op::fused_moe(X, W13, W2, topk_weights, topk_ids, type13, type2, act);
 }
+Tensor linear_runs(Tensor X, Tensor W, std::vector<int64_t> runs) { return Op::linear_runs(X, W, runs.data(), runs.size()); }
 int64_t ggml_moe_get_block_size(int64_t type) { return gguf_b200_moe_block_size((int)type); }
 
 }  // namespace
@@ -70,6 +85,7 @@ STABLE_TORCH_LIBRARY(_C_gguf, ops) {
   ops.def("ggml_moe_get_block_size(int type) -> int");
   ops.def("dequant_matmul(Tensor W, Tensor X, int type, SymInt row) -> Tensor");
   ops.def("dequantize_rows(Tensor W, Tensor ids, int type, ScalarType? dtype) -> Tensor");
+  ops.def("linear_runs(Tensor X, Tensor W, int[] runs) -> Tensor");
   ops.def("fused_moe(Tensor X, Tensor W13, Tensor W2, Tensor topk_weights, Tensor topk_ids, int type13, int type2, int act) -> Tensor");
 }
 
@@ -81,6 +97,7 @@ STABLE_TORCH_LIBRARY_IMPL(_C_gguf, CUDA, ops) {
   ops.impl("ggml_moe_a8_vec", TORCH_BOX(&ggml_moe_a8_vec));
   ops.impl("dequant_matmul", TORCH_BOX(&dequant_matmul));
   ops.impl("dequantize_rows", TORCH_BOX(&dequantize_rows));
+  ops.impl("linear_runs", TORCH_BOX(&linear_runs));
   ops.impl("fused_moe", TORCH_BOX(&fused_moe));
 }
 

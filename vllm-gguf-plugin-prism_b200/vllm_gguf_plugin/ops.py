@@ -19,6 +19,8 @@ Differences from the reference, all deliberate:
 * ``ggml_dequantize_rows`` is new: the embedding look-up (index_select of rows + ggml_dequantize,
   quantization/vocal_embeds.py:88-96) as one kernel;
 * ``ggml_fused_moe`` is new: the whole MoE step of a layer in one call;
+* ``torch.ops._C_gguf.linear_runs`` is new: the product of a merged layer whose shards are of several types, in place
+  (the reference copies every shard and concatenates the products, quantization/linear.py:246-262);
 * ``ggml_dequant_matmul`` is new: the fused form of "ggml_dequantize then x @ W.T" that the
   reference uses for IQ types above the GEMV batch threshold (quantization/linear.py:50-54).
 """
@@ -143,6 +145,11 @@ def _dequantize_rows_fake(W, ids, quant_type, dtype=None):
 @register_fake("_C_gguf::fused_moe")
 def _fused_moe_fake(X, W13, W2, topk_weights, topk_ids, type13, type2, act):
     return torch.empty_like(X)
+
+
+@register_fake("_C_gguf::linear_runs")
+def _linear_runs_fake(X, W, runs):
+    return torch.empty((X.shape[0], sum(runs[2::5])), dtype=X.dtype, device=X.device)
 
 
 @register_fake("_C_gguf::ggml_moe_a8")

@@ -21,6 +21,7 @@ from .utils import (
     IMATRIX_QUANT_TYPES,
     MMQ_QUANT_TYPES,
     MMVQ_QUANT_TYPES,
+    SUPPORTED_QUANT_SIZES,
     UNQUANTIZED_TYPES,
     quant_sizes,
 )
@@ -239,6 +240,26 @@ class GGUFLinearMethod(LinearMethodBase):
         w.gguf_runs = tuple(v for r in runs for v in r)
         _weights_complete(w)
 
+    @staticmethod
+    def _runs(layer: torch.nn.Module) -> list[int]:
+        """The runs of rows of one type: (type, first row, rows, bytes of a row, rows as the batch-size rule counts them)."""
+        w = layer.weight
+        if w.shard_id and w.gguf_one_type is None:
+            return list(w.gguf_runs)
+        rows, width = w.shape
+        return [int(w.gguf_one_type if w.shard_id else layer.weight_type.weight_type), 0, rows, width, rows]
+
+    @classmethod
+    def _has_layer_operator(cls, layer: torch.nn.Module, x: torch.Tensor) -> bool:
+        """Everything but unquantized shards, and the code-book types with fp32 activations, whose larger batches are
+        dequantized and multiplied as in the reference."""
+        w = layer.weight
+        if not (x.is_cuda and x.dim() == 2 and w.dim() == 2):
+            return False
+        types = cls._runs(layer)[0::5]
+        return (all(t in SUPPORTED_QUANT_SIZES for t in types)
+                and (x.dtype != torch.float32 or not any(t in IMATRIX_QUANT_TYPES for t in types)))
+
     def apply(self, layer: torch.nn.Module, x: torch.Tensor, bias: torch.Tensor | None = None) -> torch.Tensor:
         if self.layout is not None:
             x = self.layout.input_to_gguf(x)
@@ -250,6 +271,10 @@ class GGUFLinearMethod(LinearMethodBase):
             out = native.linear(x, weight, one_type) if one_type is not None else native.linear_runs(x, weight, weight.gguf_runs)
             if out is not None:
                 return out if bias is None else out.add_(bias)
+        if self._has_layer_operator(layer, x):
+            # ... and a compiled or traced one to the same code as one operator
+            out = torch.ops._C_gguf.linear_runs(x, layer.weight, self._runs(layer))
+            return out if bias is None else out.add_(bias)
         shard_id = layer.weight.shard_id
         if shard_id:
             shard_id = ["q", "k", "v"] if "q" in shard_id else shard_id
