@@ -684,6 +684,27 @@ def test_tp_matmul_tiles_one_gpu(case):
         assert torch.equal(ys[0], ys[1])
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("shape", [(8, 256, 20), (200, 1024, 33), (136, 4096, 130), (264, 768, 300)])
+def test_tp_matmul_stores_whole_tiles_of_every_edge(shape, dtype):
+    """A rank's column block, row tiles and token tiles ragged, between the other ranks' columns: the local product's bits, in
+    every rank's matrix, and nothing beside them."""
+    N, K, M = shape
+    t, world, rank = TYPES["Q4_K"], 3, 1
+    _, w = dev_w(t, N, K, seed=N)
+    x = dev_x(M, K, seed=M, dtype=dtype)
+    want = capi.mul_mat_a8(w, x, t, N)
+    ys = [torch.full((M, world * N), 7.0, dtype=dtype, device=DEV) for _ in range(world)]
+    flags = [torch.zeros(64, dtype=torch.int32, device=DEV) for _ in range(world)]
+    epochs = torch.zeros(64, dtype=torch.int32, device=DEV)
+    capi.matmul_tp(capi.OP_MMQ, w, x, [y.data_ptr() for y in ys], [f.data_ptr() for f in flags], epochs, 3, t, rank)
+    torch.cuda.synchronize()
+    assert capi.last_status() == 0
+    for y in ys:
+        assert torch.equal(y[:, N:2 * N], want)
+        assert bool((y[:, :N] == 7).all()) and bool((y[:, 2 * N:] == 7).all())
+
+
 def test_waits_on_other_gpus_run_out_and_report():
     """A packet that nobody sends and a flag that nobody raises: with a limit of about a millisecond
     the waiting kernels give up by themselves, the status word reads E_TIMEOUT (-8) and the

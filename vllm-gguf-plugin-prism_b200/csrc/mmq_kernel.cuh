@@ -195,20 +195,59 @@ __device__ __forceinline__ bool mmq_next_part(const MmqParams& p, MmqPart& q) {
 __device__ __forceinline__ uint16_t mmq_bits16(int dtype, float v) {
   return dtype == DT_F16 ? __half_as_ushort(__float2half_rn(v)) : __bfloat16_as_ushort(__float2bfloat16_rn(v));
 }
-// one value of an output row in the forms that are not the usual one: fp32, or this rank's column block of every rank's matrix
-__device__ __forceinline__ void mmq_store(const MmqParams& p, int64_t orow, int n, float v, float scale) {
-  if (p.tp_world > 0) {
-    const int64_t at = orow * p.ldy + p.tp_col_off + n;
-    for (int rk = 0; rk < p.tp_world; ++rk) {
-      if (p.dtype == DT_F32) static_cast<float*>(p.tp_y[rk])[at] = v;
-      else static_cast<uint16_t*>(p.tp_y[rk])[at] = mmq_bits16(p.dtype, v);
+// Sixteen tokens of a warp's 32 rows (a lane has one row) into this rank's column block of every rank's matrix.  What crosses
+// NVLink leaves in 16-byte stores: squares of eight rows by eight tokens (fp32: four by four) are transposed across the lanes
+// first, bit k of the lane against bit k of the token, so that a lane ends up with consecutive columns of one token.
+// n: the lane's row; rows come in whole groups of eight.  tokens: how many of the sixteen count.  (7168 rows of
+// Q4_K, 512 tokens, the matrices of 1 / 2 / 4 / 8 ranks all on one GPU: 55.7 / 57.9 / 56.8 / 61.1 us with a 2-byte store per value
+// and rank, 42.4 / 44.7 / 49.4 / 59.3 so.)
+__device__ __forceinline__ void mmq_store_peers(const MmqParams& p, int64_t orow, int tokens, int n, bool live, uint32_t (&acc)[16], int lane) {
+  const bool f32 = p.dtype == DT_F32;
+  const int group = f32 ? 4 : 8, l = lane & (group - 1);
+  const int64_t at = orow * p.ldy + p.tp_col_off + (n - l);
+  auto swap = [&](uint32_t& keep0, uint32_t& keep1, int bit) {   // the lane without the bit gives keep1, the one with it keep0
+    const bool up = (lane & bit) != 0;
+    const uint32_t got = __shfl_xor_sync(0xffffffffu, up ? keep0 : keep1, bit);
+    if (up) keep0 = got;
+    else keep1 = got;
+  };
+#pragma unroll 1
+  for (int t0 = 0; t0 < 16; t0 += group) {
+    uint32_t q[4];
+    if (f32) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) q[i] = acc[i];
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        q[i] = (uint32_t)mmq_bits16(p.dtype, __uint_as_float(acc[2 * i])) | (uint32_t)mmq_bits16(p.dtype, __uint_as_float(acc[2 * i + 1])) << 16;
     }
-  } else {
-    static_cast<float*>(p.y)[orow * p.ldy + n] = p.row_scale ? v * scale : v;
+    const int b1 = f32 ? 2 : 4, b0 = f32 ? 1 : 2;
+    swap(q[0], q[2], b1);
+    swap(q[1], q[3], b1);
+    swap(q[0], q[1], b0);
+    swap(q[2], q[3], b0);
+    if (!f32) {   // the last bit: halves of a register
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const uint32_t got = __shfl_xor_sync(0xffffffffu, q[i], 1);
+        q[i] = lane & 1 ? __byte_perm(got, q[i], 0x7632) : __byte_perm(q[i], got, 0x5410);
+      }
+    }
+    if (live && t0 + l < tokens) {
+      const int64_t e = at + (int64_t)(t0 + l) * p.ldy;
+#pragma unroll 1
+      for (int rk = 0; rk < p.tp_world; ++rk)
+        *reinterpret_cast<uint4*>(static_cast<uint8_t*>(p.tp_y[rk]) + e * (f32 ? 4 : 2)) = make_uint4(q[0], q[1], q[2], q[3]);
+    }
+#pragma unroll
+    for (int i = 0; i < 12; ++i) acc[i] = f32 || i >= 8 ? acc[i + 4] : acc[i + 8];   // (register indexes are static)
   }
 }
 
-template <int TYPE, typename ab_t, bool FAST>
+// TP: the tensor-parallel form, kernels of their own.  (Sixteen-byte stores to the peers as one more branch of the same epilogue
+// cost calls that never take it: 300 tokens of 8192x28672 IQ3_S 133 -> 139 us.)
+template <int TYPE, typename ab_t, bool FAST, bool TP>
 __global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_constant__ CUtensorMap bmap, const __grid_constant__ CUtensorMap wmap,
                                                              const __grid_constant__ MmqParams p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -385,7 +424,7 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_consta
           }
         }
       }
-      const bool plain = p.tp_world == 0 && p.dtype != DT_F32, rows = plain && !moe && !p.row_scale;
+      const bool plain = !TP && p.dtype != DT_F32, rows = plain && !moe && !p.row_scale;
 #pragma unroll 1
       for (int b = g; b < nb; b += MMQ_GROUPS) {
         const int orow_next = out_row(b + MMQ_GROUPS);
@@ -449,12 +488,14 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_consta
             }
             if (live && o >= 0) y[(int64_t)o * p.ldy] = v;
           }
+        } else if constexpr (TP) {
+          mmq_store_peers(p, et.x0 + 16 * b, et.rows - 16 * b, n, live, acc, lane);
         } else {
 #pragma unroll 1
           for (int j = 0; j < 16; ++j) {
             const int o = __shfl_sync(0xffffffffu, orow, j);
-            const float w = __shfl_sync(0xffffffffu, scale, j);
-            if (live && o >= 0) mmq_store(p, o, n, __uint_as_float(acc[0]), w);
+            const float w = __shfl_sync(0xffffffffu, scale, j), v = __uint_as_float(acc[0]);
+            if (live && o >= 0) static_cast<float*>(p.y)[(int64_t)o * p.ldy + n] = p.row_scale ? v * w : v;
 #pragma unroll
             for (int k = 0; k < 15; ++k) acc[k] = acc[k + 1];   // (register indexes are static)
           }
@@ -701,12 +742,12 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_consta
     __syncthreads();
   }
   if (warp == MMQ_PRODUCER_WARPS) tmem_dealloc(tmem_base, 512);
-  if (p.tp_world > 0) tp_finish(p.tp_epoch, p.tp_flag, p.tp_world, p.tp_slot, gridDim.x);
+  if constexpr (TP) tp_finish(p.tp_epoch, p.tp_flag, p.tp_world, p.tp_slot, gridDim.x);
 }
 
-template <int TYPE, typename ab_t, bool FAST>
-static int mmq_launch_form(const MmqParams& p, const CUtensorMap& bmap, const CUtensorMap& wmap, int grid, size_t smem, cudaStream_t stream) {
-  auto kern = mmq_kernel<TYPE, ab_t, FAST>;
+template <int TYPE, typename ab_t, bool FAST, bool TP>
+static int mmq_launch_kernel(const MmqParams& p, const CUtensorMap& bmap, const CUtensorMap& wmap, int grid, size_t smem, cudaStream_t stream) {
+  auto kern = mmq_kernel<TYPE, ab_t, FAST, TP>;
   static bool configured[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -715,6 +756,11 @@ static int mmq_launch_form(const MmqParams& p, const CUtensorMap& bmap, const CU
     configured[dev & 63] = true;
   }
   return launch_pdl(kern, dim3((unsigned)grid), dim3(MMQ_THREADS), smem, stream, bmap, wmap, p) == cudaSuccess ? E_OK : E_CUDA;
+}
+template <int TYPE, typename ab_t, bool FAST>
+static int mmq_launch_form(const MmqParams& p, const CUtensorMap& bmap, const CUtensorMap& wmap, int grid, size_t smem, cudaStream_t stream) {
+  return p.tp_world > 0 ? mmq_launch_kernel<TYPE, ab_t, FAST, true>(p, bmap, wmap, grid, smem, stream)
+                        : mmq_launch_kernel<TYPE, ab_t, FAST, false>(p, bmap, wmap, grid, smem, stream);
 }
 // ab: element type of the activation matrix (DT_F16, DT_BF16); fast: whole-stage decoder on dense boxes
 template <int TYPE> int mmq_launch(const MmqParams& p, const CUtensorMap& bmap, const CUtensorMap& wmap, int ab, bool fast, int grid, size_t smem,
