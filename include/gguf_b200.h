@@ -83,16 +83,15 @@ int gguf_b200_dequantize(const void* W, int type, void* out, int out_dtype, int6
 int gguf_b200_dequantize_rows(const void* W, int type, const int64_t* row_ids, int64_t n_rows, int64_t K,
                               int64_t weight_rows, void* out, int out_dtype, void* stream);
 
-/* Scratch bytes an op wants for the given sizes (rows = M, or tokens for the MoE ops).  For the
- * dense GEMM ops this includes room for fp32 partial tiles when the problem is split over K
- * (few output tiles, long rows); a smaller workspace that still holds the activations is
- * accepted and merely disables the split. */
+/* Scratch bytes of an op for the given sizes (rows = M, or tokens for the MoE ops).  For the dense GEMM ops this includes the
+ * fp32 parts of tiles that several CTAs share; a smaller workspace that still holds the activations is accepted and merely
+ * keeps every tile to one CTA. */
 int64_t gguf_b200_workspace_bytes(int op, int type, int64_t M, int64_t N, int64_t K);
 
-/* Scratch bytes with which an op is fastest, never less than the above: for batches of a few tokens
- * (gguf_b200_mul_mat_vec_a8 from three on, gguf_b200_mul_mat_a8 from three to sixteen) it adds what the
- * small-batch kernel needs, its activation tiles and partial sums; without that room these calls take
- * several passes of the one- and two-vector kernel, or the tiled kernel. */
+/* Scratch bytes with which an op is fastest, never less than the above; what a caller that can should give.  For batches of a
+ * few tokens (gguf_b200_mul_mat_vec_a8 from three on, gguf_b200_mul_mat_a8 from three to sixteen) it is what the small-batch
+ * kernel needs, its activation tiles and partial sums: without that room these calls take several passes of the one- and
+ * two-vector kernel, or the tiled kernel.  For gguf_b200_moe_a8 it adds the parts of shared tiles. */
 int64_t gguf_b200_scratch_bytes(int op, int type, int64_t M, int64_t N, int64_t K);
 
 /* Decode GEMV: Y[M][N] = q8_1(X) . dequant(W)^T, weights read once for up to 8 vectors.
@@ -250,8 +249,8 @@ int gguf_b200_tp_unpack(const void* packets_local, const uint32_t* epochs_local,
  * tile epilogue (or, when K is split over CTAs, the kernel that adds the partial tiles) stores this
  * rank's column block [rank*N_local, ...) into every rank's matrix with 16-byte stores.  The last
  * CTA then increments epochs_local[slot] and flag_peers[r][slot] on every rank (uint32 counters,
- * zero before first use, only ever growing).  Workspace: gguf_b200_workspace_bytes(op, type, M,
- * N_local, K). */
+ * zero before first use, only ever growing).  Workspace: gguf_b200_scratch_bytes(op, type, M, N_local,
+ * K) (see there for less). */
 int gguf_b200_matmul_tp(int op, const void* W, const void* X, void* const* y_peers, uint32_t* const* flag_peers,
                         uint32_t* epochs_local, int slot, void* ws, int64_t ws_bytes, int type, int dtype, int64_t M,
                         int64_t N_local, int64_t K, int rank, int world, void* stream);

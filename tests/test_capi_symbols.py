@@ -57,14 +57,19 @@ def test_geometry_and_error_codes(native_libs):
     assert lib.gguf_b200_dequantize(p, 12, p, 1, 100, null) == -3
     assert lib.gguf_b200_mul_mat_vec_a8(p, p, p, p, 0, 12, 1, 0, 8, 256, null) == 0          # empty batch
     assert b"workspace" in lib.gguf_b200_error_string(-5)
-    # dense GEMM workspace: activations (+ fp32 partial tiles when few tiles and long rows split K)
+    # dense GEMM workspace: activations, and the parts of tiles that several CTAs share: two tiles of 128 rows for each of up to
+    # 148 CTAs, in fp32, behind a counter per tile
     act = lambda m, k: (m * (k + (k // 32 + 63) // 64 * 64) * 2 + 255) // 256 * 256
-    assert lib.gguf_b200_workspace_bytes(capi.OP_MMQ, 12, 512, 14336, 4096) == act(512, 4096)              # 224 tiles: no split
-    assert lib.gguf_b200_workspace_bytes(capi.OP_MMQ, 12, 512, 4096, 14336) == act(512, 14336) + 2 * 512 * 4096 * 4
-    assert lib.gguf_b200_workspace_bytes(capi.OP_MMQ, 12, 64, 4096, 14336) == act(64, 14336) + 4 * 64 * 4096 * 4
-    assert lib.gguf_b200_workspace_bytes(capi.OP_DEQUANT_MATMUL, 16, 128, 28672, 8192) == 0
-    assert lib.gguf_b200_workspace_bytes(capi.OP_DEQUANT_MATMUL, 16, 128, 8192, 28672) == 2 * 128 * 8192 * 4
-    assert lib.gguf_b200_workspace_bytes(capi.OP_DEQUANT_MATMUL, 16, 128, 1024, 28672) == 16 * 128 * 1024 * 4   # 8 tiles: 16 K slices
+    for op, t, m, n, k, shared in ((capi.OP_MMQ, 12, 512, 14336, 4096, None), (capi.OP_MMQ, 12, 512, 4096, 14336, True), (capi.OP_MMQ, 12, 64, 4096, 14336, True),
+                                   (capi.OP_MMQ, 12, 512, 18944, 4096, None), (capi.OP_DEQUANT_MATMUL, 16, 128, 1024, 28672, True),
+                                   (capi.OP_DEQUANT_MATMUL, 16, 128, 128 * 148, 4096, False), (capi.OP_DEQUANT_MATMUL, 16, 128, 8192, 28672, True)):
+        room = lib.gguf_b200_workspace_bytes(op, t, m, n, k) - (act(m, k) if op == capi.OP_MMQ else 0)
+        assert 0 <= room <= 2 * 148 * 128 * 384 * 4 + (1 << 20) and room % 256 == 0
+        assert shared is None or (room > 0) == shared, (op, t, m, n, k, room)
+        assert lib.gguf_b200_scratch_bytes(op, t, m, n, k) == room + (act(m, k) if op == capi.OP_MMQ else 0)   # nothing allocated that no call uses
+    # a few tokens: what the small-batch kernel needs, and not also what the tiled one would
+    assert lib.gguf_b200_workspace_bytes(capi.OP_GEMV, 12, 8, 4096, 14336) < lib.gguf_b200_scratch_bytes(capi.OP_GEMV, 12, 8, 4096, 14336)
+    assert lib.gguf_b200_scratch_bytes(capi.OP_MMQ, 14, 8, 4096, 14336) == lib.gguf_b200_scratch_bytes(capi.OP_GEMV, 14, 8, 4096, 14336)
 
 
 def test_tensor_parallel_entry_points_validate_arguments(native_libs):

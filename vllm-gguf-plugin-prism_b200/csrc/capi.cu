@@ -221,34 +221,37 @@ static int64_t mmq_small_max_tokens() { return 16; }
 
 static int64_t moe_list_bytes(int64_t n_sorted) { return round_up((n_sorted / mmq_moe_block_size() + 1) * 16 + 16, 256); }
 
+static int64_t share_bytes(int type, int64_t M, int64_t N, int64_t K) {
+  const MmqShare s = mmq_share(type, M, N, K);
+  return s.counter_bytes + s.part_bytes;
+}
+
 int64_t gguf_b200_workspace_bytes(int op, int type, int64_t M, int64_t N, int64_t K) {
   if (!type_size(type) || M < 0 || K <= 0) return 0;
   switch (op) {
     case GGUF_B200_OP_GEMV:
     case GGUF_B200_OP_MOE_VEC: return q8_soa_bytes(M, K);
-    /* dense GEMM: + room for the fp32 partial tiles of a split over K (small N, long K) */
-    case GGUF_B200_OP_MMQ: return M <= mmq_gemv_max_tokens(type) ? M * mmq_ldb(type, K) * 2 : mmq_b_bytes(type, M, K) + mmq_split_scratch_bytes(M, N > 0 ? N : 0, K);
+    /* dense GEMM: + the parts of tiles that several CTAs share */
+    case GGUF_B200_OP_MMQ: return M <= mmq_gemv_max_tokens(type) ? M * mmq_ldb(type, K) * 2 : mmq_b_bytes(type, M, K) + share_bytes(type, M, N, K);
     /* M = length of sorted_token_ids; behind the activations, the work list */
     case GGUF_B200_OP_MOE: return mmq_b_bytes(type, M, K) + moe_list_bytes(M);
-    case GGUF_B200_OP_DEQUANT_MATMUL: return mmq_split_scratch_bytes(M, N > 0 ? N : 0, K);
+    case GGUF_B200_OP_DEQUANT_MATMUL: return share_bytes(type, M, N, K);
   }
   return 0;
 }
 
 int64_t gguf_b200_scratch_bytes(int op, int type, int64_t M, int64_t N, int64_t K) {
-  int64_t most = gguf_b200_workspace_bytes(op, type, M, N, K);
-  if (!type_size(type) || N <= 0 || K <= 0 || M <= 0) return most;
-  auto at_least = [&](int64_t b) { if (b > most) most = b; };
-  if (M >= small_min_tokens() && (op == GGUF_B200_OP_GEMV || (op == GGUF_B200_OP_MMQ && M <= mmq_small_max_tokens()))) at_least(small_bytes(M, N, K));
-  if (op == GGUF_B200_OP_MMQ || op == GGUF_B200_OP_DEQUANT_MATMUL) {
-    const MmqShare share = mmq_share(type, M, N, K);
-    at_least((op == GGUF_B200_OP_MMQ ? mmq_b_bytes(type, M, K) : 0) + share.counter_bytes + share.part_bytes);
+  const int64_t least = gguf_b200_workspace_bytes(op, type, M, N, K);
+  if (!type_size(type) || N <= 0 || K <= 0 || M <= 0) return least;
+  if (M >= small_min_tokens() && (op == GGUF_B200_OP_GEMV || (op == GGUF_B200_OP_MMQ && M <= mmq_small_max_tokens()))) {
+    const int64_t small = small_bytes(M, N, K);
+    return small > least ? small : least;
   }
   if (op == GGUF_B200_OP_MOE) {
     const MmqShare share = mmq_share_moe(N, M / mmq_moe_block_size() + 1, mmq_moe_block_size());
-    at_least(mmq_b_bytes(type, M, K) + moe_list_bytes(M) + share.counter_bytes + share.part_bytes);
+    return least + share.counter_bytes + share.part_bytes;
   }
-  return most;
+  return least;
 }
 
 int gguf_b200_mul_mat_vec_a8(const void* W, const void* X, void* Y, void* ws, int64_t ws_bytes, int type, int dtype,

@@ -126,7 +126,7 @@ struct MmqArgs {
   int* status;
   const MmqTp* tp;          // null: plain output y
   bool w_in_flight;         // no quantizer is ahead and earlier work may still write w (see pdl_wait)
-  // Optional: room for tiles that several CTAs share (mmq_share_bytes).  `counter` must be zero when the kernel starts.
+  // Optional: room for tiles that several CTAs share (mmq_share).  `counter` must be zero when the kernel starts.
   int* counter;
   int64_t zero_counters;    // > 0: so many words of it are cleared here first
   void* part;               // 16-byte aligned, part_bytes long
@@ -137,8 +137,6 @@ int launch_mmq(const MmqArgs& a, cudaStream_t stream);
 struct MmqShare { int64_t n_counters, counter_bytes, part_bytes; };
 MmqShare mmq_share(int type, int64_t M, int64_t N, int64_t K);   // all zero where sharing does not pay
 MmqShare mmq_share_moe(int64_t N, int64_t max_passes, int64_t pass_rows);
-// fp32 scratch that a dense M x N x K problem used to split K with (what gguf_b200_workspace_bytes reports)
-int64_t mmq_split_scratch_bytes(int64_t M, int64_t N, int64_t K);
 int launch_zero(int* p, int64_t n, cudaStream_t stream);
 int mmq_moe_block_size();
 

@@ -127,14 +127,6 @@ MmqShare mmq_share_moe(int64_t N, int64_t max_passes, int64_t pass_rows) {
   return s;
 }
 
-int64_t mmq_split_scratch_bytes(int64_t M, int64_t N, int64_t K) {
-  const int tn = M <= 32 ? 32 : (M <= 64 ? 64 : (M <= 128 ? 128 : 256));
-  const int64_t tiles = ((N + MMQ_ROWS - 1) / MMQ_ROWS) * ((M + tn - 1) / tn), nmain = (K + MMQ_BK - 1) / MMQ_BK;
-  for (int s = 16; s >= 2; --s)
-    if (tiles * s <= 148 && nmain / s >= 16) return (int64_t)s * M * N * 4;
-  return 0;
-}
-
 __global__ void __launch_bounds__(256) zero_kernel(int* p, int64_t n) {
   pdl_trigger();
   pdl_wait();
