@@ -153,3 +153,17 @@ def test_quantizers_let_the_product_start_only_behind_their_own_wait():
     assert len(kernels) == 3
     for k in kernels:
         assert 0 < k.index("pdl_wait();") < k.index("pdl_trigger();")
+
+
+def test_tiles_are_shared_where_that_pays(native_libs):
+    """The plan of the tiled kernel shows in the room it asks for: 112 row tiles on 148 SMs are not worth cutting into runs for a
+    few tokens (Q5_K, 24 tokens: 28.3 us in runs, 25.5 whole), 32 row tiles of long rows are."""
+    from gguf_b200 import capi
+
+    lib = capi.lib()
+    for t in (2, 8, 10, 12, 13):
+        for m in (17, 24, 32, 64):
+            n, k = 14336, 4096
+            columns = k + (k // 32 + 63) // 64 * 64 if t in (2, 12, 13) else k
+            assert lib.gguf_b200_workspace_bytes(capi.OP_MMQ, t, m, n, k) == (m * columns * 2 + 255) // 256 * 256, (t, m)
+            assert lib.gguf_b200_workspace_bytes(capi.OP_MMQ, t, m, 4096, 14336) > 1 << 20

@@ -36,7 +36,7 @@
 // clocks passed before a tile's first MMA and 4,800 in its epilogue, of 46,700 at 512 tokens; at 32 tokens a stage took 445
 // clocks because a B slot came back 745 clocks after its MMA and refilling it took 1,050 more, over a ring of four.
 // tcgen05.mma itself takes max(61, tn / 2) clocks per 16 values, so at 128 tokens or less a stage need not take more than 256;
-// it takes about 350 with the whole-stage decoders, 600 to 1,000 with the others, which is what bounds those.
+// it takes 450 to 540 with the whole-stage decoders and 540 to 780 with the others (mmq_decode_clocks), which is what bounds those.
 // Measured, before -> after: IQ3_S 8192 x 28672, 300 tokens 291 -> 134 us; Q6_K 37888 x 3584, 1999 tokens 668 -> 567 us;
 // IQ2_XXS 28672 x 8192, 128 tokens 108 -> 95 us; a MoE step of 256 tokens (64 experts, Q4_0) 222 -> 169 us.
 #include "mmq_kernel.cuh"
@@ -68,42 +68,67 @@ static_assert(Stage64<T_Q4_0, __half>::PERM == 1 && Stage64<T_Q4_K, __half>::PER
 //   whole    every tile is one CTA's
 //   even     few tiles: each is cut into the same number of ranges of chunks, one per CTA
 //   stream   the chunks of all tiles in equal runs over all SMs
-// A stage takes two clocks per token on the tensor core, or the time to decode it: about 420 clocks for the whole-stage
-// decoders, 600 for the others.  Reading a tile out takes 16 clocks per token (beside the next tile's work where there are two
-// accumulators); sharing, 20 clocks per token and 10 more per part where a CTA has one part, 3,000 and 50 per token where it
-// has two.  Fitted to all splits of 14 shapes: 4096 x 4096, 256 tokens of Q4_K took 30.3 us as 32 whole tiles, 33.2 in equal
-// runs and 23.1 as 64 tiles in two ranges each; 14336 x 4096 took 33.4 as 112 whole tiles and 39.9 in equal runs.
+// A stage takes 2.1 clocks per token on the tensor core, or the time to decode it (mmq_decode_clocks); reading a tile out takes
+// 19 clocks per token (beside the next tile's work where there are two accumulators), a CTA in use 59; sharing, 1,600 + 24 per
+// token + 9 per token and part where a CTA has one part of a tile, 9,000 + 19 per token + 13 per token and part where it has two
+// (6,000 by the times alone; the parts of runs also take up to 39 MB of L2: 512 tokens of 14336x4096 Q4_K in runs and in whole tiles
+// are 58.7 and 59.0 us in a row, 71.0 and 69.5 between other work).
+// Fitted by least squares to the times of every plan of 1463 problems (19 types, seven matrices of 1024x4096 to 28672x8192, 17 to
+// 1024 tokens): what it picks takes 0.4 % longer than the best plan on average, 11 % at most.  (With one decode time for the types
+// without a whole-stage decoder, nothing per CTA and cheaper runs it was 3.4 % and 37 %: 17 to 32 tokens of 14336x4096 were cut
+// into runs, 26.0 us for Q4_0 and 28.1 for Q5_K where whole tiles take 23.5 and 25.5.)
 struct MmqPlan {
   int tn;
   int64_t tt, grid;
   bool shared;
 };
+// clocks to decode a stage
+static int mmq_decode_clocks(int type) {
+  switch (type) {
+    case T_Q8_0: return 450;
+    case T_Q4_K: return 480;
+    case T_Q4_0: return 500;
+    case T_Q4_1: case T_Q5_K: return 540;
+    case T_Q5_0: case T_Q2_K: return 550;
+    case T_IQ2_XXS: case T_IQ1_S: return 610;
+    case T_Q6_K: case T_Q5_1: case T_IQ1_M: case T_IQ2_XS: return 650;
+    case T_Q3_K: return 670;
+    case T_IQ3_XXS: case T_IQ2_S: return 710;
+    case T_IQ4_XS: return 735;
+    case T_IQ3_S: return 755;
+    default: return 775;   // IQ4_NL
+  }
+}
 static int64_t mmq_stage_clocks(int type, int tn) {
-  const int decode = type == T_Q4_0 || type == T_Q8_0 || type == T_Q4_K || type == T_Q5_K ? 420 : 600;
-  return 2 * tn > decode ? 2 * tn : decode;
+  const int decode = mmq_decode_clocks(type), mma = 21 * tn / 10;
+  return mma > decode ? mma : decode;
 }
 static MmqPlan mmq_plan(int type, int64_t M, int64_t N, int64_t K, bool may_share) {
   const int64_t rt = (N + MMQ_ROWS - 1) / MMQ_ROWS, nc = (K + RAW_KC - 1) / RAW_KC;
   MmqPlan best{};
   int64_t best_t = INT64_MAX, last = 0;
   // tiles as large as the tensor memory allows, or of one instruction, or with two accumulators -- and somewhat smaller ones
-  const struct { int64_t cap, more; } sizes[3] = {{384, 4}, {256, 2}, {128, 1}};
+  const struct { int64_t cap, more; } sizes[3] = {{384, 4}, {256, 3}, {128, 3}};
   for (const auto& z : sizes) {
     for (int64_t tt = (M + z.cap - 1) / z.cap, e = tt + z.more; tt < e; ++tt) {
-      if (tt <= last) continue;
+      if (tt <= last || tt > M) continue;
       last = tt;
       const int64_t rows = (M + tt - 1) / tt;
       const int tn = (int)round_up(rows, rows > 256 ? 32 : 16);
+      if ((M + tn - 1) / tn < tt) continue;   // (rounded up, fewer tiles do)
       const int64_t tiles = rt * tt, chunk = 4 * mmq_stage_clocks(type, tn), waves = (tiles + MMQ_CTAS - 1) / MMQ_CTAS;
       const bool twin = tn <= 128;
       auto take = [&](int64_t t, int64_t grid, bool shared) {
+        t += 59 * grid;
         if (t < best_t) { best_t = t; best = {tn, tt, grid, shared}; }
       };
-      take(waves * nc * chunk + (twin ? 1 : waves) * 16 * tn, tiles < MMQ_CTAS ? tiles : MMQ_CTAS, false);
+      take(waves * nc * chunk + (twin ? 1 : waves) * 19 * tn, tiles < MMQ_CTAS ? tiles : MMQ_CTAS, false);
       if (!may_share) continue;
-      if (tiles % MMQ_CTAS != 0 && tiles * nc >= 2 * MMQ_CTAS)
-        take((tiles * nc + MMQ_CTAS - 1) / MMQ_CTAS * chunk + (twin ? 1 : tiles / MMQ_CTAS + 1) * 16 * tn + 3000 + 50 * tn, MMQ_CTAS, true);
-      for (int64_t c = 2; c * tiles <= MMQ_CTAS && 2 * c <= nc; ++c) take((nc + c - 1) / c * chunk + 1500 + tn * (36 + 10 * c), c * tiles, true);
+      if (tiles % MMQ_CTAS != 0 && tiles * nc >= 2 * MMQ_CTAS) {
+        const int64_t run = (tiles * nc + MMQ_CTAS - 1) / MMQ_CTAS;
+        take(run * chunk + (twin ? 1 : tiles / MMQ_CTAS + 1) * 19 * tn + 9000 + 19 * tn + 13 * tn * nc / run, MMQ_CTAS, true);
+      }
+      for (int64_t c = 2; c * tiles <= MMQ_CTAS && 2 * c <= nc; ++c) take((nc + c - 1) / c * chunk + 1600 + tn * (43 + 9 * c), c * tiles, true);
     }
   }
   return best;
@@ -224,7 +249,7 @@ int launch_mmq(const MmqArgs& a, cudaStream_t stream) {
     p.counter = a.counter;
   }
   // The number of passes of a MoE step is known on the device only: there tiles are shared where that saves more than it costs.
-  p.waste = a.passes ? (int)((3000 + 50 * p.tn) / (4 * mmq_stage_clocks(a.type, p.tn))) : 0;
+  p.waste = a.passes ? (int)((6000 + 45 * p.tn) / (4 * mmq_stage_clocks(a.type, p.tn))) : 0;
   if (p.part && a.zero_counters > 0) {
     const int rc = launch_zero(a.counter, a.zero_counters, stream);
     if (rc) return rc;
