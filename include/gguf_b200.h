@@ -18,7 +18,7 @@
  * Stream order: X, Y and the workspace follow the stream as usual.  Weights may be read ahead of it: gguf_b200_mul_mat_vec_a8
  * with one vector, gguf_b200_gemv_prepared and gguf_b200_dequant_matmul (plain, strided or tensor-parallel) start on W while the
  * kernel ahead of them in the stream is still finishing.  A host that writes weights on the device (loading, merging an
- * adapter) queues any other kernel behind the writes, or synchronises, before it uses them; where W comes straight out of a
+ * adapter) calls gguf_b200_weights_complete, or synchronises, before it uses them; where W comes straight out of a
  * kernel, it calls gguf_b200_mul_mat_strided with GGUF_B200_W_IN_FLIGHT.  All other entry points read W in stream order.
  */
 #ifndef GGUF_B200_H
@@ -94,7 +94,12 @@ int64_t gguf_b200_workspace_bytes(int op, int type, int64_t M, int64_t N, int64_
  * two-vector kernel, or the tiled kernel.  For gguf_b200_moe_a8 it adds the parts of shared tiles. */
 int64_t gguf_b200_scratch_bytes(int op, int type, int64_t M, int64_t N, int64_t K);
 
-/* Decode GEMV: Y[M][N] = q8_1(X) . dequant(W)^T, weights read once for up to 8 vectors.
+/* Queues an empty kernel behind the work that wrote weights: it starts when that is complete and visible, and whatever is
+ * queued behind it may read weights ahead of the stream.  For the end of loading. */
+int gguf_b200_weights_complete(void* stream);
+
+/* Decode GEMV: Y[M][N] = q8_1(X) . dequant(W)^T.  One or two vectors read the weights once; from three on the small-batch kernel
+ * reads them once for every 32 vectors, given gguf_b200_scratch_bytes of workspace (with less: once for every two to eight).
  * Replaces: ggml_mul_mat_vec_a8, gguf_kernel.cu:104-218 (+ mmvq.cuh). */
 int gguf_b200_mul_mat_vec_a8(const void* W, const void* X, void* Y, void* workspace, int64_t workspace_bytes,
                              int type, int dtype, int64_t M, int64_t N, int64_t K, void* stream);

@@ -434,6 +434,8 @@ int gguf_b200_tp_wait(const uint32_t* flags_local, const uint32_t* epochs_local,
   return launch_tp_wait(flags_local, epochs_local, slot, world, g_wait_limit_cycles, st, static_cast<cudaStream_t>(stream));
 }
 
+int gguf_b200_weights_complete(void* stream) { return launch_fence(static_cast<cudaStream_t>(stream)); }
+
 int gguf_b200_gemv_prepare(const void* X, int dtype, void* ws, int64_t ws_bytes, int type, int64_t M, int64_t K,
                            void* stream) {
   if (!type_size(type)) return E_BAD_TYPE;

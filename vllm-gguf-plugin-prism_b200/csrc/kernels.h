@@ -138,6 +138,7 @@ struct MmqShare { int64_t n_counters, counter_bytes, part_bytes; };
 MmqShare mmq_share(int type, int64_t M, int64_t N, int64_t K);   // all zero where sharing does not pay
 MmqShare mmq_share_moe(int64_t N, int64_t max_passes, int64_t pass_rows);
 int launch_zero(int* p, int64_t n, cudaStream_t stream);
+int launch_fence(cudaStream_t stream);   // an empty kernel in plain stream order (see pdl_wait)
 int mmq_moe_block_size();
 
 int64_t q8_soa_bytes(int64_t M, int64_t K);

@@ -162,6 +162,12 @@ int launch_zero(int* p, int64_t n, cudaStream_t stream) {
   return launch_pdl(zero_kernel, dim3((unsigned)((n + 255) / 256 > 64 ? 64 : (n + 255) / 256)), dim3(256), 0, stream, p, n) == cudaSuccess ? E_OK : E_CUDA;
 }
 
+__global__ void fence_kernel() {}
+int launch_fence(cudaStream_t stream) {
+  fence_kernel<<<1, 1, 0, stream>>>();
+  return cudaGetLastError() == cudaSuccess ? E_OK : E_CUDA;
+}
+
 static int mmq_aux_bytes(int type) {   // barriers, then the decoder's tables
   switch (type) {
 #define MMQ_TAB(TYPE) case TYPE: return 512 + decoder_table_bytes<TYPE>();

@@ -181,6 +181,11 @@ template <class A> struct Calls {
     return Y;
   }
 
+  static void weights_complete(const Tensor& W) {
+    const typename A::Guard guard(A::device(W));
+    check_rc(gguf_b200_weights_complete(A::stream(W)), "weights_complete");
+  }
+
   static Tensor moe_a8(const Tensor& X, const Tensor& W, const Tensor& sorted_token_ids, const Tensor& expert_ids,
                        const Tensor& num_tokens_post_padded, int64_t type, int64_t row, int64_t top_k, int64_t tokens) {
     const typename A::Guard guard(A::device(X));

@@ -70,6 +70,7 @@ Tensor fused_moe(Tensor X, Tensor W13, Tensor W2, Tensor topk_weights, Tensor to
   return Op::fused_moe(X, W13, W2, topk_weights, topk_ids, type13, type2, act);
 }
 Tensor linear_runs(Tensor X, Tensor W, std::vector<int64_t> runs) { return Op::linear_runs(X, W, runs.data(), runs.size()); }
+void weights_complete(Tensor W) { Op::weights_complete(W); }
 int64_t ggml_moe_get_block_size(int64_t type) { return gguf_b200_moe_block_size((int)type); }
 
 }  // namespace
@@ -85,6 +86,7 @@ STABLE_TORCH_LIBRARY(_C_gguf, ops) {
   ops.def("ggml_moe_get_block_size(int type) -> int");
   ops.def("dequant_matmul(Tensor W, Tensor X, int type, SymInt row) -> Tensor");
   ops.def("dequantize_rows(Tensor W, Tensor ids, int type, ScalarType? dtype) -> Tensor");
+  ops.def("weights_complete(Tensor W) -> ()");
   ops.def("linear_runs(Tensor X, Tensor W, int[] runs) -> Tensor");
   ops.def("fused_moe(Tensor X, Tensor W13, Tensor W2, Tensor topk_weights, Tensor topk_ids, int type13, int type2, int act) -> Tensor");
 }
@@ -97,6 +99,7 @@ STABLE_TORCH_LIBRARY_IMPL(_C_gguf, CUDA, ops) {
   ops.impl("ggml_moe_a8_vec", TORCH_BOX(&ggml_moe_a8_vec));
   ops.impl("dequant_matmul", TORCH_BOX(&dequant_matmul));
   ops.impl("dequantize_rows", TORCH_BOX(&dequantize_rows));
+  ops.impl("weights_complete", TORCH_BOX(&weights_complete));
   ops.impl("linear_runs", TORCH_BOX(&linear_runs));
   ops.impl("fused_moe", TORCH_BOX(&fused_moe));
 }

@@ -34,6 +34,7 @@ SIGNATURES = {
     "gguf_b200_scratch_bytes": (_L, [_I, _I, _L, _L, _L]),
     "gguf_b200_mul_mat_strided": (_I, [_P, _P, _P, _P, _L, _I, _I, _I, _L, _L, _L, _L, _L, _P]),
     "gguf_b200_mul_mat_vec_a8": (_I, [_P, _P, _P, _P, _L, _I, _I, _L, _L, _L, _P]),
+    "gguf_b200_weights_complete": (_I, [_P]),
     "gguf_b200_gemv_prepare": (_I, [_P, _I, _P, _L, _I, _L, _L, _P]),
     "gguf_b200_gemv_prepared": (_I, [_P, _P, _P, _I, _I, _L, _L, _L, _P]),
     "gguf_b200_mul_mat_a8": (_I, [_P, _P, _P, _P, _L, _I, _I, _L, _L, _L, _P]),

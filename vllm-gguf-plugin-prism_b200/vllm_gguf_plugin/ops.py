@@ -147,6 +147,11 @@ def _fused_moe_fake(X, W13, W2, topk_weights, topk_ids, type13, type2, act):
     return torch.empty_like(X)
 
 
+@register_fake("_C_gguf::weights_complete")
+def _weights_complete_fake(W):
+    return None
+
+
 @register_fake("_C_gguf::linear_runs")
 def _linear_runs_fake(X, W, runs):
     return torch.empty((X.shape[0], sum(runs[2::5])), dtype=X.dtype, device=X.device)

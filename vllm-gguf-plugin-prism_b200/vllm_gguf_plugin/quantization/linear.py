@@ -99,11 +99,11 @@ if _HAVE_VLLM:
 
 
 def _weights_complete(w: torch.Tensor) -> None:
-    """Puts an ordinary kernel behind whatever still writes a layer's weights.  A decode product starts on them while the
+    """Puts an empty kernel behind whatever still writes a layer's weights.  A decode product starts on them while the
     kernel ahead of it in the stream is finishing; with this one ahead, which starts when the writes are complete and visible,
     it never starts too soon.  (Whoever rewrites weights in place later calls process_weights_after_loading again.)"""
     if w.is_cuda:
-        torch.empty(1, dtype=torch.int32, device=w.device).fill_(1)
+        torch.ops._C_gguf.weights_complete(w)
 
 
 class GGUFWeightType(torch.nn.Parameter):
