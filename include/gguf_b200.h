@@ -151,8 +151,9 @@ int gguf_b200_moe_a8(const void* X, const void* W, void* Y, void* workspace, int
                      void* stream);
 
 /* The whole MoE step of one layer in one call: expert alignment, gate/up expert product, activation,
- * down expert product, routing weights and the sum over the top_k experts.  Up to 64 tokens, and for types
- * without a tiled kernel, on the small-batch kernel (integer dot products); otherwise on the tiled one.
+ * down expert product, routing weights and the sum over the top_k experts.  Up to 64 tokens, for types
+ * without a tiled kernel, and while an expert gets twelve slots or fewer on average, on the small-batch kernel (integer dot
+ * products); otherwise on the tiled one.
  * Replaces: both branches of _fused_moe_gguf, quantization/fused_moe.py:56-133 (moe_align_block_size,
  * ggml_moe_a8 or ggml_moe_a8_vec, apply_moe_activation, the second product, mul_ by the routing weights,
  * moe_sum: six library ops there).  Here the activation runs inside the second GEMM's activation quantizer and the routing

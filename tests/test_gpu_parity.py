@@ -944,6 +944,34 @@ def test_small_moe_step_matches_separate_products(case):
     assert rel_l2(got.float().cpu(), want.cpu()) <= 2e-3
 
 
+# beyond 64 tokens: slots per expert at the line between the kernels and on both sides of it; min terms, offsets.  The last number
+# scales the activations so that gate and up are about one: with all of them at 1/128 the results were 1e-6, where a step of fp16
+# is 1.5 % of them
+@pytest.mark.parametrize("case", [(2, 2, 64, 2, 65, 512, 256, 1), (12, 14, 32, 4, 96, 512, 256, 64), (13, 6, 16, 2, 96, 512, 256, 128),
+                                  (14, 8, 16, 2, 97, 256, 256, 64), (3, 7, 64, 8, 96, 256, 256, 1), (10, 11, 64, 1, 300, 256, 512, 4)])
+def test_moe_step_of_few_slots_an_expert_matches_the_tiled_products(case):
+    """The step against the block-aligned products of the tiled kernel, which the reference takes for these batches."""
+    from vllm_gguf_plugin import ops
+
+    t13, t2, E, k, T, H, I, scale = case
+    w13 = torch.from_numpy(np.stack([synth.make_weight(t13, 2 * I, H, seed=e) for e in range(E)])).to(DEV)
+    w2 = torch.from_numpy(np.stack([synth.make_weight(t2, H, I, seed=100 + e) for e in range(E)])).to(DEV)
+    x = (dev_x(T, H, seed=T).float() / scale).half()
+    twn, idn = synth.make_routing(T, E, k, T)
+    tw, ids = torch.from_numpy(twn).to(DEV), torch.from_numpy(idn).to(DEV).int()
+    blk = capi.lib().gguf_b200_moe_block_size(t13)
+    s, e, n = [torch.from_numpy(a).to(DEV) for a in synth.moe_align_block_size(idn, blk, E)]
+    y1 = capi.moe_a8(x, w13, s, e, n, t13, 2 * I, k, T)
+    a = (torch.nn.functional.silu(y1[:, :I].float()).half() * y1[:, I:]).contiguous()
+    y2 = capi.moe_a8(a, w2, s, e, n, t2, H, 1, T * k).view(T, k, H)
+    want = (y2.float() * tw.view(T, k, 1)).half().float().sum(1)
+    got = ops.ggml_fused_moe(x, w13, w2, tw, ids, t13, t2, "silu")
+    torch.cuda.synchronize()
+    assert capi.last_status() == 0
+    # two chained re-quantizations: see test_fused_moe_step_matches_reference_sequence
+    assert rel_l2(got.float().cpu(), want.cpu()) <= 1e-2
+
+
 # ragged last tiles, one and two accumulators, two instructions per stage, tiles whole / cut evenly / in runs over all SMs
 TILED_SHAPES = [(7, 256, 20), (259, 768, 100), (2048, 1280, 40), (77, 4096, 513), (1000, 2048, 300), (8192, 1024, 129), (14336, 512, 385)]
 

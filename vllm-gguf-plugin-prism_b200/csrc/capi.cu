@@ -206,17 +206,14 @@ int gguf_b200_dequantize_rows(const void* W, int type, const int64_t* row_ids, i
   return launch_dequantize(W, type, out, out_dtype, n_rows * K, g_q4k_contract, static_cast<cudaStream_t>(stream), row_ids, K, weight_rows);
 }
 
-// Up to this many tokens the op is bound by reading the weights once, which the GEMV kernel does
-// best; it then runs with the tiled kernels' formulas (Q4_K min term from the stored fp16 sum).
-// Measured cross-over on 14336x4096: the types with whole-stage tensor-core decoders win from 5
-// tokens on (Q4_K, 8 tokens: 26.9 us against 37.3 us through the GEMV); the others keep the GEMV
-// up to 16.
-// Largest batch that ggml_mul_mat_a8 serves with the GEMV kernels (tiled formulas) instead of the tensor cores.  Types
-// that exist only in the two-vector register-resident GEMV would need a pass per pair of tokens: beyond two passes the
-// tiled kernel (about 25 us on a 14336x4096 matrix whatever the batch) is faster.  Q6_K has the multi-vector kernel.
+// Batches that gguf_b200_mul_mat_a8 serves without the tiled kernel, with its formulas (Q4_K's min term from the stored fp16
+// sum).  Up to two tokens, and up to this many for a caller whose workspace has no room for the small-batch kernel, with the GEMV
+// kernels, two tokens a pass: beyond two passes the tiled kernel is faster (14336x4096 Q4_K, eight tokens: 25 us against 37).
 static int64_t mmq_gemv_max_tokens(int type) { return type == T_Q6_K ? 16 : 4; }
 
-// ... and that the small-batch kernel serves instead, given room for its activation tiles
+// From three tokens to this many, given room, with the small-batch kernel.  14336x4096, small-batch / tiled: at 16 tokens
+// Q4_0 20 / 23 us, Q8_0 24 / 24, Q2_K 25 / 27, Q6_K 28 / 33, Q3_K 30 / 32; at 17 (a third column tile) 26 / 23, 28 / 24, 31 / 27, 36 / 33,
+// 35 / 32, and the same order for all ten types.
 static int64_t mmq_small_max_tokens() { return 16; }
 
 static int64_t moe_list_bytes(int64_t n_sorted) { return round_up((n_sorted / mmq_moe_block_size() + 1) * 16 + 16, 256); }
@@ -623,10 +620,21 @@ FusedMoeLayout fused_moe_layout(int type13, int type2, int dtype, int64_t tokens
   L.total = o;
   return L;
 }
-// Up to this many tokens (and always for types without a tiled kernel) the step runs on the small-batch kernel: an expert
-// then sees a handful of tokens, and reading the weights of the experts in use is what it costs.
-constexpr int64_t kMoeSmallTokens = 64;
-bool moe_small(int type13, int type2, int64_t tokens) { return tokens <= kMoeSmallTokens || !is_mmq_type(type13) || !is_mmq_type(type2); }
+// Which kernel the step runs on.  Up to 64 tokens, and for a code-book type always, the reference takes its GEMV per (token,
+// expert) pair (fused_moe.py:56-133): integer products, which the small-batch kernel gives and the tiled one, whose operands are
+// rounded to 16 bits, does not.  Beyond, what decides is the slots an expert gets on average: small-batch / tiled in us, 64 experts,
+// top-8, hidden 2048, intermediate 1024, at 8 / 12 / 16 / 24 slots an expert: Q4_0 106 / 115 / 136 / 166 against 154 / 157 / 158 / 164,
+// Q8_0 121 / 131 / 156 / 172 against 141 / 143 / 145 / 148, Q6_K 153 / 165 / 209 / 255 against 213 / 215 / 217 / 221.  8, 16 and 32
+// experts, Q4_K, Q5_K, Q2_K/Q3_K: the small-batch kernel is ahead up to 12 everywhere, behind from 24 on nearly everywhere.
+constexpr int64_t kMoeSmallTokens = 64, kMoeSmallSlots = 12;
+bool moe_tiled_types(int type13, int type2) { return is_mmq_type(type13) && is_mmq_type(type2); }
+bool moe_small(int type13, int type2, int64_t tokens, int64_t top_k, int64_t E) {
+  return tokens <= kMoeSmallTokens || !moe_tiled_types(type13, type2) || tokens * top_k <= kMoeSmallSlots * E;
+}
+// (the sums that the format's minima meet: those of the reference's tiled kernels where it takes them, see gguf_b200_mul_mat_a8)
+int moe_sum_mode(int type, int type13, int type2, int64_t tokens) {
+  return tokens > kMoeSmallTokens && moe_tiled_types(type13, type2) ? (type == T_Q5_0 ? 1 : 0) : gemv_sum_mode(type);
+}
 struct MoeSmallLayout {
   int pass_tiles;
   int64_t tiles, passes, o_sorted, o_passes, o_npass, o_y1, o_y2, o_ws, total;
@@ -654,7 +662,7 @@ MoeSmallLayout moe_small_layout(int dtype, int64_t tokens, int64_t top_k, int64_
 int64_t gguf_b200_fused_moe_workspace_bytes(int type13, int type2, int dtype, int64_t tokens, int64_t top_k, int64_t n_experts,
                                             int64_t H, int64_t I) {
   if (!type_size(type13) || !type_size(type2) || tokens < 0 || top_k <= 0 || n_experts <= 0 || n_experts > 256 || H <= 0 || I <= 0) return 0;
-  if (moe_small(type13, type2, tokens)) return moe_small_layout(dtype, tokens, top_k, n_experts, H, I).total;
+  if (moe_small(type13, type2, tokens, top_k, n_experts)) return moe_small_layout(dtype, tokens, top_k, n_experts, H, I).total;
   return fused_moe_layout(type13, type2, dtype, tokens, top_k, n_experts, H, I).total;
 }
 
@@ -669,7 +677,7 @@ int gguf_b200_fused_moe(const void* X, const void* W13, const void* W2, void* Y,
   if (n_experts > 256) return E_TOO_LARGE;
   if (tokens == 0) return E_OK;
   if (!topk_ids || !topk_weights || !ws || !aligned16(ws)) return E_BAD_POINTER;
-  if (moe_small(type13, type2, tokens)) {
+  if (moe_small(type13, type2, tokens, top_k, n_experts)) {
     const MoeSmallLayout L = moe_small_layout(dtype, tokens, top_k, n_experts, H, I);
     if (ws_bytes < L.total) return E_WORKSPACE;
     if (!small_fits(n_experts * 2 * I, H) || !small_fits(n_experts * H, I)) return E_TOO_LARGE;
@@ -685,7 +693,7 @@ int gguf_b200_fused_moe(const void* X, const void* W13, const void* W2, void* Y,
     auto gemm = [&](const void* x, int64_t x_div, int act_mode, const void* w, int type, int64_t N, int64_t K, void* y, const float* scale) {
       SmallArgs a{};
       a.w = w; a.x = x; a.y = y; a.ws = base + L.o_ws;
-      a.type = type; a.dtype = dtype; a.sum_mode = gemv_sum_mode(type);
+      a.type = type; a.dtype = dtype; a.sum_mode = moe_sum_mode(type, type13, type2, tokens);
       a.m = slots; a.n = N; a.k = K;
       a.pitch = K / block_size(type) * type_size(type);
       a.ldy = N;

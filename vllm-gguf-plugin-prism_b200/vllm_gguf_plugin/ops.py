@@ -231,7 +231,7 @@ def ggml_fused_moe(X: torch.Tensor, W13: torch.Tensor, W2: torch.Tensor, topk_we
                    quant_type: int, quant_type2: int, activation: str) -> torch.Tensor:
     """The MoE step of one layer in one call: alignment, gate/up expert product, activation, down expert product, routing
     weights and the top-k sum (the reference runs six ops for it, quantization/fused_moe.py:56-133).  X [T, H] -> [T, H].
-    Up to 64 tokens, and for the code-book types, on the small-batch kernel; above that on the tiled one."""
+    Up to 64 tokens, for the code-book types, and while an expert gets few tokens, on the small-batch kernel; else on the tiled one."""
     _require(quant_type, _CUDA_GEMV_QUANT_TYPES, "ggml_fused_moe")
     _require(quant_type2, _CUDA_GEMV_QUANT_TYPES, "ggml_fused_moe")
     if topk_weights.dtype != torch.float32 or not topk_weights.is_contiguous():
