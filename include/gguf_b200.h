@@ -9,9 +9,9 @@
  * as void*).  Scratch memory is provided by the caller (gguf_b200_workspace_bytes).
  *
  * Types: GGML ids 2 (Q4_0), 3 (Q4_1), 6 (Q5_0), 7 (Q5_1), 8 (Q8_0), 10 (Q2_K), 11 (Q3_K), 12 (Q4_K), 13 (Q5_K),
- * 14 (Q6_K) -- every type of the reference's tiled kernels -- and 16 (IQ2_XXS), 20 (IQ4_NL), 23 (IQ4_XS); the
- * dequantize and the GEMV entry points (mul_mat_vec_a8, moe_a8_vec and their variants) also take 17 (IQ2_XS),
- * 18 (IQ3_XXS), 19 (IQ1_S), 21 (IQ3_S), 22 (IQ2_S), 29 (IQ1_M) -- all nineteen block types of the reference's dispatch.
+ * 14 (Q6_K) -- every type of the reference's tiled kernels, and of mul_mat_a8 and moe_a8 here; everything else also takes
+ * 16 (IQ2_XXS), 17 (IQ2_XS), 18 (IQ3_XXS), 19 (IQ1_S), 20 (IQ4_NL), 21 (IQ3_S), 22 (IQ2_S), 23 (IQ4_XS), 29 (IQ1_M) -- all
+ * nineteen block types of the reference's dispatch (dequant_matmul takes these nine).
  * Weights W are raw GGUF blocks, row-major `uint8 [N][K/QK*type_size]`, base 16-byte aligned.
  * Activations X are `[M][K]` contiguous in `dtype`; outputs Y are `[M][N]` in the same dtype.
  *
@@ -131,7 +131,7 @@ int gguf_b200_mul_mat_a8(const void* W, const void* X, void* Y, void* workspace,
 
 /* Fused dequantize + dense GEMM with unquantized activations: Y = X . dequant(W)^T.
  * Replaces the two-step route the reference takes for IQ types at larger batches
- * (quantization/linear.py:50-54: ggml_dequantize then x @ W.T).  dtype f16 or bf16.  Types 16, 20, 23. */
+ * (quantization/linear.py:50-54: ggml_dequantize then x @ W.T).  dtype f16 or bf16.  The nine IQ types. */
 int gguf_b200_dequant_matmul(const void* W, const void* X, void* Y, void* workspace, int64_t workspace_bytes,
                              int type, int dtype, int64_t M, int64_t N, int64_t K, void* stream);
 
@@ -249,7 +249,7 @@ int gguf_b200_tp_unpack_sum(const void* packets_local, const uint32_t* epochs_lo
 int gguf_b200_tp_unpack(const void* packets_local, const uint32_t* epochs_local, int slot0, int nslots,
                         int64_t slot_packets, int64_t n, void* out, int64_t out_stride, int dtype, void* stream);
 
-/* Prefill, M activation rows: op = GGUF_B200_OP_MMQ (q8_1-quantized activations, types 2/8/12/14)
+/* Prefill, M activation rows: op = GGUF_B200_OP_MMQ (q8_1-quantized activations, the types of mul_mat_a8)
  * or GGUF_B200_OP_DEQUANT_MATMUL (IQ types, f16/bf16).  y_peers[r] = rank r's gathered output
  * [M][world*N_local] in `dtype` (16-byte aligned; N_local a multiple of 8): the tensor-core kernel's
  * tile epilogue (or, when K is split over CTAs, the kernel that adds the partial tiles) stores this

@@ -203,7 +203,6 @@ int launch_mmq(const MmqArgs& a, cudaStream_t stream) {
   p.sa = p.tn <= 256 ? 8 : 4;
   p.a_col0 = p.tn <= 256 ? 256 : 384;
   p.nbuf = p.tn <= 128 ? 2 : 1;
-  p.d_step = 128;
   p.status = a.status;
   p.w_wait = a.w_in_flight ? 1 : 0;
   p.passes = static_cast<const int4*>(a.passes);

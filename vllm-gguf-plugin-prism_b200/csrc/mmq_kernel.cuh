@@ -16,10 +16,10 @@ constexpr int MMQ_BK = 64;                           // values per stage (128 by
 constexpr int MMQ_GROUPS = 4;                        // producer groups of 128 threads, one thread per weight row
 constexpr int MMQ_PRODUCER_WARPS = 4 * MMQ_GROUPS;
 constexpr int MMQ_THREADS = (MMQ_PRODUCER_WARPS + 3) * 32;   // + B loader, MMA issuer, raw-weight loader
-// Tensor memory: up to 128 tokens a tile, two accumulators of 128 columns and eight A slots of 32; beyond, 384 columns of
-// accumulator -- two of 192, or one of 384 -- and four A slots.  The stages' barriers are a ring of eight in both cases: a
+// Tensor memory: up to 256 tokens a tile, 256 columns of accumulator -- two of 128, or one beyond 128 tokens -- and eight A slots
+// of 32; up to 384 tokens, one accumulator and four A slots.  The stages' barriers are a ring of eight in both cases: a
 // group's stages are eight apart, so by the time it waits for a phase it has seen the one before complete.
-constexpr int MMQ_A_COLS = 32, MMQ_BARS = 8;
+constexpr int MMQ_A_COLS = 32, MMQ_BARS = 8, MMQ_D_STEP = 128;
 constexpr int MMQ_MAX_RAW = 8;
 // Correction values of eight chunks (64 fp16) per row, rows an odd number of 16-byte units apart
 constexpr int MMQ_CORR_CHUNKS = 8, MMQ_CORR_ROW = 144, MMQ_CORR_BYTES = MMQ_ROWS * MMQ_CORR_ROW;
@@ -34,9 +34,9 @@ struct MmqParams {
   int n, m;               // weight rows, tokens
   int k, kpad;
   int nc, corr;           // 256-value chunks of a row; 1: a stage of corrections behind every eight of them
-  int rt, tt, tn;         // row tiles, token tiles, tokens per tile (a multiple of 16, at most 256)
+  int rt, tt, tn;         // row tiles, token tiles, tokens per tile (a multiple of 16, at most 256, or of 32, at most 384)
   int sa, a_col0;         // A slots: how many (4 or 8), first column
-  int nbuf, d_step;       // accumulators, columns between them
+  int nbuf;               // accumulators, MMQ_D_STEP columns apart
   int sb, raw_stages;     // ring depths
   int raw_off, aux_off, corr_off;   // shared memory behind the B ring
   uint32_t idesc;
@@ -373,7 +373,7 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_consta
         tc_fence_after();
         pdl_wait();
       }
-      const uint32_t d = d_lane + (uint32_t)(buf * p.d_step);
+      const uint32_t d = d_lane + (uint32_t)(buf * MMQ_D_STEP);
       int first = 0, last = 0, s_first = 0;
       bool in_tmem = mode != FINISH;
       const int slot4 = p.tn * 32;            // float4s of a partial tile
@@ -690,7 +690,7 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_consta
         if (p.corr) end += (q.c1 - 1) / MMQ_CORR_CHUNKS - q.c0 / MMQ_CORR_CHUNKS + 1;
         const int buf = p.nbuf == 2 ? pi & 1 : 0, use = p.nbuf == 2 ? pi >> 1 : pi;
         ok = mbar_wait_bounded(&drained[buf], ((uint32_t)use & 1u) ^ 1u);
-        const uint32_t d = tmem_base + (uint32_t)(buf * p.d_step);
+        const uint32_t d = tmem_base + (uint32_t)(buf * MMQ_D_STEP);
         uint32_t accumulate = 0;
         for (; ok && i < end; ++i) {
           const int s = i & (MMQ_BARS - 1);

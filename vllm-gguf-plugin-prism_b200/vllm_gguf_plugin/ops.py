@@ -9,9 +9,9 @@ Differences from the reference, all deliberate:
 * no Triton backend and no CPU fallback: if the extension is missing, import fails loudly;
   ``VLLM_GGUF_USE_CUDA`` is accepted for compatibility but selects nothing;
 * supported block types are Q4_0, Q4_1, Q5_0, Q5_1, Q8_0, Q2_K, Q3_K, Q4_K, Q5_K, Q6_K (every type of the reference's
-  tiled kernels, ggml_mul_mat_a8 / ggml_moe_a8), IQ2_XXS, IQ4_NL, IQ4_XS and, for ggml_dequantize, ggml_mul_mat_vec_a8
-  and ggml_moe_a8_vec, IQ2_XS, IQ2_S, IQ3_XXS, IQ3_S, IQ1_S, IQ1_M -- with them every type of the reference's
-  dequantize dispatch (dequantize.cuh:527-571) and of its GEMV dispatch is covered; any other type raises
+  tiled kernels, ggml_mul_mat_a8 / ggml_moe_a8) and, for everything else, IQ2_XXS, IQ2_XS, IQ2_S, IQ3_XXS, IQ3_S, IQ1_S,
+  IQ1_M, IQ4_NL, IQ4_XS -- with them every type of the reference's dequantize dispatch (dequantize.cuh:527-571) and of
+  its GEMV dispatch is covered; any other type raises
   ``NotImplementedError`` (the reference silently returns zeros for an unknown type in its
   matmul switch, gguf_kernel.cu:236-289);
 * ``ggml_moe_get_block_size`` returns this library's token-block size (64, tensor-core tile)
@@ -82,7 +82,6 @@ QUANT_SIZES = {
     GGML_TYPE_IQ2_XXS: (256, 66),
     GGML_TYPE_IQ4_NL: (32, 18),
     GGML_TYPE_IQ4_XS: (256, 136),
-    # code-book types with a decode GEMV (and MoE GEMV) here; more tokens go through dequantize + matmul
     17: (256, 74),    # IQ2_XS
     22: (256, 82),    # IQ2_S
     18: (256, 98),    # IQ3_XXS

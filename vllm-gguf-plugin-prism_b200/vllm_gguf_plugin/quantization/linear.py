@@ -3,8 +3,8 @@
 
 ``_fused_mul_mat_gguf`` keeps the reference's batch-size routing (linear.py:35-58):
 GEMV for small batches, the tensor-core q8_1 GEMM for standard/K quants, and for IQ types
-above the GEMV threshold the dequantize-then-matmul route -- fused here into one kernel for
-fp16/bf16 activations.  ``GGUFLinearMethod`` keeps the reference's method signatures
+above the GEMV threshold the dequantize-then-matmul route -- one kernel here for fp16/bf16
+activations.  ``GGUFLinearMethod`` keeps the reference's method signatures
 (linear.py:80-101, 154, 221-226); weights are raw GGUF bytes ``uint8 [N, K/QK*type_size]``.
 vLLM is optional at import time: with it the method registers as a vLLM LinearMethodBase and
 the dispatcher as the custom op ``vllm::_fused_mul_mat_gguf``; without it the same Python
@@ -69,7 +69,7 @@ def _fused_mul_mat_gguf(x: torch.Tensor, weight: torch.Tensor, weight_type: int)
     elif weight_type in MMQ_QUANT_TYPES and int(weight_type) in ops._CUDA_GEMM_QUANT_TYPES:
         y = ops.ggml_mul_mat_a8(weight, x, weight_type, weight.shape[0])
     elif weight_type in DEQUANT_TYPES:
-        # the reference's route for the code-book types: dequantize, then a dense product (fused for three of them)
+        # the reference's route for the code-book types: dequantize, then a dense product (one kernel here)
         if x.dtype in (torch.float16, torch.bfloat16) and int(weight_type) in ops._DEQUANT_MATMUL_TYPES:
             y = ops.ggml_dequant_matmul(weight, x, weight_type, weight.shape[0])
         else:  # fp32 activations: the reference's two steps
