@@ -212,3 +212,63 @@ def test_layer_copies_only_what_the_kernels_cannot_read_in_place(native_libs):
             assert rel_l2(op(x, W, runs).float().cpu(), want.float().cpu()) <= 3e-4, (K, M)
     torch.cuda.synchronize()
     assert capi.last_status() == 0
+
+
+def eager_cases():
+    """(function of native.py, call through the public API, operator that the call becomes)"""
+    from vllm_gguf_plugin import ops
+    from vllm_gguf_plugin.quantization import fused_moe, vocal_embeds
+
+    w, x = weight(12, 64, 256), torch.randn(20, 256, device=DEV).half()
+    iq = weight(23, 64, 256)
+    ids = torch.arange(4, device=DEV)
+    w13, w2 = (torch.from_numpy(np.stack([synth.make_weight(2, 128, k, seed=e) for e in range(4)])).to(DEV) for k in (128, 64))
+    tw, eid = torch.ones(3, 2, device=DEV), torch.zeros(3, 2, dtype=torch.int32, device=DEV)
+    x3 = torch.randn(3, 128, device=DEV).half()
+    method, layer, _ = merged_layer((12, 12, 14), [64, 32, 32], 256)
+    one, plain, _ = merged_layer((12, 12, 12), [64, 32, 32], 256)
+    return [("mul_mat", lambda: ops.ggml_mul_mat_vec_a8(w, x, 12, 64), "ggml_mul_mat_vec_a8"), ("mul_mat", lambda: ops.ggml_mul_mat_a8(w, x, 12, 64), "ggml_mul_mat_a8"),
+            ("mul_mat", lambda: ops.ggml_dequant_matmul(iq, x, 23, 64), "dequant_matmul"),
+            ("embed", lambda: vocal_embeds._apply_gguf_embedding(ids, w, 12, 256, torch.float16), "dequantize_rows"),
+            ("moe", lambda: fused_moe._fused_moe_gguf(x3, w13, w2, tw, eid, 2, 2, "silu"), "fused_moe"),
+            ("linear_runs", lambda: method.apply(layer, x), "linear_runs"), ("linear", lambda: one.apply(plain, x), "linear_runs")]
+
+
+@pytest.mark.parametrize("i", range(7))
+def test_dispatch_modes_and_compilation_see_the_operator(native_libs, monkeypatch, i):
+    """The eager function serves the plain call; a dispatch mode, a traced and a compiled call see the registered operator and
+    get the same bits."""
+    from torch.utils._python_dispatch import TorchDispatchMode
+    from vllm_gguf_plugin import native
+
+    name, call, op = eager_cases()[i]
+    answers, function = [], getattr(native, name)
+
+    def recorded(*args):
+        answers.append(function(*args))
+        return answers[-1]
+
+    monkeypatch.setattr(native, name, recorded)
+    want = call()
+    assert len(answers) == 1 and answers[0] is not None
+    seen = []
+
+    class Mode(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            seen.append(str(func))
+            return func(*args, **(kwargs or {}))
+
+    with Mode():
+        got = call()
+    assert answers[-1] is None and f"_C_gguf.{op}.default" in seen, seen
+    assert torch.equal(got, want)
+    monkeypatch.setattr(native, name, function)
+    graphs = []
+
+    def backend(gm, inputs):
+        graphs.append([str(n.target) for n in gm.graph.nodes if n.op == "call_function"])
+        return gm.forward
+
+    torch._dynamo.reset()
+    assert torch.equal(torch.compile(call, backend=backend)(), want)
+    assert any(op in t for g in graphs for t in g), graphs

@@ -1036,3 +1036,21 @@ def test_merged_shards_of_several_types(types, K):
             assert rel_l2(method.apply(layer, x).float().cpu(), want.float().cpu()) <= tol, (M, dtype)
     torch.cuda.synchronize()
     assert capi.last_status() == 0
+
+
+@pytest.mark.parametrize("shape", TILED_SHAPES)
+def test_tiled_q5_0_product_of_every_shape(shape):
+    """Q5_0's tiled formula folds the offset into the codes, which no row-by-row product here does: against the dequantized
+    weights and the quantized activations multiplied in 64 bits."""
+    t, (N, K, M) = TYPES["Q5_0"], shape
+    _, w = dev_w(t, N, K, seed=N + K)
+    x = (dev_x(M, K, seed=M).float() / 8).half()
+    y = capi.mul_mat_a8(w, x, t, N)
+    blocks = capi.quantize_q8_1(x).view(M, -1, 36)[:, :K // 32].contiguous()
+    d = blocks[..., :2].contiguous().view(torch.float16).double()
+    xq = (blocks[..., 4:].contiguous().view(torch.int8).double() * d).reshape(M, K)
+    want = xq @ capi.dequantize(w, t, N, K, torch.float16).double().T
+    assert rel_l2(y.float().cpu(), want.cpu()) <= REL_L2_TOL
+    assert torch.equal(y, capi.mul_mat_a8(w, x, t, N))
+    torch.cuda.synchronize()
+    assert capi.last_status() == 0
