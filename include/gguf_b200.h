@@ -16,8 +16,8 @@
  * Activations X are `[M][K]` contiguous in `dtype`; outputs Y are `[M][N]` in the same dtype.
  *
  * Stream order: X, Y and the workspace follow the stream as usual.  Weights may be read ahead of it: gguf_b200_mul_mat_vec_a8
- * with one vector, gguf_b200_gemv_prepared and gguf_b200_dequant_matmul (plain, strided or tensor-parallel) start on W while the
- * kernel ahead of them in the stream is still finishing.  A host that writes weights on the device (loading, merging an
+ * with one or two vectors, gguf_b200_gemv_prepared and gguf_b200_dequant_matmul (plain, strided or tensor-parallel) start on W while
+ * the kernel ahead of them in the stream is still finishing.  A host that writes weights on the device (loading, merging an
  * adapter) calls gguf_b200_weights_complete, or synchronises, before it uses them; where W comes straight out of a
  * kernel, it calls gguf_b200_mul_mat_strided with GGUF_B200_W_IN_FLIGHT.  All other entry points read W in stream order.
  */

@@ -82,7 +82,7 @@ def test_other_threads_run_while_a_call_waits_for_the_launch_queue(native_libs, 
 
 # (operation, tokens, K): the one-launch and the two-launch GEMV, two vectors, the small-batch kernel, the tiled one, the GEMM
 # on plain activations with whole tiles and with shared ones, the GEMV per routed expert
-IN_FLIGHT = [("vec", "Q4_K", 1, 1024), ("vec", "Q6_K", 1, 8192), ("vec", "Q8_0", 2, 1024), ("vec", "IQ4_XS", 5, 1024), ("mmq", "Q4_K", 8, 1024),
+IN_FLIGHT = [("vec", "Q4_K", 1, 1024), ("vec", "Q6_K", 1, 8192), ("vec", "Q8_0", 2, 1024), ("vec", "Q4_K", 2, 8192), ("vec", "IQ4_XS", 5, 1024), ("mmq", "Q4_K", 8, 1024),
              ("mmq", "Q6_K", 40, 2048), ("dqmm", "IQ2_XXS", 300, 1024), ("dqmm", "IQ4_XS", 20, 4096), ("moe_vec", "Q4_0", 3, 1024)]
 
 

@@ -266,7 +266,9 @@ int gguf_b200_mul_mat_vec_a8(const void* W, const void* X, void* Y, void* ws, in
   if (M >= small_min_tokens() && small_fits(N, K) && ws_bytes >= small_bytes(M, N, K))
     return small_dense(W, X, Y, ws, type, dtype, gemv_sum_mode(type), M, N, K, K / block_size(type) * type_size(type), N, st, s);
   // the Q4_K / Q5_K GEMV takes its min term from the quantized codes (sum_mode 1), all others from the fp16 sum
-  rc = launch_quantize_q8_1(X, dtype, ws, M, K, Q8_MODE_SOA, gemv_sum_mode(type), 0, CORR_NONE, nullptr, 1, 0, s);
+  Q8Tp qt{};
+  qt.early = M <= 2;
+  rc = launch_quantize_q8_1(X, dtype, ws, M, K, Q8_MODE_SOA, gemv_sum_mode(type), 0, CORR_NONE, nullptr, 1, 0, s, 0, &qt);
   if (rc) return rc;
   return launch_gemv(W, ws, Y, type, dtype, M, N, K, st, s);
 }
@@ -312,6 +314,7 @@ int gguf_b200_mul_mat_vec_a8_tp(const void* W, const void* X, void* const* packe
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   Q8Tp qt{};
+  qt.early = 1;
   qt.bump = epochs_local + slot;    // this launch's number, read by the GEMV kernel behind the quantizer
   qt.status = st;
   qt.limit_cycles = g_wait_limit_cycles;
@@ -351,6 +354,7 @@ int gguf_b200_mul_mat_vec_a8_tp_rowpar(const void* W_local, const void* X_local,
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   Q8Tp qt{};
+  qt.early = 1;
   qt.bump = epochs_local + slot;
   qt.status = st;
   qt.limit_cycles = g_wait_limit_cycles;
@@ -525,7 +529,9 @@ int gguf_b200_mul_mat_strided(const void* W, const void* X, void* Y, void* ws, i
   rc = 1;
   if (op == GGUF_B200_OP_GEMV) rc = launch_gemv_fused(W, X, Y, type, dtype, M, N, K, sum_mode, st, s, pitch, in_flight);
   if (rc <= 0) return rc;
-  rc = launch_quantize_q8_1(X, dtype, ws, M, K, Q8_MODE_SOA, sum_mode, 0, CORR_NONE, nullptr, 1, 0, s);
+  Q8Tp qt{};
+  qt.early = op == GGUF_B200_OP_GEMV && !in_flight;
+  rc = launch_quantize_q8_1(X, dtype, ws, M, K, Q8_MODE_SOA, sum_mode, 0, CORR_NONE, nullptr, 1, 0, s, 0, &qt);
   if (rc) return rc;
   rc = launch_gemv1(W, ws, Y, type, dtype, N, K, st, s, nullptr, (int)M, nullptr, 0, 0, nullptr, 0, pitch, ldy);
   return rc == 1 ? E_TOO_LARGE : rc;   // rows too long for the kernels that take a pitch

@@ -26,6 +26,7 @@ struct Q8Tp {
   int add_parts = 1;                // > 1: the slot holds that many fp32 partial vectors (a row-parallel call's), add_stride
   int64_t add_stride = 0;           //      packets apart; their sum, taken in rank order, is the vector that is added
   unsigned* bump = nullptr;
+  int early = 0;                    // the product behind the quantizer may read its weights before work ahead of both is complete
   long long limit_cycles = 0;
   int* status = nullptr;
 };

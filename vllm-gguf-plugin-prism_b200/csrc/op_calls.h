@@ -110,11 +110,13 @@ template <class A> struct Calls {
     const typename A::Scratch ws(X, ws_bytes);
     void* s = A::stream(X);
     int rc = GGUF_B200_E_TOO_LARGE;
-    if (!settled && (op == GGUF_B200_OP_DEQUANT_MATMUL || (op == GGUF_B200_OP_GEMV && M == 1)))
+    if (!settled && (op == GGUF_B200_OP_DEQUANT_MATMUL || (op == GGUF_B200_OP_GEMV && M <= 2)))
       rc = gguf_b200_mul_mat_strided(W.data_ptr(), X.data_ptr(), Y.data_ptr(), ws.get(), ws_bytes, op | GGUF_B200_W_IN_FLIGHT, (int)type, code, M, row,
                                      K, W.size(W.dim() - 1), row, s);
     if (rc != GGUF_B200_E_TOO_LARGE)
-      ;   // (rows too long for that form go through a quantizer, which keeps the order)
+      ;
+    else if (!settled && op == GGUF_B200_OP_GEMV && M <= 2)   // rows too long for that form
+      check_rc(gguf_b200_weights_complete(s), name), rc = gguf_b200_mul_mat_vec_a8(W.data_ptr(), X.data_ptr(), Y.data_ptr(), ws.get(), ws_bytes, (int)type, code, M, row, K, s);
     else if (op == GGUF_B200_OP_GEMV)
       rc = gguf_b200_mul_mat_vec_a8(W.data_ptr(), X.data_ptr(), Y.data_ptr(), ws.get(), ws_bytes, (int)type, code, M, row, K, s);
     else if (op == GGUF_B200_OP_MMQ)

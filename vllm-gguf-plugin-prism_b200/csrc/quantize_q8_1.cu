@@ -30,8 +30,9 @@ __global__ void __launch_bounds__(256) quantize_q8_1_kernel(const in_t* __restri
                                                             int64_t M, int64_t K, int64_t kpad, int sum_mode,
                                                             int64_t ldb, int corr_mode, const int32_t* __restrict__ gather_ids,
                                                             int64_t gather_div, int64_t gather_limit, Q8Tp tp) {
-  pdl_wait();     // the activations (and the scratch we overwrite) belong to earlier kernels
-  pdl_trigger();  // not before: the product behind this kernel reads weights as soon as it starts (see pdl_wait)
+  if (tp.early) pdl_trigger();    // the product behind this kernel may start on its weights now (see pdl_wait)
+  pdl_wait();                     // the activations (and the scratch we overwrite) belong to earlier kernels
+  if (!tp.early) pdl_trigger();   // ... or only when whatever may still write them is complete
   // tensor-parallel decode: this launch's number for the GEMV behind it, and the tag of the
   // gathered vector (written by all ranks' GEMV kernels into this rank's memory) that is added to x
   if (MODE == Q8_MODE_SOA && tp.bump && blockIdx.x == 0 && threadIdx.x == 0) *tp.bump += 1u;
