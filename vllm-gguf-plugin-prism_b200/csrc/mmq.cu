@@ -110,12 +110,12 @@ static MmqPlan mmq_plan(int type, int64_t M, int64_t N, int64_t K, bool may_shar
   // tiles as large as the tensor memory allows, or of one instruction, or with two accumulators -- and somewhat smaller ones
   const struct { int64_t cap, more; } sizes[3] = {{384, 4}, {256, 3}, {128, 3}};
   for (const auto& z : sizes) {
-    for (int64_t tt = (M + z.cap - 1) / z.cap, e = tt + z.more; tt < e; ++tt) {
+    for (int64_t tt = (int64_t)((uint32_t)(M + z.cap - 1) / (uint32_t)z.cap), e = tt + z.more; tt < e; ++tt) {
       if (tt <= last || tt > M) continue;
       last = tt;
-      const int64_t rows = (M + tt - 1) / tt;
+      const int64_t rows = (uint32_t)(M + tt - 1) / (uint32_t)tt;
       const int tn = (int)round_up(rows, rows > 256 ? 32 : 16);
-      if ((M + tn - 1) / tn < tt) continue;   // (rounded up, fewer tiles do)
+      if ((uint32_t)(M + tn - 1) / (uint32_t)tn < tt) continue;   // (rounded up, fewer tiles do)
       const int64_t tiles = rt * tt, chunk = 4 * mmq_stage_clocks(type, tn), waves = (tiles + MMQ_CTAS - 1) / MMQ_CTAS;
       const bool twin = tn <= 128;
       auto take = [&](int64_t t, int64_t grid, bool shared) {
@@ -128,7 +128,13 @@ static MmqPlan mmq_plan(int type, int64_t M, int64_t N, int64_t K, bool may_shar
         const int64_t run = (tiles * nc + MMQ_CTAS - 1) / MMQ_CTAS;
         take(run * chunk + (twin ? 1 : tiles / MMQ_CTAS + 1) * 19 * tn + 9000 + 19 * tn + 13 * tn * nc / run, MMQ_CTAS, true);
       }
-      for (int64_t c = 2; c * tiles <= MMQ_CTAS && 2 * c <= nc; ++c) take((nc + c - 1) / c * chunk + 1600 + tn * (43 + 9 * c), c * tiles, true);
+      // (32-bit divisions: a call asks for its plan three times; a cut into more ranges of the same length only costs)
+      const int ncs = (int)nc;
+      for (int c = 2, len = 0; c * tiles <= MMQ_CTAS && 2 * c <= ncs; ++c) {
+        const int l = (ncs + c - 1) / c;
+        if (l != len) take((int64_t)l * chunk + 1600 + tn * (43 + 9 * c), c * tiles, true);
+        len = l;
+      }
     }
   }
   return best;
