@@ -310,6 +310,9 @@ template <typename T> __device__ __forceinline__ bool packet_read(const void* ba
 //     the product's CTAs no longer wait on the SMs for the activations);
 //   * the GEMV of one or two vectors, and a product that is a call's first kernel (the GEMM on plain activations), read ahead
 //     (a layer of one token 48.5 -> 48.0 us) unless their caller says that the weights are in flight (GGUF_B200_W_IN_FLIGHT).
+__device__ __forceinline__ void bulk_prefetch_l2(const void* src, uint32_t bytes) {   // (aligned as a bulk copy)
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
+}
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
