@@ -837,8 +837,7 @@ __global__ void __launch_bounds__(G1_WARPS * 32, 2) gemv1_kernel(const G1Params 
   const int my_iters = (active && nblk > 0) ? lane_iters(rl_i) : 0;
 
   // copy of the rows [r0, r0 + cnt) (this warp's slice of them) into stage st
-  // (ahead: only into L2.  That is the point where all of the chip agrees on a line, so it holds whoever writes it meanwhile.)
-  auto issue = [&](int r0, int cnt, int st, bool ahead = false) {
+  auto issue = [&](int r0, int cnt, int st) {
     uint8_t* dst = ring + (size_t)st * p.stage_bytes;
     if (contiguous) {
       if (lane == 0) {
@@ -847,9 +846,7 @@ __global__ void __launch_bounds__(G1_WARPS * 32, 2) gemv1_kernel(const G1Params 
         int64_t aend = (end + 15) & ~int64_t(15);
         if (aend > w_safe) aend = w_safe;
         const uint32_t bytes = aend > abeg ? (uint32_t)(aend - abeg) : 0u;
-        if (ahead) {
-          if (bytes) bulk_prefetch_l2(wb + abeg, bytes);
-        } else if (bytes) {
+        if (bytes) {
           mbar_expect_tx(&bars[st], bytes);
           bulk_g2s(dst, wb + abeg, bytes, &bars[st]);
         } else {
@@ -863,10 +860,6 @@ __global__ void __launch_bounds__(G1_WARPS * 32, 2) gemv1_kernel(const G1Params 
       int64_t aend = (end + 15) & ~int64_t(15);
       if (aend > w_safe) aend = w_safe;
       const uint32_t bytes = (lane < cnt && aend > abeg) ? (uint32_t)(aend - abeg) : 0u;
-      if (ahead) {
-        if (bytes) bulk_prefetch_l2(wb + abeg, bytes);
-        return;
-      }
       uint32_t total = bytes;
 #pragma unroll
       for (int m = 1; m < G1_R; m <<= 1) total += __shfl_xor_sync(0xffffffffu, total, m);  // lanes 0..3 hold the sum of lanes 0..3
@@ -884,11 +877,14 @@ __global__ void __launch_bounds__(G1_WARPS * 32, 2) gemv1_kernel(const G1Params 
   // activations are in registers.  (Filling every stage at once was slower: the memory system
   // serves what is outstanding interleaved, so every warp's FIRST item arrived later and the first
   // dot products with it -- 14336x4096 Q4_K 8.6 us against 8.0 us.)
-  if (p.w_wait) {   // the weights may still be written: they are asked for, but not read, before the wait
-    for (int i = 0; i < p.stages - 1 && i < my_iters; ++i) {
-      int r0, cnt;
-      item(rl_i, i, r0, cnt);
-      issue(r0, cnt, 0, true);
+  if (p.w_wait) {
+    // The weights may still be written: a warp's first rows go into L2, and are read behind the wait.  (L2 is where all of the chip
+    // agrees on a line, so it holds whoever writes it meanwhile.)
+    if (lane == 0 && contiguous && my_iters > 0) {
+      const int64_t beg = (int64_t)lane_row0(rl_i) * row_bytes & ~int64_t(15);
+      const int64_t room = w_safe - beg;
+      const uint32_t want = (uint32_t)(R * row_bytes) & ~15u;
+      if (room >= (int64_t)want && want > 0) bulk_prefetch_l2(wb + beg, want);
     }
     pdl_wait();
   }
