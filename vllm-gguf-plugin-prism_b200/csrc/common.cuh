@@ -134,6 +134,12 @@ __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
 __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
+__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
@@ -236,6 +242,29 @@ __device__ __forceinline__ float lds_half_f32(uint32_t saddr) {   // one fp16 va
   unsigned short h;
   asm volatile("ld.shared.u16 %0, [%1];" : "=h"(h) : "r"(saddr));
   return __half2float(__ushort_as_half(h));
+}
+// A bounded wait for threads that go on after a time-out: the word at `gave_up` (shared memory) is set, and every wait that finds it set returns.
+__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+__device__ __forceinline__ void mbar_wait_or(uint32_t bar, uint32_t parity, uint32_t gave_up, uint32_t limit_cycles = 500000000u) {
+  if (mbar_try_wait(bar, parity)) return;
+  const uint32_t t0 = (uint32_t)clock();
+  while (!mbar_try_wait(bar, parity)) {
+    if (lds32(gave_up) != 0u) return;
+    if ((uint32_t)clock() - t0 > limit_cycles) {
+      asm volatile("st.shared.u32 [%0], %1;" ::"r"(gave_up), "r"(1) : "memory");
+      return;
+    }
+  }
 }
 template <int N> __device__ __forceinline__ void lds_words_unaligned(uint32_t a, uint32_t (&w)[N]) {
   const uint32_t al = a & ~3u, sh = (a & 3u) * 8u;

@@ -22,23 +22,27 @@
 // there ([a_tmem] operand form).  Operand B (activations) is K-major in shared memory with the 128-byte swizzle, one TMA box per
 // stage.  Weight rows sit on the M axis so that small token counts do not waste the 128-row instruction.
 //
-// Warp roles: 16 producer warps in four groups of 128 threads, which take half chunks (two stages) in turn and also read the
-// accumulators out; a B loader, an MMA issuer, a raw-weight loader.  One full/empty mbarrier pair per stage serves both
-// operands.  Every wait is bounded in time and reports through the status word.  The correction values are taken from the raw
-// chunk while it is decoded, parked in shared memory, and fed to the tensor core as one stage per eight chunks (gathered from
-// global memory at the end of a tile they took 10,600 clocks of it).
+// Warp roles: 16 producer warps in four groups of 128 threads, which take items -- half chunks, two stages -- in turn and also read
+// the accumulators out; a B loader, an MMA issuer, a raw-weight loader.  An item has one full/empty barrier pair; up to 128
+// tokens a tile its activations arrive on it too, in one box.  Every wait is bounded in time and reports through the status word.
+// The correction values are taken from the raw chunk while it is decoded and written to shared memory as a tile of operand A; the
+// tensor core multiplies it once per eight chunks (gathered from global memory at the end of a tile they took 10,600 clocks of it).
 //
 // One CTA per SM lives for the whole launch, over a range of (tile, 256-value chunk) units (mmq_plan); a tile that several CTAs
 // share is added up by the last of them to arrive, in CTA order (deterministic).  While a tile's accumulator is read out the
-// loaders, the decoders (two stages per group) and, with two accumulators, the tensor core are already at work on the next one.
+// loaders, the decoders (an item per group) and, with two accumulators, the tensor core are already at work on the next one.
 //
 // What bounded the kernel before (one CTA per tile, 64 stages of a tile; clocks taken inside it, Q4_K 14336 x 4096): 5,700
 // clocks passed before a tile's first MMA and 4,800 in its epilogue, of 46,700 at 512 tokens; at 32 tokens a stage took 445
 // clocks because a B slot came back 745 clocks after its MMA and refilling it took 1,050 more, over a ring of four.
-// tcgen05.mma itself takes max(61, tn / 2) clocks per 16 values, so at 128 tokens or less a stage need not take more than 256;
-// it takes 450 to 540 with the whole-stage decoders and 540 to 780 with the others (mmq_decode_clocks), which is what bounds those.
+// tcgen05.mma itself takes max(25, tn / 2) clocks per 16 values when its operands are in uniform registers, 119 to 147 from a loop that the
+// compiler takes for divergent; a wait that is ready, with its address arithmetic, 80 to 250.  With an MMA issuer of the second sort
+// and three waits an item, no type got below 460 to 560 clocks a stage; since its warp stays converged and waits once, the decoders
+// bound the kernel at 128 tokens or less.  Clocks a stage at 48 tokens, before -> after: Q4_K 511 -> 326, Q4_0 490 -> 313, Q2_K 562 -> 397,
+// Q5_K 542 -> 429, IQ2_XXS 621 -> 459, Q3_K 684 -> 465, Q6_K 717 -> 537 (warp instructions a stage of 32 rows 279 -> 199 for Q4_K, 498 -> 346 for Q6_K).
 // Measured, before -> after: IQ3_S 8192 x 28672, 300 tokens 291 -> 134 us; Q6_K 37888 x 3584, 1999 tokens 668 -> 567 us;
-// IQ2_XXS 28672 x 8192, 128 tokens 108 -> 95 us; a MoE step of 256 tokens (64 experts, Q4_0) 222 -> 169 us.
+// IQ2_XXS 28672 x 8192, 128 tokens 108 -> 95 us; a MoE step of 256 tokens (64 experts, Q4_0) 222 -> 169 us.  By items and with the
+// converged issuer: Q6_K 3584 x 18944, 45 tokens 36.5 -> 28.0 us; the MoE step 167.6 -> 142.3; IQ2_XXS 92.5 -> 79.1; Q6_K 1999 tokens 546 -> 503.
 #include "mmq_kernel.cuh"
 
 namespace gguf_b200 {
@@ -206,7 +210,7 @@ int launch_mmq(const MmqArgs& a, cudaStream_t stream) {
   p.tn = plan.tn;
   p.tt = (int)plan.tt;
   p.idesc = umma_idesc(MMQ_ROWS, p.tn > 256 ? p.tn / 2 : p.tn, bf ? 1 : 0);
-  p.sa = p.tn <= 256 ? 8 : 4;
+  p.sa = p.tn <= 256 ? 4 : 2;
   p.a_col0 = p.tn <= 256 ? 256 : 384;
   p.nbuf = p.tn <= 128 ? 2 : 1;
   p.status = a.status;
@@ -229,30 +233,32 @@ int launch_mmq(const MmqArgs& a, cudaStream_t stream) {
       p.tp_flag[r] = a.tp->flag_peer[r];
     }
   }
-  // activations: boxes of 64 values x tn rows, zeros beyond the matrix
+  // activations as [stage of 64 values][row][value]: boxes of one or two stages x tn rows, zeros beyond the matrix
+  p.bg = p.tn <= 128 ? 2 : 1;
   EncodeTiledFn enc = tensor_map_encoder();
-  const cuuint64_t dims[2] = {(cuuint64_t)a.ldb, (cuuint64_t)a.M};
-  const cuuint64_t strides[1] = {(cuuint64_t)a.ldb * 2};
-  const cuuint32_t box[2] = {MMQ_BK, (cuuint32_t)(p.tn > 256 ? p.tn / 2 : p.tn)};
-  const cuuint32_t estr[2] = {1, 1};
-  if (!enc || enc(&bmap, bf ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(a.b), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+  const cuuint64_t dims[3] = {MMQ_BK, (cuuint64_t)a.M, (cuuint64_t)(a.ldb / MMQ_BK)};
+  const cuuint64_t strides[2] = {(cuuint64_t)a.ldb * 2, MMQ_BK * 2};
+  const cuuint32_t box[3] = {MMQ_BK, (cuuint32_t)(p.tn > 256 ? p.tn / 2 : p.tn), (cuuint32_t)p.bg};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  if (!enc || a.ldb % MMQ_BK != 0 ||
+      enc(&bmap, bf ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(a.b), dims, strides, box, estr,
+          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return E_CUDA;
-  // Shared memory: the B ring as deep as it may be (a slot is away for about 1,800 clocks between two uses: eight boxes of the
-  // shortest 244 clocks cover that, four of the longest 512), at least two raw stages, and what is left for more.
-  const int corr = p.corr ? MMQ_CORR_BYTES : 0, fixed = corr + mmq_aux_bytes(a.type), b_stage = p.tn * MMQ_BK * 2;
-  const int budget = 226 * 1024 - fixed;
+  // Shared memory: the B ring as deep as it may be (a slot is away for about 1,800 clocks between two uses: four boxes of an item of
+  // 128 tokens take 2,048, four of a stage of 384 3,072), at least two raw stages, and what is left for more.
+  const int corr = p.corr ? MMQ_CORR_BYTES : 0, fixed = corr + mmq_aux_bytes(a.type), b_box = p.bg * p.tn * MMQ_BK * 2;
+  const int budget = 226 * 1024 - fixed, most = p.bg == 2 ? MMQ_ITEMS : MMQ_MAX_B;
   int raw = 3;
-  p.sb = (budget - raw * p.raw.bytes) / b_stage;
-  if (p.sb < (p.tn > 256 ? 3 : 4)) { raw = 2; p.sb = (budget - raw * p.raw.bytes) / b_stage; }
+  p.sb = (budget - raw * p.raw.bytes) / b_box;
+  if (p.sb < (p.bg == 2 || p.tn > 256 ? 3 : 4)) { raw = 2; p.sb = (budget - raw * p.raw.bytes) / b_box; }
   if (p.sb < 2) return E_TOO_LARGE;
-  if (p.sb > MMQ_BARS) p.sb = MMQ_BARS;
-  raw = (budget - p.sb * b_stage) / p.raw.bytes;
+  if (p.sb > most) p.sb = most;
+  raw = (budget - p.sb * b_box) / p.raw.bytes;
   p.raw_stages = raw > MMQ_MAX_RAW ? MMQ_MAX_RAW : raw;
-  p.raw_off = p.sb * b_stage;
+  p.corr_off = p.sb * b_box;                      // (multiples of 2,048: the tensor core reads tiles there)
+  p.raw_off = p.corr_off + corr;
   p.aux_off = p.raw_off + p.raw_stages * p.raw.bytes;
-  p.corr_off = p.aux_off + mmq_aux_bytes(a.type);
-  const size_t smem = 1024 + (size_t)p.corr_off + corr;
+  const size_t smem = 1024 + (size_t)p.aux_off + mmq_aux_bytes(a.type);
   const int64_t tiles = a.passes ? a.max_passes * p.rt : p.rt * plan.tt;
   if (tiles * p.nc * (MMQ_CTAS + 1) >= (int64_t)1 << 31) return E_TOO_LARGE;
   if (plan.shared && a.part_bytes >= 2 * plan.grid * MMQ_ROWS * p.tn * 4) {

@@ -16,13 +16,16 @@ constexpr int MMQ_BK = 64;                           // values per stage (128 by
 constexpr int MMQ_GROUPS = 4;                        // producer groups of 128 threads, one thread per weight row
 constexpr int MMQ_PRODUCER_WARPS = 4 * MMQ_GROUPS;
 constexpr int MMQ_THREADS = (MMQ_PRODUCER_WARPS + 3) * 32;   // + B loader, MMA issuer, raw-weight loader
-// Tensor memory: up to 256 tokens a tile, 256 columns of accumulator -- two of 128, or one beyond 128 tokens -- and eight A slots
-// of 32; up to 384 tokens, one accumulator and four A slots.  The stages' barriers are a ring of eight in both cases: a
-// group's stages are eight apart, so by the time it waits for a phase it has seen the one before complete.
-constexpr int MMQ_A_COLS = 32, MMQ_BARS = 8, MMQ_D_STEP = 128;
+// Operand A moves in items: half a 256-value chunk, two stages, 64 columns of tensor memory.  Up to 256 tokens a tile there are 256
+// columns of accumulator -- two of 128 tokens, or one beyond 128 -- and four A slots; up to 384 tokens, one accumulator and two A slots.
+// The items' barriers are a ring of four in both cases: a group's items are four apart, so by the time it waits for a
+// phase it has seen the one before complete.
+constexpr int MMQ_A_COLS = 64, MMQ_ITEMS = 4, MMQ_D_STEP = 128;
+constexpr int MMQ_MAX_B = 8;
+// Activations arrive a box at a time, one stage or -- up to 128 tokens a tile, where the stages are short -- one item.
 constexpr int MMQ_MAX_RAW = 8;
-// Correction values of eight chunks (64 fp16) per row, rows an odd number of 16-byte units apart
-constexpr int MMQ_CORR_CHUNKS = 8, MMQ_CORR_ROW = 144, MMQ_CORR_BYTES = MMQ_ROWS * MMQ_CORR_ROW;
+// Correction values of eight chunks: 64 fp16 per row, a tile of operand A in shared memory (K-major, 128-byte swizzle), twice
+constexpr int MMQ_CORR_CHUNKS = 8, MMQ_CORR_TILE = MMQ_ROWS * 128, MMQ_CORR_BYTES = 2 * MMQ_CORR_TILE;
 
 struct MmqParams {
   RawPlan raw;
@@ -35,9 +38,10 @@ struct MmqParams {
   int k, kpad;
   int nc, corr;           // 256-value chunks of a row; 1: a stage of corrections behind every eight of them
   int rt, tt, tn;         // row tiles, token tiles, tokens per tile (a multiple of 16, at most 256, or of 32, at most 384)
-  int sa, a_col0;         // A slots: how many (4 or 8), first column
+  int sa, a_col0;         // A slots: how many (2 or 4), first column
   int nbuf;               // accumulators, MMQ_D_STEP columns apart
-  int sb, raw_stages;     // ring depths
+  int bg;                 // stages of an activation box: 1 or 2
+  int sb, raw_stages;     // ring depths: boxes, raw chunks
   int raw_off, aux_off, corr_off;   // shared memory behind the B ring
   uint32_t idesc;
   float* part;            // partial tiles, two slots of 128 x tn per CTA; null: every tile is one CTA's
@@ -69,6 +73,10 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+// (by the lane with `lead` set, of a converged warp)
+__device__ __forceinline__ void umma_commit(uint32_t bar, uint32_t lead) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar), "r"(lead) : "memory");
+}
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
@@ -99,14 +107,36 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-// D[tmem] (+)= A[tmem] * B[smem]: A is 128 lanes x 8 columns (16 fp16 values per row, two per column)
-__device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t b_hi, uint32_t idesc, uint32_t accumulate) {
+// A stage: four times D[tmem] (+)= A[tmem] * B[smem], issued by the lane with `lead` set.  16 values a time: eight columns of A (128 lanes
+// x 16 fp16, two per column), 32 bytes of B = +2 in the descriptor's 16-byte units.
+__device__ __forceinline__ void umma_f16_ts4(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t b_hi, uint32_t idesc, uint32_t accumulate, uint32_t lead) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t.reg .b64 b;\n\t"
-      "setp.ne.b32 p, %5, 0;\n\t"
-      "mov.b64 b, {%2, %3};\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %4, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
+      "{\n\t.reg .pred p, q, t;\n\t.reg .b64 b0, b1, b2, b3;\n\t.reg .b32 a1, a2, a3, l1, l2, l3;\n\t"
+      "setp.ne.b32 p, %5, 0;\n\tsetp.ne.b32 q, %6, 0;\n\tsetp.eq.b32 t, 0, 0;\n\t"
+      "add.u32 l1, %2, 2;\n\tadd.u32 l2, %2, 4;\n\tadd.u32 l3, %2, 6;\n\t"
+      "add.u32 a1, %1, 8;\n\tadd.u32 a2, %1, 16;\n\tadd.u32 a3, %1, 24;\n\t"
+      "mov.b64 b0, {%2, %3};\n\tmov.b64 b1, {l1, %3};\n\tmov.b64 b2, {l2, %3};\n\tmov.b64 b3, {l3, %3};\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b0, %4, p;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a1], b1, %4, t;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a2], b2, %4, t;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a3], b3, %4, t;\n\t}"
+      ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate), "r"(lead)
+      : "memory");
+}
+// ... with A from shared memory (low words of both descriptors; they share the high one)
+__device__ __forceinline__ void umma_f16_ss4(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc, uint32_t lead) {
+  asm volatile(
+      "{\n\t.reg .pred q, t;\n\t.reg .b64 a, b;\n\t.reg .b32 al, bl;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\tsetp.eq.b32 t, 0, 0;\n\t"
+      "mov.b64 a, {%1, %3};\n\tmov.b64 b, {%2, %3};\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, t;\n\t"
+      "add.u32 al, %1, 2;\n\tadd.u32 bl, %2, 2;\n\tmov.b64 a, {al, %3};\n\tmov.b64 b, {bl, %3};\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, t;\n\t"
+      "add.u32 al, %1, 4;\n\tadd.u32 bl, %2, 4;\n\tmov.b64 a, {al, %3};\n\tmov.b64 b, {bl, %3};\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, t;\n\t"
+      "add.u32 al, %1, 6;\n\tadd.u32 bl, %2, 6;\n\tmov.b64 a, {al, %3};\n\tmov.b64 b, {bl, %3};\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, t;\n\t}"
+      ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc), "r"(lead)
       : "memory");
 }
 // K-major, 128-byte swizzle: rows of 128 B, 8-row groups 1024 B apart (stride byte offset),
@@ -257,10 +287,10 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_consta
   uint8_t* sB = smem;
   uint8_t* sRaw = smem + p.raw_off;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + p.aux_off);
-  uint64_t* full = bars;                     // [8] stage i % 8: A slot and activation box filled: the four warps of a group + the B loader
-  uint64_t* empty = bars + 8;                // [8] the MMAs that read them are done
-  uint64_t* corr_full = bars + 16;           // every warp's correction values of a block of chunks are in shared memory
-  uint64_t* corr_free = bars + 17;           // ... and have been taken out
+  uint64_t* full = bars;                     // [4] item i % 4: its A slot is filled (the four warps of a group), boxes of an item: and its box is there
+  uint64_t* empty = bars + 4;                // [4] the MMAs that read it are done
+  uint64_t* b_full = bars + 8;               // [8] a box of one stage is there; boxes of an item: [0] that of a block's corrections
+  uint64_t* b_empty = bars + 16;             // [8] ... and has been read
   uint64_t* accum = bars + 24;               // [2] an accumulator is complete
   uint64_t* drained = bars + 26;             // [2] ... and has been read
   uint64_t* raw_full = bars + 28;            // [8]
@@ -270,14 +300,16 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_consta
   volatile int* s_flag = gave_up + 1;        // [2]: the last to arrive at the tile of the part just read out / of the CTA's first part
   uint8_t* s_tab = smem + p.aux_off + 512;   // decoder tables
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // (known to be the same in a warp)
   if (threadIdx.x == 0) {
-    for (int s = 0; s < MMQ_BARS; ++s) {
-      mbar_init(&full[s], MMQ_PRODUCER_WARPS / MMQ_GROUPS + 1);
+    for (int s = 0; s < MMQ_ITEMS; ++s) {
+      mbar_init(&full[s], MMQ_PRODUCER_WARPS / MMQ_GROUPS + (p.bg == 2 ? 1 : 0));
       mbar_init(&empty[s], 1);
     }
-    mbar_init(corr_full, MMQ_PRODUCER_WARPS);
-    mbar_init(corr_free, MMQ_PRODUCER_WARPS / MMQ_GROUPS);
+    for (int s = 0; s < MMQ_MAX_B; ++s) {
+      mbar_init(&b_full[s], 1);
+      mbar_init(&b_empty[s], 1);
+    }
     for (int s = 0; s < 2; ++s) {
       mbar_init(&accum[s], 1);
       mbar_init(&drained[s], MMQ_PRODUCER_WARPS);
@@ -297,13 +329,13 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_consta
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  constexpr uint32_t tmem_base = 0;   // (all 512 columns are this CTA's)
   pdl_trigger();   // the next kernel may become resident; it waits for this one before it touches anything
   // What earlier kernels write: the activations (and the work list of a MoE step), and -- cleared, or read until now -- what the
   // epilogue writes.  Everything else, decoding included, starts before they are done (the weights: see pdl_wait).
   const bool moe = p.passes != nullptr;
   if (moe) pdl_wait();
-  const int tiles = moe ? *p.n_passes * p.rt : p.rt * p.tt;
+  const int tiles = moe ? __shfl_sync(0xffffffffu, *p.n_passes, 0) * p.rt : p.rt * p.tt;
   // Units: (tile, chunk) where CTAs share tiles, whole tiles where they do not -- there is no room for parts, or the last wave
   // of whole tiles idles for less than sharing costs.  Every CTA in use has an equal contiguous range of them.
   const int rest = tiles % (int)gridDim.x;
@@ -317,36 +349,30 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_consta
     q.u1 = cta < G ? (int)((unsigned)((cta + 1) * U) / (unsigned)G) * scale : 0;
   }
   const int first_tile = (int)((unsigned)q.u / (unsigned)p.nc);
+  const uint32_t bars_s = smem_u32(bars), gave_up_s = smem_u32(const_cast<const int*>(gave_up));
+  auto bar = [&](int k) { return bars_s + 8u * (uint32_t)k; };   // (the numbers are those of the list above)
   const int half_n = p.tn > 256 ? p.tn / 2 : 0;   // tokens of one instruction and of one activation box, where a tile takes two
   bool ok = true;
 
   if (warp < MMQ_PRODUCER_WARPS) {
     // ---------------- producers and epilogue ----------------
-    // The work of a part, in order: two items per chunk (a half, 128 values, two stages) and one per block of corrections (one
-    // stage).  Group g takes the items g, g + 4, ... (counted over the whole life of the CTA); thread r of the group decodes
-    // row n0 + r.  Stage i goes to A slot i modulo their number.  The tile before is read out after every group has published
-    // its first item of the next one, so that the tensor core has eight stages of work while the accumulator goes to memory.
+    // The work of a part, in order: two items per chunk (a half, 128 values, two stages).  Group g takes the items g, g + 4, ...
+    // (counted over the whole life of the CTA); thread r of the group decodes row n0 + r.  Item i goes to A slot i modulo their
+    // number.  The tile before is read out after every group has published its first item of the next one, so that the tensor
+    // core has four items of work while the accumulator goes to memory.  What an item costs beside its decoding is kept small: one
+    // wait for the raw chunk, one for the slot and one signal for 128 values, and no work list but a stride.  (Stage by stage, with
+    // the correction stages dealt out among the groups, it was 130 to 165 instructions per stage of 32 rows, as many as the decoding of Q4_K.)
     const int r = threadIdx.x & 127, g = threadIdx.x >> 7;
     const DecodeCtx cx = decoder_context<TYPE>(s_tab, lane);
     const int nunits = p.k / 32;
     const uint32_t d_lane = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
     const uint32_t a_lane = d_lane + (uint32_t)p.a_col0;
-    const uint32_t s_corr = smem_u32(smem + p.corr_off) + (uint32_t)(r * MMQ_CORR_ROW);
+    const uint32_t s_corr = smem_u32(smem + p.corr_off) + (uint32_t)(r * 128);
     // (After a time-out the loops run on without waiting: every barrier still gets its arrivals, the result is invalid and the
     // status word says so.)
-    auto wait = [&](uint64_t* bar, uint32_t parity) {
-      if (ok) ok = mbar_wait_bounded(bar, parity);
+    auto wait = [&](uint32_t b, uint32_t parity) {
+      mbar_wait_or(b, parity, gave_up_s);
       __syncwarp();
-    };
-    auto publish = [&](const uint32_t (&v)[32], int i) {   // wait until stage i's slot is free, store the row, signal the MMA warp
-      const int o = i - p.sa;   // the stage that had the slot before
-      if (o >= 0) wait(&empty[o & (MMQ_BARS - 1)], (uint32_t)(o >> 3) & 1u);
-      tc_fence_after();
-      tmem_st32(a_lane + (uint32_t)((i & (p.sa - 1)) * MMQ_A_COLS), v);
-      tmem_st_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&full[i & (MMQ_BARS - 1)]);
     };
     // Reads out part e, the pi-th of this CTA.  Kept short: this code runs two or three times in the life of a CTA, and fetching
     // its instructions costs more than running them (unrolled over an accumulator held in 64 registers it took 10,000 clocks
@@ -369,7 +395,7 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_consta
       int orow = out_row(g);
       float scale = out_scale(orow);
       if (mode != FINISH) {
-        wait(&accum[buf], (uint32_t)use & 1u);
+        wait(bar(24 + buf), (uint32_t)use & 1u);
         tc_fence_after();
         pdl_wait();
       }
@@ -510,122 +536,116 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_consta
       }
     };
 
-    int t0 = 0, i0 = 0, pi = 0;  // first item and first stage of the block; parts so far
-    int rs0 = 0, nblk = 0;       // raw slot of the block's first chunk and its phase; blocks of corrections so far
-    uint32_t rph0 = 0;
+    // Item i is half i & 1 of the i / 2-th chunk of the CTA, so a group has the same half, slot and barriers all its life.
+    const int half = g & 1;
+    const uint32_t slot_free = bar(4 + (p.sa == 4 ? g : g ^ 2));   // `empty` of the item that had the slot before
+    uint32_t free_ph = p.sa == 2 && g >= 2 ? 0u : 1u;              // (1 at first: the slot has never been used)
+    const uint32_t a_dst = a_lane + (uint32_t)((g & (p.sa - 1)) * MMQ_A_COLS);
+    int rs = g >> 1;             // raw slot of the group's next chunk, and its phase
+    uint32_t rph = 0;
+    int i0 = 0, pi = 0;          // items before the part, parts so far
+    int blk0 = 0, end2 = -1;     // blocks of corrections before the part; last item of the last but one of them
     MmqPart prev{}, head{};      // the part before, the CTA's first part
     int mode = MORE;
-    constexpr int CI = Dec::CORR ? 1 : 0;
     for (;;) {
       const bool more = mode == MORE && mmq_next_part(p, q);
       if (!more && mode == MORE) mode = FINAL;
       const MmqTile qt = mmq_tile(p, q.tile);
       const int n = qt.n0 + r;
-      const bool live = n < p.n;
       const uint8_t* slot = sRaw + raw_slot(p.raw, r, qt.n0);
-      int cs = q.c0, ce = mmq_block_end(p, q, cs);
-      int m = (g - t0) & 3;      // this group's next item of the block
-      bool done = !more, read_out = pi > 0;
-      // On to the block that holds item m.  A group that is through with a block says so before it does anything else: the
-      // group that takes the corrections waits for it.
-      auto advance = [&]() {
-        while (!done && m >= 2 * (ce - cs) + CI) {
-          const int items = 2 * (ce - cs) + CI;
-          if constexpr (Dec::CORR) {
-            __syncwarp();
-            if (lane == 0 && m != items + 3) mbar_arrive(corr_full);   // (item items - 1 has arrived by itself)
-            ++nblk;
-          }
-          m -= items;
-          t0 += items;
-          i0 += 4 * (ce - cs) + CI;
-          rs0 += ce - cs;
-          if (rs0 >= p.raw_stages) {
-            const int laps = (int)((unsigned)rs0 / (unsigned)p.raw_stages);
-            rs0 -= laps * p.raw_stages;
-            rph0 ^= (uint32_t)laps & 1u;
-          }
-          cs = ce;
-          if (cs >= q.c1) done = true;
-          else ce = mmq_block_end(p, q, cs);
-        }
-      };
-      // With one accumulator and four slots the first items of groups two and three have no room before the tile is read out.
-      bool hold = read_out && p.nbuf == 1 && 2 * m >= p.sa;
-      advance();
+      const int items = more ? 2 * (q.c1 - q.c0) : 0;
+      int m = (g - i0) & 3;      // this group's next item of the part
+      bool read_out = pi > 0;
+      // With one accumulator and two slots the first items of groups two and three have no room before the tile is read out.
+      bool hold = read_out && p.nbuf == 1 && m >= p.sa;
       for (;;) {
-        if (!done && !hold) {
-          // this block's corrections may be written, and its arrivals counted, once the block before has been taken out
-          if constexpr (Dec::CORR) wait(corr_free, ((uint32_t)nblk & 1u) ^ 1u);
-          if (!Dec::CORR || m < 2 * (ce - cs)) {
-            const int k = m >> 1, half = m & 1;
-            int rs = rs0 + k;
-            uint32_t rph = rph0;
-            while (rs >= p.raw_stages) { rs -= p.raw_stages; rph ^= 1u; }
-            wait(&raw_full[rs], rph);
-            const uint8_t* chunk = slot + rs * p.raw.bytes + (FAST ? 0u : raw_shift(p.raw, n, qt.row0, cs + k));
-            if constexpr (Dec::CORR) {
-              const uint2 cv = live ? Dec::corr(chunk, half, nunits - 8 * (cs + k)) : make_uint2(0u, 0u);
-              asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(s_corr + (uint32_t)(16 * ((cs + k) & (MMQ_CORR_CHUNKS - 1)) + 8 * half)), "r"(cv.x), "r"(cv.y) : "memory");
-            }
+        if (m < items && !hold) {
+          const int c = q.c0 + (m >> 1), i = i0 + m;
+          // The group has seen the chunk before the last one land; with three slots that does not tell that this slot's last chunk has,
+          // and a wait that is a phase early returns at once.
+          if (p.raw_stages == 3) wait(bar(36 + rs), rph ^ 1u);
+          wait(bar(28 + rs), rph);
+          const uint8_t* chunk = slot + rs * p.raw.bytes + (FAST ? 0u : raw_shift(p.raw, n, qt.row0, c));
+          uint2 cv;
+          if constexpr (Dec::CORR) cv = Dec::corr(chunk, half, nunits - 8 * c);
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              const int s2 = 2 * half + h;      // 64-value stage of the chunk
-              uint32_t v[32];
-              if constexpr (FAST) {
-                Stage64<TYPE, ab_t>::decode(chunk, s2, v);
-              } else {
-                const int u = 2 * s2;           // units (32 values) u, u + 1 of the chunk
-                const int left = nunits - 8 * (cs + k) - u;
-                uint32_t (&v0)[16] = *reinterpret_cast<uint32_t (*)[16]>(&v[0]);
-                uint32_t (&v1)[16] = *reinterpret_cast<uint32_t (*)[16]>(&v[16]);
-                uint32_t raw[Dec::RW];
-                if (live && left > 0) {
-                  Dec::load(chunk, u, raw);
-                  Dec::decode(chunk, u, raw, cx, v0);
-                } else {
-#pragma unroll
-                  for (int j = 0; j < 32; ++j) v[j] = 0;
-                }
-                if (live && left > 1) {
-                  if constexpr (!decoder_pair_load<TYPE>()) Dec::load(chunk, u + 1, raw);   // (one load serves both)
-                  Dec::decode(chunk, u + 1, raw, cx, v1);
-                } else {
-#pragma unroll
-                  for (int j = 0; j < 16; ++j) v1[j] = 0;
-                }
-              }
-              if (h == 1) {   // this warp is done reading the raw chunk: hand the slot back to the loader
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&raw_empty[rs]);
-              }
-              publish(v, i0 + 2 * m + h);
-            }
-          } else if constexpr (Dec::CORR) {
-            // the block's corrections: every warp's values are in, zeros for the chunks that other parts have
-            __syncwarp();
-            if (lane == 0) mbar_arrive(corr_full);
-            wait(corr_full, (uint32_t)nblk & 1u);
+          for (int h = 0; h < 2; ++h) {
+            const int s2 = 2 * half + h;      // 64-value stage of the chunk
             uint32_t v[32];
+            if constexpr (FAST) {
+              Stage64<TYPE, ab_t>::decode(chunk, s2, v);
+            } else {
+              const int u = 2 * s2;           // units (32 values) u, u + 1 of the chunk
+              // (rows beyond the matrix decode what their slots happen to hold: nothing reads their sums)
+              const int left = BlockTraits<TYPE>::QK == 256 ? 2 : nunits - 8 * c - u;
+              uint32_t (&v0)[16] = *reinterpret_cast<uint32_t (*)[16]>(&v[0]);
+              uint32_t (&v1)[16] = *reinterpret_cast<uint32_t (*)[16]>(&v[16]);
+              uint32_t raw[Dec::RW];
+              if (left > 0) {
+                Dec::load(chunk, u, raw);
+                Dec::decode(chunk, u, raw, cx, v0);
+              } else {
 #pragma unroll
-            for (int c = 0; c < MMQ_CORR_CHUNKS; ++c) {
-              const uint4 x = lds128s(s_corr + 16 * c);
-              const bool have = c >= (cs & (MMQ_CORR_CHUNKS - 1)) && c <= ((ce - 1) & (MMQ_CORR_CHUNKS - 1));
-              v[4 * c] = have ? x.x : 0u; v[4 * c + 1] = have ? x.y : 0u; v[4 * c + 2] = have ? x.z : 0u; v[4 * c + 3] = have ? x.w : 0u;
+                for (int j = 0; j < 16; ++j) v0[j] = 0;
+              }
+              if (left > 1) {
+                if constexpr (!decoder_pair_load<TYPE>()) Dec::load(chunk, u + 1, raw);   // (one load serves both)
+                Dec::decode(chunk, u + 1, raw, cx, v1);
+              } else {
+#pragma unroll
+                for (int j = 0; j < 16; ++j) v1[j] = 0;
+              }
             }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(corr_free);
-            publish(v, i0 + 2 * m);
+            if (h == 1) {   // this warp is done reading the raw chunk: hand the slot back to the loader
+              __syncwarp();
+              if (lane == 0) mbar_arrive(bar(36 + rs));
+            } else {
+              wait(slot_free, free_ph);
+              free_ph ^= 1u;
+              tc_fence_after();
+            }
+            tmem_st32(a_dst + 32 * h, v);
           }
+          if constexpr (Dec::CORR) {
+            // The block's tile: multiplied before the last item of the block is handed back, and free again for the block after the
+            // next.  That item is three before this one at the earliest, and four slots wait for the fourth.
+            const int b = (c >> 3) - (q.c0 >> 3);
+            const uint32_t at = s_corr + (uint32_t)(((blk0 + b) & 1) * MMQ_CORR_TILE);
+            if (half == 0 && (c == q.c0 || (c & 7) == 0)) {   // the block's first item
+              const int e = b == 0 ? end2 : b == 1 ? i0 - 1 : i0 + 2 * ((c & ~7) - 8 - q.c0) - 1;
+              if (e >= 0 && e > i - p.sa) wait(bar(4 + (e & (MMQ_ITEMS - 1))), (uint32_t)(e >> 2) & 1u);
+              const int lo = c & 7, hi = q.c1 - (c & ~7);     // chunks that other parts have, or nobody: zeros
+              if (lo > 0 || hi < 8) {
+#pragma unroll 1
+                for (int j = 0; j < 8; ++j)
+                  if (j < lo || j >= hi) asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(at + (uint32_t)((j ^ (r & 7)) << 4)), "r"(0u) : "memory");
+              }
+            }
+            asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(at + (uint32_t)((((c & 7) ^ (r & 7)) << 4) + 8 * half)), "r"(cv.x), "r"(cv.y) : "memory");
+            fence_proxy_async();   // (the tensor core reads it)
+          }
+          tmem_st_wait();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar(g));
           m += 4;
-          advance();
+          rs += 2;
+          if (rs >= p.raw_stages) { rs -= p.raw_stages; rph ^= 1u; }
         }
         if (read_out) {
           epilogue(prev, pi - 1, mode);
           read_out = false;
         }
-        if (done) break;
+        if (m >= items) break;
         hold = false;
+      }
+      i0 += items;
+      if constexpr (Dec::CORR) {
+        if (more) {
+          const int nb = ((q.c1 - 1) >> 3) - (q.c0 >> 3) + 1;
+          end2 = nb > 1 ? i0 - 2 * (q.c1 - ((q.c1 - 1) & ~7)) - 1 : i0 - items - 1;
+          blk0 += nb;
+        }
       }
       if (!more) {
         if (mode == FINISH || head.c1 - head.c0 == p.nc || pi < 2) break;
@@ -640,29 +660,36 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_consta
       ++pi;
     }
   } else if (warp == MMQ_PRODUCER_WARPS) {
-    // ---------------- B loader: one TMA box (64 k x tn rows; two beyond 256) per stage ----------------
-    if (lane == 0) {
-      int i = 0, sb = 0;
-      pdl_wait();
-      while (ok && mmq_next_part(p, q)) {
-        const int x0 = mmq_tile(p, q.tile).x0;
-        for (int cs = q.c0, ce; ok && cs < q.c1; cs = ce) {
-          ce = mmq_block_end(p, q, cs);
-          const int nmain = 4 * (ce - cs), corr_col = p.kpad + cs / MMQ_CORR_CHUNKS * MMQ_BK;
-          for (int j = 0; j < nmain + p.corr; ++j, ++i) {
-            // B slot i % sb held stage i - sb: wait for that stage's commit
-            const int o = i - p.sb;
-            if (o >= 0 && !mbar_wait_bounded(&empty[o & (MMQ_BARS - 1)], (uint32_t)(o >> 3) & 1u)) { ok = false; break; }
-            uint64_t* fb = &full[i & (MMQ_BARS - 1)];
-            const int col = j < nmain ? cs * RAW_KC + j * MMQ_BK : corr_col;
-            mbar_expect_tx(fb, (uint32_t)b_stage);
-            raw_tma_box(sB + (size_t)sb * b_stage, &bmap, col, x0, fb);
-            if (half_n) raw_tma_box(sB + (size_t)sb * b_stage + half_n * (MMQ_BK * 2), &bmap, col, x0 + half_n, fb);
-            if (++sb == p.sb) sb = 0;
+    // ---------------- B loader: one TMA box (64 or 2 x 64 values x tn rows; two beyond 256) per stage or item ----------------
+    // (Converged like the MMA issuer below.)
+    const uint32_t lead = elect_one() ? 1u : 0u;
+    const uint32_t bytes = (uint32_t)(p.bg * b_stage), sb_s = smem_u32(sB);
+    int i = 0, sb = 0;
+    uint32_t ph = 0;
+    pdl_wait();
+    while (mmq_next_part(p, q)) {
+      const int x0 = mmq_tile(p, q.tile).x0;
+      for (int cs = q.c0, ce; cs < q.c1; cs = ce) {
+        ce = mmq_block_end(p, q, cs);
+        const int n = 2 * (ce - cs) * (p.bg == 2 ? 1 : 2);
+#pragma unroll 1
+        for (int j = 0; j < n + p.corr; ++j) {
+          mbar_wait_or(bar(16 + sb), ph ^ 1u, gave_up_s);
+          if (lds32(gave_up_s) != 0u) goto b_done;   // (no copy into a slot that may be in use)
+          __syncwarp();
+          const int stage = j < n ? 4 * cs + p.bg * j : (p.kpad >> 6) + cs / MMQ_CORR_CHUNKS;
+          const uint32_t fb = bar(p.bg == 1 ? 8 + sb : j < n ? i & (MMQ_ITEMS - 1) : 8), dst = sb_s + (uint32_t)sb * bytes;
+          if (lead) {
+            mbar_expect_tx(fb, bytes);
+            tma_box3(dst, &bmap, 0, x0, stage, fb);
+            if (half_n) tma_box3(dst + (uint32_t)(half_n * (MMQ_BK * 2)), &bmap, 0, x0 + half_n, stage, fb);
           }
+          i += j < n ? 1 : 0;
+          if (++sb == p.sb) { sb = 0; ph ^= 1u; }
         }
       }
     }
+  b_done:;
   } else if (warp == MMQ_PRODUCER_WARPS + 2) {
     // ---------------- raw-weight loader ----------------
     if (p.w_wait) pdl_wait();
@@ -671,7 +698,9 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_consta
     while (ok && mmq_next_part(p, q)) {
       const MmqTile qt = mmq_tile(p, q.tile);
       for (int c = q.c0; c < q.c1; ++c) {
-        if (!mbar_wait_bounded(&raw_empty[st], sph ^ 1u)) { ok = false; break; }
+        mbar_wait_or(bar(36 + st), sph ^ 1u, gave_up_s);
+        if (lds32(gave_up_s) != 0u) { ok = false; break; }
+        __syncwarp();
         raw_issue(p.raw, &wmap, p.w, p.w_bytes, qt.row0, qt.n0, c, sRaw + (size_t)st * p.raw.bytes, &raw_full[st], 0u, lane);
         __syncwarp();
         if (++st == p.raw_stages) { st = 0; sph ^= 1u; }
@@ -679,52 +708,75 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_consta
     }
   } else {
     // ---------------- MMA issuer ----------------
-    // One lane issues everything.  (Its loop is short: it shares its scheduler with four producer warps.)
-    if (elect_one()) {
-      int i = 0, sb = 0, pi = 0;
-      const uint64_t bd0 = umma_desc_sw128(smem_u32(sB));
-      const uint32_t b_step = (uint32_t)(b_stage >> 4), b_lo0 = (uint32_t)bd0, b_hi = (uint32_t)(bd0 >> 32);
-      uint32_t b_lo = b_lo0;
-      while (ok && mmq_next_part(p, q)) {
-        int end = i + 4 * (q.c1 - q.c0);
-        if (p.corr) end += (q.c1 - 1) / MMQ_CORR_CHUNKS - q.c0 / MMQ_CORR_CHUNKS + 1;
-        const int buf = p.nbuf == 2 ? pi & 1 : 0, use = p.nbuf == 2 ? pi >> 1 : pi;
-        ok = mbar_wait_bounded(&drained[buf], ((uint32_t)use & 1u) ^ 1u);
-        const uint32_t d = tmem_base + (uint32_t)(buf * MMQ_D_STEP);
-        uint32_t accumulate = 0;
-        for (; ok && i < end; ++i) {
-          const int s = i & (MMQ_BARS - 1);
-          ok = mbar_wait_bounded(&full[s], (uint32_t)(i >> 3) & 1u);
-          tc_fence_after();
-          const uint32_t at = tmem_base + (uint32_t)(p.a_col0 + (i & (p.sa - 1)) * MMQ_A_COLS);
-          uint32_t dh = d, bh = b_lo;
+    // The warp stays converged and its control flow depends on nothing but parameters, so that addresses, descriptors and counters
+    // live in uniform registers; one lane issues.  (With one lane in the loop, every operand went from a register to a uniform one at
+    // each instruction, and this loop was what bounded the kernel at 128 tokens or less: 460 to 560 clocks a stage whatever the decoder.)
+    const uint32_t lead = elect_one() ? 1u : 0u;
+    int i = 0, sb = 0, pi = 0, blk = 0;
+    uint32_t ph = 0;
+    const uint64_t bd0 = umma_desc_sw128(smem_u32(sB));
+    const uint32_t b_step = (uint32_t)(b_stage >> 4), b_lo0 = (uint32_t)bd0, b_hi = (uint32_t)(bd0 >> 32);
+    const uint32_t c_lo0 = (uint32_t)umma_desc_sw128(smem_u32(smem + p.corr_off));
+    const uint32_t half_lo = (uint32_t)(half_n * (MMQ_BK * 2) >> 4);
+    uint32_t b_lo = b_lo0;
+    auto box_done = [&]() {   // the box just multiplied goes back
+      umma_commit(bar(16 + sb), lead);
+      b_lo += (uint32_t)p.bg * b_step;
+      if (++sb == p.sb) { sb = 0; ph ^= 1u; b_lo = b_lo0; }
+    };
+    while (mmq_next_part(p, q)) {
+      const int buf = p.nbuf == 2 ? pi & 1 : 0, use = p.nbuf == 2 ? pi >> 1 : pi;
+      mbar_wait_or(bar(26 + buf), ((uint32_t)use & 1u) ^ 1u, gave_up_s);
+      const uint32_t d = (uint32_t)(buf * MMQ_D_STEP);
+      uint32_t accumulate = 0;
+      for (int cs = q.c0, ce; cs < q.c1; cs = ce) {
+        ce = mmq_block_end(p, q, cs);
 #pragma unroll 1
-          for (int h = half_n > 0 ? 1 : 0; h >= 0; --h) {
-#pragma unroll
-            for (int kk = 0; kk < MMQ_BK / 16; ++kk)  // 16 values = 8 columns of A, 32 bytes of B = +2 in the descriptor's 16-byte units
-              umma_f16_ts(dh, at + 8 * kk, bh + 2 * kk, b_hi, p.idesc, kk == 0 ? accumulate : 1u);
-            dh += (uint32_t)half_n;
-            bh += (uint32_t)(half_n * (MMQ_BK * 2) >> 4);
+        for (int end = i + 2 * (ce - cs); i < end; ++i) {
+          const int s = i & (MMQ_ITEMS - 1);
+          mbar_wait_or(bar(s), (uint32_t)(i >> 2) & 1u, gave_up_s);
+          const uint32_t at = (uint32_t)(p.a_col0 + (i & (p.sa - 1)) * MMQ_A_COLS);
+          if (p.bg == 2) {
+            __syncwarp();
+            tc_fence_after();
+            umma_f16_ts4(d, at, b_lo, b_hi, p.idesc, accumulate, lead);
+            umma_f16_ts4(d, at + 32, b_lo + b_step, b_hi, p.idesc, 1u, lead);
+            box_done();
+          } else {
+#pragma unroll 1
+            for (int h = 0; h < 2; ++h) {
+              mbar_wait_or(bar(8 + sb), ph, gave_up_s);
+              __syncwarp();
+              tc_fence_after();
+              umma_f16_ts4(d, at + 32 * h, b_lo, b_hi, p.idesc, accumulate | (uint32_t)h, lead);
+              if (half_n) umma_f16_ts4(d + (uint32_t)half_n, at + 32 * h, b_lo + half_lo, b_hi, p.idesc, accumulate | (uint32_t)h, lead);
+              box_done();
+            }
           }
           accumulate = 1;
-          umma_commit(&empty[s]);
-          b_lo += b_step;
-          if (++sb == p.sb) { sb = 0; b_lo = b_lo0; }
+          if (p.corr && i == end - 1) {   // the block's corrections, before its last item is handed back
+            mbar_wait_or(bar(p.bg == 2 ? 8 : 8 + sb), p.bg == 2 ? (uint32_t)blk & 1u : ph, gave_up_s);
+            __syncwarp();
+            tc_fence_after();
+            const uint32_t c_lo = c_lo0 + (uint32_t)((blk & 1) * (MMQ_CORR_TILE >> 4));
+            umma_f16_ss4(d, c_lo, b_lo, b_hi, p.idesc, lead);
+            if (half_n) umma_f16_ss4(d + (uint32_t)half_n, c_lo, b_lo + half_lo, b_hi, p.idesc, lead);
+            ++blk;
+            box_done();
+          }
+          umma_commit(bar(4 + s), lead);
         }
-        // committed in every case: the accumulator's barrier then completes once every tcgen05.mma issued so far has finished
-        umma_commit(&accum[buf]);
-        ++pi;
       }
+      umma_commit(bar(24 + buf), lead);   // completes once every tcgen05.mma issued so far has finished
+      ++pi;
     }
     __syncwarp();
   }
-  if (!ok) {   // (any lane)
-    atomicExch(p.status, E_TIMEOUT);
-    *gave_up = 1;
-  }
+  if (!ok) *gave_up = 1;   // (any lane)
   tc_fence_before();
   __syncthreads();
   if (*gave_up) {
+    if (threadIdx.x == 0) atomicExch(p.status, E_TIMEOUT);
     // A bounded wait ran out somewhere in this CTA (the result is invalid and the status word says so).  Before the tensor
     // memory is released and the CTA retires, everything it started must have finished: the commit below covers the tensor
     // pipe (bounded wait on a barrier nobody else uses any more), and the copies still in flight depend on nothing and land

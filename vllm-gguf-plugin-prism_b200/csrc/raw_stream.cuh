@@ -45,6 +45,13 @@ __device__ __forceinline__ void raw_tma_box(void* dst, const CUtensorMap* map, i
       : "memory");
 }
 
+__device__ __forceinline__ void tma_box3(uint32_t dst, const CUtensorMap* map, int x, int y, int z, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+      ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y), "r"(z)
+      : "memory");
+}
+
 // Offset, inside a stage, of row r of the tile that starts at row n0 of the matrix (whose first row is row `row0` of all
 // matrices): where its slot starts, and by how much its chunk c is displaced in it.
 __device__ __forceinline__ uint32_t raw_slot(const RawPlan& p, int r, int n0) {
