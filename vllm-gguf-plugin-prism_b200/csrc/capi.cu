@@ -124,7 +124,7 @@ static int tiled_dense(bool quantize, const void* W, const void* X, void* Y, voi
   if (quantize) {
     a.ldb = mmq_ldb(type, K);
     a.corr_mode = mmq_corr_mode(type);
-    a.perm = mmq_perm(type, K, pitch);
+    a.perm = mmq_perm(type, K, pitch, false);
     a.b = ws; a.b_dtype = DT_F16;
     const int rc = launch_quantize_q8_1(X, dtype, ws, M, K, Q8_MODE_F16, 0, a.ldb, a.corr_mode, nullptr, 1, 0, s, a.perm, nullptr, 0, 0, a.counter,
                                         a.counter ? share.n_counters : 0);
@@ -571,7 +571,7 @@ int gguf_b200_moe_a8(const void* X, const void* W, void* Y, void* ws, int64_t ws
   a.pitch = pitch; a.ldb = mmq_ldb(type, K); a.ldy = N;
   a.corr_mode = mmq_corr_mode(type);
   a.expert_gap = n_experts > 1 ? expert_stride_bytes - N * pitch : 0;
-  a.perm = a.expert_gap ? 0 : mmq_perm(type, K, pitch);
+  a.perm = mmq_perm(type, K, pitch, a.expert_gap != 0);
   a.passes = base + used;
   a.n_passes = reinterpret_cast<const int32_t*>(base + used + list - 16);
   a.sorted = sorted_token_ids;
@@ -749,7 +749,7 @@ int gguf_b200_fused_moe(const void* X, const void* W13, const void* W2, void* Y,
     a.ldb = mmq_ldb(type, K);
     a.ldy = N;
     a.corr_mode = mmq_corr_mode(type);
-    a.perm = mmq_perm(type, K, a.pitch);
+    a.perm = mmq_perm(type, K, a.pitch, false);
     a.passes = base + L.o_passes;
     a.n_passes = npass;
     a.sorted = sorted;

@@ -42,7 +42,7 @@ int launch_quantize_q8_1(const void* x, int x_dtype, void* out, int64_t M, int64
 int64_t mmq_ldb(int type, int64_t K);
 int mmq_corr_mode(int type);
 // value order the tensor-core kernel will expect in the fp16 activation matrix for this problem
-int mmq_perm(int type, int64_t K, int64_t pitch);
+int mmq_perm(int type, int64_t K, int64_t pitch, bool gap);   // gap: between one expert's matrix and the next
 
 // row_ids != null: row gather -- out row r (K values, K a multiple of 256) = weight row row_ids[r] of weight_rows
 int launch_dequantize(const void* w, int type, void* out, int out_dtype, int64_t n_elems, int q4k_contract,
@@ -116,7 +116,7 @@ struct MmqArgs {
   int64_t N, K;             // weight rows, values per row
   int64_t pitch, ldb, ldy;
   int corr_mode;            // which correction the columns behind K hold
-  int perm;                 // value order inside each group of four of b: 0 natural, 1 = (0,2,1,3) (see mmq_perm)
+  int perm;                 // value order of b (see mmq_perm)
   // MoE (null passes = dense): the work list of launch_moe_plan / launch_moe_blocks
   const void* passes;       // int4 {expert, first activation row, rows}
   const int32_t* n_passes;

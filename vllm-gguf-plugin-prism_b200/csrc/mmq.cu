@@ -62,7 +62,12 @@ int mmq_moe_block_size() { return 64; }
 static bool mmq_fast(int type, int64_t K, int64_t pitch) {
   return (type == T_Q4_0 || type == T_Q8_0 || type == T_Q4_K || type == T_Q5_K) && raw_dense(type, K, pitch);
 }
-int mmq_perm(int type, int64_t K, int64_t pitch) { return mmq_fast(type, K, pitch) && type != T_Q8_0 ? 1 : 0; }
+// The order of the values in the activation matrix: 0 as they are; 1, inside every four 0, 2, 1, 3; 2, inside every four blocks of 32
+// the blocks 0, 2, 1, 3 (Item128<T_Q6_K>).
+int mmq_perm(int type, int64_t K, int64_t pitch, bool gap) {
+  if (type == T_Q6_K) return 2;
+  return !gap && mmq_fast(type, K, pitch) && type != T_Q8_0 ? 1 : 0;
+}
 static_assert(Stage64<T_Q4_0, __half>::PERM == 1 && Stage64<T_Q4_K, __half>::PERM == 1 && Stage64<T_Q5_K, __half>::PERM == 1 &&
                   Stage64<T_Q8_0, __half>::PERM == 0,
               "mmq_perm");
@@ -192,7 +197,7 @@ int launch_mmq(const MmqArgs& a, cudaStream_t stream) {
   CUtensorMap wmap{}, bmap{};
   if (!plan_raw(a.type, a.w, a.N, a.passes ? a.experts : 1, a.K, a.pitch, p.raw, wmap, a.expert_gap)) return E_BAD_SHAPE;
   const bool fast = mmq_fast(a.type, a.K, a.pitch) && p.raw.mode == 1;
-  if (a.perm != (fast ? mmq_perm(a.type, a.K, a.pitch) : 0)) return E_BAD_SHAPE;
+  if (a.perm != mmq_perm(a.type, a.K, a.pitch, !fast)) return E_BAD_SHAPE;
   p.w = static_cast<const uint8_t*>(a.w);
   p.w_bytes = (a.N * (a.passes ? a.experts : 1) - 1) * a.pitch + p.raw.row_bytes + (a.passes ? (a.experts - 1) * p.raw.gap : 0);
   p.y = a.y;

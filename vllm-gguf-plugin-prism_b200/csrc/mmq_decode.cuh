@@ -148,6 +148,7 @@ template <int TYPE> __device__ __forceinline__ void decoder_fill_tables(uint8_t*
 }
 
 template <int TYPE, typename ab_t> struct Decoder;
+template <typename ab_t> struct Decoder<T_Q6_K, ab_t> { static constexpr bool CORR = false; };   // (see Item128)
 // types that are multiplied as dequantized weights of either 16-bit type (activations as they are)
 template <int TYPE> __host__ __device__ constexpr bool decoder_bf16() {
   return TYPE == T_IQ2_XXS || TYPE == T_IQ2_XS || TYPE == T_IQ2_S || TYPE == T_IQ3_XXS || TYPE == T_IQ3_S || TYPE == T_IQ1_S || TYPE == T_IQ1_M ||
@@ -156,7 +157,7 @@ template <int TYPE> __host__ __device__ constexpr bool decoder_bf16() {
 
 // Types whose two 32-value units of a 64-value stage (units 2j and 2j + 1 of a 256-value super-block, always
 // whole) are cut from the same words of the block: load() depends on the unit only through u >> 1.
-template <int TYPE> __host__ __device__ constexpr bool decoder_pair_load() { return TYPE == T_Q2_K || TYPE == T_Q3_K || TYPE == T_Q5_K || TYPE == T_Q6_K; }
+template <int TYPE> __host__ __device__ constexpr bool decoder_pair_load() { return TYPE == T_Q2_K || TYPE == T_Q3_K || TYPE == T_Q5_K; }
 
 // one fp16 of each of four blocks TS bytes apart, zero from block `left` on
 template <int TS> __device__ __forceinline__ uint2 block_halves(uint32_t a, int left) {
@@ -387,53 +388,6 @@ template <typename ab_t> struct Decoder<T_Q5_K, ab_t> {
   }
   // half(dmin * m) of the four sub-blocks 4 * half .. of the chunk (pairs with -s8 on the B side)
   static __device__ __forceinline__ uint2 corr(const uint8_t* blk, int half, int) { return q4k_pair_mins(lds128s(smem_u32(blk)), half); }
-};
-
-// ---- Q6_K: value = half(d * half(sc * (code - 32))) ------------------------------------------
-// unit u: super-block u>>3, group g = u&7: ip = g>>2 (128-value half), q = g&3:
-//   low 4 bits = nibble (q>>1) of ql[64ip + 32(q&1) + l], high 2 bits = bits 2q.. of qh[32ip + l], l = 0..31,
-//   scales sc[8ip + 2q] (l < 16) and sc[8ip + 2q + 1].
-// The units 2j and 2j + 1 of a stage differ in q & 1 only, so one load serves both (decoder_pair_load):
-// Raw: [0..17] the 64 bytes of ql of the half (+ cover), [18..27] 32 bytes of qh (+ cover), [28..30] the four
-// scale bytes of the pair (+ cover), [31] d.
-template <typename ab_t> struct Decoder<T_Q6_K, ab_t> {
-  static constexpr bool CORR = false;   // correction columns
-  static constexpr int RW = 32;
-  static __device__ __forceinline__ void load(const uint8_t* row, int u, uint32_t (&raw)[RW]) {
-    const uint8_t* blk = row + (int64_t)(u >> 3) * 210;
-    const int g = u & 7, ip = g >> 2, q = g & 2;
-    ldg_cover<17>(blk + 64 * ip, 64, raw);
-    raw[17] = 0;
-    ldg_cover<9>(blk + 128 + 32 * ip, 32, raw + 18);
-    raw[27] = 0;
-    ldg_cover<2>(blk + 192 + 8 * ip + 2 * q, 4, raw + 28);
-    raw[30] = 0;
-    ldg_cover<1>(blk + 208, 2, raw + 31);
-  }
-  static __device__ __forceinline__ void decode(const uint8_t* row, int u, const uint32_t (&raw)[RW], const DecodeCtx&, uint32_t (&out)[16]) {
-    const uint8_t* blk = row + (int64_t)(u >> 3) * 210;
-    const int g = u & 7, ip = g >> 2, q = g & 3;
-    const uint32_t sh_l = shift_of(blk + 64 * ip), sh_h = shift_of(blk + 128 + 32 * ip);
-    const uint32_t sc2 = (word_at(raw + 28, 0, shift_of(blk + 192 + 8 * ip + 2 * (q & 2))) >> (16 * (q & 1))) & 0xFFFFu;   // two int8 scales
-    const uint32_t du = (raw[31] >> shift_of(blk + 208)) & 0xFFFFu;
-    const __half2 d2 = u32_as_h2(du | (du << 16));
-    const __half2 off = __floats2half2_rn(1056.f, 1056.f);  // 1024 + 32
-    const __half2 s_lo = __half2half2(__int2half_rn((int)(int8_t)(sc2 & 0xFF)));
-    const __half2 s_hi = __half2half2(__int2half_rn((int)(int8_t)(sc2 >> 8)));
-    // the 6-bit code of each of a word's four values as one byte: low nibble from ql, bits 4-5 from qh
-    // rotated into place; one byte-permute per pair then builds the halves 1024 + code (0x6400 | code)
-    const uint32_t sl = 4 * (q >> 1), rot_h = (uint32_t)(2 * q - 4) & 31u;
-#pragma unroll
-    for (int wi = 0; wi < 8; ++wi) {             // word wi: values 4wi..4wi+3 of the unit
-      const uint32_t l = word_at(raw, wi + 8 * (q & 1), sh_l) >> sl;
-      const uint32_t h = word_at(raw + 18, wi, sh_h);
-      const uint32_t c = (l & 0x0F0F0F0Fu) | (__funnelshift_r(h, h, rot_h) & 0x30303030u);
-      const __half2 s2 = wi < 4 ? s_lo : s_hi;
-      const __half2 p0 = u32_as_h2(__byte_perm(c, 0x64646464u, 0x4140)), p1 = u32_as_h2(__byte_perm(c, 0x64646464u, 0x4342));
-      out[2 * wi] = h2_as_u32(hmul2_rn(d2, hmul2_rn(s2, __hsub2(p0, off))));
-      out[2 * wi + 1] = h2_as_u32(hmul2_rn(d2, hmul2_rn(s2, __hsub2(p1, off))));
-    }
-  }
 };
 
 // ---- Q2_K: value = fp32 (d*sc)*q - dmin*m rounded once (the dequantized weight itself: the 16-value
@@ -978,6 +932,85 @@ template <> struct Stage64<T_Q8_0, __half> {
       case 1: stage<1>(chunk, out); break;
       case 2: stage<2>(chunk, out); break;
       default: stage<3>(chunk, out); break;
+    }
+  }
+};
+
+// =============================================================================================
+// Item decoders: one thread turns half a 256-value chunk of its row, two stages, into operand A, whatever the row's alignment.
+// What both stages need is read once (begin), and the 32-value units are dealt to the stages as suits the format: the
+// activation matrix is written in that order (PERM, see mmq_perm).
+//
+// The N words of a row from the 2-byte aligned shared address a.  wide: every row of the tile has the same remainder modulo 16
+// (rows that are a multiple of 16 bytes, as with most K): the slots are an odd number of 16-byte units apart, so 32-bit loads of
+// 32 rows meet in eight banks, four at a time, and 16-byte loads do not.
+// =============================================================================================
+template <int N> __device__ __forceinline__ void lds_row_words(uint32_t a, bool wide, uint32_t (&w)[N]) {
+  const uint32_t sh = (a & 2u) * 8u;
+  if (wide) {
+    constexpr int Q = (N + 7) / 4;
+    uint32_t t[4 * Q];
+#pragma unroll
+    for (int i = 0; i < Q; ++i) {
+      const uint4 v = lds128s((a & ~15u) + 16u * i);
+      t[4 * i] = v.x; t[4 * i + 1] = v.y; t[4 * i + 2] = v.z; t[4 * i + 3] = v.w;
+    }
+    switch ((a >> 2) & 3u) {
+#define LDS_ROW_CASE(K) \
+  _Pragma("unroll") for (int i = 0; i < N; ++i) w[i] = __funnelshift_r(t[i + K], t[i + K + 1], sh); \
+  break
+      case 0: LDS_ROW_CASE(0);
+      case 1: LDS_ROW_CASE(1);
+      case 2: LDS_ROW_CASE(2);
+      default: LDS_ROW_CASE(3);
+#undef LDS_ROW_CASE
+    }
+  } else {
+    uint32_t r[N + 1];
+#pragma unroll
+    for (int i = 0; i <= N; ++i) r[i] = lds32((a & ~3u) + 4u * i);
+#pragma unroll
+    for (int i = 0; i < N; ++i) w[i] = __funnelshift_r(r[i], r[i + 1], sh);
+  }
+}
+
+template <int TYPE, typename ab_t> struct Item128 { static constexpr bool HAVE = false; };
+
+// ---- Q6_K: value = half(d * half(sc * (code - 32))), 210-byte blocks: ql[128] | qh[64] | sc[16] | d -----------------------
+// Half ip has four units q of 32 values: low 4 bits = nibble q >> 1 of ql[64 ip + 32 (q & 1) + l], high 2 bits = bits 2q.. of
+// qh[32 ip + l], scales sc[8 ip + 2q] (l < 16) and sc[8 ip + 2q + 1].  Stage h takes the units h and h + 2 -- both nibbles of the
+// same 32 bytes -- so 16 words give 64 values (with units h and h + 1, all 64 bytes of ql were read twice).  The code goes to bits 2-7 of a byte;
+// with 0x5C above it that is the half 256 + code, and (256 + code) * sc - 288 * sc is exact before its one rounding: 9 * 32 * sc has 11 significant bits.
+template <typename ab_t> struct Item128<T_Q6_K, ab_t> {
+  static constexpr bool HAVE = true;
+  struct State {
+    uint32_t h[8], sc[2];
+    __half2 d2;
+  };
+  static __device__ __forceinline__ void begin(uint32_t row, int ip, bool wide, State& s) {
+    lds_row_words<8>(row + 128 + 32 * ip, wide, s.h);
+    lds_words_unaligned<2>(row + 192 + 8 * ip, s.sc);
+    const uint32_t du = lds16(row + 208);
+    s.d2 = u32_as_h2(du | (du << 16));
+  }
+  template <int H> static __device__ __forceinline__ void stage(uint32_t row, int ip, bool wide, const State& s, uint32_t (&out)[32]) {
+    uint32_t l[8];
+    lds_row_words<8>(row + 64 * ip + 32 * H, wide, l);
+    __half2 sc[4], off[4];   // of the unit H, first and second 16 values, and of the unit H + 2
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      sc[i] = __hsub2(u32_as_h2(__byte_perm(s.sc[i >> 1] ^ 0x80808080u, 0x64646464u, 0x4040u + 0x0101u * (2 * H + (i & 1)))), __floats2half2_rn(1152.f, 1152.f));
+      off[i] = hmul2_rn(sc[i], __floats2half2_rn(-288.f, -288.f));
+    }
+#pragma unroll
+    for (int w = 0; w < 8; ++w) {   // values 4w .. 4w + 3 of both units
+      const uint32_t c0 = ((l[w] << 2) & 0x3C3C3C3Cu) | ((s.h[w] << (6 - 2 * H)) & 0xC0C0C0C0u);
+      const uint32_t c1 = ((l[w] >> 2) & 0x3C3C3C3Cu) | ((s.h[w] << (2 - 2 * H)) & 0xC0C0C0C0u);
+      const int i = w >> 2;
+      out[2 * w] = h2_as_u32(hmul2_rn(s.d2, __hfma2(u32_as_h2(__byte_perm(c0, 0x5C5C5C5Cu, 0x4140)), sc[i], off[i])));
+      out[2 * w + 1] = h2_as_u32(hmul2_rn(s.d2, __hfma2(u32_as_h2(__byte_perm(c0, 0x5C5C5C5Cu, 0x4342)), sc[i], off[i])));
+      out[16 + 2 * w] = h2_as_u32(hmul2_rn(s.d2, __hfma2(u32_as_h2(__byte_perm(c1, 0x5C5C5C5Cu, 0x4140)), sc[2 + i], off[2 + i])));
+      out[16 + 2 * w + 1] = h2_as_u32(hmul2_rn(s.d2, __hfma2(u32_as_h2(__byte_perm(c1, 0x5C5C5C5Cu, 0x4342)), sc[2 + i], off[2 + i])));
     }
   }
 };

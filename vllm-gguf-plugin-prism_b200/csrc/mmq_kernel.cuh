@@ -221,6 +221,10 @@ __device__ __forceinline__ bool mmq_next_part(const MmqParams& p, MmqPart& q) {
   return true;
 }
 
+template <typename I, bool HAVE = I::HAVE> struct ItemStateOf { struct type {}; };
+template <typename I> struct ItemStateOf<I, true> { using type = typename I::State; };
+template <typename I> using ItemState = typename ItemStateOf<I>::type;
+
 // bits of v in a 16-bit output type
 __device__ __forceinline__ uint16_t mmq_bits16(int dtype, float v) {
   return dtype == DT_F16 ? __half_as_ushort(__float2half_rn(v)) : __bfloat16_as_ushort(__float2bfloat16_rn(v));
@@ -538,6 +542,7 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_consta
 
     // Item i is half i & 1 of the i / 2-th chunk of the CTA, so a group has the same half, slot and barriers all its life.
     const int half = g & 1;
+    const bool wide = p.raw.mode == 2 && p.raw.cl2 == 0;           // rows of one remainder modulo 16
     const uint32_t slot_free = bar(4 + (p.sa == 4 ? g : g ^ 2));   // `empty` of the item that had the slot before
     uint32_t free_ph = p.sa == 2 && g >= 2 ? 0u : 1u;              // (1 at first: the slot has never been used)
     const uint32_t a_dst = a_lane + (uint32_t)((g & (p.sa - 1)) * MMQ_A_COLS);
@@ -568,11 +573,18 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_consta
           const uint8_t* chunk = slot + rs * p.raw.bytes + (FAST ? 0u : raw_shift(p.raw, n, qt.row0, c));
           uint2 cv;
           if constexpr (Dec::CORR) cv = Dec::corr(chunk, half, nunits - 8 * c);
+          using Item = Item128<TYPE, ab_t>;
+          ItemState<Item> state;
+          const uint32_t row_s = smem_u32(chunk);
+          if constexpr (Item::HAVE) Item::begin(row_s, half, wide, state);
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             const int s2 = 2 * half + h;      // 64-value stage of the chunk
             uint32_t v[32];
-            if constexpr (FAST) {
+            if constexpr (Item::HAVE) {
+              if (h == 0) Item::template stage<0>(row_s, half, wide, state, v);
+              else Item::template stage<1>(row_s, half, wide, state, v);
+            } else if constexpr (FAST) {
               Stage64<TYPE, ab_t>::decode(chunk, s2, v);
             } else {
               const int u = 2 * s2;           // units (32 values) u, u + 1 of the chunk

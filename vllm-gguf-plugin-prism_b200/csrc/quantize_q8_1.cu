@@ -122,8 +122,8 @@ __global__ void __launch_bounds__(256) quantize_q8_1_kernel(const in_t* __restri
 // The reference's butterfly adds element i to element i^16, then i^8, i^4, i^2, i^1; with lane
 // t of a quad holding elements 8t..8t+7 the first two levels are shuffles across the quad (lane
 // ^2, lane ^1) and the last three are adds inside the thread, in the same order, so the fp32 sum
-// has the same bits.  perm = 1 stores every group of four values in the order (0,2,1,3) (see
-// Stage64 in mmq_decode.cuh).
+// has the same bits.  perm: the order the values are stored in (see
+// mmq_perm).
 // act != 0 (fused MoE step): the input rows are [gate | up] of x_ld = 2K values and the value that
 // is quantized is act(gate) * up, formed as the reference's separate activation op forms it --
 // silu(g) = g / (1 + exp(-g)) (gelu: 0.5 g (1 + erf(g / sqrt 2))) rounded to the activation type,
@@ -220,10 +220,11 @@ __global__ void __launch_bounds__(256) quantize_f16x8_kernel(const in_t* __restr
       __half o[8];
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        const int jj = perm ? ((j & 4) | ((j & 1) << 1) | ((j >> 1) & 1)) : j;   // position jj holds value j
+        const int jj = perm == 1 ? ((j & 4) | ((j & 1) << 1) | ((j >> 1) & 1)) : j;   // position jj holds value j
         o[jj] = __float2half_rn(d8 * (float)q[j]);
       }
-      *reinterpret_cast<uint4*>(xb + row * ldb + k) = *reinterpret_cast<const uint4*>(o);
+      const int64_t at = perm == 2 ? ((kb & ~int64_t(3)) | ((kb & 1) << 1) | ((kb >> 1) & 1)) * 32 + 8 * t : k;
+      *reinterpret_cast<uint4*>(xb + row * ldb + at) = *reinterpret_cast<const uint4*>(o);
     }
     if (corr_mode != CORR_NONE) {
       qs += __shfl_xor_sync(0xffffffffu, qs, 2, 32);
