@@ -1054,3 +1054,19 @@ def test_tiled_q5_0_product_of_every_shape(shape):
     assert torch.equal(y, capi.mul_mat_a8(w, x, t, N))
     torch.cuda.synchronize()
     assert capi.last_status() == 0
+
+
+@pytest.mark.parametrize("shape", [(5120, 256, 40), (5120, 1280, 100), (640, 1280, 17), (5120, 2304, 48), (1280, 2304, 144), (5120, 2304, 300), (896, 3328, 330)])
+@pytest.mark.parametrize("name", ["Q4_K", "Q4_0", "Q5_1", "Q6_K"])
+def test_tiled_blocks_of_corrections_cut_anywhere(name, shape):
+    """One to thirteen chunks a row, most of them cut into runs that begin and end inside a block of four (blocks of one chunk among
+    them), two to four slots of operand A: against row-by-row products."""
+    t, (N, K, M) = TYPES[name], shape
+    _, w = dev_w(t, N, K, seed=N + K)
+    x = (dev_x(M, K, seed=M).float() / 8).half()
+    y = capi.mul_mat_a8(w, x, t, N)
+    want = torch.cat([capi.mul_mat_vec_a8(w, x[i:i + 16].float().contiguous(), t, N) for i in range(0, M, 16)])
+    torch.cuda.synchronize()
+    assert capi.last_status() == 0
+    assert rel_l2(y.float().cpu(), want.cpu()) <= REL_L2_TOL
+    assert torch.equal(y, capi.mul_mat_a8(w, x, t, N))

@@ -26,7 +26,7 @@
 // the accumulators out; a B loader, an MMA issuer, a raw-weight loader.  An item has one full/empty barrier pair; up to 128
 // tokens a tile its activations arrive on it too, in one box.  Every wait is bounded in time and reports through the status word.
 // The correction values are taken from the raw chunk while it is decoded and written to shared memory as a tile of operand A; the
-// tensor core multiplies it once per eight chunks (gathered from global memory at the end of a tile they took 10,600 clocks of it).
+// tensor core multiplies it once per four chunks (gathered from global memory at the end of a tile they took 10,600 clocks of it).
 //
 // One CTA per SM lives for the whole launch, over a range of (tile, 256-value chunk) units (mmq_plan); a tile that several CTAs
 // share is added up by the last of them to arrive, in CTA order (deterministic).  While a tile's accumulator is read out the
@@ -215,8 +215,8 @@ int launch_mmq(const MmqArgs& a, cudaStream_t stream) {
   p.tn = plan.tn;
   p.tt = (int)plan.tt;
   p.idesc = umma_idesc(MMQ_ROWS, p.tn > 256 ? p.tn / 2 : p.tn, bf ? 1 : 0);
-  p.sa = p.tn <= 256 ? 4 : 2;
-  p.a_col0 = p.tn <= 256 ? 256 : 384;
+  p.sa = p.tn <= 256 ? 4 : p.tn <= 320 ? 3 : 2;
+  p.a_col0 = 512 - p.sa * MMQ_A_COLS;
   p.nbuf = p.tn <= 128 ? 2 : 1;
   p.status = a.status;
   p.w_wait = a.w_in_flight ? 1 : 0;

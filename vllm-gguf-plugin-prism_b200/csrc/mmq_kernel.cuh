@@ -17,15 +17,17 @@ constexpr int MMQ_GROUPS = 4;                        // producer groups of 128 t
 constexpr int MMQ_PRODUCER_WARPS = 4 * MMQ_GROUPS;
 constexpr int MMQ_THREADS = (MMQ_PRODUCER_WARPS + 3) * 32;   // + B loader, MMA issuer, raw-weight loader
 // Operand A moves in items: half a 256-value chunk, two stages, 64 columns of tensor memory.  Up to 256 tokens a tile there are 256
-// columns of accumulator -- two of 128 tokens, or one beyond 128 -- and four A slots; up to 384 tokens, one accumulator and two A slots.
-// The items' barriers are a ring of four in both cases: a group's items are four apart, so by the time it waits for a
-// phase it has seen the one before complete.
+// columns of accumulator -- two of 128 tokens, or one beyond 128 -- and four A slots; up to 320 tokens, one accumulator and three A slots,
+// up to 384, two.  The items' barriers are a ring of four in all cases: a group's items are four apart, so by the time it
+// waits for a phase it has seen the one before complete.
 constexpr int MMQ_A_COLS = 64, MMQ_ITEMS = 4, MMQ_D_STEP = 128;
 constexpr int MMQ_MAX_B = 8;
 // Activations arrive a box at a time, one stage or -- up to 128 tokens a tile, where the stages are short -- one item.
 constexpr int MMQ_MAX_RAW = 8;
-// Correction values of eight chunks: 64 fp16 per row, a tile of operand A in shared memory (K-major, 128-byte swizzle), twice
-constexpr int MMQ_CORR_CHUNKS = 8, MMQ_CORR_TILE = MMQ_ROWS * 128, MMQ_CORR_BYTES = 2 * MMQ_CORR_TILE;
+// Correction values of a block of four chunks: 32 fp16 per row, half of a tile of operand A in shared memory (K-major, 128-byte
+// swizzle); the next block's go into the other half.  (Whole tiles of eight chunks, twice, took 16 KB more: at 256 tokens a tile that is the
+// fifth slot of the activation ring.)
+constexpr int MMQ_CORR_CHUNKS = 4, MMQ_CORR_BYTES = MMQ_ROWS * 128;
 
 struct MmqParams {
   RawPlan raw;
@@ -38,7 +40,7 @@ struct MmqParams {
   int k, kpad;
   int nc, corr;           // 256-value chunks of a row; 1: a stage of corrections behind every eight of them
   int rt, tt, tn;         // row tiles, token tiles, tokens per tile (a multiple of 16, at most 256, or of 32, at most 384)
-  int sa, a_col0;         // A slots: how many (2 or 4), first column
+  int sa, a_col0;         // A slots: how many (2 to 4), first column
   int nbuf;               // accumulators, MMQ_D_STEP columns apart
   int bg;                 // stages of an activation box: 1 or 2
   int sb, raw_stages;     // ring depths: boxes, raw chunks
@@ -123,18 +125,14 @@ __device__ __forceinline__ void umma_f16_ts4(uint32_t d_tmem, uint32_t a_tmem, u
       ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate), "r"(lead)
       : "memory");
 }
-// ... with A from shared memory (low words of both descriptors; they share the high one)
-__device__ __forceinline__ void umma_f16_ss4(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc, uint32_t lead) {
+// Half a stage with A from shared memory (low words of both descriptors; they share the high one)
+__device__ __forceinline__ void umma_f16_ss2(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc, uint32_t lead) {
   asm volatile(
       "{\n\t.reg .pred q, t;\n\t.reg .b64 a, b;\n\t.reg .b32 al, bl;\n\t"
       "setp.ne.b32 q, %5, 0;\n\tsetp.eq.b32 t, 0, 0;\n\t"
       "mov.b64 a, {%1, %3};\n\tmov.b64 b, {%2, %3};\n\t"
       "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, t;\n\t"
       "add.u32 al, %1, 2;\n\tadd.u32 bl, %2, 2;\n\tmov.b64 a, {al, %3};\n\tmov.b64 b, {bl, %3};\n\t"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, t;\n\t"
-      "add.u32 al, %1, 4;\n\tadd.u32 bl, %2, 4;\n\tmov.b64 a, {al, %3};\n\tmov.b64 b, {bl, %3};\n\t"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, t;\n\t"
-      "add.u32 al, %1, 6;\n\tadd.u32 bl, %2, 6;\n\tmov.b64 a, {al, %3};\n\tmov.b64 b, {bl, %3};\n\t"
       "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, t;\n\t}"
       ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc), "r"(lead)
       : "memory");
@@ -206,7 +204,7 @@ __device__ __forceinline__ MmqTile mmq_tile(const MmqParams& p, int tile) {
   }
   return t;
 }
-// The stages of a part come in blocks: four per chunk, and behind every run of chunks with the same c / 8 one stage of their
+// The stages of a part come in blocks: four per chunk, and behind every run of chunks with the same c / 4 half a stage of their
 // correction columns (formats without them: one block).  End of the block that starts at chunk c:
 __device__ __forceinline__ int mmq_block_end(const MmqParams& p, const MmqPart& q, int c) {
   const int e = (c | (MMQ_CORR_CHUNKS - 1)) + 1;
@@ -293,7 +291,7 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_consta
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + p.aux_off);
   uint64_t* full = bars;                     // [4] item i % 4: its A slot is filled (the four warps of a group), boxes of an item: and its box is there
   uint64_t* empty = bars + 4;                // [4] the MMAs that read it are done
-  uint64_t* b_full = bars + 8;               // [8] a box of one stage is there; boxes of an item: [0] that of a block's corrections
+  uint64_t* b_full = bars + 8;               // [8] a box of one stage is there; boxes of an item: [0], [1] those of the blocks' corrections, in turn
   uint64_t* b_empty = bars + 16;             // [8] ... and has been read
   uint64_t* accum = bars + 24;               // [2] an accumulator is complete
   uint64_t* drained = bars + 26;             // [2] ... and has been read
@@ -543,9 +541,9 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_consta
     // Item i is half i & 1 of the i / 2-th chunk of the CTA, so a group has the same half, slot and barriers all its life.
     const int half = g & 1;
     const bool wide = p.raw.mode == 2 && p.raw.cl2 == 0;           // rows of one remainder modulo 16
-    const uint32_t slot_free = bar(4 + (p.sa == 4 ? g : g ^ 2));   // `empty` of the item that had the slot before
-    uint32_t free_ph = p.sa == 2 && g >= 2 ? 0u : 1u;              // (1 at first: the slot has never been used)
-    const uint32_t a_dst = a_lane + (uint32_t)((g & (p.sa - 1)) * MMQ_A_COLS);
+    const uint32_t slot_free = bar(4 + ((g - p.sa) & 3));          // `empty` of the item that had the slot before
+    uint32_t free_ph = g >= p.sa ? 0u : 1u;                        // (1 at first: the slot has never been used)
+    int a_slot = g >= p.sa ? g - p.sa : g;                         // (four items on: the next slot of three, the same of two or four)
     int rs = g >> 1;             // raw slot of the group's next chunk, and its phase
     uint32_t rph = 0;
     int i0 = 0, pi = 0;          // items before the part, parts so far
@@ -561,7 +559,7 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_consta
       const int items = more ? 2 * (q.c1 - q.c0) : 0;
       int m = (g - i0) & 3;      // this group's next item of the part
       bool read_out = pi > 0;
-      // With one accumulator and two slots the first items of groups two and three have no room before the tile is read out.
+      // With one accumulator and fewer slots than groups the first items of the last groups have no room before the tile is read out.
       bool hold = read_out && p.nbuf == 1 && m >= p.sa;
       for (;;) {
         if (m < items && !hold) {
@@ -616,24 +614,24 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_consta
               free_ph ^= 1u;
               tc_fence_after();
             }
-            tmem_st32(a_dst + 32 * h, v);
+            tmem_st32(a_lane + (uint32_t)(a_slot * MMQ_A_COLS + 32 * h), v);
           }
           if constexpr (Dec::CORR) {
-            // The block's tile: multiplied before the last item of the block is handed back, and free again for the block after the
-            // next.  That item is three before this one at the earliest, and four slots wait for the fourth.
-            const int b = (c >> 3) - (q.c0 >> 3);
-            const uint32_t at = s_corr + (uint32_t)(((blk0 + b) & 1) * MMQ_CORR_TILE);
-            if (half == 0 && (c == q.c0 || (c & 7) == 0)) {   // the block's first item
-              const int e = b == 0 ? end2 : b == 1 ? i0 - 1 : i0 + 2 * ((c & ~7) - 8 - q.c0) - 1;
+            // The block's half tile: multiplied before the last item of the block is handed back, and free again for the block after
+            // the next.  That item is three before this one at the earliest, and four slots wait for the fourth.
+            const int b = (c >> 2) - (q.c0 >> 2);
+            const int piece0 = (blk0 + b) & 1 ? 4 ^ (r & 7) : r & 7;     // 16-byte piece of the block's first chunk, swizzled
+            if (half == 0 && (c == q.c0 || (c & 3) == 0)) {   // the block's first item
+              const int e = b == 0 ? end2 : b == 1 ? i0 - 1 : i0 + 2 * ((c & ~3) - 4 - q.c0) - 1;
               if (e >= 0 && e > i - p.sa) wait(bar(4 + (e & (MMQ_ITEMS - 1))), (uint32_t)(e >> 2) & 1u);
-              const int lo = c & 7, hi = q.c1 - (c & ~7);     // chunks that other parts have, or nobody: zeros
-              if (lo > 0 || hi < 8) {
+              const int lo = c & 3, hi = q.c1 - (c & ~3);     // chunks that other parts have, or nobody: zeros
+              if (lo > 0 || hi < 4) {
 #pragma unroll 1
-                for (int j = 0; j < 8; ++j)
-                  if (j < lo || j >= hi) asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(at + (uint32_t)((j ^ (r & 7)) << 4)), "r"(0u) : "memory");
+                for (int j = 0; j < 4; ++j)
+                  if (j < lo || j >= hi) asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(s_corr + (uint32_t)((j ^ piece0) << 4)), "r"(0u) : "memory");
               }
             }
-            asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(at + (uint32_t)((((c & 7) ^ (r & 7)) << 4) + 8 * half)), "r"(cv.x), "r"(cv.y) : "memory");
+            asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(s_corr + (uint32_t)((((c & 3) ^ piece0) << 4) + 8 * half)), "r"(cv.x), "r"(cv.y) : "memory");
             fence_proxy_async();   // (the tensor core reads it)
           }
           tmem_st_wait();
@@ -641,6 +639,7 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_consta
           __syncwarp();
           if (lane == 0) mbar_arrive(bar(g));
           m += 4;
+          if (p.sa == 3) a_slot = a_slot == 2 ? 0 : a_slot + 1;
           rs += 2;
           if (rs >= p.raw_stages) { rs -= p.raw_stages; rph ^= 1u; }
         }
@@ -654,8 +653,8 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_consta
       i0 += items;
       if constexpr (Dec::CORR) {
         if (more) {
-          const int nb = ((q.c1 - 1) >> 3) - (q.c0 >> 3) + 1;
-          end2 = nb > 1 ? i0 - 2 * (q.c1 - ((q.c1 - 1) & ~7)) - 1 : i0 - items - 1;
+          const int nb = ((q.c1 - 1) >> 2) - (q.c0 >> 2) + 1;
+          end2 = nb > 1 ? i0 - 2 * (q.c1 - ((q.c1 - 1) & ~3)) - 1 : i0 - items - 1;
           blk0 += nb;
         }
       }
@@ -676,12 +675,12 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_consta
     // (Converged like the MMA issuer below.)
     const uint32_t lead = elect_one() ? 1u : 0u;
     const uint32_t bytes = (uint32_t)(p.bg * b_stage), sb_s = smem_u32(sB);
-    int i = 0, sb = 0;
+    int i = 0, sb = 0, blk = 0;
     uint32_t ph = 0;
     pdl_wait();
     while (mmq_next_part(p, q)) {
       const int x0 = mmq_tile(p, q.tile).x0;
-      for (int cs = q.c0, ce; cs < q.c1; cs = ce) {
+      for (int cs = q.c0, ce; cs < q.c1; cs = ce, ++blk) {
         ce = mmq_block_end(p, q, cs);
         const int n = 2 * (ce - cs) * (p.bg == 2 ? 1 : 2);
 #pragma unroll 1
@@ -689,8 +688,8 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_consta
           mbar_wait_or(bar(16 + sb), ph ^ 1u, gave_up_s);
           if (lds32(gave_up_s) != 0u) goto b_done;   // (no copy into a slot that may be in use)
           __syncwarp();
-          const int stage = j < n ? 4 * cs + p.bg * j : (p.kpad >> 6) + cs / MMQ_CORR_CHUNKS;
-          const uint32_t fb = bar(p.bg == 1 ? 8 + sb : j < n ? i & (MMQ_ITEMS - 1) : 8), dst = sb_s + (uint32_t)sb * bytes;
+          const int stage = j < n ? 4 * cs + p.bg * j : (p.kpad >> 6) + (cs >> 3);   // (eight chunks' columns: a block takes its half)
+          const uint32_t fb = bar(p.bg == 1 ? 8 + sb : j < n ? i & (MMQ_ITEMS - 1) : 8 + (blk & 1)), dst = sb_s + (uint32_t)sb * bytes;
           if (lead) {
             mbar_expect_tx(fb, bytes);
             tma_box3(dst, &bmap, 0, x0, stage, fb);
@@ -724,7 +723,7 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_consta
     // live in uniform registers; one lane issues.  (With one lane in the loop, every operand went from a register to a uniform one at
     // each instruction, and this loop was what bounded the kernel at 128 tokens or less: 460 to 560 clocks a stage whatever the decoder.)
     const uint32_t lead = elect_one() ? 1u : 0u;
-    int i = 0, sb = 0, pi = 0, blk = 0;
+    int i = 0, sb = 0, pi = 0, blk = 0, a_slot = 0;
     uint32_t ph = 0;
     const uint64_t bd0 = umma_desc_sw128(smem_u32(sB));
     const uint32_t b_step = (uint32_t)(b_stage >> 4), b_lo0 = (uint32_t)bd0, b_hi = (uint32_t)(bd0 >> 32);
@@ -747,7 +746,8 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_consta
         for (int end = i + 2 * (ce - cs); i < end; ++i) {
           const int s = i & (MMQ_ITEMS - 1);
           mbar_wait_or(bar(s), (uint32_t)(i >> 2) & 1u, gave_up_s);
-          const uint32_t at = (uint32_t)(p.a_col0 + (i & (p.sa - 1)) * MMQ_A_COLS);
+          const uint32_t at = (uint32_t)(p.a_col0 + a_slot * MMQ_A_COLS);
+          if (++a_slot == p.sa) a_slot = 0;
           if (p.bg == 2) {
             __syncwarp();
             tc_fence_after();
@@ -767,12 +767,12 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_consta
           }
           accumulate = 1;
           if (p.corr && i == end - 1) {   // the block's corrections, before its last item is handed back
-            mbar_wait_or(bar(p.bg == 2 ? 8 : 8 + sb), p.bg == 2 ? (uint32_t)blk & 1u : ph, gave_up_s);
+            mbar_wait_or(bar(8 + (p.bg == 2 ? blk & 1 : sb)), p.bg == 2 ? (uint32_t)(blk >> 1) & 1u : ph, gave_up_s);
             __syncwarp();
             tc_fence_after();
-            const uint32_t c_lo = c_lo0 + (uint32_t)((blk & 1) * (MMQ_CORR_TILE >> 4));
-            umma_f16_ss4(d, c_lo, b_lo, b_hi, p.idesc, lead);
-            if (half_n) umma_f16_ss4(d + (uint32_t)half_n, c_lo, b_lo + half_lo, b_hi, p.idesc, lead);
+            const uint32_t c_lo = c_lo0 + 4u * (uint32_t)(blk & 1), x_lo = b_lo + 4u * (uint32_t)((cs >> 2) & 1);   // halves of 64 bytes
+            umma_f16_ss2(d, c_lo, x_lo, b_hi, p.idesc, lead);
+            if (half_n) umma_f16_ss2(d + (uint32_t)half_n, c_lo, x_lo + half_lo, b_hi, p.idesc, lead);
             ++blk;
             box_done();
           }

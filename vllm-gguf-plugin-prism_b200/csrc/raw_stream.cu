@@ -29,7 +29,7 @@ bool plan_raw(int type, const void* w, int64_t n_rows, int64_t copies, int64_t K
   p.gap = copies > 1 ? gap : 0;
   p.nrows = p.nfull = (int)n_rows;
   if (pitch % raw_type_align(type) != 0 || pitch < p.row_bytes) return false;
-  const int s16 = (p.rbc + 30) / 16 + 1;
+  const int s16 = (p.rbc + 30) / 16;   // the chunk, displaced by up to 15 bytes
   p.slot = (s16 % 2 ? s16 : s16 + 1) * 16;
   EncodeTiledFn enc = tensor_map_encoder();
   auto encode = [&](int64_t inner, int64_t row, int64_t rows, int box0, int box1) {
