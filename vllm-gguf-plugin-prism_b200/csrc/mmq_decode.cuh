@@ -64,28 +64,33 @@ __device__ __forceinline__ uint32_t shift_of(const uint8_t* p) { return (uint32_
 // thread's copy; the larger code books have room for fewer copies.
 struct DecodeCtx {
   uint32_t grid;      // code book: byte-permute selectors of value pairs (IQ2), magnitudes (IQ3), codes (IQ1)
-  uint32_t sgn;       // per sign index, the sign-bit masks of the four value pairs (16 bytes)
+  uint32_t sgn;       // per 7-bit sign index, the signs of the four value pairs (iq_pair_signs)
 };
-template <int TYPE> struct DecodeTables {   // GRID entries of GB bytes in GC copies; SGN sign entries in SC copies
-  static constexpr int GRID = 0, GB = 0, GC = 0, SGN = 0, SC = 0;
+template <int TYPE> struct DecodeTables {   // GRID entries of GB bytes in GC copies; SGN sign words in 32 copies
+  static constexpr int GRID = 0, GB = 0, GC = 0, SGN = 0;
 };
-template <> struct DecodeTables<T_IQ2_XXS> { static constexpr int GRID = 256, GB = 8, GC = 16, SGN = 128, SC = 8; };
-template <> struct DecodeTables<T_IQ2_XS> { static constexpr int GRID = 512, GB = 8, GC = 4, SGN = 128, SC = 8; };
-template <> struct DecodeTables<T_IQ2_S> { static constexpr int GRID = 1024, GB = 8, GC = 2, SGN = 256, SC = 4; };
-template <> struct DecodeTables<T_IQ3_XXS> { static constexpr int GRID = 256, GB = 4, GC = 16, SGN = 128, SC = 8; };
-template <> struct DecodeTables<T_IQ3_S> { static constexpr int GRID = 512, GB = 4, GC = 8, SGN = 256, SC = 4; };
-template <> struct DecodeTables<T_IQ1_S> { static constexpr int GRID = 2048, GB = 4, GC = 2, SGN = 0, SC = 0; };
+template <> struct DecodeTables<T_IQ2_XXS> { static constexpr int GRID = 256, GB = 16, GC = 8, SGN = 128; };
+template <> struct DecodeTables<T_IQ2_XS> { static constexpr int GRID = 512, GB = 16, GC = 4, SGN = 128; };
+template <> struct DecodeTables<T_IQ2_S> { static constexpr int GRID = 1024, GB = 16, GC = 2, SGN = 0; };
+template <> struct DecodeTables<T_IQ3_XXS> { static constexpr int GRID = 256, GB = 8, GC = 16, SGN = 128; };
+template <> struct DecodeTables<T_IQ3_S> { static constexpr int GRID = 512, GB = 8, GC = 8, SGN = 0; };
+template <> struct DecodeTables<T_IQ1_S> { static constexpr int GRID = 2048, GB = 4, GC = 2, SGN = 0; };
 template <> struct DecodeTables<T_IQ1_M> : DecodeTables<T_IQ1_S> {};
 template <int TYPE> __host__ __device__ constexpr int decoder_table_bytes() {
   using D = DecodeTables<TYPE>;
-  return D::GRID * D::GB * D::GC + D::SGN * 16 * D::SC;
+  return D::GRID * D::GB * D::GC + D::SGN * 4 * 32;
 }
 template <int TYPE> __device__ __forceinline__ DecodeCtx decoder_context(const uint8_t* tab, int lane) {
   using D = DecodeTables<TYPE>;
   DecodeCtx cx{0, 0};
   if constexpr (D::GRID > 0) cx.grid = smem_u32(tab) + (uint32_t)(D::GB * (lane & (D::GC - 1)));
-  if constexpr (D::SGN > 0) cx.sgn = smem_u32(tab) + (uint32_t)(D::GRID * D::GB * D::GC + 16 * (lane & (D::SC - 1)));
+  if constexpr (D::SGN > 0) cx.sgn = smem_u32(tab) + (uint32_t)(D::GRID * D::GB * D::GC + 4 * lane);
   return cx;
+}
+template <int TYPE> __device__ __forceinline__ uint4 grid128(const DecodeCtx& cx, uint32_t i) {
+  uint4 v;
+  asm("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(cx.grid + (uint32_t)(16 * DecodeTables<TYPE>::GC) * i));
+  return v;
 }
 template <int TYPE> __device__ __forceinline__ uint2 grid64(const DecodeCtx& cx, uint32_t i) {
   uint2 v;
@@ -97,58 +102,72 @@ template <int TYPE> __device__ __forceinline__ uint32_t grid32(const DecodeCtx& 
   asm("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(cx.grid + (uint32_t)(4 * DecodeTables<TYPE>::GC) * i));
   return v;
 }
-template <int TYPE> __device__ __forceinline__ uint4 sign_masks(const DecodeCtx& cx, uint32_t i) {
-  uint4 v;
-  asm("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(cx.sgn + (uint32_t)(16 * DecodeTables<TYPE>::SC) * i));
+// Signs of eight values, two ways.  Both multiply where they could shift: the integer pipe that shifts, masks and permutes is
+// what bounds these decoders, the one that multiplies has room.  `negate` takes the word whose bits 15 and 31 are those of pair P.
+__device__ __forceinline__ uint32_t negate(uint32_t pair, uint32_t bits) { return pair ^ (bits & 0x80008000u); }
+// ... from the sign bits themselves, s < 256: bit 2P to bit 15, bit 2P + 1 to bit 31 (the two products do not overlap)
+template <int P> __device__ __forceinline__ uint32_t sign_bits8(uint32_t s) { return s * ((1u << (15 - 2 * P)) + (1u << (30 - 2 * P))); }
+// ... from the table word of a 7-bit index: bits 15 - P and 31 - P
+__device__ __forceinline__ uint32_t sign_word(const DecodeCtx& cx, uint32_t i) {
+  uint32_t v;
+  asm("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(cx.sgn + 128u * i));
   return v;
 }
-// Shared-memory tables of the IQ2 decoders, built once per CTA from the formats' grid and
-// sign tables.  A grid entry holds eight magnitudes, each one of {8, 25, 43}; with the three
-// products d*8, d*25, d*43 of a 32-value group rounded to 16 bits and parked in two registers,
-// every PAIR of decoded values is one byte-permute whose 16-bit selector depends only on the grid
-// entry -- those selectors are what the table holds -- and the signs are one XOR per pair.
-__device__ __forceinline__ uint2 iq2xxs_pair_selectors(uint64_t grid_entry) {
-  uint32_t s[2] = {0u, 0u};
+template <int P> __device__ __forceinline__ uint32_t sign_bits(uint32_t word) { return word * (1u << P); }
+__device__ __forceinline__ uint32_t iq_pair_signs(uint32_t sign_bits) {
+  uint32_t w = 0;
+#pragma unroll
+  for (int p = 0; p < 4; ++p) w |= ((sign_bits >> (2 * p)) & 1u) << (15 - p) | ((sign_bits >> (2 * p + 1)) & 1u) << (31 - p);
+  return w;
+}
+// Shared-memory tables of the code-book decoders, built once per CTA from the formats' grid and sign tables.  An IQ2 grid entry
+// holds eight magnitudes, each one of {8, 25, 43}; with the three products d*8, d*25, d*43 of a 32-value group rounded to 16 bits
+// and parked in two registers, every PAIR of decoded values is one byte-permute whose selector depends only on the
+// grid entry -- those selectors are what the table holds.
+__device__ __forceinline__ uint4 iq2_pair_selectors(uint64_t grid_entry) {
+  uint32_t s[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     const uint32_t m = (uint32_t)(grid_entry >> (8 * j)) & 0xFFu;
     const uint32_t c = (m > 8u ? 1u : 0u) + (m > 25u ? 1u : 0u);   // which of the three magnitudes
     const uint32_t nib = (2u * c) | ((2u * c + 1u) << 4);           // its two bytes in the register pair
-    s[j >> 2] |= nib << (8 * (j & 3));
+    s[j >> 1] |= nib << (8 * (j & 1));
   }
-  return make_uint2(s[0], s[1]);
+  return make_uint4(s[0], s[1], s[2], s[3]);
 }
-__device__ __forceinline__ uint4 iq2xxs_pair_signs(uint32_t sign_bits) {
-  uint32_t m[4];
-#pragma unroll
-  for (int p = 0; p < 4; ++p) m[p] = (((sign_bits >> (2 * p)) & 1u) << 15) | (((sign_bits >> (2 * p + 1)) & 1u) << 31);
-  return make_uint4(m[0], m[1], m[2], m[3]);
+// An IQ3 entry: its four magnitudes (at most 62) as 16-bit values, for fp16 divided by 256 (see iq3_pair).
+template <typename ab_t> __device__ __forceinline__ uint2 iq3_magnitudes(uint32_t g) {
+  const float f = std::is_same<ab_t, __half>::value ? 1.f / 256.f : 1.f;
+  return make_uint2(pack2<ab_t>(f * (float)(g & 0xFFu), f * (float)((g >> 8) & 0xFFu)), pack2<ab_t>(f * (float)((g >> 16) & 0xFFu), f * (float)(g >> 24)));
 }
 
-template <int TYPE> __device__ __forceinline__ void decoder_fill_tables(uint8_t* tab) {
+template <int TYPE, typename ab_t> __device__ __forceinline__ void decoder_fill_tables(uint8_t* tab) {
   using D = DecodeTables<TYPE>;
   if constexpr (D::GRID > 0) {
     for (int i = threadIdx.x; i < D::GRID * D::GC; i += blockDim.x) {
       const int e = i / D::GC;
-      if constexpr (TYPE == T_IQ2_XXS) reinterpret_cast<uint2*>(tab)[i] = iq2xxs_pair_selectors(d_iq2xxs_grid[e]);
-      if constexpr (TYPE == T_IQ2_XS) reinterpret_cast<uint2*>(tab)[i] = iq2xxs_pair_selectors(d_iq2xs_grid[e]);
-      if constexpr (TYPE == T_IQ2_S) reinterpret_cast<uint2*>(tab)[i] = iq2xxs_pair_selectors(d_iq2s_grid[e]);
-      if constexpr (TYPE == T_IQ3_XXS) reinterpret_cast<uint32_t*>(tab)[i] = d_iq3xxs_grid[e];
-      if constexpr (TYPE == T_IQ3_S) reinterpret_cast<uint32_t*>(tab)[i] = d_iq3s_grid[e];
+      if constexpr (TYPE == T_IQ2_XXS) reinterpret_cast<uint4*>(tab)[i] = iq2_pair_selectors(d_iq2xxs_grid[e]);
+      if constexpr (TYPE == T_IQ2_XS) reinterpret_cast<uint4*>(tab)[i] = iq2_pair_selectors(d_iq2xs_grid[e]);
+      if constexpr (TYPE == T_IQ2_S) reinterpret_cast<uint4*>(tab)[i] = iq2_pair_selectors(d_iq2s_grid[e]);
+      if constexpr (TYPE == T_IQ3_XXS) reinterpret_cast<uint2*>(tab)[i] = iq3_magnitudes<ab_t>(d_iq3xxs_grid[e]);
+      if constexpr (TYPE == T_IQ3_S) reinterpret_cast<uint2*>(tab)[i] = iq3_magnitudes<ab_t>(d_iq3s_grid[e]);
       if constexpr (TYPE == T_IQ1_S || TYPE == T_IQ1_M) reinterpret_cast<uint32_t*>(tab)[i] = d_iq1s_grid[e];
     }
   }
   if constexpr (D::SGN > 0) {
-    uint4* sgn = reinterpret_cast<uint4*>(tab + D::GRID * D::GB * D::GC);
-    for (int i = threadIdx.x; i < D::SGN * D::SC; i += blockDim.x) {
-      const int e = i / D::SC;
-      sgn[i] = iq2xxs_pair_signs(D::SGN == 128 ? (uint32_t)d_ksigns_iq2xs[e] : (uint32_t)e);
-    }
+    uint32_t* sgn = reinterpret_cast<uint32_t*>(tab + D::GRID * D::GB * D::GC);
+    for (int i = threadIdx.x; i < D::SGN * 32; i += blockDim.x) sgn[i] = iq_pair_signs(d_ksigns_iq2xs[i >> 5]);
   }
 }
 
 template <int TYPE, typename ab_t> struct Decoder;
-template <typename ab_t> struct Decoder<T_Q6_K, ab_t> { static constexpr bool CORR = false; };   // (see Item128)
+// formats decoded by the item (see Item128)
+template <typename ab_t> struct Decoder<T_Q6_K, ab_t> { static constexpr bool CORR = false; };
+template <typename ab_t> struct Decoder<T_IQ2_XXS, ab_t> { static constexpr bool CORR = false; };
+template <typename ab_t> struct Decoder<T_IQ2_XS, ab_t> { static constexpr bool CORR = false; };
+template <typename ab_t> struct Decoder<T_IQ2_S, ab_t> { static constexpr bool CORR = false; };
+template <typename ab_t> struct Decoder<T_IQ3_XXS, ab_t> { static constexpr bool CORR = false; };
+template <typename ab_t> struct Decoder<T_IQ3_S, ab_t> { static constexpr bool CORR = false; };
 // types that are multiplied as dequantized weights of either 16-bit type (activations as they are)
 template <int TYPE> __host__ __device__ constexpr bool decoder_bf16() {
   return TYPE == T_IQ2_XXS || TYPE == T_IQ2_XS || TYPE == T_IQ2_S || TYPE == T_IQ3_XXS || TYPE == T_IQ3_S || TYPE == T_IQ1_S || TYPE == T_IQ1_M ||
@@ -533,143 +552,6 @@ template <typename ab_t> struct Decoder<T_IQ4_NL, ab_t> {
   }
 };
 
-// ---- IQ2_XXS: fp32 d*(0.5+s)*0.25*grid*sign rounded once; unit = 32-value group ib = u&7 ----------
-// (value = +-round(d * magnitude): the product is formed in fp32 and rounded once, as in the
-// reference; multiplying by -1.f afterwards is exact, so flipping the sign bit is the same)
-template <typename ab_t> struct Decoder<T_IQ2_XXS, ab_t> {
-  static constexpr bool CORR = false;   // correction columns
-  static constexpr int RW = 5;   // [0] word holding d, [1..3] the group's 8 bytes (+ cover), [4] pad
-  static __device__ __forceinline__ void load(const uint8_t* row, int u, uint32_t (&raw)[RW]) {
-    const uint8_t* blk = row + (int64_t)(u >> 3) * 66;
-    ldg_cover<1>(blk, 2, raw);
-    ldg_cover<3>(blk + 2 + 8 * (u & 7), 8, raw + 1);
-    raw[4] = 0;
-  }
-  static __device__ __forceinline__ void decode(const uint8_t* row, int u, const uint32_t (&raw)[RW], const DecodeCtx& cx, uint32_t (&out)[16]) {
-    const uint8_t* blk = row + (int64_t)(u >> 3) * 66;
-    const float dh = __half2float(__ushort_as_half((unsigned short)((raw[0] >> shift_of(blk)) & 0xFFFFu)));
-    const uint32_t sh = shift_of(blk + 2 + 8 * (u & 7));
-    const uint32_t idx = word_at(raw + 1, 0, sh), aux = word_at(raw + 1, 1, sh);
-    const float d = dh * (0.5f + (float)(aux >> 28)) * 0.25f;
-    // the three possible magnitudes of this group, each rounded once (the sign flips only the top bit)
-    const uint32_t r0 = pack2<ab_t>(d * 8.f, d * 25.f), r1 = pack2<ab_t>(d * 43.f, 0.f);
-#pragma unroll
-    for (int il = 0; il < 4; ++il) {
-      const uint2 sel = grid64<T_IQ2_XXS>(cx, (idx >> (8 * il)) & 0xFF);
-      const uint4 sg = sign_masks<T_IQ2_XXS>(cx, (aux >> (7 * il)) & 127);
-      out[4 * il + 0] = __byte_perm(r0, r1, sel.x) ^ sg.x;
-      out[4 * il + 1] = __byte_perm(r0, r1, sel.x >> 16) ^ sg.y;
-      out[4 * il + 2] = __byte_perm(r0, r1, sel.y) ^ sg.z;
-      out[4 * il + 3] = __byte_perm(r0, r1, sel.y >> 16) ^ sg.w;
-    }
-  }
-};
-
-// ---- the other code-book formats (bit-identical to the standalone dequantize: one fp32 product, one rounding) ----
-// 8 values of an IQ2 entry whose three possible magnitudes are parked in r0, r1 (see Decoder<T_IQ2_XXS>)
-__device__ __forceinline__ void iq2_entry(uint2 sel, uint4 sg, uint32_t r0, uint32_t r1, uint32_t* out) {
-  out[0] = __byte_perm(r0, r1, sel.x) ^ sg.x;
-  out[1] = __byte_perm(r0, r1, sel.x >> 16) ^ sg.y;
-  out[2] = __byte_perm(r0, r1, sel.y) ^ sg.z;
-  out[3] = __byte_perm(r0, r1, sel.y >> 16) ^ sg.w;
-}
-template <typename ab_t> struct Decoder<T_IQ2_XS, ab_t> {   // half d | u16 qs[32] | u8 scales[8], 74 bytes
-  static constexpr bool CORR = false;
-  static constexpr int RW = 5;   // [0] d, [1..3] the group's 8 bytes (+ cover), [4] its scale byte
-  static __device__ __forceinline__ void load(const uint8_t* blk, int u, uint32_t (&raw)[RW]) {
-    ldg_cover<1>(blk, 2, raw);
-    ldg_cover<3>(blk + 2 + 8 * u, 8, raw + 1);
-    raw[4] = lds8(smem_u32(blk) + 66 + u);
-  }
-  static __device__ __forceinline__ void decode(const uint8_t* blk, int u, const uint32_t (&raw)[RW], const DecodeCtx& cx, uint32_t (&out)[16]) {
-    const float dh = __half2float(__ushort_as_half((unsigned short)((raw[0] >> shift_of(blk)) & 0xFFFFu)));
-    const uint32_t sh = shift_of(blk + 2 + 8 * u);
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const float d = dh * (0.5f + (float)((raw[4] >> (4 * h)) & 0xF)) * 0.25f;
-      const uint32_t r0 = pack2<ab_t>(d * 8.f, d * 25.f), r1 = pack2<ab_t>(d * 43.f, 0.f), q = word_at(raw + 1, h, sh);
-#pragma unroll
-      for (int l = 0; l < 2; ++l)
-        iq2_entry(grid64<T_IQ2_XS>(cx, (q >> (16 * l)) & 511u), sign_masks<T_IQ2_XS>(cx, (q >> (16 * l + 9)) & 127u), r0, r1, out + 8 * h + 4 * l);
-    }
-  }
-};
-template <typename ab_t> struct Decoder<T_IQ2_S, ab_t> {   // half d | u8 qs[32] | u8 signs[32] | u8 qh[8] | u8 scales[8], 82 bytes
-  static constexpr bool CORR = false;
-  static constexpr int RW = 7;
-  static __device__ __forceinline__ void load(const uint8_t* blk, int u, uint32_t (&raw)[RW]) {
-    ldg_cover<1>(blk, 2, raw);
-    ldg_cover<2>(blk + 2 + 4 * u, 4, raw + 1);
-    ldg_cover<2>(blk + 34 + 4 * u, 4, raw + 3);
-    raw[5] = lds8(smem_u32(blk) + 66 + u);
-    raw[6] = lds8(smem_u32(blk) + 74 + u);
-  }
-  static __device__ __forceinline__ void decode(const uint8_t* blk, int u, const uint32_t (&raw)[RW], const DecodeCtx& cx, uint32_t (&out)[16]) {
-    const float dh = __half2float(__ushort_as_half((unsigned short)((raw[0] >> shift_of(blk)) & 0xFFFFu)));
-    const uint32_t q = word_at(raw + 1, 0, shift_of(blk + 2 + 4 * u)), sg = word_at(raw + 3, 0, shift_of(blk + 34 + 4 * u));
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const float d = dh * (0.5f + (float)((raw[6] >> (4 * h)) & 0xF)) * 0.25f;
-      const uint32_t r0 = pack2<ab_t>(d * 8.f, d * 25.f), r1 = pack2<ab_t>(d * 43.f, 0.f);
-#pragma unroll
-      for (int l2 = 0; l2 < 2; ++l2) {
-        const int l = 2 * h + l2;
-        iq2_entry(grid64<T_IQ2_S>(cx, ((q >> (8 * l)) & 0xFFu) | ((raw[5] << (8 - 2 * l)) & 0x300u)), sign_masks<T_IQ2_S>(cx, (sg >> (8 * l)) & 0xFFu), r0,
-                  r1, out + 4 * l);
-      }
-    }
-  }
-};
-// 8 values of two IQ3 entries: magnitude bytes, scaled in fp32 (d * (2^23 + byte) - d * 2^23 is d * byte rounded once)
-template <typename ab_t> __device__ __forceinline__ void iq3_entries(uint32_t g0, uint32_t g1, uint4 sg, float d, float off, uint32_t* out) {
-  auto v = [&](uint32_t g, int k) { return fmaf(d, byte_2p23(g, k), off); };
-  out[0] = pack2<ab_t>(v(g0, 0), v(g0, 1)) ^ sg.x;
-  out[1] = pack2<ab_t>(v(g0, 2), v(g0, 3)) ^ sg.y;
-  out[2] = pack2<ab_t>(v(g1, 0), v(g1, 1)) ^ sg.z;
-  out[3] = pack2<ab_t>(v(g1, 2), v(g1, 3)) ^ sg.w;
-}
-template <typename ab_t> struct Decoder<T_IQ3_XXS, ab_t> {   // half d | u8 qs[64] | u32 scale_and_signs[8], 98 bytes
-  static constexpr bool CORR = false;
-  static constexpr int RW = 6;
-  static __device__ __forceinline__ void load(const uint8_t* blk, int u, uint32_t (&raw)[RW]) {
-    ldg_cover<1>(blk, 2, raw);
-    ldg_cover<3>(blk + 2 + 8 * u, 8, raw + 1);
-    ldg_cover<2>(blk + 66 + 4 * u, 4, raw + 4);
-  }
-  static __device__ __forceinline__ void decode(const uint8_t* blk, int u, const uint32_t (&raw)[RW], const DecodeCtx& cx, uint32_t (&out)[16]) {
-    const float dh = __half2float(__ushort_as_half((unsigned short)((raw[0] >> shift_of(blk)) & 0xFFFFu)));
-    const uint32_t sh = shift_of(blk + 2 + 8 * u), aux = word_at(raw + 4, 0, shift_of(blk + 66 + 4 * u));
-    const float d = dh * (0.5f + (float)(aux >> 28)) * 0.5f, off = -8388608.f * d;
-#pragma unroll
-    for (int l = 0; l < 4; ++l) {
-      const uint32_t e = word_at(raw + 1, l >> 1, sh) >> (16 * (l & 1));
-      iq3_entries<ab_t>(grid32<T_IQ3_XXS>(cx, e & 0xFFu), grid32<T_IQ3_XXS>(cx, (e >> 8) & 0xFFu), sign_masks<T_IQ3_XXS>(cx, (aux >> (7 * l)) & 127u), d,
-                        off, out + 4 * l);
-    }
-  }
-};
-template <typename ab_t> struct Decoder<T_IQ3_S, ab_t> {   // half d | u8 qs[64] | u8 qh[8] | u8 signs[32] | u8 scales[4], 110 bytes
-  static constexpr bool CORR = false;
-  static constexpr int RW = 8;
-  static __device__ __forceinline__ void load(const uint8_t* blk, int u, uint32_t (&raw)[RW]) {
-    ldg_cover<1>(blk, 2, raw);
-    ldg_cover<3>(blk + 2 + 8 * u, 8, raw + 1);
-    ldg_cover<2>(blk + 74 + 4 * u, 4, raw + 4);
-    raw[6] = lds8(smem_u32(blk) + 66 + u);
-    raw[7] = lds8(smem_u32(blk) + 106 + (u >> 1));
-  }
-  static __device__ __forceinline__ void decode(const uint8_t* blk, int u, const uint32_t (&raw)[RW], const DecodeCtx& cx, uint32_t (&out)[16]) {
-    const float dh = __half2float(__ushort_as_half((unsigned short)((raw[0] >> shift_of(blk)) & 0xFFFFu)));
-    const uint32_t sh = shift_of(blk + 2 + 8 * u), sg = word_at(raw + 4, 0, shift_of(blk + 74 + 4 * u));
-    const float d = dh * (0.5f + (float)((raw[7] >> (4 * (u & 1))) & 0xFu)) * 0.5f, off = -8388608.f * d;
-#pragma unroll
-    for (int l = 0; l < 4; ++l) {
-      const uint32_t e = word_at(raw + 1, l >> 1, sh) >> (16 * (l & 1));
-      iq3_entries<ab_t>(grid32<T_IQ3_S>(cx, (e & 0xFFu) | ((raw[6] << (8 - 2 * l)) & 256u)), grid32<T_IQ3_S>(cx, ((e >> 8) & 0xFFu) | ((raw[6] << (7 - 2 * l)) & 256u)),
-                        sign_masks<T_IQ3_S>(cx, (sg >> (8 * l)) & 0xFFu), d, off, out + 4 * l);
-    }
-  }
-};
 // 8 values of an IQ1 entry (codes 0, 1, 2 in nibbles: values 0-3 low, 4-7 high): the group has three possible values d * (code +
 // delta), rounded once each and parked in r0, r1; a pair is one byte-permute whose selector is its codes times 0x22 plus 0x1010
 __device__ __forceinline__ void iq1_entry(uint32_t g, uint32_t r0, uint32_t r1, uint32_t* out) {
@@ -993,7 +875,7 @@ template <typename ab_t> struct Item128<T_Q6_K, ab_t> {
     const uint32_t du = lds16(row + 208);
     s.d2 = u32_as_h2(du | (du << 16));
   }
-  template <int H> static __device__ __forceinline__ void stage(uint32_t row, int ip, bool wide, const State& s, uint32_t (&out)[32]) {
+  template <int H> static __device__ __forceinline__ void stage(uint32_t row, int ip, bool wide, const DecodeCtx&, const State& s, uint32_t (&out)[32]) {
     uint32_t l[8];
     lds_row_words<8>(row + 64 * ip + 32 * H, wide, l);
     __half2 sc[4], off[4];   // of the unit H, first and second 16 values, and of the unit H + 2
@@ -1011,6 +893,216 @@ template <typename ab_t> struct Item128<T_Q6_K, ab_t> {
       out[2 * w + 1] = h2_as_u32(hmul2_rn(s.d2, __hfma2(u32_as_h2(__byte_perm(c0, 0x5C5C5C5Cu, 0x4342)), sc[i], off[i])));
       out[16 + 2 * w] = h2_as_u32(hmul2_rn(s.d2, __hfma2(u32_as_h2(__byte_perm(c1, 0x5C5C5C5Cu, 0x4140)), sc[2 + i], off[2 + i])));
       out[16 + 2 * w + 1] = h2_as_u32(hmul2_rn(s.d2, __hfma2(u32_as_h2(__byte_perm(c1, 0x5C5C5C5Cu, 0x4342)), sc[2 + i], off[2 + i])));
+    }
+  }
+};
+
+__device__ __forceinline__ uint32_t byte_of(uint32_t w, int k) { return __byte_perm(w, 0u, 0x4440u | (uint32_t)k); }
+// byte K of w with byte K of `high`, 0 or 1, above it, in one permute (a selector with bit 3 set replicates that byte's sign: zero)
+template <int K> __device__ __forceinline__ uint32_t byte_of9(uint32_t w, uint32_t high) {
+  uint32_t r;
+  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(w), "r"(high), "n"(K | (4 + K) << 4 | (12 + K) << 8 | (12 + K) << 12));
+  return r;
+}
+__device__ __forceinline__ uint32_t spread_bits4(uint32_t b) { return ((b & 0xFu) * 0x00204081u) & 0x01010101u; }   // bit j -> bit 0 of byte j
+
+// ---- the IQ2 formats: value = +-round(d * magnitude), d = dh * (0.5 + s) * 0.25 in fp32, rounded once as in the reference (multiplying
+// by -1.f afterwards is exact, so flipping the sign bit is the same) ----
+template <typename ab_t> struct Iq2Group {   // the three possible magnitudes of a group, each rounded once
+  uint32_t r0, r1;
+  __device__ __forceinline__ void set(float dh, uint32_t s) {
+    const float d = dh * (0.5f + (float)s) * 0.25f;
+    r0 = pack2<ab_t>(d * 8.f, d * 25.f);
+    r1 = pack2<ab_t>(d * 43.f, 0.f);
+  }
+};
+template <typename ab_t> __device__ __forceinline__ void iq2_entry(const Iq2Group<ab_t>& g, uint4 sel, uint32_t word, uint32_t* out) {
+  out[0] = negate(__byte_perm(g.r0, g.r1, sel.x), sign_bits<0>(word));
+  out[1] = negate(__byte_perm(g.r0, g.r1, sel.y), sign_bits<1>(word));
+  out[2] = negate(__byte_perm(g.r0, g.r1, sel.z), sign_bits<2>(word));
+  out[3] = negate(__byte_perm(g.r0, g.r1, sel.w), sign_bits<3>(word));
+}
+template <typename ab_t> struct Item128<T_IQ2_XXS, ab_t> {   // half d | per 32 values: four grid bytes, four 7-bit sign indices and a 4-bit scale; 66 bytes
+  static constexpr bool HAVE = true;
+  struct State { uint32_t q[8]; float dh; };
+  static __device__ __forceinline__ void begin(uint32_t row, int ip, bool wide, State& s) {
+    lds_row_words<8>(row + 2 + 32 * ip, wide, s.q);
+    s.dh = lds_half_f32(row);
+  }
+  template <int H> static __device__ __forceinline__ void stage(uint32_t, int, bool, const DecodeCtx& cx, const State& s, uint32_t (&out)[32]) {
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const uint32_t idx = s.q[4 * H + 2 * u], aux = s.q[4 * H + 2 * u + 1];
+      Iq2Group<ab_t> g;
+      g.set(s.dh, aux >> 28);
+#pragma unroll
+      for (int l = 0; l < 4; ++l)
+        iq2_entry<ab_t>(g, grid128<T_IQ2_XXS>(cx, byte_of(idx, l)), sign_word(cx, (aux >> (7 * l)) & 127u), out + 16 * u + 4 * l);
+    }
+  }
+};
+template <typename ab_t> struct Item128<T_IQ2_XS, ab_t> {   // half d | u16 qs[32] | u8 scales[8], 74 bytes
+  static constexpr bool HAVE = true;
+  struct State { uint32_t q[8], sc; float dh; };
+  static __device__ __forceinline__ void begin(uint32_t row, int ip, bool wide, State& s) {
+    lds_row_words<8>(row + 2 + 32 * ip, wide, s.q);
+    uint32_t w[1];
+    lds_words_unaligned<1>(row + 66 + 4 * ip, w);
+    s.sc = w[0];
+    s.dh = lds_half_f32(row);
+  }
+  template <int H> static __device__ __forceinline__ void stage(uint32_t, int, bool, const DecodeCtx& cx, const State& s, uint32_t (&out)[32]) {
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {   // 16 values: a word of indices, half a byte of scales
+      const uint32_t q = s.q[4 * H + v];
+      Iq2Group<ab_t> g;
+      g.set(s.dh, (s.sc >> (16 * H + 4 * v)) & 0xFu);
+#pragma unroll
+      for (int l = 0; l < 2; ++l)
+        iq2_entry<ab_t>(g, grid128<T_IQ2_XS>(cx, (q >> (16 * l)) & 511u), sign_word(cx, (q >> (16 * l + 9)) & 127u), out + 8 * v + 4 * l);
+    }
+  }
+};
+template <typename ab_t> struct Item128<T_IQ2_S, ab_t> {   // half d | u8 qs[32] | u8 signs[32] | u8 qh[8] | u8 scales[8], 82 bytes
+  static constexpr bool HAVE = true;
+  struct State { uint32_t q[4], sg[4], qh, sc; float dh; };
+  static __device__ __forceinline__ void begin(uint32_t row, int ip, bool wide, State& s) {
+    lds_row_words<4>(row + 2 + 16 * ip, wide, s.q);
+    lds_row_words<4>(row + 34 + 16 * ip, wide, s.sg);
+    uint32_t w[1];
+    lds_words_unaligned<1>(row + 66 + 4 * ip, w);
+    s.qh = w[0];
+    lds_words_unaligned<1>(row + 74 + 4 * ip, w);
+    s.sc = w[0];
+    s.dh = lds_half_f32(row);
+  }
+  template <int H> static __device__ __forceinline__ void stage(uint32_t, int, bool, const DecodeCtx& cx, const State& s, uint32_t (&out)[32]) {
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const uint32_t q = s.q[2 * H + u], sg = s.sg[2 * H + u], qh = s.qh >> (16 * H + 8 * u);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        Iq2Group<ab_t> g;
+        g.set(s.dh, (s.sc >> (16 * H + 8 * u + 4 * h)) & 0xFu);
+#pragma unroll
+        for (int l2 = 0; l2 < 2; ++l2) {
+          const int l = 2 * h + l2;
+          const uint4 sel = grid128<T_IQ2_S>(cx, byte_of(q, l) | ((qh << (8 - 2 * l)) & 0x300u));
+          const uint32_t sb = byte_of(sg, l);
+          uint32_t* o = out + 16 * u + 4 * l;
+          o[0] = negate(__byte_perm(g.r0, g.r1, sel.x), sign_bits8<0>(sb));
+          o[1] = negate(__byte_perm(g.r0, g.r1, sel.y), sign_bits8<1>(sb));
+          o[2] = negate(__byte_perm(g.r0, g.r1, sel.z), sign_bits8<2>(sb));
+          o[3] = negate(__byte_perm(g.r0, g.r1, sel.w), sign_bits8<3>(sb));
+        }
+      }
+    }
+  }
+};
+
+// ---- the IQ3 formats: value = +-round(d * magnitude), d = dh * (0.5 + s) * 0.5 in fp32 (at most 16 significant bits) ----
+// (8192x28672, 300 tokens, bf16: 121.4 -> 112.5 us with the same plan, 165 -> about 100 shared-memory wavefronts a stage of 32 rows; the
+// IQ2 formats with their signs as above, IQ2_XXS 28672x8192, 128 tokens: 67.9 -> 61.8 us.)
+// Two 16-bit instructions a pair instead of two permutes, two fp32 multiply-adds and a conversion: d is the sum of two 16-bit
+// numbers, and fma(m, hi, m * lo) rounds the sum once.  Only m * lo is rounded before, by 2^-12 (bf16: 2^-9) of what is at
+// most half a unit in the last place of the result, so the result is the correctly rounded one but for sums that
+// close to the middle between two numbers.  For fp16 the magnitudes are held divided by 256 and d times 256, which keeps lo clear of the
+// subnormals; a d beyond that range (`big`) takes the fp32 form.
+template <typename ab_t> struct Iq3Group {
+  using V = typename std::conditional<std::is_same<ab_t, __half>::value, __half2, __nv_bfloat162>::type;
+  V hi, lo;
+  float d;
+  bool big;
+  __device__ __forceinline__ void set(float dh, uint32_t s) {
+    d = dh * (0.5f + (float)s) * 0.5f;
+    if constexpr (std::is_same<ab_t, __half>::value) {
+      d *= 256.f;
+      hi = __float2half2_rn(d);
+      lo = __float2half2_rn(d - __low2float(hi));
+      big = !(fabsf(d) < 60000.f);
+    } else {
+      hi = __float2bfloat162_rn(d);
+      lo = __float2bfloat162_rn(d - __low2float(hi));
+      big = !(fabsf(d) < 1e36f);
+    }
+  }
+  __device__ __forceinline__ uint32_t pair(uint32_t m) const {
+    const V v = *reinterpret_cast<const V*>(&m), r = __hfma2(v, hi, __hmul2_rn(v, lo));
+    return *reinterpret_cast<const uint32_t*>(&r);
+  }
+  __device__ __forceinline__ uint32_t pair32(uint32_t m) const {
+    const V v = *reinterpret_cast<const V*>(&m);
+    return pack2<ab_t>(d * __low2float(v), d * __high2float(v));
+  }
+};
+template <typename ab_t> struct Item128<T_IQ3_XXS, ab_t> {   // half d | u8 qs[64] | per 32 values four 7-bit sign indices and a 4-bit scale; 98 bytes
+  static constexpr bool HAVE = true;
+  struct State { uint32_t q[8], aux[4]; float dh; };
+  static __device__ __forceinline__ void begin(uint32_t row, int ip, bool wide, State& s) {
+    lds_row_words<8>(row + 2 + 32 * ip, wide, s.q);
+    lds_row_words<4>(row + 66 + 16 * ip, wide, s.aux);
+    s.dh = lds_half_f32(row);
+  }
+  template <int H> static __device__ __forceinline__ void stage(uint32_t, int, bool, const DecodeCtx& cx, const State& s, uint32_t (&out)[32]) {
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const uint32_t aux = s.aux[2 * H + u];
+      Iq3Group<ab_t> g;
+      g.set(s.dh, aux >> 28);
+      auto go = [&](auto value) {
+#pragma unroll
+        for (int l = 0; l < 4; ++l) {
+          const uint32_t w = s.q[4 * H + 2 * u + (l >> 1)], sw = sign_word(cx, (aux >> (7 * l)) & 127u);
+          const uint2 a = grid64<T_IQ3_XXS>(cx, byte_of(w, 2 * (l & 1))), b = grid64<T_IQ3_XXS>(cx, byte_of(w, 2 * (l & 1) + 1));
+          uint32_t* o = out + 16 * u + 4 * l;
+          o[0] = negate(value(a.x), sign_bits<0>(sw));
+          o[1] = negate(value(a.y), sign_bits<1>(sw));
+          o[2] = negate(value(b.x), sign_bits<2>(sw));
+          o[3] = negate(value(b.y), sign_bits<3>(sw));
+        }
+      };
+      if (!g.big) go([&](uint32_t m) { return g.pair(m); });
+      else go([&](uint32_t m) { return g.pair32(m); });
+    }
+  }
+};
+template <typename ab_t> struct Item128<T_IQ3_S, ab_t> {   // half d | u8 qs[64] | u8 qh[8] | u8 signs[32] | u8 scales[4], 110 bytes
+  static constexpr bool HAVE = true;
+  struct State { uint32_t q[8], sg[4], qh, sc; float dh; };
+  static __device__ __forceinline__ void begin(uint32_t row, int ip, bool wide, State& s) {
+    lds_row_words<8>(row + 2 + 32 * ip, wide, s.q);
+    lds_row_words<4>(row + 74 + 16 * ip, wide, s.sg);
+    uint32_t w[1];
+    lds_words_unaligned<1>(row + 66 + 4 * ip, w);
+    s.qh = w[0];
+    s.sc = lds16(row + 106 + 2 * ip);
+    s.dh = lds_half_f32(row);
+  }
+  template <int H> static __device__ __forceinline__ void stage(uint32_t, int, bool, const DecodeCtx& cx, const State& s, uint32_t (&out)[32]) {
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const uint32_t qh = s.qh >> (16 * H + 8 * u), sg = s.sg[2 * H + u];
+      Iq3Group<ab_t> g;
+      g.set(s.dh, (s.sc >> (8 * H + 4 * u)) & 0xFu);
+      auto go = [&](auto value) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {   // a word of indices: 16 values
+          const uint32_t w = s.q[4 * H + 2 * u + h], top = spread_bits4(qh >> (4 * h));
+          const uint2 e[4] = {grid64<T_IQ3_S>(cx, byte_of9<0>(w, top)), grid64<T_IQ3_S>(cx, byte_of9<1>(w, top)),
+                              grid64<T_IQ3_S>(cx, byte_of9<2>(w, top)), grid64<T_IQ3_S>(cx, byte_of9<3>(w, top))};
+#pragma unroll
+          for (int l = 0; l < 2; ++l) {
+            const uint32_t sb = byte_of(sg, 2 * h + l);
+            uint32_t* o = out + 16 * u + 8 * h + 4 * l;
+            o[0] = negate(value(e[2 * l].x), sign_bits8<0>(sb));
+            o[1] = negate(value(e[2 * l].y), sign_bits8<1>(sb));
+            o[2] = negate(value(e[2 * l + 1].x), sign_bits8<2>(sb));
+            o[3] = negate(value(e[2 * l + 1].y), sign_bits8<3>(sb));
+          }
+        }
+      };
+      if (!g.big) go([&](uint32_t m) { return g.pair(m); });
+      else go([&](uint32_t m) { return g.pair32(m); });
     }
   }
 };

@@ -323,7 +323,7 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_consta
     *gave_up = 0;
     fence_barrier_init();
   }
-  decoder_fill_tables<TYPE>(s_tab);
+  decoder_fill_tables<TYPE, ab_t>(s_tab);
   if (warp == MMQ_PRODUCER_WARPS) {
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
@@ -580,8 +580,8 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_consta
             const int s2 = 2 * half + h;      // 64-value stage of the chunk
             uint32_t v[32];
             if constexpr (Item::HAVE) {
-              if (h == 0) Item::template stage<0>(row_s, half, wide, state, v);
-              else Item::template stage<1>(row_s, half, wide, state, v);
+              if (h == 0) Item::template stage<0>(row_s, half, wide, cx, state, v);
+              else Item::template stage<1>(row_s, half, wide, cx, state, v);
             } else if constexpr (FAST) {
               Stage64<TYPE, ab_t>::decode(chunk, s2, v);
             } else {
