@@ -333,10 +333,9 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_consta
   tc_fence_after();
   constexpr uint32_t tmem_base = 0;   // (all 512 columns are this CTA's)
   pdl_trigger();   // the next kernel may become resident; it waits for this one before it touches anything
-  // What earlier kernels write: the activations (and the work list of a MoE step), and -- cleared, or read until now -- what the
-  // epilogue writes.  Everything else, decoding included, starts before they are done (the weights: see pdl_wait).
+  // What the kernel ahead writes: the activations, and -- cleared, or read until now -- what the epilogue writes.  Everything else, decoding
+  // included, starts before it is done (the weights: see pdl_wait; the work list of a MoE step is older than the quantizer's trigger).
   const bool moe = p.passes != nullptr;
-  if (moe) pdl_wait();
   const int tiles = moe ? __shfl_sync(0xffffffffu, *p.n_passes, 0) * p.rt : p.rt * p.tt;
   // Units: (tile, chunk) where CTAs share tiles, whole tiles where they do not -- there is no room for parts, or the last wave
   // of whole tiles idles for less than sharing costs.  Every CTA in use has an equal contiguous range of them.

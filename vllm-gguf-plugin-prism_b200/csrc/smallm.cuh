@@ -137,7 +137,9 @@ __global__ void __launch_bounds__(SM_THREADS, 2) smallm_kernel(const __grid_cons
   const bool moe = p.passes != nullptr;
   const bool producer = warp == SM_WARPS;
   pdl_trigger();   // the next kernel may become resident; it waits for this one before it touches anything
-  if (moe || !producer) pdl_wait();   // (the producer of a dense product first asks for weights: see pdl_wait)
+  // The producer asks for weights first.  (Those of a MoE step too: the quantizer ahead let this kernel start when its own wait was
+  // over, and the passes are older than that.  A step of eight tokens over 64 experts of Q4_0: 66.6 -> 61.6 us.)
+  if (!producer) pdl_wait();
   // units: chunk by chunk, row tile by row tile, pass by pass; CTA i owns the units [i * U / G, (i + 1) * U / G)
   // (the host sees to it that U * G fits 31 bits: everything here is 32-bit arithmetic, and divisions are few -- a 64-bit
   // division costs as much as a block of the product)
@@ -172,7 +174,7 @@ __global__ void __launch_bounds__(SM_THREADS, 2) smallm_kernel(const __grid_cons
     Cursor held = cur;        // first unit whose activations have not been asked for
     int n_held = 0, st = 0;
     uint32_t ph = 0;
-    bool waited = moe;
+    bool waited = false;
     auto release = [&]() {    // the activations exist now
       pdl_wait();
       waited = true;
