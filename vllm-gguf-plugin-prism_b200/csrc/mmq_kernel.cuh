@@ -176,33 +176,55 @@ __device__ __forceinline__ void tp_finish(unsigned* epoch, unsigned* const* flag
   }
 }
 
-// A CTA's work: the units (tile, chunk) [u0, u1) in parts of one tile each.  Every role of the CTA walks the same parts.
+// A CTA's work: a range of units (tile, chunk) in parts of one tile each.  Every role of the CTA walks the same parts.
 struct MmqPart {
-  int u, u1;                 // next unit, end
-  int tile, c0, c1;          // chunks [c0, c1) of the tile
+  int left;                  // units behind this part
+  int tile, outer, inner;    // tile = outer * (row tiles of a pass, or token tiles of a row tile) + inner
+  int c0, c1;                // chunks [c0, c1) of the tile
 };
 struct MmqTile {
   int n0;                    // first row
   int x0, rows;              // first activation row, rows that count
   int row0;                  // MoE: first row of the expert's matrix among all rows
 };
-__device__ __forceinline__ MmqTile mmq_tile(const MmqParams& p, int tile) {
+__device__ __forceinline__ MmqTile mmq_tile(const MmqParams& p, const MmqPart& q) {
   MmqTile t;
   if (p.passes) {
-    const int ps = (int)((unsigned)tile / (unsigned)p.rt);
-    const int4 info = p.passes[ps];
-    t.n0 = (tile - ps * p.rt) * MMQ_ROWS;
+    const int4 info = p.passes[q.outer];
+    t.n0 = q.inner * MMQ_ROWS;
     t.row0 = info.x * p.n;
     t.x0 = info.y;
     t.rows = info.z;
-  } else {
-    const int r = (int)((unsigned)tile / (unsigned)p.tt);   // token tiles of a row tile are neighbours: they share its weights in L2
-    t.n0 = r * MMQ_ROWS;
+  } else {   // token tiles of a row tile are neighbours: they share its weights in L2
+    t.n0 = q.outer * MMQ_ROWS;
     t.row0 = 0;
-    t.x0 = (tile - r * p.tt) * p.tn;
+    t.x0 = q.inner * p.tn;
     t.rows = p.m - t.x0 < p.tn ? p.m - t.x0 : p.tn;
   }
   return t;
+}
+// The units from u on, `units` of them, before the first part.  (The only divisions: a part behind another begins a tile.)
+__device__ __forceinline__ MmqPart mmq_parts(const MmqParams& p, int u, int units) {
+  const int d = p.passes ? p.rt : p.tt;
+  MmqPart q;
+  q.left = units;
+  q.tile = (int)((unsigned)u / (unsigned)p.nc);
+  q.c0 = u - q.tile * p.nc;
+  q.outer = (int)((unsigned)q.tile / (unsigned)d);
+  q.inner = q.tile - q.outer * d;
+  q.c1 = -1;                 // (no part yet)
+  return q;
+}
+__device__ __forceinline__ bool mmq_next_part(const MmqParams& p, MmqPart& q) {
+  if (q.left <= 0) return false;
+  if (q.c1 >= 0) {
+    ++q.tile;
+    if (++q.inner == (p.passes ? p.rt : p.tt)) { q.inner = 0; ++q.outer; }
+    q.c0 = 0;
+  }
+  q.c1 = q.left < p.nc - q.c0 ? q.c0 + q.left : p.nc;
+  q.left -= q.c1 - q.c0;
+  return true;
 }
 // The stages of a part come in blocks: four per chunk, and behind every run of chunks with the same c / 4 half a stage of their
 // correction columns (formats without them: one block).  End of the block that starts at chunk c:
@@ -210,15 +232,6 @@ __device__ __forceinline__ int mmq_block_end(const MmqParams& p, const MmqPart& 
   const int e = (c | (MMQ_CORR_CHUNKS - 1)) + 1;
   return p.corr && e < q.c1 ? e : q.c1;
 }
-__device__ __forceinline__ bool mmq_next_part(const MmqParams& p, MmqPart& q) {
-  if (q.u >= q.u1) return false;
-  q.tile = (int)((unsigned)q.u / (unsigned)p.nc);
-  q.c0 = q.u - q.tile * p.nc;
-  q.c1 = q.u1 - q.u < p.nc - q.c0 ? q.c0 + (q.u1 - q.u) : p.nc;
-  q.u += q.c1 - q.c0;
-  return true;
-}
-
 template <typename I, bool HAVE = I::HAVE> struct ItemStateOf { struct type {}; };
 template <typename I> struct ItemStateOf<I, true> { using type = typename I::State; };
 template <typename I> using ItemState = typename ItemStateOf<I>::type;
@@ -342,14 +355,10 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_consta
   const int rest = tiles % (int)gridDim.x;
   const bool split = p.part && rest != 0 && (unsigned)p.nc * (unsigned)((int)gridDim.x - rest) > (unsigned)p.waste * gridDim.x;
   const int U = split ? tiles * p.nc : tiles, G = U < (int)gridDim.x ? U : (int)gridDim.x;
-  MmqPart q{};
-  const int cta = (int)blockIdx.x;
-  {
-    const int scale = split ? 1 : p.nc;
-    q.u = cta < G ? (int)((unsigned)(cta * U) / (unsigned)G) * scale : 0;
-    q.u1 = cta < G ? (int)((unsigned)((cta + 1) * U) / (unsigned)G) * scale : 0;
-  }
-  const int first_tile = (int)((unsigned)q.u / (unsigned)p.nc);
+  const int cta = (int)blockIdx.x, scale = split ? 1 : p.nc;
+  const int u0 = cta < G ? (int)((unsigned)(cta * U) / (unsigned)G) * scale : 0;
+  MmqPart q = mmq_parts(p, u0, cta < G ? (int)((unsigned)((cta + 1) * U) / (unsigned)G) * scale - u0 : 0);
+  const int first_tile = q.tile;
   const uint32_t bars_s = smem_u32(bars), gave_up_s = smem_u32(const_cast<const int*>(gave_up));
   auto bar = [&](int k) { return bars_s + 8u * (uint32_t)k; };   // (the numbers are those of the list above)
   const int half_n = p.tn > 256 ? p.tn / 2 : 0;   // tokens of one instruction and of one activation box, where a tile takes two
@@ -380,7 +389,7 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_consta
     // instead of 4,000, most of them for the first time through).  FINISH: the parts of e's tile are all in memory.
     enum : int { MORE, FINAL, FINISH };
     auto epilogue = [&](const MmqPart& e, int pi, int mode) {
-      const MmqTile et = mmq_tile(p, e.tile);
+      const MmqTile et = mmq_tile(p, e);
       const int buf = p.nbuf == 2 ? pi & 1 : 0, use = p.nbuf == 2 ? pi >> 1 : pi;
       const int n = et.n0 + r, nb = p.tn / 16;
       const bool live = n < p.n;
@@ -503,17 +512,33 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_consta
               h[7] >>= 16;
             }
           }
-        } else if (plain) {
-          uint16_t* y = static_cast<uint16_t*>(p.y) + n;
+        } else if (plain) {   // rows of their own: lane j of each sixteen has the number and the weight of row j
+          uint32_t h[8];
+          if (p.dtype == DT_F16) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) h[j] = pack2<__half>(__uint_as_float(acc[2 * j]), __uint_as_float(acc[2 * j + 1]));
+          } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) h[j] = pack2<__nv_bfloat16>(__uint_as_float(acc[2 * j]), __uint_as_float(acc[2 * j + 1]));
+          }
+          if (p.row_scale) {   // applied as the reference applies it: to the rounded value, rounded again
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              const float s0 = __shfl_sync(0xffffffffu, scale, 2 * j), s1 = __shfl_sync(0xffffffffu, scale, 2 * j + 1);
+              if (p.dtype == DT_F16) {
+                const float2 f = __half22float2(u32_as_h2(h[j]));
+                h[j] = pack2<__half>(f.x * s0, f.y * s1);
+              } else {
+                h[j] = pack2<__nv_bfloat16>(__uint_as_float(h[j] << 16) * s0, __uint_as_float(h[j] & 0xFFFF0000u) * s1);
+              }
+            }
+          }
+          uint8_t* y = static_cast<uint8_t*>(p.y) + 2 * (int64_t)n;
+          const uint32_t pitch = 2u * (uint32_t)p.ldy;
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
             const int o = __shfl_sync(0xffffffffu, orow, j);
-            uint16_t v = mmq_bits16(p.dtype, __uint_as_float(acc[j]));
-            if (p.row_scale) {   // applied as the reference applies it: to the rounded value, rounded again
-              const float f = p.dtype == DT_F16 ? __half2float(__ushort_as_half(v)) : __bfloat162float(__ushort_as_bfloat16(v));
-              v = mmq_bits16(p.dtype, f * __shfl_sync(0xffffffffu, scale, j));
-            }
-            if (live && o >= 0) y[(int64_t)o * p.ldy] = v;
+            if (live && o >= 0) *reinterpret_cast<uint16_t*>(y + (uint64_t)(uint32_t)o * pitch) = (uint16_t)(j & 1 ? h[j >> 1] >> 16 : h[j >> 1]);
           }
         } else if constexpr (TP) {
           mmq_store_peers(p, et.x0 + 16 * b, et.rows - 16 * b, n, live, acc, lane);
@@ -552,7 +577,7 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_consta
     for (;;) {
       const bool more = mode == MORE && mmq_next_part(p, q);
       if (!more && mode == MORE) mode = FINAL;
-      const MmqTile qt = mmq_tile(p, q.tile);
+      const MmqTile qt = mmq_tile(p, q);
       const int n = qt.n0 + r;
       const uint8_t* slot = sRaw + raw_slot(p.raw, r, qt.n0);
       const int items = more ? 2 * (q.c1 - q.c0) : 0;
@@ -678,7 +703,7 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_consta
     uint32_t ph = 0;
     pdl_wait();
     while (mmq_next_part(p, q)) {
-      const int x0 = mmq_tile(p, q.tile).x0;
+      const int x0 = mmq_tile(p, q).x0;
       for (int cs = q.c0, ce; cs < q.c1; cs = ce, ++blk) {
         ce = mmq_block_end(p, q, cs);
         const int n = 2 * (ce - cs) * (p.bg == 2 ? 1 : 2);
@@ -706,7 +731,7 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_consta
     int st = 0;
     uint32_t sph = 0;
     while (ok && mmq_next_part(p, q)) {
-      const MmqTile qt = mmq_tile(p, q.tile);
+      const MmqTile qt = mmq_tile(p, q);
       for (int c = q.c0; c < q.c1; ++c) {
         mbar_wait_or(bar(36 + st), sph ^ 1u, gave_up_s);
         if (lds32(gave_up_s) != 0u) { ok = false; break; }
