@@ -1070,3 +1070,35 @@ def test_tiled_blocks_of_corrections_cut_anywhere(name, shape):
     assert capi.last_status() == 0
     assert rel_l2(y.float().cpu(), want.cpu()) <= REL_L2_TOL
     assert torch.equal(y, capi.mul_mat_a8(w, x, t, N))
+
+
+@pytest.mark.parametrize("name", ["Q4_K", "Q6_K", "Q8_0"])
+def test_tiled_activations_of_every_value(name):
+    """The activation matrix of the tiled product: ties, zeros of both signs, subnormal blocks and NaN give what the q8_1 records say
+    (a NaN counts as zero), in every order the formats want."""
+    t, K, M = TYPES[name], 512, 40
+    _, w = dev_w(t, 512, K, seed=1)
+    x = dev_x(M, K, seed=2, dtype=torch.float32)
+    x[0, :64] = torch.arange(64, device=DEV) - 31.5           # ties: amax 32 and steps of 0.5
+    x[1, :32] = 0.0
+    x[2, :32] = -0.0
+    x[3, :32] = 1e-39                                          # d underflows
+    x[4, 5] = float("nan")
+    x[5, :] = 127.0
+    x[5, ::2] = 0.5                                            # halfway between codes 0 and 1
+    y = capi.mul_mat_a8(w, x, t, 512)
+    blocks = capi.quantize_q8_1(x).view(M, -1, 36)[:, :K // 32].contiguous()
+    d = blocks[..., :2].contiguous().view(torch.float16).double()
+    xq = (blocks[..., 4:].contiguous().view(torch.int8).double() * d).half().double().reshape(M, K)
+    wd = capi.dequantize(w, t, 512, K, torch.float32).double()
+    want = xq @ wd.T
+    torch.cuda.synchronize()
+    assert capi.last_status() == 0
+    keep = torch.ones(M, dtype=torch.bool, device=DEV)
+    if name == "Q4_K":   # its minima meet the sums of the unquantized values: not a number in row 4, another value elsewhere
+        keep[4] = False
+        want = torch.cat([capi.mul_mat_vec_a8(w, x[i:i + 16].contiguous(), t, 512) for i in range(0, M, 16)]).double()
+    assert torch.isfinite(y[keep]).all()
+    assert rel_l2(y[keep].cpu(), want[keep].float().cpu()) <= REL_L2_TOL
+    for i in (0, 5):
+        assert rel_l2(y[i].cpu(), want[i].float().cpu()) <= REL_L2_TOL
