@@ -2,7 +2,7 @@
 // eight 32-value blocks) of each of 128 consecutive rows.  Shared by the kernels that walk 128-row
 // tiles.  Three forms, chosen per matrix by plan_raw():
 //
-//   dense   row pitch and chunk size multiples of 16 bytes: one 2-D TMA box per stage, rows back to back
+//   dense   row pitch and chunk size multiples of 16 bytes: one 2-D TMA box per stage, rows an odd number of 16-byte units apart
 //   class   anything else (rows of 210, 110, 66 ... bytes): P = 16 / gcd(16, pitch) alignment classes.
 //           The tensor map views the matrix as rows of P weight rows (P * pitch IS a multiple of 16), so
 //           the rows of one class share the remainder of their chunk starts modulo 16 and ONE box per
@@ -12,7 +12,7 @@
 //   rows    one bulk copy per row (a copy costs about 90 clocks of the SM's copy engine: only for
 //           matrices that the other two cannot describe)
 //
-// Slots are an odd number of 16-byte units where the format allows it, so that eight rows read at
+// Slots are an odd number of 16-byte units, so that eight rows read at
 // the same offset fall into different banks.  Nothing is read past the caller's buffer.
 #pragma once
 
