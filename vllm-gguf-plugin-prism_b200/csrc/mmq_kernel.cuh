@@ -564,7 +564,7 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_consta
 
     // Item i is half i & 1 of the i / 2-th chunk of the CTA, so a group has the same half, slot and barriers all its life.
     const int half = g & 1;
-    const bool wide = p.raw.mode == 2 && p.raw.cl2 == 0;           // rows of one remainder modulo 16
+    const bool wide = p.raw.mode == 1 || (p.raw.mode == 2 && p.raw.cl2 == 0);   // rows of one remainder modulo 16
     const uint32_t slot_free = bar(4 + ((g - p.sa) & 3));          // `empty` of the item that had the slot before
     uint32_t free_ph = g >= p.sa ? 0u : 1u;                        // (1 at first: the slot has never been used)
     int a_slot = g >= p.sa ? g - p.sa : g;                         // (four items on: the next slot of three, the same of two or four)
@@ -598,7 +598,7 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_consta
           using Item = Item128<TYPE, ab_t>;
           ItemState<Item> state;
           const uint32_t row_s = smem_u32(chunk);
-          if constexpr (Item::HAVE) Item::begin(row_s, half, wide, state);
+          if constexpr (Item::HAVE) Item::begin(row_s, half, wide, nunits - 8 * c - 4 * half, state);
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             const int s2 = 2 * half + h;      // 64-value stage of the chunk
