@@ -25,7 +25,6 @@ namespace gguf_b200 {
 
 constexpr int G1_WARPS = 8;
 constexpr int G1_BATCH = 32;   // row iterations between two flushes of the slice partials
-constexpr int G1_TAB_COPIES = 16;   // bank-conflict-free copies of the IQ2_XXS code books (see the kernel)
 
 __device__ __forceinline__ __half2 u32_as_half2(uint32_t u) { return *reinterpret_cast<__half2*>(&u); }
 __device__ __forceinline__ int dp4a_us1(uint32_t a, uint32_t b, int c) {
@@ -83,6 +82,52 @@ struct Tab1 {
 };
 
 // Per type: UPB units per block, XW activation words and XD floats held per unit.
+// Code books in shared memory: GRID entries of GB bytes in GC copies, then SGN sign masks (eight bytes: all ones where the value is
+// negative) in SC copies.  Copy c of an entry lies in column c of its line, and lane l reads copy l modulo their number: the lanes
+// that are served together then sit in different banks whatever entries they ask for, or all but (32 unrelated entries of one copy
+// conflict three- to fourfold on almost every look-up).  48 KB of tables leave two CTAs on an SM.
+template <int TYPE> struct G1Tab { static constexpr int GRID = 0, GB = 0, GC = 0, SGN = 0, SC = 0; };
+template <> struct G1Tab<T_IQ2_XXS> { static constexpr int GRID = 256, GB = 8, GC = 16, SGN = 128, SC = 16; };
+template <> struct G1Tab<T_IQ2_XS> { static constexpr int GRID = 512, GB = 8, GC = 8, SGN = 128, SC = 16; };
+template <> struct G1Tab<T_IQ2_S> { static constexpr int GRID = 1024, GB = 8, GC = 4, SGN = 256, SC = 8; };
+template <> struct G1Tab<T_IQ3_XXS> { static constexpr int GRID = 256, GB = 4, GC = 32, SGN = 128, SC = 16; };
+template <> struct G1Tab<T_IQ3_S> { static constexpr int GRID = 512, GB = 4, GC = 16, SGN = 256, SC = 8; };
+template <int TYPE> __host__ __device__ constexpr int g1_grid_bytes() { return G1Tab<TYPE>::GRID * G1Tab<TYPE>::GB * G1Tab<TYPE>::GC; }
+template <int TYPE> __host__ __device__ constexpr int g1_tab_bytes() { return g1_grid_bytes<TYPE>() + G1Tab<TYPE>::SGN * 8 * G1Tab<TYPE>::SC; }
+template <int TYPE> __device__ __forceinline__ uint2 g1_grid64(const Tab1& t, uint32_t i) { return pl64(t.grid + i * (uint32_t)(8 * G1Tab<TYPE>::GC)); }
+template <int TYPE> __device__ __forceinline__ uint32_t g1_grid32(const Tab1& t, uint32_t i) { return pl32(t.grid + i * (uint32_t)(4 * G1Tab<TYPE>::GC)); }
+template <int TYPE> __device__ __forceinline__ uint2 g1_signs(const Tab1& t, uint32_t i) { return pl64(t.smask + i * (uint32_t)(8 * G1Tab<TYPE>::SC)); }
+// Eight magnitudes g times eight activations into sp, and those of the negative values into sn: the signed sum is sp - 2 sn, exactly.
+__device__ __forceinline__ void g1_dot8(uint32_t g0, uint32_t g1, uint2 m, uint32_t x0, uint32_t x1, int& sp, int& sn) {
+  sp = dp4a_us1(g0, x0, sp);
+  sp = dp4a_us1(g1, x1, sp);
+  sn = dp4a_us1(g0 & m.x, x0, sn);
+  sn = dp4a_us1(g1 & m.y, x1, sn);
+}
+template <int TYPE> __device__ __forceinline__ void g1_fill_tables(uint8_t* tab) {
+  using D = G1Tab<TYPE>;
+  for (int i = threadIdx.x; i < D::GRID * D::GC; i += blockDim.x) {
+    const int e = i / D::GC;
+    if constexpr (D::GB == 8) {
+      const uint64_t v = TYPE == T_IQ2_XXS ? d_iq2xxs_grid[e & 255] : TYPE == T_IQ2_XS ? d_iq2xs_grid[e & 511] : d_iq2s_grid[e & 1023];
+      reinterpret_cast<uint2*>(tab)[i] = make_uint2((uint32_t)v, (uint32_t)(v >> 32));
+    } else {
+      reinterpret_cast<uint32_t*>(tab)[i] = TYPE == T_IQ3_XXS ? d_iq3xxs_grid[e & 255] : d_iq3s_grid[e & 511];
+    }
+  }
+  uint2* sgn = reinterpret_cast<uint2*>(tab + g1_grid_bytes<TYPE>());
+  for (int i = threadIdx.x; i < D::SGN * D::SC; i += blockDim.x) {
+    const uint32_t e = (uint32_t)(i / D::SC), b = D::SGN == 128 ? (uint32_t)d_ksigns_iq2xs[e & 127u] : e;
+    uint32_t lo = 0, hi = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      lo |= ((b >> j) & 1u) ? (0xFFu << (8 * j)) : 0u;
+      hi |= ((b >> (4 + j)) & 1u) ? (0xFFu << (8 * j)) : 0u;
+    }
+    sgn[i] = make_uint2(lo, hi);
+  }
+}
+
 template <int TYPE> struct G1;
 
 // ---- Q8_0: unit = block of 32 -----------------------------------------------------------
@@ -281,35 +326,22 @@ template <> struct G1<T_IQ2_XXS> {
     int sp = 0, sn = 0;
 #pragma unroll
     for (int il = 0; il < 4; ++il) {
-      const uint2 gr = pl64(t.grid + ((q[0] >> (8 * il)) & 0xFF) * (8 * G1_TAB_COPIES));     // this lane's copy of the entry
-      const uint2 sm = pl64(t.smask + ((aux >> (7 * il)) & 127) * (8 * G1_TAB_COPIES));
-      sp = dp4a_us1(gr.x, x[2 * il], sp);
-      sp = dp4a_us1(gr.y, x[2 * il + 1], sp);
-      sn = dp4a_us1(gr.x & sm.x, x[2 * il], sn);
-      sn = dp4a_us1(gr.y & sm.y, x[2 * il + 1], sn);
+      const uint2 gr = g1_grid64<T_IQ2_XXS>(t, (q[0] >> (8 * il)) & 0xFF);
+      g1_dot8(gr.x, gr.y, g1_signs<T_IQ2_XXS>(t, (aux >> (7 * il)) & 127), x[2 * il], x[2 * il + 1], sp, sn);
     }
     return d * (0.5f + (float)(aux >> 28)) * 0.25f * xd[0] * (float)(sp - 2 * sn);
   }
 };
 
 // ---- the other code-book types: IQ2_XS, IQ2_S, IQ3_XXS, IQ3_S, IQ1_S, IQ1_M ---------------------
-// unit ib = 32 values (one q8_1 block).  Their code books (1 to 8 KB each) are read from global
-// memory through the read-only path, as the reference's vec_dot_iq*_q8_1 do (vecdotq.cuh:1554-1750):
-// these formats trade arithmetic for size and are bound by the look-ups, not by the weight stream.
+// unit ib = 32 values (one q8_1 block; vecdotq.cuh:1554-1750).  The IQ2 and IQ3 books are in shared memory like IQ2_XXS's, with the signs as
+// masks beside them; those of IQ1 (8 KB) are read from global memory through the read-only path.  (All of them that way, with the
+// masks computed and byte-wise negations: 14336x4096, one vector: IQ2_XS
+// 19.3 -> 12.5 us, IQ2_S 19.6 -> 16.0, IQ3_XXS 21.8 -> 14.0, IQ3_S 22.4 -> 16.1; 3072x1024: 6.5 -> 4.7, 6.7 -> 4.7, 6.8 -> 5.7, 7.5 -> 5.3.)
 __device__ __forceinline__ uint32_t pl8(uint32_t a) {
   uint32_t v;
   asm("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(a));
   return v;
-}
-// bit j of a nibble -> byte j of a word all ones (the reference's __vcmpeq4 form, vecdotq.cuh:1598-1599)
-__device__ __forceinline__ uint32_t sign_mask4(uint32_t nib) { return __vcmpeq4(((nib & 0xfu) * 0x01010101u) & 0x08040201u, 0x08040201u); }
-// seven sign bits + the eighth that makes the parity even (the ksigns_iq2xs table, computed)
-__device__ __forceinline__ uint32_t signs_from7(uint32_t s7) { return s7 | ((__popc(s7) & 1u) << 7); }
-// dot product of eight signed code-book magnitudes (two words, sign bit j = value j negative) with eight int8 activations
-__device__ __forceinline__ int dot8_signed(uint32_t g0, uint32_t g1, uint32_t signs, uint32_t x0, uint32_t x1, int acc) {
-  const uint32_t m0 = sign_mask4(signs), m1 = sign_mask4(signs >> 4);
-  acc = __dp4a((int)__vsub4(g0 ^ m0, m0), (int)x0, acc);
-  return __dp4a((int)__vsub4(g1 ^ m1, m1), (int)x1, acc);
 }
 
 template <> struct G1<T_IQ2_XS> {   // half d | u16 qs[32] | u8 scales[8]   (vecdotq.cuh:1554-1583)
@@ -317,19 +349,19 @@ template <> struct G1<T_IQ2_XS> {   // half d | u16 qs[32] | u8 scales[8]   (vec
   static __device__ __forceinline__ void load_x(const uint8_t* qs, const float2* ds, int u, int b, uint32_t (&x)[XW], float (&xd)[XD]) {
     G1<T_Q8_0>::load_x(qs, ds, u, b, x, xd);
   }
-  static __device__ __forceinline__ float unit(uint32_t blk, int ib, const uint32_t (&x)[XW], const float (&xd)[XD], const Tab1&) {
+  static __device__ __forceinline__ float unit(uint32_t blk, int ib, const uint32_t (&x)[XW], const float (&xd)[XD], const Tab1& t) {
     const float d = plh(blk);
     uint32_t q[2];
     lds_a2<2>(blk + 2 + 8 * ib, q);
     const uint32_t sc = pl8(blk + 66 + ib);
-    int s1 = 0, s2 = 0;
+    int s1 = 0, s2 = 0, n1 = 0, n2 = 0;
 #pragma unroll
     for (int l = 0; l < 4; ++l) {
-      const uint32_t idx = (q[l >> 1] >> (16 * (l & 1))) & 0xFFFFu;
-      const uint64_t g = __ldg(&d_iq2xs_grid[idx & 511]);
-      const int v = dot8_signed((uint32_t)g, (uint32_t)(g >> 32), signs_from7(idx >> 9), x[2 * l], x[2 * l + 1], 0);
-      if (l < 2) s1 += v; else s2 += v;
+      const uint2 g = g1_grid64<T_IQ2_XS>(t, (q[l >> 1] >> (16 * (l & 1))) & 511u);
+      g1_dot8(g.x, g.y, g1_signs<T_IQ2_XS>(t, (q[l >> 1] >> (16 * (l & 1) + 9)) & 127u), x[2 * l], x[2 * l + 1], l < 2 ? s1 : s2, l < 2 ? n1 : n2);
     }
+    s1 -= 2 * n1;
+    s2 -= 2 * n2;
     return d * xd[0] * 0.25f * ((0.5f + (float)(sc & 0xf)) * (float)s1 + (0.5f + (float)(sc >> 4)) * (float)s2);
   }
 };
@@ -339,19 +371,20 @@ template <> struct G1<T_IQ2_S> {   // half d | u8 qs[32] | u8 signs[32] | u8 qh[
   static __device__ __forceinline__ void load_x(const uint8_t* qs, const float2* ds, int u, int b, uint32_t (&x)[XW], float (&xd)[XD]) {
     G1<T_Q8_0>::load_x(qs, ds, u, b, x, xd);
   }
-  static __device__ __forceinline__ float unit(uint32_t blk, int ib, const uint32_t (&x)[XW], const float (&xd)[XD], const Tab1&) {
+  static __device__ __forceinline__ float unit(uint32_t blk, int ib, const uint32_t (&x)[XW], const float (&xd)[XD], const Tab1& t) {
     const float d = plh(blk);
     uint32_t q[1], sg[1];
     lds_a2<1>(blk + 2 + 4 * ib, q);
     lds_a2<1>(blk + 34 + 4 * ib, sg);
     const uint32_t qh = pl8(blk + 66 + ib), sc = pl8(blk + 74 + ib);
-    int s1 = 0, s2 = 0;
+    int s1 = 0, s2 = 0, n1 = 0, n2 = 0;
 #pragma unroll
     for (int l = 0; l < 4; ++l) {
-      const uint64_t g = __ldg(&d_iq2s_grid[((q[0] >> (8 * l)) & 0xFF) | ((qh << (8 - 2 * l)) & 0x300)]);
-      const int v = dot8_signed((uint32_t)g, (uint32_t)(g >> 32), (sg[0] >> (8 * l)) & 0xFF, x[2 * l], x[2 * l + 1], 0);
-      if (l < 2) s1 += v; else s2 += v;
+      const uint2 g = g1_grid64<T_IQ2_S>(t, ((q[0] >> (8 * l)) & 0xFF) | ((qh << (8 - 2 * l)) & 0x300));
+      g1_dot8(g.x, g.y, g1_signs<T_IQ2_S>(t, (sg[0] >> (8 * l)) & 0xFF), x[2 * l], x[2 * l + 1], l < 2 ? s1 : s2, l < 2 ? n1 : n2);
     }
+    s1 -= 2 * n1;
+    s2 -= 2 * n2;
     return d * xd[0] * 0.25f * ((0.5f + (float)(sc & 0xf)) * (float)s1 + (0.5f + (float)(sc >> 4)) * (float)s2);
   }
 };
@@ -361,20 +394,20 @@ template <> struct G1<T_IQ3_XXS> {   // half d | u8 qs[64] | u32 scale_and_signs
   static __device__ __forceinline__ void load_x(const uint8_t* qs, const float2* ds, int u, int b, uint32_t (&x)[XW], float (&xd)[XD]) {
     G1<T_Q8_0>::load_x(qs, ds, u, b, x, xd);
   }
-  static __device__ __forceinline__ float unit(uint32_t blk, int ib, const uint32_t (&x)[XW], const float (&xd)[XD], const Tab1&) {
+  static __device__ __forceinline__ float unit(uint32_t blk, int ib, const uint32_t (&x)[XW], const float (&xd)[XD], const Tab1& t) {
     const float d = plh(blk);
     uint32_t q[2], a[1];
     lds_a2<2>(blk + 2 + 8 * ib, q);
     lds_a2<1>(blk + 66 + 4 * ib, a);
     const uint32_t aux = a[0];
-    int s = 0;
+    int s = 0, n = 0;
 #pragma unroll
     for (int l = 0; l < 4; ++l) {
       const uint32_t w = q[l >> 1] >> (16 * (l & 1));
-      const uint32_t g0 = __ldg(&d_iq3xxs_grid[w & 0xFF]), g1 = __ldg(&d_iq3xxs_grid[(w >> 8) & 0xFF]);
-      s = dot8_signed(g0, g1, signs_from7((aux >> (7 * l)) & 127), x[2 * l], x[2 * l + 1], s);
+      g1_dot8(g1_grid32<T_IQ3_XXS>(t, w & 0xFF), g1_grid32<T_IQ3_XXS>(t, (w >> 8) & 0xFF), g1_signs<T_IQ3_XXS>(t, (aux >> (7 * l)) & 127), x[2 * l],
+              x[2 * l + 1], s, n);
     }
-    return d * (0.5f + (float)(aux >> 28)) * xd[0] * 0.5f * (float)s;
+    return d * (0.5f + (float)(aux >> 28)) * xd[0] * 0.5f * (float)(s - 2 * n);
   }
 };
 
@@ -383,22 +416,21 @@ template <> struct G1<T_IQ3_S> {   // half d | u8 qs[64] | u8 qh[8] | u8 signs[3
   static __device__ __forceinline__ void load_x(const uint8_t* qs, const float2* ds, int u, int b, uint32_t (&x)[XW], float (&xd)[XD]) {
     G1<T_Q8_0>::load_x(qs, ds, u, b, x, xd);
   }
-  static __device__ __forceinline__ float unit(uint32_t blk, int ib, const uint32_t (&x)[XW], const float (&xd)[XD], const Tab1&) {
+  static __device__ __forceinline__ float unit(uint32_t blk, int ib, const uint32_t (&x)[XW], const float (&xd)[XD], const Tab1& t) {
     const float d = plh(blk);
     uint32_t q[2], sg[1];
     lds_a2<2>(blk + 2 + 8 * ib, q);
     lds_a2<1>(blk + 74 + 4 * ib, sg);
     const uint32_t qh = pl8(blk + 66 + ib);
     const uint32_t sc = (pl8(blk + 106 + (ib >> 1)) >> (4 * (ib & 1))) & 0xf;
-    int s = 0;
+    int s = 0, n = 0;
 #pragma unroll
     for (int l = 0; l < 4; ++l) {
       const uint32_t w = q[l >> 1] >> (16 * (l & 1));
-      const uint32_t g0 = __ldg(&d_iq3s_grid[(w & 0xFF) | ((qh << (8 - 2 * l)) & 256)]);
-      const uint32_t g1 = __ldg(&d_iq3s_grid[((w >> 8) & 0xFF) | ((qh << (7 - 2 * l)) & 256)]);
-      s = dot8_signed(g0, g1, (sg[0] >> (8 * l)) & 0xFF, x[2 * l], x[2 * l + 1], s);
+      g1_dot8(g1_grid32<T_IQ3_S>(t, (w & 0xFF) | ((qh << (8 - 2 * l)) & 256)), g1_grid32<T_IQ3_S>(t, ((w >> 8) & 0xFF) | ((qh << (7 - 2 * l)) & 256)),
+              g1_signs<T_IQ3_S>(t, (sg[0] >> (8 * l)) & 0xFF), x[2 * l], x[2 * l + 1], s, n);
     }
-    return d * (0.5f + (float)sc) * xd[0] * 0.5f * (float)s;
+    return d * (0.5f + (float)sc) * xd[0] * 0.5f * (float)(s - 2 * n);
   }
 };
 
@@ -496,9 +528,19 @@ template <> struct G1<T_Q2_K> {
 // ---- Q3_K: hmask[32] | qs[64] | scales[12] | d; unit g = 32 values (vecdotq.cuh:269-300, 1024-1048) ----
 // value 128n + 32i + l = ((qs[32n + l] >> 2i) & 3) - (bit 4n+i of hmask[l] ? 0 : 4); 6-bit scales minus 32.
 template <> struct G1<T_Q3_K> {
-  static constexpr int UPB = 8, XW = 8, XD = 2, UMAX = 4;
+  static constexpr int UPB = 8, XW = 10, XD = 2, UMAX = 4;   // x[8], x[9]: 4 * the sums of the two sub-blocks' codes
   static __device__ __forceinline__ void load_x(const uint8_t* qs, const float2* ds, int u, int b, uint32_t (&x)[XW], float (&xd)[XD]) {
-    G1<T_Q8_0>::load_x(qs, ds, u, b, x, xd);
+    uint32_t n[8];
+    G1<T_Q8_0>::load_x(qs, ds, u, b, n, xd);
+    int c0 = 0, c1 = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      x[i] = n[i];
+      if (i < 4) c0 = __dp4a((int)n[i], 0x04040404, c0);
+      else c1 = __dp4a((int)n[i], 0x04040404, c1);
+    }
+    x[8] = (uint32_t)c0;
+    x[9] = (uint32_t)c1;
   }
   static __device__ __forceinline__ float unit(uint32_t blk, int g, const uint32_t (&x)[XW], const float (&xd)[XD], const Tab1&) {
     uint32_t hm[8], q[8];
@@ -506,13 +548,15 @@ template <> struct G1<T_Q3_K> {
     lds_a2<8>(blk + 32 + 32 * (g >> 2), q);
     const uint32_t lo = pl16(blk + 96 + ((2 * g) & 7)) >> (4 * (g >> 2)), hi = pl16(blk + 104 + ((2 * g) & 3)) >> (2 * (g >> 1));
     const int sc0 = (int)((lo & 0xF) | ((hi & 3) << 4)) - 32, sc1 = (int)(((lo >> 8) & 0xF) | (((hi >> 8) & 3) << 4)) - 32;
-    const uint32_t sh = 2 * (g & 3);
-    int a0 = 0, a1 = 0;
+    // codes 0 to 7, and 4 less in the sum: (c - 4) . x = c . x - 4 sum(x).  (Byte-wise subtractions take several
+    // instructions a word: 14336x4096 16.8 -> 13.8 us.)
+    const uint32_t sh = 2 * (g & 3), rot = (uint32_t)(g - 2) & 31u;
+    int a0 = -(int)x[8], a1 = -(int)x[9];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      const uint32_t v = __vsub4((q[i] >> sh) & 0x03030303u, ((~hm[i] >> g) << 2) & 0x04040404u);
-      if (i < 4) a0 = __dp4a((int)v, (int)x[i], a0);
-      else a1 = __dp4a((int)v, (int)x[i], a1);
+      const uint32_t v = ((q[i] >> sh) & 0x03030303u) | (__funnelshift_r(hm[i], hm[i], rot) & 0x04040404u);
+      if (i < 4) a0 = dp4a_us1(v, x[i], a0);
+      else a1 = dp4a_us1(v, x[i], a1);
     }
     return plh(blk + 108) * xd[0] * (float)(a0 * sc0 + a1 * sc1);
   }
@@ -772,18 +816,10 @@ __global__ void __launch_bounds__(G1_WARPS * 32, 2) gemv1_kernel(const G1Params 
   Tab1 tb;
   tb.grid = 0;
   tb.smask = 0;
-  if (TYPE == T_IQ2_XXS) {
-    // Both code books are stored G1_TAB_COPIES times, copy c in the 8-byte column c of every
-    // 128-byte line: lane l reads copy l % 16, and since a 64-bit shared load is served one
-    // half-warp at a time, the 16 lanes of a half-warp hit 16 different bank pairs whatever
-    // entries they ask for.  (One copy costs a 3- to 4-way bank conflict on almost every look-up:
-    // 32 unrelated 8-byte entries per load.  Eight copies -- half the shared memory, room for larger
-    // work items -- measured slower: 28672x8192 36.7 us against 29.5 us with sixteen.)
-    uint2* g = reinterpret_cast<uint2*>(cur);
-    uint2* sm = g + 256 * G1_TAB_COPIES;
-    cur += (256 + 128) * 8 * G1_TAB_COPIES;
-    tb.grid = smem_u32(g + (lane & (G1_TAB_COPIES - 1)));
-    tb.smask = smem_u32(sm + (lane & (G1_TAB_COPIES - 1)));
+  if constexpr (G1Tab<TYPE>::GRID > 0) {   // (IQ2_XXS with eight copies -- half the shared memory, room for larger work items -- 36.7 us against 29.5 at 28672x8192)
+    tb.grid = smem_u32(cur) + (uint32_t)(G1Tab<TYPE>::GB * (lane & (G1Tab<TYPE>::GC - 1)));
+    tb.smask = smem_u32(cur) + (uint32_t)(g1_grid_bytes<TYPE>() + 8 * (lane & (G1Tab<TYPE>::SC - 1)));
+    cur += g1_tab_bytes<TYPE>();
   }
   if (TYPE == T_IQ4_XS || TYPE == T_IQ4_NL) {
     const uint32_t* kv = reinterpret_cast<const uint32_t*>(d_kvalues_iq4nl);
@@ -899,24 +935,7 @@ __global__ void __launch_bounds__(G1_WARPS * 32, 2) gemv1_kernel(const G1Params 
     }
   }
 
-  if (TYPE == T_IQ2_XXS) {   // fill the code-book copies while the first weight copies are in flight
-    uint2* tab_g = reinterpret_cast<uint2*>(smem);
-    uint2* tab_s = tab_g + 256 * G1_TAB_COPIES;
-    for (int i = threadIdx.x; i < 256 * G1_TAB_COPIES; i += blockDim.x) {
-      const uint64_t v = d_iq2xxs_grid[i / G1_TAB_COPIES];
-      tab_g[i] = make_uint2((uint32_t)v, (uint32_t)(v >> 32));
-    }
-    for (int i = threadIdx.x; i < 128 * G1_TAB_COPIES; i += blockDim.x) {
-      const uint32_t s = d_ksigns_iq2xs[i / G1_TAB_COPIES];
-      uint32_t lo = 0, hi = 0;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        lo |= ((s >> j) & 1u) ? (0xFFu << (8 * j)) : 0u;
-        hi |= ((s >> (4 + j)) & 1u) ? (0xFFu << (8 * j)) : 0u;
-      }
-      tab_s[i] = make_uint2(lo, hi);
-    }
-  }
+  if constexpr (G1Tab<TYPE>::GRID > 0) g1_fill_tables<TYPE>(smem);   // while the first weight copies are in flight
   // The copies above read nothing but weights; everything below reads or writes what earlier kernels may use.
   pdl_wait();
   const unsigned tag = p.world > 0 ? (sizeof(out_t) == 2 ? (p.epoch[p.slot] & 0xFFFFu) : p.epoch[p.slot]) : 0u;
@@ -1016,7 +1035,7 @@ __global__ void __launch_bounds__(G1_WARPS * 32, 2) gemv1_kernel(const G1Params 
       }
     }
   }
-  if (TYPE == T_IQ2_XXS) __syncthreads();  // tables staged
+  if (G1Tab<TYPE>::GRID > 0) __syncthreads();  // tables staged
   if (p.x_alias) {   // every warp has read its activations: the stage they sat in may now take weights
     __syncthreads();
     fence_proxy_async();
@@ -1185,10 +1204,10 @@ static int launch_g1(G1Params p, cudaStream_t stream) {
   const int slice_bytes = (p.slice_q + (p.slice_r ? 1 : 0)) * TS;   // the longest slice
   int R = rows_env < 1 ? 1 : (rows_env > G1_R ? G1_R : rows_env);
   // An item is as large as two stages per warp allow with two CTAs on an SM (16 stages in 113 KB less
-  // the tables, the staged results and the barriers: 6.9 KB, 3.9 KB with the 48 KB of IQ2_XXS code-book
+  // the tables, the staged results and the barriers: 6.9 KB, 3.9 KB with 48 KB of code-book
   // copies).  Larger items mean fewer barrier round trips per warp: 57344x4096 Q4_K 25.1 -> 21.8 us,
   // 14336x4096 8.3 -> 7.8 us with three rows instead of two.
-  const size_t tables = TYPE == T_IQ2_XXS ? (size_t)(256 + 128) * 8 * G1_TAB_COPIES : 0;
+  const size_t tables = g1_tab_bytes<TYPE>();
   p.partial_bytes = (ks > 1 || p.world > 0) ? G1_BATCH * 8 * G1_R * MV * 4 : 0;
   const int room2 = (int)(((size_t)113 * 1024 - tables - (size_t)p.partial_bytes - (size_t)G1_WARPS * 8 * 16) / (2 * G1_WARPS)) - 48;
   const int item_cap = item_env < room2 ? item_env : room2;
