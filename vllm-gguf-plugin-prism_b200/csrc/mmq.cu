@@ -77,39 +77,41 @@ static_assert(Stage64<T_Q4_0, __half>::PERM == 1 && Stage64<T_Q4_K, __half>::PER
 //   whole    every tile is one CTA's
 //   even     few tiles: each is cut into the same number of ranges of chunks, one per CTA
 //   stream   the chunks of all tiles in equal runs over all SMs
-// A stage takes 2.1 clocks per token on the tensor core, or the time to decode it (mmq_decode_clocks); reading a tile out takes
-// 19 clocks per token (beside the next tile's work where there are two accumulators), a CTA in use 59; sharing, 1,600 + 24 per
-// token + 9 per token and part where a CTA has one part of a tile, 9,000 + 19 per token + 13 per token and part where it has two
-// (6,000 by the times alone; the parts of runs also take up to 39 MB of L2: 512 tokens of 14336x4096 Q4_K in runs and in whole tiles
-// are 58.7 and 59.0 us in a row, 71.0 and 69.5 between other work).
-// Fitted by least squares to the times of every plan of 1463 problems (19 types, seven matrices of 1024x4096 to 28672x8192, 17 to
-// 1024 tokens): what it picks takes 0.4 % longer than the best plan on average, 11 % at most.  (With one decode time for the types
-// without a whole-stage decoder, nothing per CTA and cheaper runs it was 3.4 % and 37 %: 17 to 32 tokens of 14336x4096 were cut
-// into runs, 26.0 us for Q4_0 and 28.1 for Q5_K where whole tiles take 23.5 and 25.5.)
+// A stage takes the time to decode it (mmq_decode_clocks) or that of its product and its activations (mmq_stage_clocks); reading a tile
+// out takes 29 clocks per token, 11 where there are two accumulators (beside the next tile's work); a CTA in use 68; sharing, 4,000 + 36 per
+// token + 9.5 per token and part where a CTA has one part of a tile, 7,000 + 33 per token + 11 per token and part where it has two (5,500
+// by the times alone; the parts of runs also take up to 39 MB of L2: 512 tokens of 14336x4096 Q4_K in runs and in whole tiles are 55.9
+// and 56.0 us in a row, and runs lose 2 % between other work).
+// Fitted by least squares, then by what is lost, to the times of every plan of 1501 problems (19 types, seven matrices of 1024x4096 to
+// 28672x8192, 17 to 1999 tokens): what it picks takes 0.5 % longer than the best plan on average, 10 % at most.
 struct MmqPlan {
   int tn;
   int64_t tt, grid;
   bool shared;
 };
-// clocks to decode a stage
+// clocks to decode a stage, with what a CTA of many tokens leaves of its issue slots and shared memory (3 / 8 per token)
 static int mmq_decode_clocks(int type) {
   switch (type) {
-    case T_Q8_0: return 450;
-    case T_Q4_K: return 480;
-    case T_Q4_0: return 500;
-    case T_Q4_1: case T_Q5_K: return 540;
-    case T_Q5_0: case T_Q2_K: return 550;
-    case T_IQ2_XXS: case T_IQ1_S: return 610;
-    case T_Q6_K: case T_Q5_1: case T_IQ1_M: case T_IQ2_XS: return 650;
-    case T_Q3_K: return 670;
-    case T_IQ3_XXS: case T_IQ2_S: return 710;
-    case T_IQ4_XS: return 735;
-    case T_IQ3_S: return 755;
-    default: return 775;   // IQ4_NL
+    case T_Q8_0: return 340;
+    case T_Q4_0: return 360;
+    case T_Q4_K: return 365;
+    case T_Q4_1: return 400;
+    case T_IQ2_XXS: return 410;
+    case T_Q6_K: return 430;
+    case T_Q2_K: return 440;
+    case T_Q5_K: case T_Q5_1: return 460;
+    case T_IQ3_XXS: case T_IQ2_S: return 475;
+    case T_IQ1_S: case T_IQ2_XS: case T_IQ3_S: return 480;
+    case T_Q3_K: return 485;
+    case T_Q5_0: return 520;
+    case T_IQ1_M: return 540;
+    default: return 565;   // IQ4_NL, IQ4_XS
   }
 }
+// (the product itself takes two clocks per token; the rest is the activations' way from L2 and, beyond 256 tokens, the few A slots)
 static int64_t mmq_stage_clocks(int type, int tn) {
-  const int decode = mmq_decode_clocks(type), mma = 21 * tn / 10;
+  const int decode = mmq_decode_clocks(type) + (tn <= 256 ? 3 * tn / 8 : 0);
+  const int mma = tn <= 128 ? 290 + 11 * tn / 8 : tn <= 256 ? 177 + 8 * tn / 5 : tn <= 320 ? 500 + 7 * tn / 8 : 500 + 23 * tn / 20;
   return mma > decode ? mma : decode;
 }
 static MmqPlan mmq_plan(int type, int64_t M, int64_t N, int64_t K, bool may_share) {
@@ -128,20 +130,20 @@ static MmqPlan mmq_plan(int type, int64_t M, int64_t N, int64_t K, bool may_shar
       const int64_t tiles = rt * tt, chunk = 4 * mmq_stage_clocks(type, tn), waves = (tiles + MMQ_CTAS - 1) / MMQ_CTAS;
       const bool twin = tn <= 128;
       auto take = [&](int64_t t, int64_t grid, bool shared) {
-        t += 59 * grid;
+        t += 68 * grid;
         if (t < best_t) { best_t = t; best = {tn, tt, grid, shared}; }
       };
-      take(waves * nc * chunk + (twin ? 1 : waves) * 19 * tn, tiles < MMQ_CTAS ? tiles : MMQ_CTAS, false);
+      take(waves * nc * chunk + (twin ? 11 : waves * 29) * tn, tiles < MMQ_CTAS ? tiles : MMQ_CTAS, false);
       if (!may_share) continue;
       if (tiles % MMQ_CTAS != 0 && tiles * nc >= 2 * MMQ_CTAS) {
         const int64_t run = (tiles * nc + MMQ_CTAS - 1) / MMQ_CTAS;
-        take(run * chunk + (twin ? 1 : tiles / MMQ_CTAS + 1) * 19 * tn + 9000 + 19 * tn + 13 * tn * nc / run, MMQ_CTAS, true);
+        take(run * chunk + (twin ? 11 : (tiles / MMQ_CTAS + 1) * 29) * tn + 7000 + 33 * tn + 11 * tn * nc / run, MMQ_CTAS, true);
       }
       // (32-bit divisions: a call asks for its plan three times; a cut into more ranges of the same length only costs)
       const int ncs = (int)nc;
       for (int c = 2, len = 0; c * tiles <= MMQ_CTAS && 2 * c <= ncs; ++c) {
         const int l = (ncs + c - 1) / c;
-        if (l != len) take((int64_t)l * chunk + 1600 + tn * (43 + 9 * c), c * tiles, true);
+        if (l != len) take((int64_t)l * chunk + 4000 + tn * (72 + 19 * c) / 2, c * tiles, true);
         len = l;
       }
     }
