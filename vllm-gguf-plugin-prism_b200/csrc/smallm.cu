@@ -75,6 +75,11 @@ int launch_smallm(const SmallArgs& a, cudaStream_t stream) {
   if (stages > SM_MAX_STAGES) stages = SM_MAX_STAGES;
   if (stages < 2) return E_TOO_LARGE;
   p.stages = stages;
+  // A CTA asks for up to 60 KB of weights at a time.  The memory system serves what is outstanding interleaved: with whole rings asked
+  // for -- most of a 33 MB matrix -- every CTA's first stage arrived with the last, 3.6 us into the wait (14336x4096, eight tokens, all / four /
+  // three / two / one stage: Q4_K, 18 KB a stage, 17.4 / 16.7 / 16.2 / 15.7 / 16.4 us; Q6_K, 31 KB, 22.9 / 22.7 / 22.8 / 21.8 / 21.1).
+  p.ahead = 60 * 1024 / p.raw.bytes;
+  p.ahead = p.ahead < 1 ? 1 : p.ahead > stages ? stages : p.ahead;
   const size_t smem = 256 + (size_t)table + (size_t)stages * p.stage_bytes;
   const int64_t units = (int64_t)a.max_passes * p.rt * p.nc;
   if (units * (SM_GRID + 1) >= (int64_t)1 << 31) return E_TOO_LARGE;

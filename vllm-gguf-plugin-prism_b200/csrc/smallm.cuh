@@ -26,6 +26,7 @@ struct SmParams {
   int nblk, nc, rt;       // 32-value blocks, chunks, row tiles of a row / matrix
   int tiles;              // column tiles in x
   int stages, stage_bytes;
+  int ahead;              // stages asked for and not there yet, at most
   float* part;            // partial tiles, two slots per CTA
   int* counter;           // arrivals per output tile, zero at the start
   int* status;
@@ -172,8 +173,8 @@ __global__ void __launch_bounds__(SM_THREADS, 2) smallm_kernel(const __grid_cons
     cur.r = first_tile - cur.pass * p.rt;
     load_pass(cur);
     Cursor held = cur;        // first unit whose activations have not been asked for
-    int n_held = 0, st = 0;
-    uint32_t ph = 0;
+    int n_held = 0, st = 0, st_in = 0;   // st_in: the stage that has to be there before the next one is asked for
+    uint32_t ph = 0, ph_in = 0;
     bool waited = false;
     auto release = [&]() {    // the activations exist now
       pdl_wait();
@@ -181,7 +182,15 @@ __global__ void __launch_bounds__(SM_THREADS, 2) smallm_kernel(const __grid_cons
       for (int v = 0; v < n_held; ++v) { x_copy(held, v); advance(held); }
     };
     for (int u = u0; u < u1; ++u) {
-      if (!waited && n_held == p.stages) release();   // the ring is full of weights
+      if (!waited && n_held == p.ahead) release();
+      if (u - u0 >= p.ahead) {
+        if (!mbar_wait_bounded(&full[st_in], ph_in)) {
+          if (lane == 0) atomicExch(p.status, E_TIMEOUT);
+          drain_pause();
+          break;
+        }
+        if (++st_in == p.stages) { st_in = 0; ph_in ^= 1u; }
+      }
       if (!mbar_wait_bounded(&empty[st], ph ^ 1u)) {
         if (lane == 0) atomicExch(p.status, E_TIMEOUT);
         drain_pause();
