@@ -7,7 +7,7 @@
 // cores.  At these batches the instruction count decides, not the tensor rate: one instruction replaces the 128 dp4a of a
 // 16 x 32 block and eight tokens, a block's codes are unpacked once for all tokens, and what is left per block, token
 // tile and lane is 8 (no minimum) to 12 floating-point instructions.  (tcgen05 needs the codes as a 128-row operand in
-// tensor memory and the scales folded into 16-bit operands; its instruction costs at least 61 clocks however few tokens it
+// tensor memory and the scales folded into 16-bit operands; its instruction costs at least 25 clocks however few tokens it
 // has, and the fp16 rounding of the operands is not what this entry point promises.)
 //
 // Work: a CTA (eight warps x 16 rows, one warp that issues copies) streams stages of 256 values x 128 rows (raw_stream.cuh)
