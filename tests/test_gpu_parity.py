@@ -1102,3 +1102,26 @@ def test_tiled_activations_of_every_value(name):
     assert rel_l2(y[keep].cpu(), want[keep].float().cpu()) <= REL_L2_TOL
     for i in (0, 5):
         assert rel_l2(y[i].cpu(), want[i].float().cpu()) <= REL_L2_TOL
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("name,large", [("IQ3_S", 140.0), ("IQ3_XXS", 130.0), ("IQ4_XS", 16.0), ("IQ4_NL", 500.0)])
+def test_tiled_scales_of_every_size(name, large, dtype):
+    """Scales beyond the range of the split in two 16-bit numbers (the fp32 form), on both sides of it, and down to where the weights are
+    subnormal in fp16: against the dequantized weights."""
+    # The largest weight has to be finite in fp16 (65504): it is 465 d for IQ3_S (31 x 15), 480.5 d for IQ3_XXS (15.5 / 2 x 62),
+    # 4064 d for IQ4_XS (32 x 127) and 127 d for IQ4_NL; the fp32 form starts at group scales of 60000 / 256 (IQ3) and 60000 / 128 (IQ4).
+    t, N, K, M = TYPES[name], 136, 1024, 40
+    wn = synth.make_weight(t, N, K, seed=9)
+    size = capi.lib().gguf_b200_type_size(t)
+    x = dev_x(M, K, seed=5, dtype=dtype) / 1024
+    for d in (large, large / 8, 1e-3, 2e-6):
+        blocks = wn.reshape(-1, size).copy()
+        blocks[:, 0:2] = np.full(len(blocks), d, np.float16).view(np.uint8).reshape(-1, 2)
+        w = torch.from_numpy(blocks.reshape(N, -1)).to(DEV)
+        y = capi.dequant_matmul(w, x * (1 if d > 1e-3 else 2 ** 10), t, N)
+        want = (x.double() * (1 if d > 1e-3 else 2 ** 10)) @ capi.dequantize(w, t, N, K, dtype).double().T
+        torch.cuda.synchronize()
+        assert capi.last_status() == 0 and torch.isfinite(y).all()
+        # the output's own rounding: 2^-11 (bf16 2^-8) of each value, and for the smallest scale fp16 outputs that are subnormal themselves
+        assert rel_l2(y.float().cpu(), want.float().cpu()) <= (6e-3 if dtype == torch.bfloat16 or d < 1e-5 else REL_L2_TOL), d

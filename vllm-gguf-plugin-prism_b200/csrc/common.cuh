@@ -337,6 +337,7 @@ template <typename T> __device__ __forceinline__ bool packet_read(const void* ba
 //   * an activation quantizer calls pdl_trigger() after its own pdl_wait(), so a product behind it does not even start before
 //     all work ahead of the call is complete and visible (a decoder layer of 8 tokens 83.7 -> 80.3 us, of 45 tokens 124.5 -> 126.6:
 //     the product's CTAs no longer wait on the SMs for the activations);
+//     A MoE product reads its work list at its start for the same reason: that is older than the quantizer's trigger;
 //   * the GEMV of one or two vectors, and a product that is a call's first kernel (the GEMM on plain activations), read ahead
 //     (a layer of one token 48.5 -> 48.0 us) unless their caller says that the weights are in flight (GGUF_B200_W_IN_FLIGHT).
 __device__ __forceinline__ void bulk_prefetch_l2(const void* src, uint32_t bytes) {   // (aligned as a bulk copy)

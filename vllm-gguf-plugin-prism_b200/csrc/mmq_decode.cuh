@@ -1,7 +1,8 @@
 // Weight decoders of the tensor-core GEMM (mmq.cu): one 32-value group of one weight row
 // ("unit" u = values 32u..32u+31) -> 16 packed 16-bit pairs = 64 bytes of the row in the A tile.
-// A producer thread owns one row of a 64-value stage and calls a decoder for its two units
-// (the whole-stage decoders at the end of this file replace that for Q4_K / Q4_0 / Q8_0).
+// A producer thread owns one row of a 64-value stage and calls a decoder for its two units; towards the end of this file,
+// whole-stage decoders replace that for Q4_K / Q5_K / Q4_0 / Q8_0 in dense stages, and decoders of an item (two stages) for Q6_K,
+// IQ2_*, IQ3_* and, with fp16 activations, IQ4_*.
 //
 // Each decoder is split in two:
 //   load()   fetches a unit's raw bytes (from the shared-memory raw ring) into registers,
@@ -9,8 +10,8 @@
 //
 // Values are bit-identical to the reference's standalone dequantize for the types that are fed
 // to the MMA as dequantized weights (Q4_0, Q8_0, Q6_K: dequantize.cuh:3-15, 69-78, 232-256;
-// IQ4_XS, IQ2_XXS: dequantize.cuh:420-435, 258-275).  Q4_K feeds half(d*sc*q) and carries its
-// min term in the correction columns (see mmq.cu).
+// IQ2_XXS: dequantize.cuh:258-275), but for IQ3 and IQ4 values that lie closer to the middle between two numbers than
+// Iq3Group says.  Q4_K feeds half(d*sc*q) and carries its min term in the correction columns (see mmq.cu).
 //
 // Blocks of Q4_0 / Q8_0 / Q6_K / IQ2_XXS are only 2-byte aligned: raw bytes are fetched as the
 // aligned 32-bit words that cover them and realigned with funnel shifts.
