@@ -1110,7 +1110,7 @@ def test_tiled_scales_of_every_size(name, large, dtype):
     """Scales beyond the range of the split in two 16-bit numbers (the fp32 form), on both sides of it, and down to where the weights are
     subnormal in fp16: against the dequantized weights."""
     # The largest weight has to be finite in fp16 (65504): it is 465 d for IQ3_S (31 x 15), 480.5 d for IQ3_XXS (15.5 / 2 x 62),
-    # 4064 d for IQ4_XS (32 x 127) and 127 d for IQ4_NL; the fp32 form starts at group scales of 60000 / 256 (IQ3) and 60000 / 128 (IQ4).
+    # 4064 d for IQ4_XS (32 x 127) and 127 d for IQ4_NL; the fp32 form of fp16 starts at group scales of 60000 / 256 (IQ3_S) and 60000 / 128 (IQ4).
     t, N, K, M = TYPES[name], 136, 1024, 40
     wn = synth.make_weight(t, N, K, seed=9)
     size = capi.lib().gguf_b200_type_size(t)
@@ -1125,3 +1125,22 @@ def test_tiled_scales_of_every_size(name, large, dtype):
         assert capi.last_status() == 0 and torch.isfinite(y).all()
         # the output's own rounding: 2^-11 (bf16 2^-8) of each value, and for the smallest scale fp16 outputs that are subnormal themselves
         assert rel_l2(y.float().cpu(), want.float().cpu()) <= (6e-3 if dtype == torch.bfloat16 or d < 1e-5 else REL_L2_TOL), d
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("name", ["IQ3_S", "IQ3_XXS"])
+def test_tiled_iq3_weights_are_rounded_once(name, dtype):
+    """Every weight as the tiled kernel uses it, read out with unit vectors: the fp32 product rounded once, bit for bit."""
+    t, N, K, M = TYPES[name], 128, 512, 64
+    wn = synth.make_weight(t, N, K, seed=3)
+    size = capi.lib().gguf_b200_type_size(t)
+    d = np.random.default_rng(3).uniform(np.log(2e-6), np.log(100.0), wn.size // size)   # scales of every size, subnormal ones too
+    blocks = wn.reshape(-1, size).copy()
+    blocks[:, 0:2] = np.exp(d).astype(np.float16).view(np.uint8).reshape(-1, 2)
+    w = torch.from_numpy(blocks.reshape(N, -1)).to(DEV)
+    # dequantize to fp32 is the exact product: at most 11 + 5 + 5 significant bits
+    want = capi.dequantize(w, t, N, K, torch.float32).to(dtype).T
+    eye = torch.eye(K, dtype=dtype, device=DEV)
+    for k in range(0, K, M):   # one non-zero product a sum: exact in the accumulator
+        y = capi.dequant_matmul(w, eye[k:k + M].contiguous(), t, N)
+        assert torch.equal(y, want[k:k + M]), k

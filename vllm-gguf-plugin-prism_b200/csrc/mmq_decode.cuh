@@ -10,8 +10,9 @@
 //
 // Values are bit-identical to the reference's standalone dequantize for the types that are fed
 // to the MMA as dequantized weights (Q4_0, Q8_0, Q6_K: dequantize.cuh:3-15, 69-78, 232-256;
-// IQ2_XXS: dequantize.cuh:258-275), but for IQ3 and IQ4 values that lie closer to the middle between two numbers than
-// Iq3Group says.  Q4_K feeds half(d*sc*q) and carries its min term in the correction columns (see mmq.cu).
+// IQ2_XXS: dequantize.cuh:258-275), and so are the IQ3 and IQ4 values (of the split scales of fp16 every
+// finite scale, sub-scale and level was compared).  Q4_K feeds half(d*sc*q) and carries its min term in
+// the correction columns (see mmq.cu).
 //
 // Blocks of Q4_0 / Q8_0 / Q6_K / IQ2_XXS are only 2-byte aligned: raw bytes are fetched as the
 // aligned 32-bit words that cover them and realigned with funnel shifts.
@@ -136,7 +137,7 @@ __device__ __forceinline__ uint4 iq2_pair_selectors(uint64_t grid_entry) {
   }
   return make_uint4(s[0], s[1], s[2], s[3]);
 }
-// An IQ3 entry: its four magnitudes (at most 62) as 16-bit values, for fp16 divided by 256 (see iq3_pair).
+// An IQ3 entry: its four magnitudes (at most 62) as 16-bit values, for fp16 divided by 256; those of IQ3_XXS are bf16 always (see Iq3Group).
 template <typename ab_t> __device__ __forceinline__ uint2 iq3_magnitudes(uint32_t g) {
   const float f = std::is_same<ab_t, __half>::value ? 1.f / 256.f : 1.f;
   return make_uint2(pack2<ab_t>(f * (float)(g & 0xFFu), f * (float)((g >> 8) & 0xFFu)), pack2<ab_t>(f * (float)((g >> 16) & 0xFFu), f * (float)(g >> 24)));
@@ -150,7 +151,7 @@ template <int TYPE, typename ab_t> __device__ __forceinline__ void decoder_fill_
       if constexpr (TYPE == T_IQ2_XXS) reinterpret_cast<uint4*>(tab)[i] = iq2_pair_selectors(d_iq2xxs_grid[e]);
       if constexpr (TYPE == T_IQ2_XS) reinterpret_cast<uint4*>(tab)[i] = iq2_pair_selectors(d_iq2xs_grid[e]);
       if constexpr (TYPE == T_IQ2_S) reinterpret_cast<uint4*>(tab)[i] = iq2_pair_selectors(d_iq2s_grid[e]);
-      if constexpr (TYPE == T_IQ3_XXS) reinterpret_cast<uint2*>(tab)[i] = iq3_magnitudes<ab_t>(d_iq3xxs_grid[e]);
+      if constexpr (TYPE == T_IQ3_XXS) reinterpret_cast<uint2*>(tab)[i] = iq3_magnitudes<__nv_bfloat16>(d_iq3xxs_grid[e]);
       if constexpr (TYPE == T_IQ3_S) reinterpret_cast<uint2*>(tab)[i] = iq3_magnitudes<ab_t>(d_iq3s_grid[e]);
       if constexpr (TYPE == T_IQ1_S || TYPE == T_IQ1_M) reinterpret_cast<uint32_t*>(tab)[i] = d_iq1s_grid[e];
     }
@@ -1002,38 +1003,47 @@ template <typename ab_t> struct Item128<T_IQ2_S, ab_t> {   // half d | u8 qs[32]
 };
 
 // ---- the IQ3 formats: value = +-round(d * magnitude), d = dh * (0.5 + s) * 0.5 in fp32 (at most 16 significant bits) ----
-// (8192x28672, 300 tokens, bf16: 121.4 -> 112.5 us with the same plan, 165 -> about 100 shared-memory wavefronts a stage of 32 rows; the
+// (8192x28672, 300 tokens, bf16, products split in bf16 at the time: 121.4 -> 112.5 us with the same plan; in fp32 as now the call keeps its gain, 149.9 -> 138.5 against 148.4 -> 137.1; 165 -> about 100 shared-memory wavefronts a stage of 32 rows; the
 // IQ2 formats with their signs as above, IQ2_XXS 28672x8192, 128 tokens: 67.9 -> 61.8 us.)
-// Two 16-bit instructions a pair instead of two permutes, two fp32 multiply-adds and a conversion: d is the sum of two 16-bit
-// numbers, and fma(m, hi, m * lo) rounds the sum once.  Only m * lo is rounded before, by 2^-12 (bf16: 2^-9) of what is at
-// most half a unit in the last place of the result, so the result is the correctly rounded one but for sums that
-// close to the middle between two numbers.  For fp16 the magnitudes are held divided by 256 and d times 256, which keeps lo clear of the
-// subnormals; a d beyond that range (`big`) takes the fp32 form.
-template <typename ab_t> struct Iq3Group {
-  using V = typename std::conditional<std::is_same<ab_t, __half>::value, __half2, __nv_bfloat162>::type;
-  V hi, lo;
-  float d;
-  bool big;
+// IQ3_S with fp16: two 16-bit instructions a pair instead of two permutes, two fp32 multiply-adds and a conversion.  d is the sum of two 16-bit
+// numbers and fma(m, hi, m * lo) rounds the sum once: lo has at most five significant bits, m four, so m * lo is exact and the result the correctly
+// rounded one.  The magnitudes are held divided by 256 and d times 256, which keeps lo clear of the subnormals; a d beyond that range takes the
+// fp32 form (`wide`).
+// bf16, and IQ3_XXS: the product in fp32, exact in 21 bits, two values an instruction, rounded once; the magnitudes are held in bf16 (five bits).
+// Split in bf16, m * lo would be rounded to eight bits before the sum (0.502 of a last place against 0.500, one weight in 2500); of IQ3_XXS in fp16 62 / 256 * lo can be
+// an odd multiple of 2^-25, half of fp16's last place, where dh is below 2^-13, and taking the fp32 form only there made warps run both
+// (14336x4096, 512 tokens: 70.7 us against 63.1 before all this).
+template <int TYPE, typename ab_t> struct Iq3Group {
+  static constexpr bool SPLIT = TYPE == T_IQ3_S && std::is_same<ab_t, __half>::value;
+  __half2 hi, lo;
+  uint64_t d2;   // (d, d) in fp32
+  bool wide;
   __device__ __forceinline__ void set(float dh, uint32_t s) {
-    d = dh * (0.5f + (float)s) * 0.5f;
-    if constexpr (std::is_same<ab_t, __half>::value) {
+    float d = dh * (0.5f + (float)s) * 0.5f;
+    wide = true;
+    if constexpr (SPLIT) {
       d *= 256.f;
       hi = __float2half2_rn(d);
       lo = __float2half2_rn(d - __low2float(hi));
-      big = !(fabsf(d) < 60000.f);
-    } else {
-      hi = __float2bfloat162_rn(d);
-      lo = __float2bfloat162_rn(d - __low2float(hi));
-      big = !(fabsf(d) < 1e36f);
+      wide = !(fabsf(d) < 60000.f);
     }
+    asm("mov.b64 %0, {%1, %1};" : "=l"(d2) : "r"(__float_as_uint(d)));
   }
   __device__ __forceinline__ uint32_t pair(uint32_t m) const {
-    const V v = *reinterpret_cast<const V*>(&m), r = __hfma2(v, hi, __hmul2_rn(v, lo));
-    return *reinterpret_cast<const uint32_t*>(&r);
+    const __half2 v = u32_as_h2(m);
+    return h2_as_u32(__hfma2(v, hi, __hmul2_rn(v, lo)));
   }
   __device__ __forceinline__ uint32_t pair32(uint32_t m) const {
-    const V v = *reinterpret_cast<const V*>(&m);
-    return pack2<ab_t>(d * __low2float(v), d * __high2float(v));
+    float a, b;
+    if constexpr (SPLIT) {
+      a = __low2float(u32_as_h2(m));
+      b = __high2float(u32_as_h2(m));
+    } else {
+      a = __uint_as_float(m << 16);
+      b = __uint_as_float(m & 0xFFFF0000u);
+    }
+    asm("{.reg .b64 t;\n\tmov.b64 t, {%0, %1};\n\tmul.rn.f32x2 t, t, %2;\n\tmov.b64 {%0, %1}, t;}" : "+f"(a), "+f"(b) : "l"(d2));
+    return pack2<ab_t>(a, b);
   }
 };
 template <typename ab_t> struct Item128<T_IQ3_XXS, ab_t> {   // half d | u8 qs[64] | per 32 values four 7-bit sign indices and a 4-bit scale; 98 bytes
@@ -1048,7 +1058,7 @@ template <typename ab_t> struct Item128<T_IQ3_XXS, ab_t> {   // half d | u8 qs[6
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
       const uint32_t aux = s.aux[2 * H + u];
-      Iq3Group<ab_t> g;
+      Iq3Group<T_IQ3_XXS, ab_t> g;
       g.set(s.dh, aux >> 28);
       auto go = [&](auto value) {
 #pragma unroll
@@ -1062,7 +1072,7 @@ template <typename ab_t> struct Item128<T_IQ3_XXS, ab_t> {   // half d | u8 qs[6
           o[3] = negate(value(b.y), sign_bits<3>(sw));
         }
       };
-      if (!g.big) go([&](uint32_t m) { return g.pair(m); });
+      if (Iq3Group<T_IQ3_XXS, ab_t>::SPLIT && !g.wide) go([&](uint32_t m) { return g.pair(m); });
       else go([&](uint32_t m) { return g.pair32(m); });
     }
   }
@@ -1083,7 +1093,7 @@ template <typename ab_t> struct Item128<T_IQ3_S, ab_t> {   // half d | u8 qs[64]
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
       const uint32_t qh = s.qh >> (16 * H + 8 * u), sg = s.sg[2 * H + u];
-      Iq3Group<ab_t> g;
+      Iq3Group<T_IQ3_S, ab_t> g;
       g.set(s.dh, (s.sc >> (8 * H + 4 * u)) & 0xFu);
       auto go = [&](auto value) {
 #pragma unroll
@@ -1102,7 +1112,7 @@ template <typename ab_t> struct Item128<T_IQ3_S, ab_t> {   // half d | u8 qs[64]
           }
         }
       };
-      if (!g.big) go([&](uint32_t m) { return g.pair(m); });
+      if (Iq3Group<T_IQ3_S, ab_t>::SPLIT && !g.wide) go([&](uint32_t m) { return g.pair(m); });
       else go([&](uint32_t m) { return g.pair32(m); });
     }
   }
