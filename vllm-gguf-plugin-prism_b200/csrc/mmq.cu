@@ -185,6 +185,16 @@ int launch_fence(cudaStream_t stream) {
   return cudaGetLastError() == cudaSuccess ? E_OK : E_CUDA;
 }
 
+// Three activation boxes of the largest tile have to fit beside the tables and two raw stages of rows of any pitch (an odd number of
+// 16-byte units each, with the rows that a class map leaves over).  With two, 1152 tokens of 37888x3584 IQ3_XXS took 281 us instead of 231.
+template <int TYPE> constexpr bool mmq_three_boxes() {
+  constexpr int units = (RAW_KC / BlockTraits<TYPE>::QK * BlockTraits<TYPE>::TS + 30) / 16 | 1;
+  constexpr int raw = (RAW_ROWS + RAW_EXTRA) * units * 16 + 128, corr = Decoder<TYPE, __half>::CORR ? MMQ_CORR_BYTES : 0;
+  return 226 * 1024 - 512 - decoder_table_bytes<TYPE>() - corr - 2 * raw >= 3 * 384 * MMQ_BK * 2;
+}
+#define MMQ_FITS(TYPE) static_assert(mmq_three_boxes<TYPE>(), #TYPE);
+MMQ_TYPES(MMQ_FITS)
+
 static int mmq_aux_bytes(int type) {   // barriers, then the decoder's tables
   switch (type) {
 #define MMQ_TAB(TYPE) case TYPE: return 512 + decoder_table_bytes<TYPE>();

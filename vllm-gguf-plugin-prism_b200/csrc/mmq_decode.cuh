@@ -64,29 +64,31 @@ __device__ __forceinline__ uint32_t shift_of(const uint8_t* p) { return (uint32_
 // that share a 128-byte access phase then sit in different columns of the 128 bytes whatever entries they look up (random
 // look-ups into a single copy averaged 2.5 to 3 bank conflicts per access).  The addresses below already point at this
 // thread's copy; the larger code books have room for fewer copies.
+// IQ3_XXS has 16 copies of the signs, of which half a warp's share a bank: with 32 the tables left two activation boxes at 384 tokens a
+// tile and two raw stages at 256.  14336x4096, 32 -> 16 copies: 384 tokens 43.5 -> 41.0 us, 256 tokens 31.4 -> 29.9, 128 tokens 24.2 -> 24.4.
 struct DecodeCtx {
   uint32_t grid;      // code book: byte-permute selectors of value pairs (IQ2), magnitudes (IQ3), codes (IQ1)
   uint32_t sgn;       // per 7-bit sign index, the signs of the four value pairs (iq_pair_signs)
 };
-template <int TYPE> struct DecodeTables {   // GRID entries of GB bytes in GC copies; SGN sign words in 32 copies
-  static constexpr int GRID = 0, GB = 0, GC = 0, SGN = 0;
+template <int TYPE> struct DecodeTables {   // GRID entries of GB bytes in GC copies; SGN sign words in SC copies
+  static constexpr int GRID = 0, GB = 0, GC = 0, SGN = 0, SC = 0;
 };
-template <> struct DecodeTables<T_IQ2_XXS> { static constexpr int GRID = 256, GB = 16, GC = 8, SGN = 128; };
-template <> struct DecodeTables<T_IQ2_XS> { static constexpr int GRID = 512, GB = 16, GC = 4, SGN = 128; };
-template <> struct DecodeTables<T_IQ2_S> { static constexpr int GRID = 1024, GB = 16, GC = 2, SGN = 0; };
-template <> struct DecodeTables<T_IQ3_XXS> { static constexpr int GRID = 256, GB = 8, GC = 16, SGN = 128; };
-template <> struct DecodeTables<T_IQ3_S> { static constexpr int GRID = 512, GB = 8, GC = 8, SGN = 0; };
-template <> struct DecodeTables<T_IQ1_S> { static constexpr int GRID = 2048, GB = 4, GC = 2, SGN = 0; };
+template <> struct DecodeTables<T_IQ2_XXS> { static constexpr int GRID = 256, GB = 16, GC = 8, SGN = 128, SC = 32; };
+template <> struct DecodeTables<T_IQ2_XS> { static constexpr int GRID = 512, GB = 16, GC = 4, SGN = 128, SC = 32; };
+template <> struct DecodeTables<T_IQ2_S> { static constexpr int GRID = 1024, GB = 16, GC = 2, SGN = 0, SC = 0; };
+template <> struct DecodeTables<T_IQ3_XXS> { static constexpr int GRID = 256, GB = 8, GC = 16, SGN = 128, SC = 16; };
+template <> struct DecodeTables<T_IQ3_S> { static constexpr int GRID = 512, GB = 8, GC = 8, SGN = 0, SC = 0; };
+template <> struct DecodeTables<T_IQ1_S> { static constexpr int GRID = 2048, GB = 4, GC = 2, SGN = 0, SC = 0; };
 template <> struct DecodeTables<T_IQ1_M> : DecodeTables<T_IQ1_S> {};
 template <int TYPE> __host__ __device__ constexpr int decoder_table_bytes() {
   using D = DecodeTables<TYPE>;
-  return D::GRID * D::GB * D::GC + D::SGN * 4 * 32;
+  return D::GRID * D::GB * D::GC + D::SGN * 4 * D::SC;
 }
 template <int TYPE> __device__ __forceinline__ DecodeCtx decoder_context(const uint8_t* tab, int lane) {
   using D = DecodeTables<TYPE>;
   DecodeCtx cx{0, 0};
   if constexpr (D::GRID > 0) cx.grid = smem_u32(tab) + (uint32_t)(D::GB * (lane & (D::GC - 1)));
-  if constexpr (D::SGN > 0) cx.sgn = smem_u32(tab) + (uint32_t)(D::GRID * D::GB * D::GC + 4 * lane);
+  if constexpr (D::SGN > 0) cx.sgn = smem_u32(tab) + (uint32_t)(D::GRID * D::GB * D::GC + 4 * (lane & (D::SC - 1)));
   return cx;
 }
 template <int TYPE> __device__ __forceinline__ uint4 grid128(const DecodeCtx& cx, uint32_t i) {
@@ -110,9 +112,9 @@ __device__ __forceinline__ uint32_t negate(uint32_t pair, uint32_t bits) { retur
 // ... from the sign bits themselves, s < 256: bit 2P to bit 15, bit 2P + 1 to bit 31 (the two products do not overlap)
 template <int P> __device__ __forceinline__ uint32_t sign_bits8(uint32_t s) { return s * ((1u << (15 - 2 * P)) + (1u << (30 - 2 * P))); }
 // ... from the table word of a 7-bit index: bits 15 - P and 31 - P
-__device__ __forceinline__ uint32_t sign_word(const DecodeCtx& cx, uint32_t i) {
+template <int TYPE> __device__ __forceinline__ uint32_t sign_word(const DecodeCtx& cx, uint32_t i) {
   uint32_t v;
-  asm("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(cx.sgn + 128u * i));
+  asm("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(cx.sgn + (uint32_t)(4 * DecodeTables<TYPE>::SC) * i));
   return v;
 }
 template <int P> __device__ __forceinline__ uint32_t sign_bits(uint32_t word) { return word * (1u << P); }
@@ -158,7 +160,7 @@ template <int TYPE, typename ab_t> __device__ __forceinline__ void decoder_fill_
   }
   if constexpr (D::SGN > 0) {
     uint32_t* sgn = reinterpret_cast<uint32_t*>(tab + D::GRID * D::GB * D::GC);
-    for (int i = threadIdx.x; i < D::SGN * 32; i += blockDim.x) sgn[i] = iq_pair_signs(d_ksigns_iq2xs[i >> 5]);
+    for (int i = threadIdx.x; i < D::SGN * D::SC; i += blockDim.x) sgn[i] = iq_pair_signs(d_ksigns_iq2xs[i / D::SC]);
   }
 }
 
@@ -939,7 +941,7 @@ template <typename ab_t> struct Item128<T_IQ2_XXS, ab_t> {   // half d | per 32 
       g.set(s.dh, aux >> 28);
 #pragma unroll
       for (int l = 0; l < 4; ++l)
-        iq2_entry<ab_t>(g, grid128<T_IQ2_XXS>(cx, byte_of(idx, l)), sign_word(cx, (aux >> (7 * l)) & 127u), out + 16 * u + 4 * l);
+        iq2_entry<ab_t>(g, grid128<T_IQ2_XXS>(cx, byte_of(idx, l)), sign_word<T_IQ2_XXS>(cx, (aux >> (7 * l)) & 127u), out + 16 * u + 4 * l);
     }
   }
 };
@@ -961,7 +963,7 @@ template <typename ab_t> struct Item128<T_IQ2_XS, ab_t> {   // half d | u16 qs[3
       g.set(s.dh, (s.sc >> (16 * H + 4 * v)) & 0xFu);
 #pragma unroll
       for (int l = 0; l < 2; ++l)
-        iq2_entry<ab_t>(g, grid128<T_IQ2_XS>(cx, (q >> (16 * l)) & 511u), sign_word(cx, (q >> (16 * l + 9)) & 127u), out + 8 * v + 4 * l);
+        iq2_entry<ab_t>(g, grid128<T_IQ2_XS>(cx, (q >> (16 * l)) & 511u), sign_word<T_IQ2_XS>(cx, (q >> (16 * l + 9)) & 127u), out + 8 * v + 4 * l);
     }
   }
 };
@@ -1063,7 +1065,7 @@ template <typename ab_t> struct Item128<T_IQ3_XXS, ab_t> {   // half d | u8 qs[6
       auto go = [&](auto value) {
 #pragma unroll
         for (int l = 0; l < 4; ++l) {
-          const uint32_t w = s.q[4 * H + 2 * u + (l >> 1)], sw = sign_word(cx, (aux >> (7 * l)) & 127u);
+          const uint32_t w = s.q[4 * H + 2 * u + (l >> 1)], sw = sign_word<T_IQ3_XXS>(cx, (aux >> (7 * l)) & 127u);
           const uint2 a = grid64<T_IQ3_XXS>(cx, byte_of(w, 2 * (l & 1))), b = grid64<T_IQ3_XXS>(cx, byte_of(w, 2 * (l & 1) + 1));
           uint32_t* o = out + 16 * u + 4 * l;
           o[0] = negate(value(a.x), sign_bits<0>(sw));
