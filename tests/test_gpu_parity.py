@@ -1144,3 +1144,38 @@ def test_tiled_iq3_weights_are_rounded_once(name, dtype):
     for k in range(0, K, M):   # one non-zero product a sum: exact in the accumulator
         y = capi.dequant_matmul(w, eye[k:k + M].contiguous(), t, N)
         assert torch.equal(y, want[k:k + M]), k
+
+
+def _scales_of_every_size(name, largest, n, k, seed):
+    """Random blocks whose fp16 scales run from the subnormals to `largest`, a tenth of them just below it."""
+    size = capi.lib().gguf_b200_type_size(TYPES[name])
+    wn = synth.make_weight(TYPES[name], n, k, seed=seed)
+    rng = np.random.default_rng(seed)
+    d = np.exp(rng.uniform(np.log(2e-6), np.log(largest), wn.size // size))
+    d = np.where(rng.random(d.size) < 0.1, largest * rng.uniform(0.9, 1.0, d.size), d).astype(np.float16)
+    at = 208 if name == "Q6_K" else 0
+    blocks = wn.reshape(-1, size).copy()
+    blocks[:, at:at + 2] = d.view(np.uint8).reshape(-1, 2)
+    return torch.from_numpy(blocks.reshape(n, -1)).to(DEV)
+
+
+# The largest scale leaves every weight finite in fp16: 127 d for IQ4_NL, 4064 d for IQ4_XS (both beyond 60000 / 128, where fp16 takes the fp32
+# form), 15.5 / 4 x 43 d for the IQ2 types, 15.5 / 2 x 62 d for IQ3_XXS, 31 x 15 d for IQ3_S.
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("name,largest,k", [("IQ4_NL", 510.0, 320), ("IQ4_NL", 510.0, 2048), ("IQ4_XS", 16.0, 768), ("IQ4_XS", 16.0, 1024), ("IQ2_XXS", 390.0, 768),
+                                            ("IQ2_XXS", 390.0, 2048), ("IQ2_XS", 390.0, 768), ("IQ2_XS", 390.0, 2048), ("IQ2_S", 390.0, 768),
+                                            ("IQ2_S", 390.0, 2048), ("IQ3_XXS", 135.0, 768), ("IQ3_S", 140.0, 768)])
+def test_tiled_code_book_weights_are_rounded_once(name, largest, k, dtype):
+    """Every weight as the tiled kernel uses it, read out with unit vectors, in rows of every pitch and rows that end inside a chunk: the fp32
+    product rounded once, bit for bit."""
+    t, N, M = TYPES[name], 136, 64
+    w = _scales_of_every_size(name, largest, N, k, seed=k)
+    # dequantize to fp32 is the exact product: at most 24 significant bits (IQ4_XS: 11 of d, 6 of the sub-scale, 7 of the level)
+    want = capi.dequantize(w, t, N, k, torch.float32).to(dtype).T
+    assert torch.isfinite(want).all()
+    eye = torch.eye(k, dtype=dtype, device=DEV)
+    for i in range(0, k, M):   # one non-zero product a sum: exact in the accumulator
+        y = capi.dequant_matmul(w, eye[i:i + M].contiguous(), t, N)
+        assert torch.equal(y, want[i:i + M]), i
+    torch.cuda.synchronize()
+    assert capi.last_status() == 0

@@ -1123,7 +1123,7 @@ template <typename ab_t> struct Item128<T_IQ3_S, ab_t> {   // half d | u8 qs[64]
 // ---- the IQ4 formats with fp16 activations: value = round(dl * level), dl in fp32 (at most 17 significant bits) ----
 // As IQ3: the level, divided by 128, is 1024 + (level + 128) made by a permute, times 1/128, minus 9 -- exact -- and dl times 128 is split
 // in two.  (bf16 has no room for the byte under a power of two; those activations keep iq4_word.  14336x4096, 48 tokens:
-// IQ4_XS 26.2 -> 24.1 us, IQ4_NL 29.7 -> 27.4.)
+// IQ4_XS 26.2 -> 24.1 us, IQ4_NL 29.7 -> 23.9.)
 struct Iq4Group {
   __half2 hi, lo;
   float dl;
@@ -1137,10 +1137,20 @@ struct Iq4Group {
   }
   // a word of indices: values 4i .. 4i + 3 in the low nibbles, 16 + 4i .. in the high ones
   __device__ __forceinline__ void word(uint32_t w, uint32_t* o_lo, uint32_t* o_hi) const {
+    if (big) iq4_word<__half>(w, dl, o_lo, o_hi);
+    else word16(w, o_lo, o_hi);
+  }
+  // the 32 values of four words, with one branch
+  __device__ __forceinline__ void words(const uint32_t (&w)[4], uint32_t* o) const {
     if (big) {
-      iq4_word<__half>(w, dl, o_lo, o_hi);
-      return;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) iq4_word<__half>(w[i], dl, o + 2 * i, o + 8 + 2 * i);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) word16(w[i], o + 2 * i, o + 8 + 2 * i);
     }
+  }
+  __device__ __forceinline__ void word16(uint32_t w, uint32_t* o_lo, uint32_t* o_hi) const {
     const uint32_t q3 = w & 0x77777777u, sel = ((w >> 1) & 0x44444444u) | 0x32103210u;
     const uint32_t a = iq4_levels4(q3, sel), b = iq4_levels4(q3 >> 16, sel >> 16);   // bytes (4i, 16+4i, 4i+1, 17+4i) and (4i+2, ...)
     auto v = [&](uint32_t x) {
@@ -1177,20 +1187,26 @@ template <> struct Item128<T_IQ4_XS, __half> {   // half d | u16 scales_h | u8 s
     }
   }
 };
+// IQ4_NL: the words of both stages at once and one branch a block.  (Read by the stage, with a branch a word, the decoder held the few A slots of the
+// largest tiles for too long: 384 tokens of 14336x4096 44.3 us against 40.2 with unit decoders, now 39.2; 17 tokens 26.9 -> 23.5.)
 template <> struct Item128<T_IQ4_NL, __half> {   // blocks of 18 bytes: half d | u8 qs[16]
   static constexpr bool HAVE = true;
-  struct State { int left; };
-  static __device__ __forceinline__ void begin(uint32_t, int, bool, int left, State& s) { s.left = left; }
-  template <int H> static __device__ __forceinline__ void stage(uint32_t row, int ip, bool wide, const DecodeCtx&, const State& s, uint32_t (&out)[32]) {
-    uint32_t w[9];
-    lds_row_words<9>(row + 72 * ip + 36 * H, wide, w);
+  struct State { uint32_t w[18]; int left; };
+  static __device__ __forceinline__ void begin(uint32_t row, int ip, bool wide, int left, State& s) {
+    lds_row_words<18>(row + 72 * ip, wide, s.w);
+    s.left = left;
+  }
+  template <int H> static __device__ __forceinline__ void stage(uint32_t, int, bool, const DecodeCtx&, const State& s, uint32_t (&out)[32]) {
+    const uint32_t* w = s.w + 9 * H;
 #pragma unroll
     for (int u = 0; u < 2; ++u) {   // the second block starts 18 bytes on: its d in the upper half of word four
       const float d = __half2float(__ushort_as_half((unsigned short)(u ? w[4] >> 16 : w[0] & 0xFFFFu)));
       Iq4Group g;
       g.set(2 * H + u < s.left ? d : 0.f);   // (beyond the row: what follows it)
+      uint32_t q[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) g.word(u ? w[5 + i] : __funnelshift_r(w[i], w[i + 1], 16), out + 16 * u + 2 * i, out + 16 * u + 8 + 2 * i);
+      for (int i = 0; i < 4; ++i) q[i] = u ? w[5 + i] : __funnelshift_r(w[i], w[i + 1], 16);
+      g.words(q, out + 16 * u);
     }
   }
 };
