@@ -1179,3 +1179,18 @@ def test_tiled_code_book_weights_are_rounded_once(name, largest, k, dtype):
         assert torch.equal(y, want[i:i + M]), i
     torch.cuda.synchronize()
     assert capi.last_status() == 0
+
+
+@pytest.mark.parametrize("name,largest,k", [("Q6_K", 15.0, 768), ("Q6_K", 15.0, 2048), ("Q8_0", 500.0, 320), ("Q8_0", 500.0, 1024)])
+def test_tiled_weights_are_the_dequantized_ones(name, largest, k):
+    """As above for weights that meet q8_1 activations: 127 is stored as code 127 with scale 1, and 127 times an fp16 weight has 18 bits."""
+    t, N, M = TYPES[name], 136, 64
+    w = _scales_of_every_size(name, largest, N, k, seed=k)
+    want = capi.dequantize(w, t, N, k, torch.float16).float().T * 127
+    assert torch.isfinite(want).all()
+    eye = 127 * torch.eye(k, dtype=torch.float32, device=DEV)
+    for i in range(0, k, M):
+        y = capi.mul_mat_a8(w, eye[i:i + M].contiguous(), t, N)
+        assert torch.equal(y, want[i:i + M]), i
+    torch.cuda.synchronize()
+    assert capi.last_status() == 0
