@@ -2,7 +2,7 @@
 // ("unit" u = values 32u..32u+31) -> 16 packed 16-bit pairs = 64 bytes of the row in the A tile.
 // A producer thread owns one row of a 64-value stage and calls a decoder for its two units; towards the end of this file,
 // whole-stage decoders replace that for Q4_K / Q5_K / Q4_0 / Q8_0 in dense stages, and decoders of an item (two stages) for Q6_K,
-// IQ2_*, IQ3_* and, with fp16 activations, IQ4_*.
+// IQ2_*, IQ3_*, IQ4_NL and, with fp16 activations, IQ4_XS.
 //
 // Each decoder is split in two:
 //   load()   fetches a unit's raw bytes (from the shared-memory raw ring) into registers,
@@ -172,6 +172,8 @@ template <typename ab_t> struct Decoder<T_IQ2_XS, ab_t> { static constexpr bool 
 template <typename ab_t> struct Decoder<T_IQ2_S, ab_t> { static constexpr bool CORR = false; };
 template <typename ab_t> struct Decoder<T_IQ3_XXS, ab_t> { static constexpr bool CORR = false; };
 template <typename ab_t> struct Decoder<T_IQ3_S, ab_t> { static constexpr bool CORR = false; };
+template <typename ab_t> struct Decoder<T_IQ4_NL, ab_t> { static constexpr bool CORR = false; };
+template <> struct Decoder<T_IQ4_XS, __half> { static constexpr bool CORR = false; };
 // types that are multiplied as dequantized weights of either 16-bit type (activations as they are)
 template <int TYPE> __host__ __device__ constexpr bool decoder_bf16() {
   return TYPE == T_IQ2_XXS || TYPE == T_IQ2_XS || TYPE == T_IQ2_S || TYPE == T_IQ3_XXS || TYPE == T_IQ3_S || TYPE == T_IQ1_S || TYPE == T_IQ1_M ||
@@ -519,8 +521,8 @@ template <typename ab_t> __device__ __forceinline__ void iq4_word(uint32_t w, fl
   hi[1] = pack2<ab_t>(v(b, 1), v(b, 3));
 }
 
-// ---- IQ4_XS: fp32 d*(ls-32)*level rounded once to ab_t; unit = 32-value group ib = u&7 -----------
-template <typename ab_t> struct Decoder<T_IQ4_XS, ab_t> {
+// ---- IQ4_XS with bf16 activations: fp32 d*(ls-32)*level rounded once; unit = 32-value group ib = u&7 -----------
+template <> struct Decoder<T_IQ4_XS, __nv_bfloat16> {
   static constexpr bool CORR = false;
   static constexpr int RW = 6;   // header (8 bytes) + 16 index bytes, 8-byte aligned
   static __device__ __forceinline__ void load(const uint8_t* row, int u, uint32_t (&raw)[RW]) {
@@ -535,24 +537,7 @@ template <typename ab_t> struct Decoder<T_IQ4_XS, ab_t> {
     const int ls = (int)(((raw[1] >> (4 * ib)) & 0xF) | ((((raw[0] >> 16) >> (2 * ib)) & 3) << 4)) - 32;
     const float dl = d * (float)ls;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) iq4_word<ab_t>(raw[2 + i], dl, out + 2 * i, out + 8 + 2 * i);
-  }
-};
-
-// ---- IQ4_NL: fp32 d*level rounded once to ab_t; unit = one 18-byte block (2-byte aligned) ----------
-template <typename ab_t> struct Decoder<T_IQ4_NL, ab_t> {
-  static constexpr bool CORR = false;
-  static constexpr int RW = 7;
-  static __device__ __forceinline__ void load(const uint8_t* row, int u, uint32_t (&raw)[RW]) {
-    ldg_cover<RW - 1>(row + (int64_t)u * 18, 18, raw);
-    raw[RW - 1] = 0;
-  }
-  static __device__ __forceinline__ void decode(const uint8_t* row, int u, const uint32_t (&raw)[RW], const DecodeCtx&, uint32_t (&out)[16]) {
-    const uint32_t sh = shift_of(row + (int64_t)u * 18);
-    const float d = __half2float(__ushort_as_half((unsigned short)(word_at(raw, 0, sh) & 0xFFFFu)));
-#pragma unroll
-    for (int i = 0; i < 4; ++i)   // the indices start 2 bytes into the block
-      iq4_word<ab_t>(__funnelshift_r(word_at(raw, i, sh), word_at(raw, i + 1, sh), 16), d, out + 2 * i, out + 8 + 2 * i);
+    for (int i = 0; i < 4; ++i) iq4_word<__nv_bfloat16>(raw[2 + i], dl, out + 2 * i, out + 8 + 2 * i);
   }
 };
 
@@ -1122,7 +1107,7 @@ template <typename ab_t> struct Item128<T_IQ3_S, ab_t> {   // half d | u8 qs[64]
 
 // ---- the IQ4 formats with fp16 activations: value = round(dl * level), dl in fp32 (at most 17 significant bits) ----
 // As IQ3: the level, divided by 128, is 1024 + (level + 128) made by a permute, times 1/128, minus 9 -- exact -- and dl times 128 is split
-// in two.  (bf16 has no room for the byte under a power of two; those activations keep iq4_word.  14336x4096, 48 tokens:
+// in two.  (bf16 has no room for the byte under a power of two: iq4_word.  14336x4096, 48 tokens:
 // IQ4_XS 26.2 -> 24.1 us, IQ4_NL 29.7 -> 23.9.)
 struct Iq4Group {
   __half2 hi, lo;
@@ -1188,8 +1173,9 @@ template <> struct Item128<T_IQ4_XS, __half> {   // half d | u16 scales_h | u8 s
   }
 };
 // IQ4_NL: the words of both stages at once and one branch a block.  (Read by the stage, with a branch a word, the decoder held the few A slots of the
-// largest tiles for too long: 384 tokens of 14336x4096 44.3 us against 40.2 with unit decoders, now 39.2; 17 tokens 26.9 -> 23.5.)
-template <> struct Item128<T_IQ4_NL, __half> {   // blocks of 18 bytes: half d | u8 qs[16]
+// largest tiles for too long: 384 tokens of 14336x4096 44.3 us against 40.2 with unit decoders, now 39.2; 17 tokens 26.9 -> 23.5.  The unit
+// decoder that bf16 had fetched every block's bytes by itself: 384 tokens 40.9 -> 38.9, 17 tokens 29.4 -> 26.4, same arithmetic.)
+template <typename ab_t> struct Item128<T_IQ4_NL, ab_t> {   // blocks of 18 bytes: half d | u8 qs[16]
   static constexpr bool HAVE = true;
   struct State { uint32_t w[18]; int left; };
   static __device__ __forceinline__ void begin(uint32_t row, int ip, bool wide, int left, State& s) {
@@ -1201,12 +1187,18 @@ template <> struct Item128<T_IQ4_NL, __half> {   // blocks of 18 bytes: half d |
 #pragma unroll
     for (int u = 0; u < 2; ++u) {   // the second block starts 18 bytes on: its d in the upper half of word four
       const float d = __half2float(__ushort_as_half((unsigned short)(u ? w[4] >> 16 : w[0] & 0xFFFFu)));
-      Iq4Group g;
-      g.set(2 * H + u < s.left ? d : 0.f);   // (beyond the row: what follows it)
+      const float dl = 2 * H + u < s.left ? d : 0.f;   // (beyond the row: what follows it)
       uint32_t q[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) q[i] = u ? w[5 + i] : __funnelshift_r(w[i], w[i + 1], 16);
-      g.words(q, out + 16 * u);
+      if constexpr (std::is_same<ab_t, __half>::value) {
+        Iq4Group g;
+        g.set(dl);
+        g.words(q, out + 16 * u);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) iq4_word<ab_t>(q[i], dl, out + 16 * u + 2 * i, out + 16 * u + 8 + 2 * i);
+      }
     }
   }
 };
