@@ -3,6 +3,8 @@
 import ctypes
 import re
 
+import pytest
+
 from helpers import ROOT
 
 
@@ -169,3 +171,19 @@ def test_tiles_are_shared_where_that_pays(native_libs):
             columns = k + (k // 32 + 63) // 64 * 64 if t in (2, 12, 13) else k
             assert lib.gguf_b200_workspace_bytes(capi.OP_MMQ, t, m, n, k) == (m * columns * 2 + 255) // 256 * 256, (t, m)
             assert lib.gguf_b200_workspace_bytes(capi.OP_MMQ, t, m, 4096, 14336) > 1 << 20
+
+
+@pytest.mark.parametrize("t,m,n,k,tile", [(8, 272, 8192, 28672, 288), (8, 300, 8192, 28672, 320), (2, 300, 8192, 28672, 320), (3, 352, 8192, 28672, 352),
+                                          (21, 700, 8192, 28672, 352), (8, 700, 28672, 8192, 352)])
+def test_tiles_beyond_256_tokens_where_they_pay(native_libs, t, m, n, k, tile):
+    """Tiles of 257 to 384 tokens take less time than two or three smaller ones in these calls (8192x28672: Q8_0, 272 tokens 135 us in one tile, 155 in
+    two; 300 tokens 137 and 157; Q4_0 135 and 147; Q4_1, 352 tokens 154 and 162; IQ3_S, 700 tokens 251 in two and 263 in three)."""
+    from gguf_b200 import capi
+
+    op = capi.OP_DEQUANT_MATMUL if t == 21 else capi.OP_MMQ
+    columns = k + ((k // 32 + 63) // 64 * 64 if t in (2, 3) else 0)
+    activations = 0 if t == 21 else (m * columns * 2 + 255) // 256 * 256
+    tiles = (n // 128) * ((m + tile - 1) // tile)
+    counters = (tiles * 4 + 255) // 256 * 256
+    # runs over all SMs: two parts of 128 rows by a tile's tokens for each of 148 CTAs
+    assert capi.lib().gguf_b200_workspace_bytes(op, t, m, n, k) == activations + counters + 2 * 148 * 128 * tile * 4

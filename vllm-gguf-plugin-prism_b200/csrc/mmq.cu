@@ -78,40 +78,44 @@ static_assert(Stage64<T_Q4_0, __half>::PERM == 1 && Stage64<T_Q4_K, __half>::PER
 //   even     few tiles: each is cut into the same number of ranges of chunks, one per CTA
 //   stream   the chunks of all tiles in equal runs over all SMs
 // A stage takes the time to decode it (mmq_decode_clocks) or that of its product and its activations (mmq_stage_clocks); reading a tile
-// out takes 29 clocks per token, 11 where there are two accumulators (beside the next tile's work); a CTA in use 68; sharing, 4,000 + 36 per
-// token + 9.5 per token and part where a CTA has one part of a tile, 7,000 + 33 per token + 11 per token and part where it has two (5,500
-// by the times alone; the parts of runs also take up to 39 MB of L2: 512 tokens of 14336x4096 Q4_K in runs and in whole tiles are 55.9
-// and 56.0 us in a row, and runs lose 2 % between other work).
-// Fitted by least squares, then by what is lost, to the times of every plan of 1501 problems (19 types, seven matrices of 1024x4096 to
-// 28672x8192, 17 to 1999 tokens): what it picks takes 0.5 % longer than the best plan on average, 10 % at most.
+// out takes 13.5 clocks per token, 6 where there are two accumulators (beside the next tile's work); a CTA in use 50; sharing, 1,800 + 44 per
+// token + 11 per token and part where a CTA has one part of a tile, 6,300 + 34 per token + 16.5 per token and part where it has two.
+// Fitted by least squares, then by what is lost, to the times of every plan of 3,500 problems (19 types, eight matrices of 1024x4096 to
+// 28672x8192, 17 to 1999 tokens, weights from memory, plans timed in turn; those beyond 256 tokens on three GPUs, which the power limit holds back
+// to different degrees): what it picks takes 0.5 % longer than the best plan on average, 15 % at most.  (The clocks before these had tiles of
+// more than 256 tokens too long by a tenth and those of up to 256 too short: 300 tokens of 8192x28672 Q8_0 were cut into two tiles, 157 us
+// where one takes 137; 700 of 37888x3584 IQ2_S into three, 151 where two take 145.)
 struct MmqPlan {
   int tn;
   int64_t tt, grid;
   bool shared;
 };
-// clocks to decode a stage, with what a CTA of many tokens leaves of its issue slots and shared memory (3 / 8 per token)
+// clocks to decode a stage, with what a CTA of many tokens leaves of its issue slots and shared memory (half a clock per token).  One number a type,
+// between those of fp16 and bf16 activations (IQ4_XS 560 and 620, IQ4_NL 570 and 650, alike or within 1 % for the others): a workspace's size
+// follows from the plan, and the caller who asks for it names no activation type.
 static int mmq_decode_clocks(int type) {
   switch (type) {
-    case T_Q8_0: return 340;
-    case T_Q4_0: return 360;
-    case T_Q4_K: return 365;
-    case T_Q4_1: return 400;
-    case T_IQ2_XXS: return 410;
-    case T_Q6_K: return 430;
-    case T_Q2_K: return 440;
-    case T_Q5_K: case T_Q5_1: return 460;
-    case T_IQ3_XXS: case T_IQ2_S: return 475;
-    case T_IQ1_S: case T_IQ2_XS: case T_IQ3_S: return 480;
-    case T_Q3_K: return 485;
-    case T_Q5_0: return 520;
-    case T_IQ1_M: return 540;
-    default: return 565;   // IQ4_NL, IQ4_XS
+    case T_Q8_0: return 300;
+    case T_Q4_K: return 305;
+    case T_Q4_0: return 310;
+    case T_Q4_1: return 425;
+    case T_Q2_K: return 430;
+    case T_IQ2_XXS: return 445;
+    case T_Q6_K: return 450;
+    case T_IQ2_S: return 460;
+    case T_Q5_0: case T_Q5_1: case T_Q5_K: case T_IQ2_XS: return 475;
+    case T_IQ1_S: return 480;
+    case T_IQ3_XXS: case T_IQ3_S: return 490;
+    case T_Q3_K: return 510;
+    case T_IQ1_M: return 530;
+    case T_IQ4_XS: return 590;
+    default: return 610;   // IQ4_NL
   }
 }
 // (the product itself takes two clocks per token; the rest is the activations' way from L2 and, beyond 256 tokens, the few A slots)
 static int64_t mmq_stage_clocks(int type, int tn) {
-  const int decode = mmq_decode_clocks(type) + (tn <= 256 ? 3 * tn / 8 : 0);
-  const int mma = tn <= 128 ? 290 + 11 * tn / 8 : tn <= 256 ? 177 + 8 * tn / 5 : tn <= 320 ? 500 + 7 * tn / 8 : 500 + 23 * tn / 20;
+  const int decode = mmq_decode_clocks(type) + (tn <= 256 ? tn : 256) / 2;
+  const int mma = tn <= 128 ? 250 + 3 * tn / 2 : tn <= 256 ? 190 + 7 * tn / 4 : tn <= 320 ? 300 + 13 * tn / 8 : 170 + 33 * tn / 16;
   return mma > decode ? mma : decode;
 }
 static MmqPlan mmq_plan(int type, int64_t M, int64_t N, int64_t K, bool may_share) {
@@ -130,20 +134,20 @@ static MmqPlan mmq_plan(int type, int64_t M, int64_t N, int64_t K, bool may_shar
       const int64_t tiles = rt * tt, chunk = 4 * mmq_stage_clocks(type, tn), waves = (tiles + MMQ_CTAS - 1) / MMQ_CTAS;
       const bool twin = tn <= 128;
       auto take = [&](int64_t t, int64_t grid, bool shared) {
-        t += 68 * grid;
+        t += 50 * grid;
         if (t < best_t) { best_t = t; best = {tn, tt, grid, shared}; }
       };
-      take(waves * nc * chunk + (twin ? 11 : waves * 29) * tn, tiles < MMQ_CTAS ? tiles : MMQ_CTAS, false);
+      take(waves * nc * chunk + (twin ? 12 : waves * 27) * tn / 2, tiles < MMQ_CTAS ? tiles : MMQ_CTAS, false);
       if (!may_share) continue;
       if (tiles % MMQ_CTAS != 0 && tiles * nc >= 2 * MMQ_CTAS) {
         const int64_t run = (tiles * nc + MMQ_CTAS - 1) / MMQ_CTAS;
-        take(run * chunk + (twin ? 11 : (tiles / MMQ_CTAS + 1) * 29) * tn + 7000 + 33 * tn + 11 * tn * nc / run, MMQ_CTAS, true);
+        take(run * chunk + (twin ? 12 : (tiles / MMQ_CTAS + 1) * 27) * tn / 2 + 6300 + 34 * tn + 33 * tn * nc / (2 * run), MMQ_CTAS, true);
       }
       // (32-bit divisions: a call asks for its plan three times; a cut into more ranges of the same length only costs)
       const int ncs = (int)nc;
       for (int c = 2, len = 0; c * tiles <= MMQ_CTAS && 2 * c <= ncs; ++c) {
         const int l = (ncs + c - 1) / c;
-        if (l != len) take((int64_t)l * chunk + 4000 + tn * (72 + 19 * c) / 2, c * tiles, true);
+        if (l != len) take((int64_t)l * chunk + 1800 + tn * (44 + 11 * c), c * tiles, true);
         len = l;
       }
     }
