@@ -187,3 +187,14 @@ def test_tiles_beyond_256_tokens_where_they_pay(native_libs, t, m, n, k, tile):
     counters = (tiles * 4 + 255) // 256 * 256
     # runs over all SMs: two parts of 128 rows by a tile's tokens for each of 148 CTAs
     assert capi.lib().gguf_b200_workspace_bytes(op, t, m, n, k) == activations + counters + 2 * 148 * 128 * tile * 4
+
+
+def test_moe_products_read_their_work_list_past_l1():
+    """The products of a MoE step read the work list (and the routing in the tiled kernel's epilogue) ahead of their own griddepcontrol.wait: only
+    loads that do not take the L1's word may do that, since the list lies at the same addresses in every step."""
+    csrc = ROOT / "vllm-gguf-plugin-prism_b200" / "csrc"
+    for name, fields in (("mmq_kernel.cuh", "passes|n_passes|sorted|row_scale"), ("smallm.cuh", "passes|n_passes")):
+        src = (csrc / name).read_text()
+        assert not re.search(rf"p\.({fields})\[|(?<![\w*] )\*p\.({fields})\b|__ldg\(p\.({fields})\b", src), name
+        assert len(re.findall(rf"ld_older\(p\.(?:{fields})\b", src)) >= 4, name
+    assert (csrc / "common.cuh").read_text().count("ld.relaxed.gpu.global") == 3

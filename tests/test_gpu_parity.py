@@ -1194,3 +1194,36 @@ def test_tiled_weights_are_the_dequantized_ones(name, largest, k):
         assert torch.equal(y, want[i:i + M]), i
     torch.cuda.synchronize()
     assert capi.last_status() == 0
+
+
+@pytest.mark.parametrize("t,T,top_k", [(2, 8, 4), (12, 8, 4), (2, 96, 2), (12, 96, 2)])
+def test_moe_steps_in_a_row_on_one_workspace(t, T, top_k):
+    """Steps with other routes and weights each, launched without a pause on one workspace, give what each gives by itself: no step works from
+    the list of the one before."""
+    E, H, I, steps = 16, 512, 256, 48
+    w13 = torch.from_numpy(np.stack([synth.make_weight(t, 2 * I, H, seed=e) for e in range(E)])).to(DEV)
+    w2 = torch.from_numpy(np.stack([synth.make_weight(t, H, I, seed=100 + e) for e in range(E)])).to(DEV)
+    x = (dev_x(T, H, seed=3).float() / 64).half()
+    routes = []
+    for s in range(steps):   # from a handful of experts to all of them: lists of every length
+        tw, ids = synth.make_routing(T, max(top_k, E * (s % 5 + 1) // 5), top_k, s)
+        routes.append((torch.from_numpy(tw).to(DEV), torch.from_numpy((ids + s) % E).to(DEV)))
+    nbytes = capi.lib().gguf_b200_fused_moe_workspace_bytes(t, t, capi.F16, T, top_k, E, H, I)
+    ws = torch.empty(nbytes, dtype=torch.uint8, device=DEV)
+    got, alone = torch.empty(2, steps, T, H, dtype=torch.float16, device=DEV)
+
+    def step(s, out):
+        tw, ids = routes[s]
+        rc = capi.lib().gguf_b200_fused_moe(x.data_ptr(), w13.data_ptr(), w2.data_ptr(), out[s].data_ptr(), ids.data_ptr(), tw.data_ptr(), ws.data_ptr(), nbytes, t, t,
+                                            capi.F16, capi.ACT_SILU, T, top_k, E, H, I, torch.cuda.current_stream().cuda_stream)
+        assert rc == 0
+
+    for s in range(steps):
+        step(s, got)
+    torch.cuda.synchronize()
+    for s in range(steps):
+        step(s, alone)
+        torch.cuda.synchronize()
+    assert capi.last_status() == 0 and bool(torch.isfinite(got).all())
+    for s in range(steps):
+        assert torch.equal(got[s], alone[s]), s

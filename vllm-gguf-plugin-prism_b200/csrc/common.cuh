@@ -337,11 +337,30 @@ template <typename T> __device__ __forceinline__ bool packet_read(const void* ba
 //   * an activation quantizer calls pdl_trigger() after its own pdl_wait(), so a product behind it does not even start before
 //     all work ahead of the call is complete and visible (a decoder layer of 8 tokens 83.7 -> 80.3 us, of 45 tokens 124.5 -> 126.6:
 //     the product's CTAs no longer wait on the SMs for the activations);
-//     A MoE product reads its work list at its start for the same reason: that is older than the quantizer's trigger;
+//     A MoE product reads its work list and its routing at its start for the same reason, through ld_older(): the kernel that wrote them is
+//     complete and its writes visible to all of the quantizer's grid, on every SM, before any of its CTAs triggers, and the product's first CTA starts
+//     after the last trigger.  What that does not promise is that the product's own L1 holds nothing older from those addresses, which are
+//     the same in every step: its own griddepcontrol.wait would.  So until then these loads are made where all SMs meet, in L2;
 //   * the GEMV of one or two vectors, and a product that is a call's first kernel (the GEMM on plain activations), read ahead
 //     (a layer of one token 48.5 -> 48.0 us) unless their caller says that the weights are in flight (GGUF_B200_W_IN_FLIGHT).
 __device__ __forceinline__ void bulk_prefetch_l2(const void* src, uint32_t bytes) {   // (aligned as a bulk copy)
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
+}
+// Loads, ahead of pdl_wait(), of what was complete before the kernel ahead triggered (see above)
+__device__ __forceinline__ int32_t ld_older(const int32_t* p) {
+  int32_t v;
+  asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ float ld_older(const float* p) {
+  float v;
+  asm volatile("ld.relaxed.gpu.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ int4 ld_older(const int4* p) {
+  int4 v;
+  asm volatile("ld.relaxed.gpu.global.v4.s32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+  return v;
 }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

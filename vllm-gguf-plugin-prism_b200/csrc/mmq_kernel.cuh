@@ -190,7 +190,7 @@ struct MmqTile {
 __device__ __forceinline__ MmqTile mmq_tile(const MmqParams& p, const MmqPart& q) {
   MmqTile t;
   if (p.passes) {
-    const int4 info = p.passes[q.outer];
+    const int4 info = ld_older(p.passes + q.outer);
     t.n0 = q.inner * MMQ_ROWS;
     t.row0 = info.x * p.n;
     t.x0 = info.y;
@@ -349,7 +349,7 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_consta
   // What the kernel ahead writes: the activations, and -- cleared, or read until now -- what the epilogue writes.  Everything else, decoding
   // included, starts before it is done (the weights: see pdl_wait; the work list of a MoE step is older than the quantizer's trigger).
   const bool moe = p.passes != nullptr;
-  const int tiles = moe ? __shfl_sync(0xffffffffu, *p.n_passes, 0) * p.rt : p.rt * p.tt;
+  const int tiles = moe ? __shfl_sync(0xffffffffu, ld_older(p.n_passes), 0) * p.rt : p.rt * p.tt;
   // Units: (tile, chunk) where CTAs share tiles, whole tiles where they do not -- there is no room for parts, or the last wave
   // of whole tiles idles for less than sharing costs.  Every CTA in use has an equal contiguous range of them.
   const int rest = tiles % (int)gridDim.x;
@@ -398,10 +398,10 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_consta
       auto out_row = [&](int b) {
         const int t = 16 * b + (lane & 15);
         int o = b < nb && t < et.rows ? et.x0 + t : -1;
-        if (moe && o >= 0) o = p.sorted[o];
+        if (moe && o >= 0) o = ld_older(p.sorted + o);
         return o < p.rows_out ? o : -1;
       };
-      auto out_scale = [&](int o) { return p.row_scale && o >= 0 ? p.row_scale[o] : 1.f; };
+      auto out_scale = [&](int o) { return p.row_scale && o >= 0 ? ld_older(p.row_scale + o) : 1.f; };
       int orow = out_row(g);
       float scale = out_scale(orow);
       if (mode != FINISH) {
