@@ -139,15 +139,18 @@ __global__ void __launch_bounds__(SM_THREADS, 2) smallm_kernel(const __grid_cons
   const bool producer = warp == SM_WARPS;
   pdl_trigger();   // the next kernel may become resident; it waits for this one before it touches anything
   // The producer asks for weights first.  (Those of a MoE step too: the quantizer ahead let this kernel start when its own wait was
-  // over, and the passes are older than that.  A step of eight tokens over 64 experts of Q4_0: 66.6 -> 61.6 us.)
-  if (!producer) pdl_wait();
+  // over, and the passes are older than that.  A step of eight tokens over 64 experts of Q4_0: 66.6 -> 61.6 us.)  The others wait when
+  // they know their first tile.
   // units: chunk by chunk, row tile by row tile, pass by pass; CTA i owns the units [i * U / G, (i + 1) * U / G)
   // (the host sees to it that U * G fits 31 bits: everything here is 32-bit arithmetic, and divisions are few -- a 64-bit
   // division costs as much as a block of the product)
   const int U = (moe ? ld_older(p.n_passes) : 1) * p.rt * p.nc;
   const int G = U < (int)gridDim.x ? U : (int)gridDim.x;
   const int cta = (int)blockIdx.x;
-  if (cta >= G) return;
+  if (cta >= G) {
+    pdl_wait();   // (not even a grid without work may complete before the kernels ahead of it)
+    return;
+  }
   const int u0 = (int)((unsigned)(cta * U) / (unsigned)G), u1 = (int)((unsigned)((cta + 1) * U) / (unsigned)G);
   const int first_tile = (int)((unsigned)u0 / (unsigned)p.nc);
 
@@ -252,6 +255,7 @@ __global__ void __launch_bounds__(SM_THREADS, 2) smallm_kernel(const __grid_cons
   int u = u0, tile = first_tile, c0 = u0 - first_tile * p.nc;
   int pass = moe ? first_tile / p.rt : 0, r = first_tile - pass * p.rt;
   int4 pi = moe ? ld_older(p.passes + pass) : make_int4(0, 0, p.tiles, 0), pi_next = pi;
+  pdl_wait();
   for (; u < u1; ++tile) {
     const int c1 = u1 - u < p.nc - c0 ? c0 + (u1 - u) : p.nc;
     const int nt = pi.z, x0 = pi.y, row0 = pi.x * p.n;
