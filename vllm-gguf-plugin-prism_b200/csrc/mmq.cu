@@ -79,7 +79,8 @@ static_assert(Stage64<T_Q4_0, __half>::PERM == 1 && Stage64<T_Q4_K, __half>::PER
 //   stream   the chunks of all tiles in equal runs over all SMs
 // A stage takes the time to decode it (mmq_decode_clocks) or that of its product and its activations (mmq_stage_clocks); reading a tile
 // out takes 13.5 clocks per token, 6 where there are two accumulators (beside the next tile's work); a CTA in use 50; sharing, 1,800 + 44 per
-// token + 11 per token and part where a CTA has one part of a tile, 6,300 + 34 per token + 16.5 per token and part where it has two.
+// token + 11 per token and part where a CTA has one part of a tile, 7,000 + 34 per token + 16.5 per token and part where it has two (6,300 by
+// the times of graphs of one product; between other work 512 tokens of 14336x4096 Q4_K take 67.4 us in whole tiles and 68.3 in runs).
 // Fitted by least squares, then by what is lost, to the times of every plan of 3,500 problems (19 types, eight matrices of 1024x4096 to
 // 28672x8192, 17 to 1999 tokens, weights from memory, plans timed in turn; those beyond 256 tokens on three GPUs, which the power limit holds back
 // to different degrees): what it picks takes 0.5 % longer than the best plan on average, 15 % at most.  (The clocks before these had tiles of
@@ -141,7 +142,7 @@ static MmqPlan mmq_plan(int type, int64_t M, int64_t N, int64_t K, bool may_shar
       if (!may_share) continue;
       if (tiles % MMQ_CTAS != 0 && tiles * nc >= 2 * MMQ_CTAS) {
         const int64_t run = (tiles * nc + MMQ_CTAS - 1) / MMQ_CTAS;
-        take(run * chunk + (twin ? 12 : (tiles / MMQ_CTAS + 1) * 27) * tn / 2 + 6300 + 34 * tn + 33 * tn * nc / (2 * run), MMQ_CTAS, true);
+        take(run * chunk + (twin ? 12 : (tiles / MMQ_CTAS + 1) * 27) * tn / 2 + 7000 + 34 * tn + 33 * tn * nc / (2 * run), MMQ_CTAS, true);
       }
       // (32-bit divisions: a call asks for its plan three times; a cut into more ranges of the same length only costs)
       const int ncs = (int)nc;
