@@ -1100,8 +1100,9 @@ def test_tiled_activations_of_every_value(name):
         want = torch.cat([capi.mul_mat_vec_a8(w, x[i:i + 16].contiguous(), t, 512) for i in range(0, M, 16)]).double()
     assert torch.isfinite(y[keep]).all()
     assert rel_l2(y[keep].cpu(), want[keep].float().cpu()) <= REL_L2_TOL
-    for i in (0, 5):
-        assert rel_l2(y[i].cpu(), want[i].float().cpu()) <= REL_L2_TOL
+    for i in range(M):   # row by row: the large row outweighs the others, and one wrong code of 512 is a twentieth of its row
+        if keep[i]:
+            assert rel_l2(y[i].cpu(), want[i].float().cpu()) <= REL_L2_TOL, i
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
