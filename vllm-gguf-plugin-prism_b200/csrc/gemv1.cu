@@ -76,12 +76,11 @@ template <int N> __device__ __forceinline__ void lds_a2(uint32_t a, uint32_t (&w
 }
 
 struct Tab1 {
-  uint32_t grid;    // shared-window addresses of this lane's copies of the IQ2_XXS code books
-  uint32_t smask;
+  uint32_t grid;    // shared-window addresses of this lane's copies of the IQ2 and IQ3 code books
+  uint32_t smask;   // ... and of their signs
   uint32_t kv[4];
 };
 
-// Per type: UPB units per block, XW activation words and XD floats held per unit.
 // Code books in shared memory: GRID entries of GB bytes in GC copies, then SGN sign masks (eight bytes: all ones where the value is
 // negative) in SC copies.  Copy c of an entry lies in column c of its line, and lane l reads copy l modulo their number: the lanes
 // that are served together then sit in different banks whatever entries they ask for, or all but (32 unrelated entries of one copy
@@ -128,6 +127,7 @@ template <int TYPE> __device__ __forceinline__ void g1_fill_tables(uint8_t* tab)
   }
 }
 
+// Per type: UPB units per block, XW activation words and XD floats held per unit.
 template <int TYPE> struct G1;
 
 // ---- Q8_0: unit = block of 32 -----------------------------------------------------------

@@ -39,7 +39,7 @@
 // compiler takes for divergent; a wait that is ready, with its address arithmetic, 80 to 250.  With an MMA issuer of the second sort
 // and three waits an item, no type got below 460 to 560 clocks a stage; since its warp stays converged and waits once, the decoders
 // bound the kernel at 128 tokens or less.  Clocks a stage at 48 tokens, before -> after: Q4_K 511 -> 326, Q4_0 490 -> 313, Q2_K 562 -> 397,
-// Q5_K 542 -> 429, IQ2_XXS 621 -> 459, Q3_K 684 -> 465, Q6_K 717 -> 537 (warp instructions a stage of 32 rows 279 -> 199 for Q4_K, 498 -> 346 for Q6_K).
+// Q5_K 542 -> 429, IQ2_XXS 621 -> 459, Q3_K 684 -> 465, Q6_K 717 -> 405 (its unit decoder 537).
 // Measured, before -> after: IQ3_S 8192 x 28672, 300 tokens 291 -> 134 us; Q6_K 37888 x 3584, 1999 tokens 668 -> 567 us;
 // IQ2_XXS 28672 x 8192, 128 tokens 108 -> 95 us; a MoE step of 256 tokens (64 experts, Q4_0) 222 -> 169 us.  By items and with the
 // converged issuer: Q6_K 3584 x 18944, 45 tokens 36.5 -> 28.0 us; the MoE step 167.6 -> 142.3; IQ2_XXS 92.5 -> 79.1; Q6_K 1999 tokens 546 -> 503.

@@ -139,7 +139,7 @@ __device__ __forceinline__ uint4 iq2_pair_selectors(uint64_t grid_entry) {
   }
   return make_uint4(s[0], s[1], s[2], s[3]);
 }
-// An IQ3 entry: its four magnitudes (at most 62) as 16-bit values, for fp16 divided by 256; those of IQ3_XXS are bf16 always (see Iq3Group).
+// An IQ3 entry: its four magnitudes (at most 62) as 16-bit values, for fp16 divided by 256; those of IQ3_XXS are bf16 always (see Iq3Scale).
 template <typename ab_t> __device__ __forceinline__ uint2 iq3_magnitudes(uint32_t g) {
   const float f = std::is_same<ab_t, __half>::value ? 1.f / 256.f : 1.f;
   return make_uint2(pack2<ab_t>(f * (float)(g & 0xFFu), f * (float)((g >> 8) & 0xFFu)), pack2<ab_t>(f * (float)((g >> 16) & 0xFFu), f * (float)(g >> 24)));
@@ -1000,29 +1000,13 @@ template <typename ab_t> struct Item128<T_IQ2_S, ab_t> {   // half d | u8 qs[32]
 // Split in bf16, m * lo would be rounded to eight bits before the sum (0.502 of a last place against 0.500, one weight in 2500); of IQ3_XXS in fp16 62 / 256 * lo can be
 // an odd multiple of 2^-25, half of fp16's last place, where dh is below 2^-13, and taking the fp32 form only there made warps run both
 // (14336x4096, 512 tokens: 70.7 us against 63.1 before all this).
-template <int TYPE, typename ab_t> struct Iq3Group {
-  static constexpr bool SPLIT = TYPE == T_IQ3_S && std::is_same<ab_t, __half>::value;
-  __half2 hi, lo;
-  uint64_t d2;   // (d, d) in fp32
-  bool wide;
-  __device__ __forceinline__ void set(float dh, uint32_t s) {
-    float d = dh * (0.5f + (float)s) * 0.5f;
-    wide = true;
-    if constexpr (SPLIT) {
-      d *= 256.f;
-      hi = __float2half2_rn(d);
-      lo = __float2half2_rn(d - __low2float(hi));
-      wide = !(fabsf(d) < 60000.f);
-    }
-    asm("mov.b64 %0, {%1, %1};" : "=l"(d2) : "r"(__float_as_uint(d)));
-  }
-  __device__ __forceinline__ uint32_t pair(uint32_t m) const {
-    const __half2 v = u32_as_h2(m);
-    return h2_as_u32(__hfma2(v, hi, __hmul2_rn(v, lo)));
-  }
+// Iq3Scale: magnitudes in MT times d in fp32, as ab_t
+template <typename MT, typename ab_t> struct Iq3Scale {
+  uint64_t d2;   // (d, d)
+  __device__ __forceinline__ void set(float d) { asm("mov.b64 %0, {%1, %1};" : "=l"(d2) : "r"(__float_as_uint(d))); }
   __device__ __forceinline__ uint32_t pair32(uint32_t m) const {
     float a, b;
-    if constexpr (SPLIT) {
+    if constexpr (std::is_same<MT, __half>::value) {
       a = __low2float(u32_as_h2(m));
       b = __high2float(u32_as_h2(m));
     } else {
@@ -1031,6 +1015,19 @@ template <int TYPE, typename ab_t> struct Iq3Group {
     }
     asm("{.reg .b64 t;\n\tmov.b64 t, {%0, %1};\n\tmul.rn.f32x2 t, t, %2;\n\tmov.b64 {%0, %1}, t;}" : "+f"(a), "+f"(b) : "l"(d2));
     return pack2<ab_t>(a, b);
+  }
+};
+struct Iq3Split {   // d * 256 in two fp16 numbers
+  __half2 hi, lo;
+  bool wide;
+  __device__ __forceinline__ void set(float d) {
+    hi = __float2half2_rn(d);
+    lo = __float2half2_rn(d - __low2float(hi));
+    wide = !(fabsf(d) < 60000.f);
+  }
+  __device__ __forceinline__ uint32_t pair(uint32_t m) const {
+    const __half2 v = u32_as_h2(m);
+    return h2_as_u32(__hfma2(v, hi, __hmul2_rn(v, lo)));
   }
 };
 template <typename ab_t> struct Item128<T_IQ3_XXS, ab_t> {   // half d | u8 qs[64] | per 32 values four 7-bit sign indices and a 4-bit scale; 98 bytes
@@ -1045,22 +1042,18 @@ template <typename ab_t> struct Item128<T_IQ3_XXS, ab_t> {   // half d | u8 qs[6
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
       const uint32_t aux = s.aux[2 * H + u];
-      Iq3Group<T_IQ3_XXS, ab_t> g;
-      g.set(s.dh, aux >> 28);
-      auto go = [&](auto value) {
+      Iq3Scale<__nv_bfloat16, ab_t> g;
+      g.set(s.dh * (0.5f + (float)(aux >> 28)) * 0.5f);
 #pragma unroll
-        for (int l = 0; l < 4; ++l) {
-          const uint32_t w = s.q[4 * H + 2 * u + (l >> 1)], sw = sign_word<T_IQ3_XXS>(cx, (aux >> (7 * l)) & 127u);
-          const uint2 a = grid64<T_IQ3_XXS>(cx, byte_of(w, 2 * (l & 1))), b = grid64<T_IQ3_XXS>(cx, byte_of(w, 2 * (l & 1) + 1));
-          uint32_t* o = out + 16 * u + 4 * l;
-          o[0] = negate(value(a.x), sign_bits<0>(sw));
-          o[1] = negate(value(a.y), sign_bits<1>(sw));
-          o[2] = negate(value(b.x), sign_bits<2>(sw));
-          o[3] = negate(value(b.y), sign_bits<3>(sw));
-        }
-      };
-      if (Iq3Group<T_IQ3_XXS, ab_t>::SPLIT && !g.wide) go([&](uint32_t m) { return g.pair(m); });
-      else go([&](uint32_t m) { return g.pair32(m); });
+      for (int l = 0; l < 4; ++l) {
+        const uint32_t w = s.q[4 * H + 2 * u + (l >> 1)], sw = sign_word<T_IQ3_XXS>(cx, (aux >> (7 * l)) & 127u);
+        const uint2 a = grid64<T_IQ3_XXS>(cx, byte_of(w, 2 * (l & 1))), b = grid64<T_IQ3_XXS>(cx, byte_of(w, 2 * (l & 1) + 1));
+        uint32_t* o = out + 16 * u + 4 * l;
+        o[0] = negate(g.pair32(a.x), sign_bits<0>(sw));
+        o[1] = negate(g.pair32(a.y), sign_bits<1>(sw));
+        o[2] = negate(g.pair32(b.x), sign_bits<2>(sw));
+        o[3] = negate(g.pair32(b.y), sign_bits<3>(sw));
+      }
     }
   }
 };
@@ -1080,8 +1073,10 @@ template <typename ab_t> struct Item128<T_IQ3_S, ab_t> {   // half d | u8 qs[64]
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
       const uint32_t qh = s.qh >> (16 * H + 8 * u), sg = s.sg[2 * H + u];
-      Iq3Group<T_IQ3_S, ab_t> g;
-      g.set(s.dh, (s.sc >> (8 * H + 4 * u)) & 0xFu);
+      constexpr bool SPLIT = std::is_same<ab_t, __half>::value;
+      const float d = s.dh * (0.5f + (float)((s.sc >> (8 * H + 4 * u)) & 0xFu)) * (SPLIT ? 128.f : 0.5f);   // (the magnitudes are divided by 256)
+      Iq3Scale<ab_t, ab_t> g;
+      g.set(d);
       auto go = [&](auto value) {
 #pragma unroll
         for (int h = 0; h < 2; ++h) {   // a word of indices: 16 values
@@ -1099,8 +1094,15 @@ template <typename ab_t> struct Item128<T_IQ3_S, ab_t> {   // half d | u8 qs[64]
           }
         }
       };
-      if (Iq3Group<T_IQ3_S, ab_t>::SPLIT && !g.wide) go([&](uint32_t m) { return g.pair(m); });
-      else go([&](uint32_t m) { return g.pair32(m); });
+      if constexpr (SPLIT) {
+        Iq3Split h;
+        h.set(d);
+        if (!h.wide) {
+          go([&](uint32_t m) { return h.pair(m); });
+          continue;
+        }
+      }
+      go([&](uint32_t m) { return g.pair32(m); });
     }
   }
 };

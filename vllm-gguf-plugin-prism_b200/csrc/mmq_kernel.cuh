@@ -38,7 +38,7 @@ struct MmqParams {
   int dtype;              // of y
   int n, m;               // weight rows, tokens
   int k, kpad;
-  int nc, corr;           // 256-value chunks of a row; 1: a stage of corrections behind every eight of them
+  int nc, corr;           // 256-value chunks of a row; 1: half a stage of corrections behind every four of them
   int rt, tt, tn;         // row tiles, token tiles, tokens per tile (a multiple of 16, at most 256, or of 32, at most 384)
   int sa, a_col0;         // A slots: how many (2 to 4), first column
   int nbuf;               // accumulators, MMQ_D_STEP columns apart
