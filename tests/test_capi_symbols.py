@@ -190,11 +190,24 @@ def test_tiles_beyond_256_tokens_where_they_pay(native_libs, t, m, n, k, tile):
 
 
 def test_moe_products_read_their_work_list_past_l1():
-    """The products of a MoE step read the work list (and the routing in the tiled kernel's epilogue) ahead of their own griddepcontrol.wait: only
-    loads that do not take the L1's word may do that, since the list lies at the same addresses in every step."""
+    """The products of a MoE step read the work list ahead of their own griddepcontrol.wait: only loads that do not take the L1's word may do that,
+    since the list lies at the same addresses in every step.  Plain loads of it, and of the routing, stand behind the wait."""
     csrc = ROOT / "vllm-gguf-plugin-prism_b200" / "csrc"
-    for name, fields in (("mmq_kernel.cuh", "passes|n_passes|sorted|row_scale"), ("smallm.cuh", "passes|n_passes")):
-        src = (csrc / name).read_text()
-        assert not re.search(rf"p\.({fields})\[|(?<![\w*] )\*p\.({fields})\b|__ldg\(p\.({fields})\b", src), name
-        assert len(re.findall(rf"ld_older\(p\.(?:{fields})\b", src)) >= 4, name
-    assert (csrc / "common.cuh").read_text().count("ld.relaxed.gpu.global") == 3
+    plain = r"p\.(?:passes|sorted|row_scale)\[|(?<![\w*] )\*p\.n_passes\b|__ldg\(p\.(?:sorted|row_scale)\b"
+    mmq = (csrc / "mmq_kernel.cuh").read_text()
+    at = mmq.index("waited ? p.passes[q.outer] : ld_older(p.passes + q.outer)")
+    epilogue = mmq.index("pdl_wait();", mmq.index("auto epilogue = "))
+    for m in re.finditer(plain, mmq):
+        assert m.start() == at + len("waited ? ") or m.start() > epilogue, m.group()
+    assert mmq[epilogue:].index("mmq_tile(p, e, true)") < 60                     # the epilogue's tile: right behind its wait
+    calls = [m.start() for m in re.finditer(r"mmq_tile\(p, q, (?:true|waited)\)", mmq)]
+    assert len(calls) == 2                                                        # the decoders' and the activation loader's
+    for c in calls:
+        assert 0 < c - mmq.rindex("pdl_wait();", 0, c) < 250
+    small = (csrc / "smallm.cuh").read_text()
+    producer, consumers = small.index("if (producer) {"), small.index("  pdl_wait();\n  for (; u < u1; ++tile)")
+    for m in re.finditer(plain, small):
+        before = small[m.start() - len("waited ? "):m.start()]
+        assert before == "waited ? " or m.start() > consumers or "auto outputs" in small[producer:m.start()], m.group()
+    assert small.count("ld_older(p.n_passes)") == 1 and mmq.count("ld_older(p.n_passes)") == 1
+    assert (csrc / "common.cuh").read_text().count("ld.relaxed.gpu.global") == 2

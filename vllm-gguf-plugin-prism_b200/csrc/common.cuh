@@ -346,20 +346,17 @@ template <typename T> __device__ __forceinline__ bool packet_read(const void* ba
 __device__ __forceinline__ void bulk_prefetch_l2(const void* src, uint32_t bytes) {   // (aligned as a bulk copy)
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
 }
-// Loads, ahead of pdl_wait(), of what was complete before the kernel ahead triggered (see above)
+// Loads, ahead of pdl_wait(), of what was complete before the kernel ahead triggered (see above).  Nothing writes there while this kernel runs, so the
+// compiler may move, merge and drop them.  Behind its own wait a thread takes plain loads, which are near when a neighbour has asked before (a MoE
+// step of 512 tokens over 64 experts of Q6_K, hidden 1024: 86.0 -> 85.0 us).
 __device__ __forceinline__ int32_t ld_older(const int32_t* p) {
   int32_t v;
-  asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ float ld_older(const float* p) {
-  float v;
-  asm volatile("ld.relaxed.gpu.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+  asm("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p));
   return v;
 }
 __device__ __forceinline__ int4 ld_older(const int4* p) {
   int4 v;
-  asm volatile("ld.relaxed.gpu.global.v4.s32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+  asm("ld.relaxed.gpu.global.v4.s32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
   return v;
 }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

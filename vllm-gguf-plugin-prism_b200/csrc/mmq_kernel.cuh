@@ -187,10 +187,11 @@ struct MmqTile {
   int x0, rows;              // first activation row, rows that count
   int row0;                  // MoE: first row of the expert's matrix among all rows
 };
-__device__ __forceinline__ MmqTile mmq_tile(const MmqParams& p, const MmqPart& q) {
+// (waited: behind this thread's pdl_wait)
+__device__ __forceinline__ MmqTile mmq_tile(const MmqParams& p, const MmqPart& q, bool waited) {
   MmqTile t;
   if (p.passes) {
-    const int4 info = ld_older(p.passes + q.outer);
+    const int4 info = waited ? p.passes[q.outer] : ld_older(p.passes + q.outer);
     t.n0 = q.inner * MMQ_ROWS;
     t.row0 = info.x * p.n;
     t.x0 = info.y;
@@ -389,7 +390,8 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_consta
     // instead of 4,000, most of them for the first time through).  FINISH: the parts of e's tile are all in memory.
     enum : int { MORE, FINAL, FINISH };
     auto epilogue = [&](const MmqPart& e, int pi, int mode) {
-      const MmqTile et = mmq_tile(p, e);
+      pdl_wait();
+      const MmqTile et = mmq_tile(p, e, true);
       const int buf = p.nbuf == 2 ? pi & 1 : 0, use = p.nbuf == 2 ? pi >> 1 : pi;
       const int n = et.n0 + r, nb = p.tn / 16;
       const bool live = n < p.n;
@@ -398,16 +400,15 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_consta
       auto out_row = [&](int b) {
         const int t = 16 * b + (lane & 15);
         int o = b < nb && t < et.rows ? et.x0 + t : -1;
-        if (moe && o >= 0) o = ld_older(p.sorted + o);
+        if (moe && o >= 0) o = p.sorted[o];
         return o < p.rows_out ? o : -1;
       };
-      auto out_scale = [&](int o) { return p.row_scale && o >= 0 ? ld_older(p.row_scale + o) : 1.f; };
+      auto out_scale = [&](int o) { return p.row_scale && o >= 0 ? p.row_scale[o] : 1.f; };
       int orow = out_row(g);
       float scale = out_scale(orow);
       if (mode != FINISH) {
         wait(bar(24 + buf), (uint32_t)use & 1u);
         tc_fence_after();
-        pdl_wait();
       }
       const uint32_t d = d_lane + (uint32_t)(buf * MMQ_D_STEP);
       int first = 0, last = 0, s_first = 0;
@@ -577,7 +578,9 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_consta
     for (;;) {
       const bool more = mode == MORE && mmq_next_part(p, q);
       if (!more && mode == MORE) mode = FINAL;
-      const MmqTile qt = mmq_tile(p, q);
+      const bool waited = pi > 0;
+      if (moe && waited) pdl_wait();   // (over: the part before has had its activations)
+      const MmqTile qt = mmq_tile(p, q, waited);
       const int n = qt.n0 + r;
       const uint8_t* slot = sRaw + raw_slot(p.raw, r, qt.n0);
       const int items = more ? 2 * (q.c1 - q.c0) : 0;
@@ -703,7 +706,7 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_consta
     uint32_t ph = 0;
     pdl_wait();
     while (mmq_next_part(p, q)) {
-      const int x0 = mmq_tile(p, q).x0;
+      const int x0 = mmq_tile(p, q, true).x0;
       for (int cs = q.c0, ce; cs < q.c1; cs = ce, ++blk) {
         ce = mmq_block_end(p, q, cs);
         const int n = 2 * (ce - cs) * (p.bg == 2 ? 1 : 2);
@@ -731,7 +734,7 @@ __global__ void __launch_bounds__(MMQ_THREADS, 1) mmq_kernel(const __grid_consta
     int st = 0;
     uint32_t sph = 0;
     while (ok && mmq_next_part(p, q)) {
-      const MmqTile qt = mmq_tile(p, q);
+      const MmqTile qt = mmq_tile(p, q, false);
       for (int c = q.c0; c < q.c1; ++c) {
         mbar_wait_or(bar(36 + st), sph ^ 1u, gave_up_s);
         if (lds32(gave_up_s) != 0u) { ok = false; break; }

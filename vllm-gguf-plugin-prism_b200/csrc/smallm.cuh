@@ -144,7 +144,8 @@ __global__ void __launch_bounds__(SM_THREADS, 2) smallm_kernel(const __grid_cons
   // units: chunk by chunk, row tile by row tile, pass by pass; CTA i owns the units [i * U / G, (i + 1) * U / G)
   // (the host sees to it that U * G fits 31 bits: everything here is 32-bit arithmetic, and divisions are few -- a 64-bit
   // division costs as much as a block of the product)
-  const int U = (moe ? ld_older(p.n_passes) : 1) * p.rt * p.nc;
+  const int n_passes = moe ? ld_older(p.n_passes) : 1;
+  const int U = n_passes * p.rt * p.nc;
   const int G = U < (int)gridDim.x ? U : (int)gridDim.x;
   const int cta = (int)blockIdx.x;
   if (cta >= G) {
@@ -159,11 +160,12 @@ __global__ void __launch_bounds__(SM_THREADS, 2) smallm_kernel(const __grid_cons
       int c, r, pass;
       int4 info;      // {expert, first column tile, column tiles}
     };
-    auto load_pass = [&](Cursor& q) { q.info = moe ? ld_older(p.passes + q.pass) : make_int4(0, 0, p.tiles, 0); };
+    bool waited = false;
+    auto load_pass = [&](Cursor& q) { q.info = !moe ? make_int4(0, 0, p.tiles, 0) : waited ? p.passes[q.pass] : ld_older(p.passes + q.pass); };
     auto advance = [&](Cursor& q) {
       if (++q.c == p.nc) {
         q.c = 0;
-        if (++q.r == p.rt) { q.r = 0; ++q.pass; if (moe && q.pass < ld_older(p.n_passes)) load_pass(q); }
+        if (++q.r == p.rt) { q.r = 0; ++q.pass; if (q.pass < n_passes) load_pass(q); }
       }
     };
     auto x_copy = [&](const Cursor& q, int s) {
@@ -178,7 +180,6 @@ __global__ void __launch_bounds__(SM_THREADS, 2) smallm_kernel(const __grid_cons
     Cursor held = cur;        // first unit whose activations have not been asked for
     int n_held = 0, st = 0, st_in = 0;   // st_in: the stage that has to be there before the next one is asked for
     uint32_t ph = 0, ph_in = 0;
-    bool waited = false;
     auto release = [&]() {    // the activations exist now
       pdl_wait();
       waited = true;
@@ -259,7 +260,7 @@ __global__ void __launch_bounds__(SM_THREADS, 2) smallm_kernel(const __grid_cons
   for (; u < u1; ++tile) {
     const int c1 = u1 - u < p.nc - c0 ? c0 + (u1 - u) : p.nc;
     const int nt = pi.z, x0 = pi.y, row0 = pi.x * p.n;
-    if (moe && r + 1 == p.rt && u + (c1 - c0) < u1) pi_next = ld_older(p.passes + pass + 1);   // (for the tile after this one)
+    if (moe && r + 1 == p.rt && u + (c1 - c0) < u1) pi_next = p.passes[pass + 1];   // (for the tile after this one)
     Out out_rows;
     constexpr bool early = T <= 2;   // (four column tiles have no registers left for it)
     if (early && c1 - c0 == p.nc) outputs(out_rows, x0, nt);
